@@ -146,6 +146,9 @@ struct sg_ctx {
           *mlp_gpart = nullptr, *mlp_lpart = nullptr, *mlp_loss = nullptr, *mlp_X = nullptr,
           *mlp_Y = nullptr, *mlp_out = nullptr;
     int* mlp_idx = nullptr;
+    float* mlp_hist = nullptr;  // loss of each iteration of a training run
+    size_t mlp_idx_cap = 0;
+    int mlp_hist_cap = 0;
     void* mlp_wbf = nullptr;
     int mlp_cap = 0;
     // CUNBODY slot buffers
@@ -1206,6 +1209,7 @@ int sg_destroy(sg_ctx* ctx) {
                    ctx->mlp_lpart, ctx->mlp_loss, ctx->mlp_X, ctx->mlp_Y, ctx->mlp_out};
     for (float* f : mf) cudaFree(f);
     cudaFree(ctx->mlp_idx);
+    cudaFree(ctx->mlp_hist);
     cudaFree(ctx->mlp_wbf);
     cudaFree(ctx->cb_xj);
     cudaFree(ctx->cb_mj);
@@ -2017,8 +2021,8 @@ int mlp_reserve(sg_ctx* ctx, int n) {
         CK(dalloc(&ctx->mlp_m1, SG_MLP_NP));
         CK(dalloc(&ctx->mlp_m2, SG_MLP_NP));
         CK(dalloc(&ctx->mlp_grad, SG_MLP_NP));
-        CK(dalloc(&ctx->mlp_gpart, (size_t)SG_MLP_NP * 64));
-        CK(dalloc(&ctx->mlp_lpart, 64));
+        CK(dalloc(&ctx->mlp_gpart, (size_t)SG_MLP_NP * SG_MLP_BLOCKS));
+        CK(dalloc(&ctx->mlp_lpart, SG_MLP_BLOCKS));
         CK(dalloc(&ctx->mlp_loss, 1));
         CK(cudaMalloc(&ctx->mlp_wbf, SG_MLP_NP * 2));
     }
@@ -2026,14 +2030,33 @@ int mlp_reserve(sg_ctx* ctx, int n) {
         cudaFree(ctx->mlp_X);
         cudaFree(ctx->mlp_Y);
         cudaFree(ctx->mlp_out);
-        cudaFree(ctx->mlp_idx);
         ctx->mlp_X = ctx->mlp_Y = ctx->mlp_out = nullptr;
-        ctx->mlp_idx = nullptr;
+        ctx->mlp_cap = 0;
         CK(dalloc(&ctx->mlp_X, (size_t)n * SG_MLP_IN));
         CK(dalloc(&ctx->mlp_Y, (size_t)n));
         CK(dalloc(&ctx->mlp_out, (size_t)n));
-        CK(dalloc(&ctx->mlp_idx, (size_t)n));
         ctx->mlp_cap = n;
+    }
+    return SG_OK;
+}
+
+// minibatch rows drawn ahead at most (16 MB of indices): a run of training iterations
+constexpr long long kMlpRunRows = 1ll << 22;
+
+int mlp_reserve_run(sg_ctx* ctx, size_t rows, int iters) {
+    if (rows > ctx->mlp_idx_cap) {
+        cudaFree(ctx->mlp_idx);
+        ctx->mlp_idx = nullptr;
+        ctx->mlp_idx_cap = 0;
+        CK(dalloc(&ctx->mlp_idx, rows));
+        ctx->mlp_idx_cap = rows;
+    }
+    if (iters > ctx->mlp_hist_cap) {
+        cudaFree(ctx->mlp_hist);
+        ctx->mlp_hist = nullptr;
+        ctx->mlp_hist_cap = 0;
+        CK(dalloc(&ctx->mlp_hist, (size_t)iters));
+        ctx->mlp_hist_cap = iters;
     }
     return SG_OK;
 }
@@ -2068,9 +2091,8 @@ int sg_mlp_grad(sg_ctx* ctx, int n, const float* X, const float* Y, const float*
     CK(sg_mlp_to_bf16_launch(ctx->mlp_wm, ctx->mlp_wbf, ctx->stream));
     CK(cudaMemcpyAsync(ctx->mlp_X, X, sizeof(float) * n * SG_MLP_IN, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->mlp_Y, Y, sizeof(float) * n, cudaMemcpyHostToDevice, ctx->stream));
-    const int nb = std::min(64, std::max(1, n / 32));
     CK(sg_mlp_grad_launch(ctx->mlp_wbf, ctx->mlp_X, ctx->mlp_Y, nullptr, n, ctx->mlp_gpart,
-                          ctx->mlp_lpart, nb, ctx->mlp_grad, ctx->mlp_loss, ctx->stream));
+                          ctx->mlp_lpart, ctx->mlp_grad, ctx->mlp_loss, ctx->stream));
     CK(cudaMemcpyAsync(grad, ctx->mlp_grad, SG_MLP_NP * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(loss, ctx->mlp_loss, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -2090,8 +2112,9 @@ int sg_mlp_train(sg_ctx* ctx, int n, const float* X, const float* Y, int iters, 
     CK(sg_mlp_to_bf16_launch(ctx->mlp_wm, ctx->mlp_wbf, ctx->stream));
     CK(cudaMemcpyAsync(ctx->mlp_X, X, sizeof(float) * n * SG_MLP_IN, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->mlp_Y, Y, sizeof(float) * n, cudaMemcpyHostToDevice, ctx->stream));
-    // minibatches: a seeded permutation per epoch (splitmix64), uploaded per iteration
-    std::vector<int> perm(n), idx(batch);
+    // minibatches: a seeded permutation per epoch (splitmix64), drawn and uploaded for
+    // kMlpRun iterations at a time, so that the host waits once per run of iterations
+    std::vector<int> perm(n);
     for (int i = 0; i < n; i++) perm[i] = i;
     uint64_t s = seed;
     auto next = [&s]() {
@@ -2102,33 +2125,36 @@ int sg_mlp_train(sg_ctx* ctx, int n, const float* X, const float* Y, int iters, 
         return z ^ (z >> 31);
     };
     int pos = n;
-    std::vector<float> losses(iters > 0 ? iters : 1);
-    const int nb = std::min(64, std::max(1, batch / 32));
-    for (int it = 0; it < iters; it++) {
-        for (int b = 0; b < batch; b++) {
+    const int run = (int)std::min<long long>(std::max(iters, 1), std::max(1ll, kMlpRunRows / batch));
+    st = mlp_reserve_run(ctx, (size_t)run * batch, run);
+    if (st != SG_OK) return st;
+    std::vector<int> idx((size_t)run * batch);
+    std::vector<float> losses(run);
+    for (int it0 = 0; it0 < iters; it0 += run) {
+        const int k = std::min(run, iters - it0);
+        for (size_t b = 0; b < (size_t)k * batch; b++) {
             if (pos >= n) {
                 for (int i = n - 1; i > 0; i--) std::swap(perm[i], perm[next() % (uint64_t)(i + 1)]);
                 pos = 0;
             }
             idx[b] = perm[pos++];
         }
-        CK(cudaMemcpyAsync(ctx->mlp_idx, idx.data(), sizeof(int) * batch, cudaMemcpyHostToDevice,
-                           ctx->stream));
-        CK(sg_mlp_grad_launch(ctx->mlp_wbf, ctx->mlp_X, ctx->mlp_Y, ctx->mlp_idx, batch,
-                              ctx->mlp_gpart, ctx->mlp_lpart, nb, ctx->mlp_grad, ctx->mlp_loss,
-                              ctx->stream));
-        CK(sg_mlp_adam_launch(ctx->mlp_wm, ctx->mlp_wbf, ctx->mlp_m1, ctx->mlp_m2, ctx->mlp_grad, lr,
-                              it + 1, ctx->stream));
+        CK(cudaMemcpyAsync(ctx->mlp_idx, idx.data(), sizeof(int) * (size_t)k * batch,
+                           cudaMemcpyHostToDevice, ctx->stream));
+        for (int it = 0; it < k; it++)
+            CK(sg_mlp_train_launch(ctx->mlp_wm, ctx->mlp_wbf, ctx->mlp_m1, ctx->mlp_m2, ctx->mlp_X,
+                                   ctx->mlp_Y, ctx->mlp_idx + (size_t)it * batch, batch,
+                                   ctx->mlp_gpart, ctx->mlp_lpart, ctx->mlp_hist + it, lr,
+                                   it0 + it + 1, ctx->stream));
         if (loss_hist)
-            CK(cudaMemcpyAsync(&losses[it], ctx->mlp_loss, sizeof(float), cudaMemcpyDeviceToHost,
-                               ctx->stream));
-        // the index buffer is reused next iteration: wait for this one's upload to land
+            CK(cudaMemcpyAsync(losses.data(), ctx->mlp_hist, sizeof(float) * k,
+                               cudaMemcpyDeviceToHost, ctx->stream));
+        // the index and loss buffers are reused by the next run of iterations
         CK(cudaStreamSynchronize(ctx->stream));
+        if (loss_hist) std::copy(losses.begin(), losses.begin() + k, loss_hist + it0);
     }
     CK(cudaMemcpyAsync(w, ctx->mlp_wm, SG_MLP_NP * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (loss_hist)
-        for (int it = 0; it < iters; it++) loss_hist[it] = losses[it];
     return SG_OK;
 }
 

@@ -21,6 +21,8 @@
 // previous step of the step size that would have met the tolerance exactly.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "sg_internal.cuh"
 
 namespace {
@@ -162,76 +164,139 @@ __global__ void proposer_kernel(const SgCloud* __restrict__ clouds, SgCtrl* __re
 
 // ---- training ----------------------------------------------------------------
 // Forward + backward of a batch; block b takes samples [b*per, (b+1)*per) (of the
-// index list idx) and writes its gradient partial to gpart[b][SG_MLP_NP] and its
-// squared-error sum to lpart[b].  MSE loss L = (1/B) sum (o - y)^2.
-constexpr int kTrainThreads = 128;
+// index list idx), kTrainChunk at a time, and writes its gradient partial to
+// gpart[b][SG_MLP_NP] and its squared-error sum to lpart[b].  MSE loss
+// L = (1/B) sum (o - y)^2.
+//
+// Latency-bound: a minibatch of 256 is 4 M multiply-adds.  Each layer of a chunk is one
+// product with a thread per (sample, unit), the weights (FP32 images of the BF16 values)
+// and activations in shared memory, W2 with a row stride of 65 words so that both
+// W2[u][m] over u (forward) and over m (backward) are conflict-free; each thread keeps
+// the 16 + 4 weight gradients it owns in registers.  With one thread per whole sample
+// and shared-memory atomics for every weight gradient (32 busy threads in each of 8
+// blocks, activations in local memory) a minibatch of 256 took 7,347 us; this form, 64
+// blocks of one chunk, takes 13.5 us.
+constexpr int kTrainThreads = 256;
+constexpr int kTrainChunk = 4;  // kTrainThreads / SG_MLP_H samples in flight per block
+constexpr int kW2Stride = SG_MLP_H + 1;
+
+struct TrainShared {
+    float W1[SG_MLP_H][SG_MLP_IN + 1];
+    float W2[SG_MLP_H * kW2Stride];
+    float B1[SG_MLP_H], B2[SG_MLP_H], W3[SG_MLP_H];
+    float x[kTrainChunk][SG_MLP_IN];
+    float h1[kTrainChunk][SG_MLP_H], h2[kTrainChunk][SG_MLP_H];
+    float gz1[kTrainChunk][SG_MLP_H], gz2[kTrainChunk][SG_MLP_H];
+    float osum[kTrainThreads / 32];
+    float go[kTrainChunk];
+};
 
 __global__ void __launch_bounds__(kTrainThreads) mlp_grad_kernel(
     const __nv_bfloat16* __restrict__ w, const float* __restrict__ X, const float* __restrict__ Y,
     const int* __restrict__ idx, int B, int per, float* __restrict__ gpart,
     float* __restrict__ lpart) {
     sg_griddep_wait();
-    __shared__ float g[SG_MLP_NP];
-    __shared__ float lsum[kTrainThreads / 32];
-    for (int k = threadIdx.x; k < SG_MLP_NP; k += blockDim.x) g[k] = 0.f;
-    __syncthreads();
-    float lerr = 0.f;
-    const int s0 = blockIdx.x * per;
-    for (int si = s0 + threadIdx.x; si < min(B, s0 + per); si += blockDim.x) {
-        const int sidx = idx ? idx[si] : si;
-        const float* x = X + (size_t)sidx * SG_MLP_IN;
-        float xv[SG_MLP_IN];
+    __shared__ TrainShared sh;
+    const int tid = threadIdx.x;
+    for (int k = tid; k < SG_MLP_H * SG_MLP_IN; k += kTrainThreads)
+        sh.W1[k / SG_MLP_IN][k % SG_MLP_IN] = __bfloat162float(w[SG_MLP_W1 + k]);
+    for (int k = tid; k < SG_MLP_H * SG_MLP_H; k += kTrainThreads)
+        sh.W2[k / SG_MLP_H * kW2Stride + k % SG_MLP_H] = __bfloat162float(w[SG_MLP_W2 + k]);
+    if (tid < SG_MLP_H) {
+        sh.B1[tid] = __bfloat162float(w[SG_MLP_B1 + tid]);
+        sh.B2[tid] = __bfloat162float(w[SG_MLP_B2 + tid]);
+        sh.W3[tid] = __bfloat162float(w[SG_MLP_W3 + tid]);
+    }
+    const float b3 = __bfloat162float(w[SG_MLP_B3]);
+    const int u = tid % SG_MLP_H, s = tid / SG_MLP_H;  // unit, sample of the chunk
+    // this thread's weight gradients: W2[s*16 + r][u], W1[tid / 4][(tid % 4) * 4 + r]
+    float g2[SG_MLP_H / kTrainChunk], g1[SG_MLP_H * SG_MLP_IN / kTrainThreads];
+    float gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, lerr = 0.f;
 #pragma unroll
-        for (int k = 0; k < SG_MLP_IN; k++) xv[k] = x[k];
-        float z1[SG_MLP_H], h1[SG_MLP_H], z2[SG_MLP_H], h2[SG_MLP_H];
-        for (int u = 0; u < SG_MLP_H; u++) {
-            float z = __bfloat162float(w[SG_MLP_B1 + u]);
+    for (int r = 0; r < SG_MLP_H / kTrainChunk; r++) g2[r] = 0.f;
 #pragma unroll
-            for (int k = 0; k < SG_MLP_IN; k++)
-                z = fmaf(__bfloat162float(w[SG_MLP_W1 + u * SG_MLP_IN + k]), xv[k], z);
-            z1[u] = z;
-            h1[u] = silu(z);
+    for (int r = 0; r < SG_MLP_H * SG_MLP_IN / kTrainThreads; r++) g1[r] = 0.f;
+    const int s0 = blockIdx.x * per, s1 = min(B, s0 + per);
+    for (int c0 = s0; c0 < s1; c0 += kTrainChunk) {
+        const int nc = min(kTrainChunk, s1 - c0);
+        __syncthreads();  // weights loaded; the previous chunk's arrays are free
+        if (tid < kTrainChunk * SG_MLP_IN) {
+            const int q = tid / SG_MLP_IN;
+            const int at = q < nc ? (idx ? idx[c0 + q] : c0 + q) : -1;
+            sh.x[q][tid % SG_MLP_IN] = at >= 0 ? X[(size_t)at * SG_MLP_IN + tid % SG_MLP_IN] : 0.f;
         }
-        for (int u = 0; u < SG_MLP_H; u++) {
-            float z = __bfloat162float(w[SG_MLP_B2 + u]);
-            for (int m = 0; m < SG_MLP_H; m++)
-                z = fmaf(__bfloat162float(w[SG_MLP_W2 + u * SG_MLP_H + m]), h1[m], z);
-            z2[u] = z;
-            h2[u] = silu(z);
-        }
-        float o = __bfloat162float(w[SG_MLP_B3]);
-        for (int u = 0; u < SG_MLP_H; u++) o = fmaf(__bfloat162float(w[SG_MLP_W3 + u]), h2[u], o);
-        const float d = o - Y[sidx];
-        lerr += d * d;
-        const float go = 2.0f * d / (float)B;
-        atomicAdd(&g[SG_MLP_B3], go);
-        float gz2[SG_MLP_H];
-        for (int u = 0; u < SG_MLP_H; u++) {
-            atomicAdd(&g[SG_MLP_W3 + u], go * h2[u]);
-            gz2[u] = go * __bfloat162float(w[SG_MLP_W3 + u]) * silu_grad(z2[u]);
-            atomicAdd(&g[SG_MLP_B2 + u], gz2[u]);
-        }
-        for (int m = 0; m < SG_MLP_H; m++) {
-            float gh = 0.f;
-            for (int u = 0; u < SG_MLP_H; u++) {
-                atomicAdd(&g[SG_MLP_W2 + u * SG_MLP_H + m], gz2[u] * h1[m]);
-                gh = fmaf(__bfloat162float(w[SG_MLP_W2 + u * SG_MLP_H + m]), gz2[u], gh);
+        __syncthreads();
+        float z1 = sh.B1[u];
+#pragma unroll
+        for (int k = 0; k < SG_MLP_IN; k++) z1 = fmaf(sh.W1[u][k], sh.x[s][k], z1);
+        sh.h1[s][u] = silu(z1);
+        __syncthreads();
+        float z2 = sh.B2[u];
+#pragma unroll 16
+        for (int m = 0; m < SG_MLP_H; m++) z2 = fmaf(sh.W2[u * kW2Stride + m], sh.h1[s][m], z2);
+        const float h2 = silu(z2);
+        sh.h2[s][u] = h2;
+        float o = sh.W3[u] * h2;
+        for (int off = 16; off > 0; off >>= 1) o += __shfl_xor_sync(0xffffffffu, o, off);
+        if ((tid & 31) == 0) sh.osum[tid >> 5] = o;
+        __syncthreads();
+        if (tid < kTrainChunk) {
+            float go = 0.f;
+            if (tid < nc) {
+                const int at = idx ? idx[c0 + tid] : c0 + tid;
+                const float d = sh.osum[2 * tid] + sh.osum[2 * tid + 1] + b3 - Y[at];
+                lerr += d * d;
+                go = 2.0f * d / (float)B;
             }
-            const float gz1 = gh * silu_grad(z1[m]);
-            atomicAdd(&g[SG_MLP_B1 + m], gz1);
+            sh.go[tid] = go;  // 0 past the batch: no gradient from there
+            gb3 += go;
+        }
+        __syncthreads();
+        sh.gz2[s][u] = sh.go[s] * sh.W3[u] * silu_grad(z2);
+        __syncthreads();
+        float gh = 0.f;
+#pragma unroll 16
+        for (int q = 0; q < SG_MLP_H; q++) gh = fmaf(sh.W2[q * kW2Stride + u], sh.gz2[s][q], gh);
+        sh.gz1[s][u] = gh * silu_grad(z1);
+        __syncthreads();
 #pragma unroll
-            for (int k = 0; k < SG_MLP_IN; k++) atomicAdd(&g[SG_MLP_W1 + m * SG_MLP_IN + k], gz1 * xv[k]);
+        for (int q = 0; q < kTrainChunk; q++) {
+            const float hm = sh.h1[q][u];
+#pragma unroll
+            for (int r = 0; r < SG_MLP_H / kTrainChunk; r++)
+                g2[r] = fmaf(sh.gz2[q][s * (SG_MLP_H / kTrainChunk) + r], hm, g2[r]);
+            const float g = sh.gz1[q][tid / 4];
+#pragma unroll
+            for (int r = 0; r < SG_MLP_H * SG_MLP_IN / kTrainThreads; r++)
+                g1[r] = fmaf(g, sh.x[q][(tid % 4) * 4 + r], g1[r]);
+            if (s == 0) {
+                gb1 += sh.gz1[q][u];
+                gb2 += sh.gz2[q][u];
+                gw3 = fmaf(sh.go[q], sh.h2[q][u], gw3);
+            }
         }
     }
-    for (int o = 16; o > 0; o >>= 1) lerr += __shfl_down_sync(0xffffffffu, lerr, o);
-    if ((threadIdx.x & 31) == 0) lsum[threadIdx.x >> 5] = lerr;
-    __syncthreads();
-    for (int k = threadIdx.x; k < SG_MLP_NP; k += blockDim.x)
-        gpart[(size_t)blockIdx.x * SG_MLP_NP + k] = g[k];
-    if (threadIdx.x == 0) {
-        float s = 0.f;
-        for (int q = 0; q < kTrainThreads / 32; q++) s += lsum[q];
-        lpart[blockIdx.x] = s;
+    float* gp = gpart + (size_t)blockIdx.x * SG_MLP_NP;
+#pragma unroll
+    for (int r = 0; r < SG_MLP_H / kTrainChunk; r++)
+        gp[SG_MLP_W2 + (s * (SG_MLP_H / kTrainChunk) + r) * SG_MLP_H + u] = g2[r];
+#pragma unroll
+    for (int r = 0; r < SG_MLP_H * SG_MLP_IN / kTrainThreads; r++)
+        gp[SG_MLP_W1 + (tid / 4) * SG_MLP_IN + (tid % 4) * 4 + r] = g1[r];
+    if (s == 0) {
+        gp[SG_MLP_B1 + u] = gb1;
+        gp[SG_MLP_B2 + u] = gb2;
+        gp[SG_MLP_W3 + u] = gw3;
+    }
+    if (tid < 32) {  // the chunk's per-sample threads are lanes 0-3 of this warp
+        for (int off = 2; off > 0; off >>= 1) {
+            lerr += __shfl_down_sync(0xffffffffu, lerr, off);
+            gb3 += __shfl_down_sync(0xffffffffu, gb3, off);
+        }
+        if (tid == 0) {
+            gp[SG_MLP_B3] = gb3;
+            lpart[blockIdx.x] = lerr;
+        }
     }
 }
 
@@ -252,24 +317,35 @@ __global__ void mlp_reduce_kernel(const float* __restrict__ gpart, const float* 
     }
 }
 
-// Adam on the FP32 master weights, then the BF16 copy used by the forward pass.
+// One training iteration's end: the gradient (block partials in a fixed order), Adam on
+// the FP32 master weights, the BF16 copy used by the next forward pass, and the loss into
+// the iteration's history entry.  One launch: with the sums, Adam and the loss read-back
+// apart, an iteration was 3 launches, a copy and a host wait.
 __global__ void mlp_adam_kernel(float* __restrict__ wm, __nv_bfloat16* __restrict__ wb,
                                 float* __restrict__ m1, float* __restrict__ m2,
-                                const float* __restrict__ grad, float lr, float b1, float b2,
-                                float eps, int step) {
+                                const float* __restrict__ gpart, const float* __restrict__ lpart,
+                                int nb, int B, float* __restrict__ loss, float lr, float b1,
+                                float b2, float eps, int step) {
     sg_griddep_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= SG_MLP_NP) return;
-    const float g = grad[k];
-    const float a = b1 * m1[k] + (1.f - b1) * g;
-    const float v = b2 * m2[k] + (1.f - b2) * g * g;
-    m1[k] = a;
-    m2[k] = v;
-    const float ah = a / (1.f - powf(b1, (float)step));
-    const float vh = v / (1.f - powf(b2, (float)step));
-    const float nw = wm[k] - lr * ah / (sqrtf(vh) + eps);
-    wm[k] = nw;
-    wb[k] = __float2bfloat16_rn(nw);
+    if (k < SG_MLP_NP) {
+        float g = 0.f;
+#pragma unroll 16
+        for (int b = 0; b < nb; b++) g += gpart[(size_t)b * SG_MLP_NP + k];
+        const float a = b1 * m1[k] + (1.f - b1) * g;
+        const float v = b2 * m2[k] + (1.f - b2) * g * g;
+        m1[k] = a;
+        m2[k] = v;
+        const float ah = a / (1.f - powf(b1, (float)step));
+        const float vh = v / (1.f - powf(b2, (float)step));
+        const float nw = wm[k] - lr * ah / (sqrtf(vh) + eps);
+        wm[k] = nw;
+        wb[k] = __float2bfloat16_rn(nw);
+    } else if (k == SG_MLP_NP) {  // a thread of its own
+        float s = 0.f;
+        for (int b = 0; b < nb; b++) s += lpart[b];
+        *loss = s / (float)B;
+    }
 }
 
 __global__ void mlp_to_bf16_kernel(const float* __restrict__ wm, __nv_bfloat16* __restrict__ wb) {
@@ -304,20 +380,31 @@ cudaError_t sg_proposer_launch(const SgCloud* clouds, SgCtrl* ctrl, const double
     return cudaGetLastError();
 }
 
+// Blocks of a forward + backward pass over B samples: one chunk of samples each while
+// that fits the partial-gradient array (64 blocks for a minibatch of 256: one wave).
+static int train_blocks(int B) {
+    return std::max(1, std::min(SG_MLP_BLOCKS, (B + kTrainChunk - 1) / kTrainChunk));
+}
+
 cudaError_t sg_mlp_grad_launch(const void* wbf, const float* X, const float* Y, const int* idx,
-                               int B, float* gpart, float* lpart, int nb, float* grad, float* loss,
+                               int B, float* gpart, float* lpart, float* grad, float* loss,
                                cudaStream_t st) {
-    const int per = (B + nb - 1) / nb;
+    const int nb = train_blocks(B);
     sg_launch(mlp_grad_kernel, nb, kTrainThreads, 0, st, static_cast<const __nv_bfloat16*>(wbf), X, Y, idx,
-                                                  B, per, gpart, lpart);
+                                                  B, (B + nb - 1) / nb, gpart, lpart);
     sg_launch(mlp_reduce_kernel, (SG_MLP_NP + 255) / 256, 256, 0, st, gpart, lpart, nb, B, grad, loss);
     return cudaGetLastError();
 }
 
-cudaError_t sg_mlp_adam_launch(float* wm, void* wbf, float* m1, float* m2, const float* grad,
-                               float lr, int step, cudaStream_t st) {
-    sg_launch(mlp_adam_kernel, (SG_MLP_NP + 255) / 256, 256, 0, st, 
-        wm, static_cast<__nv_bfloat16*>(wbf), m1, m2, grad, lr, 0.9f, 0.999f, 1e-8f, step);
+cudaError_t sg_mlp_train_launch(float* wm, void* wbf, float* m1, float* m2, const float* X,
+                                const float* Y, const int* idx, int B, float* gpart, float* lpart,
+                                float* loss, float lr, int step, cudaStream_t st) {
+    const int nb = train_blocks(B);
+    __nv_bfloat16* wb = static_cast<__nv_bfloat16*>(wbf);
+    sg_launch(mlp_grad_kernel, nb, kTrainThreads, 0, st, (const __nv_bfloat16*)wb, X, Y, idx, B,
+              (B + nb - 1) / nb, gpart, lpart);
+    sg_launch(mlp_adam_kernel, SG_MLP_NP / 128 + 1, 128, 0, st, wm, wb, m1, m2,
+              (const float*)gpart, (const float*)lpart, nb, B, loss, lr, 0.9f, 0.999f, 1e-8f, step);
     return cudaGetLastError();
 }
 

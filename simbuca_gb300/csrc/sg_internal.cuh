@@ -250,6 +250,7 @@ __host__ __device__ inline int sg_start_ops(SgCtrl& cs, sg_field_params& fp, con
 #define SG_MLP_W3 (SG_MLP_B2 + SG_MLP_H)
 #define SG_MLP_B3 (SG_MLP_W3 + SG_MLP_H)
 #define SG_MLP_NP (SG_MLP_B3 + 1)
+#define SG_MLP_BLOCKS 128  // gradient partials of a training pass at most
 
 // Per-cloud proposer state: features of the current step start and step history.
 struct SgProposerState {
@@ -467,10 +468,12 @@ cudaError_t sg_proposer_launch(const SgCloud* clouds, SgCtrl* ctrl, const double
                                double* log_num, int log_cap, int use_mlp, double safety,
                                int n_clouds, cudaStream_t st);
 cudaError_t sg_mlp_grad_launch(const void* wbf, const float* X, const float* Y, const int* idx,
-                               int B, float* gpart, float* lpart, int nb, float* grad, float* loss,
+                               int B, float* gpart, float* lpart, float* grad, float* loss,
                                cudaStream_t st);
-cudaError_t sg_mlp_adam_launch(float* wm, void* wbf, float* m1, float* m2, const float* grad,
-                               float lr, int step, cudaStream_t st);
+// one training iteration: forward, backward, Adam; the loss goes to *loss (device)
+cudaError_t sg_mlp_train_launch(float* wm, void* wbf, float* m1, float* m2, const float* X,
+                                const float* Y, const int* idx, int B, float* gpart, float* lpart,
+                                float* loss, float lr, int step, cudaStream_t st);
 cudaError_t sg_mlp_to_bf16_launch(const float* wm, void* wbf, cudaStream_t st);
 cudaError_t sg_mlp_forward_launch(const void* wbf, const float* X, int n, float* out,
                                   cudaStream_t st);

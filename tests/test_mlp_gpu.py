@@ -153,3 +153,26 @@ def test_controller_safety_mode(ctx):
     low = proposer.run_controller(ctx, ev, 1e-6, controller_safety=0.7)
     assert low["status"] == 0 and low["done"] == 1
     assert low["mean_h"] < ref["mean_h"]
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 127, 513, 1030])
+def test_training_pass_at_block_edges(ctx, n):
+    """The forward-backward kernel takes 4 samples at a time over up to 128 blocks: batches
+    below one chunk, ragged ones, and past the block cap.  FP32 sums of up to 1,030 terms
+    against the float64 oracle: the bounds of the gradient test above.  One training
+    iteration over the whole set is one Adam step, w - lr g / (|g| + 1e-8), wherever the
+    gradient's sign is resolved."""
+    rng = np.random.default_rng(n)
+    X = rng.normal(0, 1, (n, 16)).astype(np.float32)
+    Y = rng.normal(0, 1, n).astype(np.float32)
+    w = rand_weights(n)
+    rloss, rg = omlp.loss_and_grad(X, Y, w)
+    loss, g = ctx.mlp_grad(X, Y, w)
+    assert loss == pytest.approx(rloss, rel=1e-5)
+    assert np.abs(g - rg).max() <= 1e-4 * np.abs(rg).max()
+    w1, hist = ctx.mlp_train(X, Y, w, iters=1, batch=n, lr=1e-3)
+    assert hist[0] == pytest.approx(rloss, rel=1e-5)
+    big = np.abs(rg) > 1e-2 * np.abs(rg).max()
+    step = w.astype(np.float64) - 1e-3 * rg / (np.abs(rg) + 1e-8)
+    # |dg| <= 1e-4 max|g| moves g/(|g|+eps) by < 1e-4 there; plus one FP32 rounding of w
+    assert np.abs(w1 - step)[big].max() <= 1e-3 * 1e-4 + np.abs(w).max() * 2.0 ** -23
