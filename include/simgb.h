@@ -164,7 +164,7 @@ int sg_force(sg_ctx* ctx, int precision, int n, const double* pos, const double*
  * from a host framework's pool.  pos [n][3], q [n], kq [n] and acc [n][3] are DEVICE
  * buffers owned by the caller; the result is the FP64 form of sg_coulomb_accel.  Work
  * is queued on `stream` (a cudaStream_t, NULL = legacy default stream) of the current
- * device and the call returns without waiting.  Scratch lives in a fixed 1.8 MB device
+ * device and the call returns without waiting.  Scratch lives in a fixed 13 MB device
  * array of the library: n <= 8192, else SG_TOO_LARGE.  The array has one address per
  * CUDA context: the first call made in a context looks it up and keeps it under that
  * context's unique id (make that first call before capturing any stream).  n = 0

@@ -25,6 +25,7 @@ struct Problem {
     int variant = 0;  // FP32c launch shape the items were planned for
     int method = 5;   // 5 Dormand-Prince, 4 Cash-Karp (every cloud of a batch)
     bool any_coulomb = false;
+    bool sym = false;  // FP64: items take each unordered pair once
     bool uploaded = false;
     std::vector<SgCloud> hc;
     std::vector<SgCtrl> hctrl0;
@@ -154,6 +155,8 @@ struct sg_ctx {
     // CUNBODY slot buffers
     double *cb_xj = nullptr, *cb_mj = nullptr, *cb_xi = nullptr, *cb_ai = nullptr;
     double* cb_host = nullptr;
+    double* cb_part = nullptr;  // partial sums
+    size_t cb_part_cap = 0;
     int cb_ni = 0, cb_nj = 0;
 };
 
@@ -235,6 +238,60 @@ int auto_variant(const std::vector<int>& counts, int requested) {
     return big < 24000 ? 5 : 9;
 }
 
+// FP64 items that take each unordered pair once: i-block b (128 ions) against the j-tiles
+// (32 ions) from its own diagonal up, K tiles per item, or 1/bands of the rotation steps
+// of one tile when that leaves the device short of items.  A block keeps all four FP64
+// pipes of an SM busy whatever else it does, so the items only have to be small against
+// one SM's share of the work (at least 4 items per SM) and large against the ~1 us it
+// takes to start one (a tile is 20 us of FP64).
+void plan_sym(Problem& P, int n_sm) {
+    const int TB = SG_SYM_IB / SG_SYM_JT;
+    double tiles = 0.0;
+    for (int c = 0; c < P.n_clouds; c++) {
+        if (!(P.hc[c].fp.flags & SG_F_COULOMB)) continue;
+        const int nj = P.hc[c].npad / SG_SYM_JT;
+        for (int b = 0; b * TB < nj; b++) tiles += nj - b * TB;
+    }
+    int bands = 1, K = 1;
+    while (bands < 8 && tiles * bands < 4.0 * n_sm) bands *= 2;
+    if (bands == 1) K = (int)std::min(64.0, std::max(1.0, std::floor(tiles / (16.0 * n_sm))));
+    P.max_slots = 0;
+    for (int c = 0; c < P.n_clouds; c++) {
+        SgCloud& cl = P.hc[c];
+        cl.nslots = 0;
+        if (!(cl.fp.flags & SG_F_COULOMB) || cl.n == 0) continue;
+        P.any_coulomb = true;
+        cl.sym_k = K;
+        cl.sym_bands = bands;
+        const int nj = cl.npad / SG_SYM_JT;
+        for (int b = 0; b * TB < nj; b++)
+            for (int t = b * TB, q = 0; t < nj; t += K, q++)
+                for (int band = 0; band < bands; band++) {
+                    SgWorkItem it;
+                    memset(&it, 0, sizeof it);
+                    it.cloud = c;
+                    it.i0 = cl.poff + b * SG_SYM_IB;
+                    it.ni = std::min(SG_SYM_IB, cl.npad - b * SG_SYM_IB);
+                    it.j0 = cl.poff + t * SG_SYM_JT;
+                    it.nj = std::min(K, nj - t) * SG_SYM_JT;
+                    it.slot = (b + 1 + q) * bands + band;
+                    it.jslot = b * bands + band;
+                    const int step = SG_SYM_JT / bands;
+                    it.s01 = band * step | (band + 1) * step << 16;
+                    P.hitems.push_back(it);
+                }
+        for (int p = 0; p < cl.npad; p += SG_SYM_IB)
+            cl.nslots = std::max(cl.nslots, sg_sym_slots(cl, p));
+        P.max_slots = std::max(P.max_slots, cl.nslots);
+        P.cloud_inter[c] = (double)cl.n * (cl.n - 1);
+    }
+    // diagonal items (about half a tile's work each) last
+    std::stable_sort(P.hitems.begin(), P.hitems.end(), [](const SgWorkItem& a, const SgWorkItem& b) {
+        return (a.j0 >= a.i0 + SG_SYM_IB) > (b.j0 >= b.i0 + SG_SYM_IB);
+    });
+    P.n_items = (int)P.hitems.size();
+}
+
 // Partition clouds into row blocks and Coulomb work items.  Items are sized so that
 // (a) there are several waves of blocks on the device and (b) no single item is a
 // large share of the total work; they are issued largest first.
@@ -275,7 +332,7 @@ void plan(Problem& P, int n_sm) {
             rb.cloud = c;
             rb.i0 = off + i;
             rb.n = std::min(rows, cl.n - i);
-            rb.pad = 0;
+            rb.cap = rows;
             P.hrows.push_back(rb);
         }
         cl.nrb = (int)P.hrows.size() - cl.rb0;
@@ -288,6 +345,16 @@ void plan(Problem& P, int n_sm) {
     P.n_rows = (int)P.hrows.size();
 
     const bool f32 = P.precision == SG_PREC_FP32C;
+    P.sym = false;
+    if (!f32) {
+        P.sym = true;
+        for (int c = 0; c < C; c++)
+            if (P.hc[c].npad > SG_SYM_MAX_IONS) P.sym = false;
+    }
+    if (P.sym) {
+        plan_sym(P, n_sm);
+        return;
+    }
     const int ib = f32 ? sg_coulomb_fp32c_ib(P.variant) : SG_C64_IB;
     const int per_sm = f32 ? std::max(1, 2048 / ib) : 4;
     const double conc = (double)n_sm * per_sm;
@@ -306,16 +373,14 @@ void plan(Problem& P, int n_sm) {
     }
     // j-chunks are whole 128-ion tiles, or smaller ones (plain shapes only: the k-d
     // ordered kernels test whole tiles) when 128-ion chunks would leave fewer than two
-    // blocks per SM.  FP32c: 64-ion chunks -- a 1,000-ion cloud runs 512 one-warp blocks
-    // instead of 256 (7 % faster per step than 32-ion chunks, whose 32 partial-sum slots
-    // made the reduction dearer than the extra parallelism paid).  FP64: 32-ion chunks,
-    // its pair kernel being bound by the FP64 pipe of every SM it can reach (1,000 ions:
-    // 23 sim-us/s with 32-ion chunks, 14.5 with 64).
+    // blocks per SM: 64-ion chunks -- a 1,000-ion cloud runs 512 one-warp blocks instead of
+    // 256 (7 % faster per step than 32-ion chunks, whose 32 partial-sum slots made the
+    // reduction dearer than the extra parallelism paid).
     long long full_split = 0;
     for (int c = 0; c < C; c++)
         if (S[c] > 0)
             full_split += (long long)((P.hc[c].n + ib - 1) / ib) * std::max(1, P.hc[c].npad / 128);
-    const int jgran = (!P.sorted && full_split < 2LL * n_sm) ? (f32 ? 64 : 32) : 128;
+    const int jgran = (!P.sorted && full_split < 2LL * n_sm) ? 64 : 128;
     const double target = conc * 4.0;
     if (items > 0 && items < target) {
         const int f = (int)std::ceil(target / (double)items);
@@ -443,7 +508,7 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     CK(dalloc(&P.y, 6 * N));
     CK(dalloc(&P.ys, 6 * N));
     CK(dalloc(&P.k, 42 * N));
-    CK(dalloc(&P.part, (size_t)std::max(P.max_slots, 1) * SG_PART_ARRAYS * NP));
+    CK(dalloc(&P.part, (size_t)std::max(P.max_slots, 1) * SG_PART_DOUBLES * NP));
     CK(dalloc(&P.coulS, 3 * N));
     CK(dalloc(&P.coul1, 3 * N));
     CK(dalloc(&P.coul7, 3 * N));
@@ -504,7 +569,7 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     for (int i = 0; i < P.n; i++) P.perm[i] = i;
     CK(cudaMemcpy(P.dperm, P.perm.data(), sizeof(int) * P.n, cudaMemcpyHostToDevice));
     CK(cudaMemset(P.coul1, 0, 3 * N * sizeof(double)));
-    CK(cudaMemset(P.part, 0, (size_t)std::max(P.max_slots, 1) * SG_PART_ARRAYS * NP * sizeof(double)));
+    CK(cudaMemset(P.part, 0, (size_t)std::max(P.max_slots, 1) * SG_PART_DOUBLES * NP * sizeof(double)));
     CK(cudaMemset(P.coulS, 0, 3 * N * sizeof(double)));
     CK(cudaMallocHost((void**)&P.hctrl, sizeof(SgCtrl) * (size_t)std::max(P.n_clouds, 1)));
     CK(cudaMemcpy(P.drows, P.hrows.data(), sizeof(SgRowBlock) * P.hrows.size(),
@@ -689,6 +754,7 @@ int launch_coulomb(sg_ctx* ctx, Problem& P, bool with_ctrl, double inter, double
     ca.npad_total = P.npad;
     ca.errword = P.flags;
     ca.variant = P.variant;
+    ca.sym = P.sym ? 1 : 0;
     ca.bbox = P.bbox;
     ca.fix_list = P.fix_list;
     ca.fix_part = P.fix_part;
@@ -723,8 +789,8 @@ int launch_coulomb(sg_ctx* ctx, Problem& P, bool with_ctrl, double inter, double
         CK(cudaEventRecord(tl.b, ctx->stream));
         ctx->pending.push_back(tl);
     }
-    CK(sg_launch_coulomb_reduce(ca, P.drows, P.n_rows, f32 ? 1 : 0, out, P.n, P.flags + 2,
-                                ctx->stream));
+    CK(sg_launch_coulomb_reduce(ca, P.drows, P.n_rows, P.hrows[0].cap, f32 ? 1 : 0, out, P.n,
+                                P.flags + 2, ctx->stream));
     return SG_OK;
 }
 
@@ -1090,6 +1156,7 @@ int upload_state(sg_ctx* ctx, Problem& P, const double* pos, const double* vel,
     }
     for (int c = 0; c < P.n_clouds; c++) {
         set_frame(P.hc[c], pos, P.hc[c].off);
+        P.hc[c].psc = -(P.hc[c].invL * P.hc[c].invL) * P.hc[c].qscale;
         if (P.kfar_prior > 0.0) P.hc[c].kfar2 = (float)(P.kfar_prior * P.kfar_prior);
         double v2 = 0.0;
         if (vel)
@@ -1215,6 +1282,7 @@ int sg_destroy(sg_ctx* ctx) {
     cudaFree(ctx->cb_mj);
     cudaFree(ctx->cb_xi);
     cudaFree(ctx->cb_ai);
+    cudaFree(ctx->cb_part);
     if (ctx->cb_host) cudaFreeHost(ctx->cb_host);
     cudaFreeHost(ctx->herr);
     cudaStreamDestroy(ctx->stream);
@@ -2359,7 +2427,23 @@ int cb_begin(double xj[][3], double mj[], double xi[][3], double eps2, int ni, i
     CK(cudaMemcpyAsync(ctx->cb_xj, xj, 3 * sizeof(double) * nj, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->cb_mj, mj, sizeof(double) * nj, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->cb_xi, xi, 3 * sizeof(double) * ni, cudaMemcpyHostToDevice, ctx->stream));
-    CK(sg_cunbody_launch(ctx->cb_xj, ctx->cb_mj, ctx->cb_xi, eps2, ctx->cb_ai, ni, nj, ctx->stream));
+    // one set against itself, bit for bit, takes each unordered pair once; comparing the
+    // arrays costs the host ~10 us per 10,000 ions, the pairs it saves milliseconds
+    const int same = ni == nj && ni <= SG_SYM_MAX_IONS &&
+                     memcmp(xj, xi, 3 * sizeof(double) * (size_t)ni) == 0;
+    int uniform = same && mj[0] != 0.0 && std::isfinite(mj[0]);
+    for (int j = 1; uniform && j < nj; j++) uniform = mj[j] == mj[0];
+    const size_t need = sg_cunbody_scratch(ni, nj, same, ctx->n_sm);
+    if (need > ctx->cb_part_cap) {
+        cudaStreamSynchronize(ctx->stream);
+        cudaFree(ctx->cb_part);
+        ctx->cb_part = nullptr;
+        ctx->cb_part_cap = 0;
+        CK(dalloc(&ctx->cb_part, need));
+        ctx->cb_part_cap = need;
+    }
+    CK(sg_cunbody_launch(ctx->cb_xj, ctx->cb_mj, ctx->cb_xi, eps2, ctx->cb_ai, ni, nj, same,
+                         uniform, same ? mj[0] : 0.0, ctx->cb_part, ctx->n_sm, ctx->stream));
     CK(cudaMemcpyAsync(ctx->cb_host, ctx->cb_ai, 3 * sizeof(double) * ni, cudaMemcpyDeviceToHost,
                        ctx->stream));
     return SG_OK;

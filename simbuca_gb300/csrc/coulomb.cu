@@ -19,12 +19,15 @@
 // consecutive j-ions.  j-tiles are fetched with TMA bulk copies (cp.async.bulk) into
 // a 4-stage shared-memory ring guarded by mbarriers.
 //
-// FP64 (coulomb_fp64_kernel): the plain form, every operation in FP64; 1/sqrt(r^2)
-// is an FP32 SFU seed refined by one third-order step of the binomial series
-// 1/sqrt(1-e) = 1 + e/2 + 3e^2/8 (e = 1 - r^2 y0^2), accurate to ~1 ulp.
+// FP64 (coulomb_fp64_sym_kernel, fp64_pairs.cuh): the plain form, every operation in
+// FP64, each unordered pair evaluated once; 1/r^3 is the SFU's FP64 seed refined by one
+// third-order step of the binomial series (inv_r3_fp64), accurate to ~1 ulp.
 #include <stdio.h>
 
+#include <algorithm>
+
 #include "fp32c_math.cuh"
+#include "fp64_pairs.cuh"
 #include "sg_internal.cuh"
 
 namespace {
@@ -89,54 +92,142 @@ __device__ __forceinline__ void fence_proxy_async() {
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-// Close pairs of one flagged ion against one shared-memory tile, evaluated by the
-// whole warp (lanes stride over the tile): pairs whose FP32 1/r^3 exceeded wc get their
-// exact FP64 term, minus the capped FP32 term the main loop already summed (a product
-// of two floats, exact in FP64).  Returns the warp-reduced correction (all lanes) and,
-// in ymx, the tile's strongest FP32 term as a y3 (pairs below the cap, capped terms:
-// capped_term_y3), which the main loop's y3max cannot give for a tile with a close pair.
-template <int TL>
-__device__ __forceinline__ void close_pairs_warp(const float (*tl)[TL], int len, int j0,
-                                                 int ig, float xih, float yih, float zih,
-                                                 float xil, float yil, float zil, float wc,
-                                                 double invL2, double qscale,
-                                                 const double* __restrict__ c64,
-                                                 int npad_total, double& ox, double& oy,
-                                                 double& oz, float& ymx) {
+// Close pairs of one flagged ion (lane src's, padded index ig) among the j-ions
+// [jb, je) of one shared-memory tile, by the whole warp (lanes stride over the j-ions):
+// pairs whose FP32 1/r^3 exceeded wc get their exact term minus the capped FP32 term the
+// main loop already summed, added in lane order to the ion's float-float corrections
+// corr[0..5][li] (hi x, y, z, lo x, y, z; frame units) by lane src.  Returns the strongest
+// FP32 term of these j-ions as a y3 (pairs below the cap, capped terms: capped_term_y3),
+// which the main loop's y3max cannot give where there is a close pair.
+template <int TL, int NI>
+__device__ __forceinline__ float close_pairs_warp(const float (*tl)[TL], int jb, int je, int j0,
+                                                  int ig, float xih, float yih, float zih,
+                                                  float xil, float yil, float zil, float wc,
+                                                  double sc, const double* __restrict__ c64,
+                                                  int npad_total, int src, float (*corr)[NI],
+                                                  int li) {
     const int lane = threadIdx.x & 31;
-    const double xi = c64[ig], yi = c64[npad_total + ig], zi = c64[2 * (size_t)npad_total + ig];
-    double cx = 0.0, cy = 0.0, cz = 0.0;
     float ym = 0.f;
-    for (int jj = lane; jj < len; jj += 32) {
-        const PairF p = pair_f32(tl[0][jj], tl[1][jj], tl[2][jj], tl[4][jj], tl[5][jj],
-                                 tl[6][jj], xih, yih, zih, xil, yil, zil);
-        const int jg = j0 + jj;
-        if (jg != ig && tl[3][jj] != 0.f)
-            ym = fmaxf(ym, p.y3 > wc ? capped_term_y3(p.y3, wc) : p.y3);
-        if (p.y3 > wc && jg != ig) {
-            const float wf = __fmul_rn(tl[3][jj], wc);
-            const double rx = xi - c64[jg];
-            const double ry = yi - c64[npad_total + jg];
-            const double rz = zi - c64[2 * (size_t)npad_total + jg];
-            const double r2d = rx * rx + ry * ry + rz * rz;
-            const double inv = rsqrt_fp64(r2d);
-            const double wq = c64[3 * (size_t)npad_total + jg] * inv * inv * inv;
-            const double wsc = invL2 * qscale * (double)wf;
-            cx += wq * rx + wsc * (double)p.dx;
-            cy += wq * ry + wsc * (double)p.dy;
-            cz += wq * rz + wsc * (double)p.dz;
+    for (int j1 = jb; j1 < je; j1 += 32) {
+        const int jj = j1 + lane;
+        bool close = false;
+        ff cx{0.f, 0.f}, cy{0.f, 0.f}, cz{0.f, 0.f};
+        if (jj < je) {
+            const float xh = tl[0][jj], yh = tl[1][jj], zh = tl[2][jj], q = tl[3][jj];
+            const float xl = tl[4][jj], yl = tl[5][jj], zl = tl[6][jj];
+            const PairF p = pair_f32(xh, yh, zh, xl, yl, zl, xih, yih, zih, xil, yil, zil);
+            const int jg = j0 + jj;
+            if (jg != ig && q != 0.f) {
+                close = p.y3 > wc;
+                ym = fmaxf(ym, close ? capped_term_y3(p.y3, wc) : p.y3);
+            }
+            if (close) {
+                const float wf = __fmul_rn(q, wc);
+                if (p.y3 <= kVeryClose) {
+                    close_term_ff(ff_diff(xh, xl, xih, xil), ff_diff(yh, yl, yih, yil),
+                                  ff_diff(zh, zl, zih, zil), q, wf, p, cx, cy, cz);
+                } else {
+                    const size_t NP = (size_t)npad_total;
+                    const double rx = c64[ig] - c64[jg], ry = c64[NP + ig] - c64[NP + jg],
+                                 rz = c64[2 * NP + ig] - c64[2 * NP + jg];
+                    const double w = c64[3 * NP + jg] * inv_r3_fp64(rx * rx + ry * ry + rz * rz);
+                    const double c[3] = {w * rx / sc - (double)wf * (double)p.dx,
+                                         w * ry / sc - (double)wf * (double)p.dy,
+                                         w * rz / sc - (double)wf * (double)p.dz};
+                    cx.h = (float)c[0];
+                    cx.l = (float)(c[0] - (double)cx.h);
+                    cy.h = (float)c[1];
+                    cy.l = (float)(c[1] - (double)cy.h);
+                    cz.h = (float)c[2];
+                    cz.l = (float)(c[2] - (double)cz.h);
+                }
+            }
+        }
+        unsigned m = __ballot_sync(0xffffffffu, close);
+        while (m) {
+            const int from = __ffs(m) - 1;
+            m &= m - 1;
+            ff a, b, c;
+            a.h = __shfl_sync(0xffffffffu, cx.h, from);
+            a.l = __shfl_sync(0xffffffffu, cx.l, from);
+            b.h = __shfl_sync(0xffffffffu, cy.h, from);
+            b.l = __shfl_sync(0xffffffffu, cy.l, from);
+            c.h = __shfl_sync(0xffffffffu, cz.h, from);
+            c.l = __shfl_sync(0xffffffffu, cz.l, from);
+            if (lane == src) {
+                a = ff_add({corr[0][li], corr[3][li]}, a);
+                b = ff_add({corr[1][li], corr[4][li]}, b);
+                c = ff_add({corr[2][li], corr[5][li]}, c);
+                corr[0][li] = a.h;
+                corr[1][li] = b.h;
+                corr[2][li] = c.h;
+                corr[3][li] = a.l;
+                corr[4][li] = b.l;
+                corr[5][li] = c.l;
+            }
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        cx += __shfl_xor_sync(0xffffffffu, cx, o);
-        cy += __shfl_xor_sync(0xffffffffu, cy, o);
-        cz += __shfl_xor_sync(0xffffffffu, cz, o);
-    }
-    ox = cx;
-    oy = cy;
-    oz = cz;
     // non-negative floats order as their bit patterns
-    ymx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ym)));
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ym)));
+}
+
+// The conditioning estimate's strongest FP32 term of the j-ions [jb, je) just summed
+// (fmx), and their close pairs: one flagged ion at a time by the whole warp.  y3max: per
+// ion the largest 1/r^3 of these j-ions, the self pair left out; reset here.  LI(k): the
+// thread's k-th ion in the corrections array.
+template <int IPT, int TL, int NI, typename LI>
+__device__ __forceinline__ void fold_close(const float (*tl)[TL], int jb, int je, int j0,
+                                           const int* ipad, const f2* xh, const f2* yh,
+                                           const f2* zh, const f2* xl, const f2* yl, const f2* zl,
+                                           float wc, double sc, const double* __restrict__ c64,
+                                           int npad_total, float (*corr)[NI], float* y3max,
+                                           float* fmx, LI li) {
+#pragma unroll
+    for (int k = 0; k < IPT; k++) {
+        const bool hit = y3max[k] > wc;
+        if (!hit) fmx[k] = fmaxf(fmx[k], y3max[k]);
+        y3max[k] = 0.f;
+        unsigned m = __ballot_sync(0xffffffffu, hit && ipad[k] >= 0);
+        while (m) {
+            const int src = __ffs(m) - 1;
+            m &= m - 1;
+            float a, dummy;
+            upk(xh[k], a, dummy);
+            const float xih = __shfl_sync(0xffffffffu, a, src);
+            upk(yh[k], a, dummy);
+            const float yih = __shfl_sync(0xffffffffu, a, src);
+            upk(zh[k], a, dummy);
+            const float zih = __shfl_sync(0xffffffffu, a, src);
+            upk(xl[k], a, dummy);
+            const float xil = __shfl_sync(0xffffffffu, a, src);
+            upk(yl[k], a, dummy);
+            const float yil = __shfl_sync(0xffffffffu, a, src);
+            upk(zl[k], a, dummy);
+            const float zil = __shfl_sync(0xffffffffu, a, src);
+            const int igs = __shfl_sync(0xffffffffu, ipad[k], src);
+            const float ymx = close_pairs_warp<TL, NI>(tl, jb, je, j0, igs, xih, yih, zih, xil, yil,
+                                                       zil, wc, sc, c64, npad_total, src, corr,
+                                                       li(k));
+            if ((threadIdx.x & 31) == src) fmx[k] = fmaxf(fmx[k], ymx);
+        }
+    }
+}
+
+// One ion's partial sums of a slot: the float-float sum hi x, y, z, lo x, y, z of the
+// Kahan accumulator and the close-pair corrections in frame units, and the conditioning
+// estimate s2.  No FP64: converting and scaling here cost every warp ~25 FP64
+// instructions of 64 cycles per slot; the reduction does it once per ion.
+template <int NI>
+__device__ __forceinline__ void store_partial(float* __restrict__ P, size_t NP, int ig,
+                                              const float* ks, const float* kc,
+                                              float (*corr)[NI], int li, float s2, float fmx) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const ff v = ff_add({ks[c], -kc[c]}, {corr[c][li], corr[3 + c][li]});
+        P[c * NP + ig] = v.h;
+        P[(3 + c) * NP + ig] = v.l;
+    }
+    P[6 * NP + ig] = conditioning_s2(s2, fmx);
 }
 
 // Main loop over one shared-memory j-tile for the IPT ions of a thread: packed FP32x2
@@ -252,17 +343,16 @@ __global__ void __launch_bounds__(NT) coulomb_fp32c_kernel(const float* __restri
     __shared__ __align__(128) float tile[SG_STAGES][7][T];
     __shared__ __align__(8) uint64_t full[SG_STAGES];
     __shared__ __align__(8) uint64_t never;  // the wait test's barrier
-    __shared__ double corr[3][NT * IPT];
+    __shared__ float corr[6][NT * IPT];
 
     const SgWorkItem it = items[blockIdx.x];
     const int wtest = errword ? errword[SG_FLAG_WAIT_TILE] : 0;
     if (ctrl != nullptr && (ctrl[it.cloud].done || ctrl[it.cloud].hold || ctrl[it.cloud].status != SG_OK)) return;
     const SgCloud& cl = clouds[it.cloud];
     const float wc = cl.wc;
-    const double invL2 = cl.invL * cl.invL;
     // uniform-charge clouds hold q_j / qscale (1 for ions, 0 for padding): tiles without
     // padding skip the charge product and the sums are scaled once at the end
-    const double qscale = cl.qscale;
+    const double sc = cl.psc;
     const int j_real_end = cl.poff + cl.n;
     const int tid = threadIdx.x;
     const float* X = c32;
@@ -287,9 +377,8 @@ __global__ void __launch_bounds__(NT) coulomb_fp32c_kernel(const float* __restri
         xl[k] = pk(d, d);
         yl[k] = pk(e, e);
         zl[k] = pk(f, f);
-        corr[0][li] = 0.0;
-        corr[1][li] = 0.0;
-        corr[2][li] = 0.0;
+#pragma unroll
+        for (int c = 0; c < 6; c++) corr[c][li] = 0.f;
     }
     float ks[IPT][3], kc[IPT][3], s2[IPT], fmx[IPT];
 #pragma unroll
@@ -390,45 +479,8 @@ __global__ void __launch_bounds__(NT) coulomb_fp32c_kernel(const float* __restri
                 // sum of squared partial sums: estimates sum_j |f_ij|^2 (conditioning test)
                 s2[k] = fmaf(tx_, tx_, fmaf(ty_, ty_, fmaf(tz_, tz_, s2[k])));
             }
-        }
-        // the strongest single FP32 term so far (conditioning estimate); a tile with a
-        // close pair gives its strongest term below the cap from the close-pair pass
-#pragma unroll
-        for (int k = 0; k < IPT; k++)
-            if (y3max[k] <= wc) fmx[k] = fmaxf(fmx[k], y3max[k]);
-        // close pairs of this tile, one flagged ion at a time by the whole warp
-#pragma unroll
-        for (int k = 0; k < IPT; k++) {
-            unsigned m = __ballot_sync(0xffffffffu, y3max[k] > wc && ipad[k] >= 0);
-            while (m) {
-                const int src = __ffs(m) - 1;
-                m &= m - 1;
-                float a, dummy;
-                upk(xh[k], a, dummy);
-                const float xih = __shfl_sync(0xffffffffu, a, src);
-                upk(yh[k], a, dummy);
-                const float yih = __shfl_sync(0xffffffffu, a, src);
-                upk(zh[k], a, dummy);
-                const float zih = __shfl_sync(0xffffffffu, a, src);
-                upk(xl[k], a, dummy);
-                const float xil = __shfl_sync(0xffffffffu, a, src);
-                upk(yl[k], a, dummy);
-                const float yil = __shfl_sync(0xffffffffu, a, src);
-                upk(zl[k], a, dummy);
-                const float zil = __shfl_sync(0xffffffffu, a, src);
-                const int igs = __shfl_sync(0xffffffffu, ipad[k], src);
-                double ox, oy, oz;
-                float ymx;
-                close_pairs_warp(tile[s], len, j0, igs, xih, yih, zih, xil, yil, zil, wc, invL2, qscale,
-                                 c64, npad_total, ox, oy, oz, ymx);
-                if ((tid & 31) == src) {
-                    fmx[k] = fmaxf(fmx[k], ymx);
-                    const int li = tid + k * NT;
-                    corr[0][li] += ox;
-                    corr[1][li] += oy;
-                    corr[2][li] += oz;
-                }
-            }
+            fold_close<IPT>(tile[s], jb, je, j0, ipad, xh, yh, zh, xl, yl, zl, wc, sc, c64,
+                            npad_total, corr, y3max, fmx, [tid](int k) { return tid + k * NT; });
         }
         __syncthreads();  // every thread is done with ring slot s
         if (tid == 0 && t + SG_STAGES < ntiles) {
@@ -442,20 +494,13 @@ __global__ void __launch_bounds__(NT) coulomb_fp32c_kernel(const float* __restri
         }
     }
     if (!ok) return;
-    double* P = part + (size_t)it.slot * SG_PART_ARRAYS * npad_total;
+    const size_t NP = (size_t)npad_total;
+    float* P = reinterpret_cast<float*>(part) + (size_t)it.slot * SG_PART_F32 * NP;
 #pragma unroll
     for (int k = 0; k < IPT; k++) {
         if (ipad[k] < 0) continue;
-        const int li = tid + k * NT;
-        const int ig = ipad[k];
-        P[3 * (size_t)npad_total + ig] = (double)conditioning_s2(s2[k], fmx[k]) * (qscale * qscale);
-        P[4 * (size_t)npad_total + ig] = 0.0;  // no far tiles in this form
-        // P_i = sum q_j (x_i - x_j)/r^3 = -invL^2 qscale sum w (u_j - u_i) + close-pair
-        // terms, w carrying the charges q_j / qscale
-        const double sc = -invL2 * qscale;
-        P[ig] = sc * ((double)ks[k][0] - (double)kc[k][0]) + corr[0][li];
-        P[npad_total + ig] = sc * ((double)ks[k][1] - (double)kc[k][1]) + corr[1][li];
-        P[2 * (size_t)npad_total + ig] = sc * ((double)ks[k][2] - (double)kc[k][2]) + corr[2][li];
+        store_partial(P, NP, ipad[k], ks[k], kc[k], corr, tid + k * NT, s2[k], fmx[k]);
+        P[7 * NP + ipad[k]] = 0.f;  // no far tiles in this form
     }
 }
 
@@ -501,17 +546,16 @@ __global__ void __launch_bounds__(NT, MINB) coulomb_fp32c_sorted_kernel(const fl
     __shared__ __align__(128) float tile[STAGES][7][T];
     __shared__ __align__(8) uint64_t full[STAGES];
     __shared__ __align__(8) uint64_t never;  // the wait test's barrier
-    __shared__ double corr[3][NT * IPT];
+    __shared__ float corr[6][NT * IPT];
 
     const SgWorkItem it = items[blockIdx.x];
     const int wtest = errword ? errword[SG_FLAG_WAIT_TILE] : 0;
     if (ctrl != nullptr && (ctrl[it.cloud].done || ctrl[it.cloud].hold || ctrl[it.cloud].status != SG_OK)) return;
     const SgCloud& cl = clouds[it.cloud];
     const float wc = cl.wc;
-    const double invL2 = cl.invL * cl.invL;
     // uniform-charge clouds hold q_j / qscale (1 for ions, 0 for padding): tiles without
     // padding skip the charge product and the sums are scaled once at the end
-    const double qscale = cl.qscale;
+    const double sc = cl.psc;
     const int j_real_end = cl.poff + cl.n;
     const int tid = threadIdx.x;
     const float* X = c32;
@@ -536,9 +580,8 @@ __global__ void __launch_bounds__(NT, MINB) coulomb_fp32c_sorted_kernel(const fl
         xl[k] = pk(d, d);
         yl[k] = pk(e, e);
         zl[k] = pk(f, f);
-        corr[0][li] = 0.0;
-        corr[1][li] = 0.0;
-        corr[2][li] = 0.0;
+#pragma unroll
+        for (int c = 0; c < 6; c++) corr[c][li] = 0.f;
     }
     float ks[IPT][3], kc[IPT][3], s2[IPT], s2f[IPT], fmx[IPT];
 #pragma unroll
@@ -651,45 +694,10 @@ __global__ void __launch_bounds__(NT, MINB) coulomb_fp32c_sorted_kernel(const fl
                     tile_pairs<IPT, true>(tx, ty, tz, tq, txl, tyl, tzl, jb, je, j0, ipad, xh, yh,
                                           zh, xl, yl, zl, tiny2, wc, ax, ay, az, y3max);
                 fold_partials<IPT, S2F>(ax, ay, az, ks, kc, s2, s2f, !far);
-            }
-        }
-        // the strongest single FP32 term so far (conditioning estimate); a tile with a
-        // close pair gives its strongest term below the cap from the close-pair pass
-#pragma unroll
-        for (int k = 0; k < IPT; k++)
-            if (y3max[k] <= wc) fmx[k] = fmaxf(fmx[k], y3max[k]);
-        // close pairs of this tile, one flagged ion at a time by the whole warp
-#pragma unroll
-        for (int k = 0; k < IPT; k++) {
-            unsigned m = __ballot_sync(0xffffffffu, y3max[k] > wc && ipad[k] >= 0);
-            while (m) {
-                const int src = __ffs(m) - 1;
-                m &= m - 1;
-                float a, dummy;
-                upk(xh[k], a, dummy);
-                const float xih = __shfl_sync(0xffffffffu, a, src);
-                upk(yh[k], a, dummy);
-                const float yih = __shfl_sync(0xffffffffu, a, src);
-                upk(zh[k], a, dummy);
-                const float zih = __shfl_sync(0xffffffffu, a, src);
-                upk(xl[k], a, dummy);
-                const float xil = __shfl_sync(0xffffffffu, a, src);
-                upk(yl[k], a, dummy);
-                const float yil = __shfl_sync(0xffffffffu, a, src);
-                upk(zl[k], a, dummy);
-                const float zil = __shfl_sync(0xffffffffu, a, src);
-                const int igs = __shfl_sync(0xffffffffu, ipad[k], src);
-                double ox, oy, oz;
-                float ymx;
-                close_pairs_warp(tile[s], len, j0, igs, xih, yih, zih, xil, yil, zil, wc, invL2, qscale,
-                                 c64, npad_total, ox, oy, oz, ymx);
-                if ((tid & 31) == src) {
-                    fmx[k] = fmaxf(fmx[k], ymx);
-                    const int li = IPT * tid + k;
-                    corr[0][li] += ox;
-                    corr[1][li] += oy;
-                    corr[2][li] += oz;
-                }
+                if (!far)
+                    fold_close<IPT>(tile[s], jb, je, j0, ipad, xh, yh, zh, xl, yl, zl, wc, sc,
+                                    c64, npad_total, corr, y3max, fmx,
+                                    [tid](int k) { return IPT * tid + k; });
             }
         }
         __syncthreads();  // every thread is done with ring slot s
@@ -704,27 +712,42 @@ __global__ void __launch_bounds__(NT, MINB) coulomb_fp32c_sorted_kernel(const fl
         }
     }
     if (!ok) return;
-    double* P = part + (size_t)it.slot * SG_PART_ARRAYS * npad_total;
+    const size_t NP = (size_t)npad_total;
+    float* P = reinterpret_cast<float*>(part) + (size_t)it.slot * SG_PART_F32 * NP;
 #pragma unroll
     for (int k = 0; k < IPT; k++) {
         if (ipad[k] < 0) continue;
-        const int li = IPT * tid + k;
-        const int ig = ipad[k];
-        P[3 * (size_t)npad_total + ig] = (double)conditioning_s2(s2[k], fmx[k]) * (qscale * qscale);
-        if (S2F) P[4 * (size_t)npad_total + ig] = (double)s2f[k] * (qscale * qscale);
-        // P_i = sum q_j (x_i - x_j)/r^3 = -invL^2 qscale sum w (u_j - u_i) + close-pair
-        // terms, w carrying the charges q_j / qscale
-        const double sc = -invL2 * qscale;
-        P[ig] = sc * ((double)ks[k][0] - (double)kc[k][0]) + corr[0][li];
-        P[npad_total + ig] = sc * ((double)ks[k][1] - (double)kc[k][1]) + corr[1][li];
-        P[2 * (size_t)npad_total + ig] = sc * ((double)ks[k][2] - (double)kc[k][2]) + corr[2][li];
+        store_partial(P, NP, ipad[k], ks[k], kc[k], corr, IPT * tid + k, s2[k], fmx[k]);
+        if (S2F) P[7 * NP + ipad[k]] = s2f[k];
     }
 }
 
 // ---------------------------------------------------------------------------
-// FP64 kernel (plain form).  c64 = 4 double arrays (x, y, z, q) in SI units.
+// FP64 kernels (plain form).  c64 = 4 double arrays (x, y, z, q) in SI units.
 // ---------------------------------------------------------------------------
 
+// Every unordered pair once (fp64_pairs.cuh): a work item is one 128-ion i-block against
+// nj j-ions, rotation steps [s0, s1) of each 32-ion j-tile.
+__global__ void __launch_bounds__(SG_SYM_IB) coulomb_fp64_sym_kernel(
+    const double* __restrict__ c64, const SgWorkItem* __restrict__ items,
+    const SgCloud* __restrict__ clouds, const SgCtrl* __restrict__ ctrl,
+    double* __restrict__ part, int npad_total) {
+    sg_griddep_wait();
+    __shared__ Fp64SymShared sh;
+    const SgWorkItem it = items[blockIdx.x];
+    if (ctrl != nullptr && (ctrl[it.cloud].done || ctrl[it.cloud].hold || ctrl[it.cloud].status != SG_OK)) return;
+    const SgCloud& cl = clouds[it.cloud];
+    const int s0 = it.s01 & 0xffff, s1 = it.s01 >> 16;
+    const size_t NP = (size_t)npad_total;
+    const double* c = c64 + cl.poff;
+    fp64_sym_block<false>([c, NP](int a, int k) { return c[a * NP + k]; }, cl.n, cl.npad,
+                          it.i0 - cl.poff, it.j0 - cl.poff, it.nj, s0, s1, cl.quniform != 0,
+                          cl.qscale, 0.0, part + (size_t)it.slot * 3 * NP + cl.poff,
+                          part + (size_t)it.jslot * 3 * NP + cl.poff, NP, sh);
+}
+
+// Every ordered pair, for clouds whose symmetric partial sums would not fit
+// (SG_SYM_MAX_IONS).
 template <int NT, int IPT>
 __global__ void __launch_bounds__(NT) coulomb_fp64_kernel(const double* __restrict__ c64,
                                                            const SgWorkItem* __restrict__ items,
@@ -769,9 +792,7 @@ __global__ void __launch_bounds__(NT) coulomb_fp64_kernel(const double* __restri
 #pragma unroll
             for (int k = 0; k < IPT; k++) {
                 const double rx = xi[k] - xj, ry = yi[k] - yj, rz = zi[k] - zj;
-                const double r2 = rx * rx + ry * ry + rz * rz;
-                const double y = rsqrt_fp64(r2);
-                double w = qj * (y * y * y);
+                double w = qj * inv_r3_fp64(rx * rx + ry * ry + rz * rz);
                 w = (jg == ipad[k]) ? 0.0 : w;
                 ax[k] = fma(w, rx, ax[k]);
                 ay[k] = fma(w, ry, ay[k]);
@@ -779,12 +800,10 @@ __global__ void __launch_bounds__(NT) coulomb_fp64_kernel(const double* __restri
             }
         }
     }
-    double* P = part + (size_t)it.slot * SG_PART_ARRAYS * npad_total;
+    double* P = part + (size_t)it.slot * 3 * npad_total;
 #pragma unroll
     for (int k = 0; k < IPT; k++) {
         if (ipad[k] < 0) continue;
-        P[3 * (size_t)npad_total + ipad[k]] = 0.0;
-        P[4 * (size_t)npad_total + ipad[k]] = 0.0;
         P[ipad[k]] = ax[k];
         P[npad_total + ipad[k]] = ay[k];
         P[2 * (size_t)npad_total + ipad[k]] = az[k];
@@ -810,12 +829,12 @@ __global__ void __launch_bounds__(NT) coulomb_fp64_kernel(const double* __restri
 // s2f > SgCloud::kfar2 |P_i|^2 gets the exact first-order correction of every far pair
 // term (fixup_ion), which leaves it at the near tiles' FP32 accuracy.
 // ---------------------------------------------------------------------------
-constexpr double kKappa2 = 2.25;
+constexpr float kKappa2 = 2.25f;
 // Clouds of up to kSmallRow padded ions flag at sqrt(s2) > |P| instead: their FP64 row
 // is cheap, and with few terms per ion the error per unit of sqrt(s2)/|P| ran up to
 // ~9e-7 (an unflagged ion at 1.37 measured 1.2e-6 in the 512-cloud scan's small clouds;
 // 2.5e-7 at most on the 65,536-ion cloud).  Their flagged rows are one work unit each.
-constexpr double kKappa2Small = 1.0;
+constexpr float kKappa2Small = 1.0f;
 constexpr int kSmallRow = 4096;
 // kinds of fix-up of a flagged ion
 constexpr int kFixNear = 1, kFixFar = 2;
@@ -891,8 +910,7 @@ __device__ Corr3 fixup_row(const SgCloud& cl, int i, const double* __restrict__ 
         const int jg = cl.poff + j;
         if (jg == igk) continue;
         const double rx = xi - c64[jg], ry = yi - c64[NP + jg], rz = zi - c64[2 * NP + jg];
-        const double inv = rsqrt_fp64(rx * rx + ry * ry + rz * rz);
-        const double wq = c64[3 * NP + jg] * inv * inv * inv;
+        const double wq = c64[3 * NP + jg] * inv_r3_fp64(rx * rx + ry * ry + rz * rz);
         ax = fma(wq, rx, ax);
         ay = fma(wq, ry, ay);
         az = fma(wq, rz, az);
@@ -986,13 +1004,30 @@ __device__ void fixup_ion(const SgCloud& cl, int i, int kind, const float* __res
     __syncthreads();
 }
 
-// Sums the j-chunk partials of each ion (x, y, z and the FP32c conditioning estimates
-// s2, s2f) into out.  FP32c: an ion whose near terms cancel strongly (sqrt(s2) > 1.5 |P|,
-// > |P| in clouds of up to kSmallRow ions) or whose far terms are large next to |P|
-// (s2f > SgCloud::kfar2 |P|^2) is fixed up (fixup_ion): INBLOCK, by this block right away
-// (small batches, where a second launch costs more than the work); otherwise it is put
-// on a work list of coulomb_fixup_kernel (ion index; cloud | kind << 28): the ions whose
-// row is re-evaluated in one list, the far-only ones in the other.
+// The G threads of a row (thread li sums slots li / R, li / R + G, ... of row li % R, R
+// rows in the block): their parts combined in a fixed order by the row's first thread.
+struct SlotShared {
+    float v[SG_ROWS][8];  // FP32c: hi x, y, z, lo x, y, z, s2, s2f
+};
+struct SlotShared64 {
+    double v[SG_ROWS][3];
+};
+
+// Sums the partial-sum slots of each ion into out[3][N] (SI, m^-2), R rows per block with
+// SG_ROWS / R threads each.
+//
+// FP32c: the slots hold float-float sums in frame units (store_partial); they are added
+// in float-float and converted once.  An ion whose near terms cancel strongly
+// (sqrt(s2) > 1.5 |P|, > |P| in clouds of up to kSmallRow ions) or whose far terms are
+// large next to |P| (s2f > SgCloud::kfar2 |P|^2) is fixed up (fixup_ion): INBLOCK, by this
+// block right away (small batches, where a second launch costs more than the work);
+// otherwise it is put on a work list of coulomb_fixup_kernel (ion index; cloud | kind <<
+// 28): the ions whose row is re-evaluated in one list, the far-only ones in the other.
+//
+// Latency-bound for small clouds: an FP64 addition takes a warp 64 cycles, so one thread
+// per row over 32 slots of five FP64 values spent ~5 us on additions alone.  Batches of
+// up to kInBlockFixupMax ions take 16 rows a block, 16 threads each (and the flagged rows
+// of more ions in parallel); larger ones 64 rows of 4 threads.
 template <bool F32, bool INBLOCK>
 __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
     const SgRowBlock* __restrict__ rows, const SgCloud* __restrict__ clouds,
@@ -1000,46 +1035,111 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
     double* __restrict__ out, int n_total, int* __restrict__ counters,
     int* __restrict__ fix_list, const float* __restrict__ c32,
     const double* __restrict__ c64, const float* __restrict__ bbox, float* __restrict__ risk,
-    int* __restrict__ ran, const SgCheck* __restrict__ chk) {
+    int* __restrict__ ran, const SgCheck* __restrict__ chk, int split) {
     sg_griddep_wait();
-    const SgRowBlock rb = rows[blockIdx.x];
+    // this block's share of its row block: cap / split rows
+    SgRowBlock rb = rows[blockIdx.x / split];
+    const int R = rb.cap / split, G = SG_ROWS / R;  // powers of two
+    const int first = (int)(blockIdx.x % split) * R;
+    rb.i0 += first;
+    rb.n = min(rb.n - first, R);
+    if (rb.n <= 0) return;
     if (ctrl != nullptr &&
         (ctrl[rb.cloud].done || ctrl[rb.cloud].hold || ctrl[rb.cloud].status != SG_OK))
         return;
     const SgCloud& cl = clouds[rb.cloud];
     if (!(cl.fp.flags & SG_F_COULOMB)) return;
     const int li = threadIdx.x;
-    const int i = rb.i0 + li;
+    const int row = li & (R - 1), g = li / R;
+    const size_t NP = (size_t)npad_total;
+    const int ig = cl.poff + (rb.i0 - cl.off) + row;  // padded index (row < rb.n)
     int kind = 0;
-    double pf = 0.0;
-    if (li < rb.n) {
-        const int ig = cl.poff + (i - cl.off);
-        const size_t NP = (size_t)npad_total;
-        double px = 0.0, py = 0.0, pz = 0.0, s2 = 0.0, s2f = 0.0;
-        for (int sl = 0; sl < cl.nslots; sl++) {
-            const double* P = part + (size_t)sl * SG_PART_ARRAYS * NP;
-            px += P[ig];
-            py += P[NP + ig];
-            pz += P[2 * NP + ig];
-            if (F32) {
-                s2 += P[3 * NP + ig];
-                s2f += P[4 * NP + ig];
+    const int i = rb.i0 + li;
+    if constexpr (F32) {
+        __shared__ SlotShared ss;
+        ff px{0.f, 0.f}, py{0.f, 0.f}, pz{0.f, 0.f};
+        float s2 = 0.f, s2f = 0.f;
+        if (row < rb.n) {
+            const float* P = reinterpret_cast<const float*>(part) + ig;
+#pragma unroll 4
+            for (int sl = g; sl < cl.nslots; sl += G) {
+                const float* Q = P + (size_t)sl * SG_PART_F32 * NP;
+                px = ff_add(px, {Q[0], Q[3 * NP]});
+                py = ff_add(py, {Q[NP], Q[4 * NP]});
+                pz = ff_add(pz, {Q[2 * NP], Q[5 * NP]});
+                s2 += Q[6 * NP];
+                s2f += Q[7 * NP];
             }
         }
-        out[i] = px;
-        out[(size_t)n_total + i] = py;
-        out[2 * (size_t)n_total + i] = pz;
-        if (F32) {
-            pf = sqrt(px * px + py * py + pz * pz) * (cl.L * cl.L);  // frame units
-            // the far threshold: the prior of the frame set-up, or the measured one
-            const double kf2 = chk ? fmin((double)cl.kfar2, (double)chk[rb.cloud].kfar2)
-                                   : (double)cl.kfar2;
-            const double kap2 = cl.npad <= kSmallRow ? kKappa2Small : kKappa2;
-            kind = (s2 > kap2 * pf * pf ? kFixNear : 0) | (s2f > kf2 * pf * pf ? kFixFar : 0);
-            if (risk != nullptr) {
-                risk[i] = kind ? -1.f : (float)(sqrt(s2f) / pf);
-                risk[(size_t)n_total + i] = kind ? -1.f : (float)(sqrt(s2) / pf);
+        if (G > 1) {
+            float* v = ss.v[li];
+            v[0] = px.h;
+            v[1] = py.h;
+            v[2] = pz.h;
+            v[3] = px.l;
+            v[4] = py.l;
+            v[5] = pz.l;
+            v[6] = s2;
+            v[7] = s2f;
+            __syncthreads();
+        }
+        if (li < rb.n) {
+            for (int q = 1; q < G; q++) {
+                const float* v = ss.v[li + q * R];
+                px = ff_add(px, {v[0], v[3]});
+                py = ff_add(py, {v[1], v[4]});
+                pz = ff_add(pz, {v[2], v[5]});
+                s2 += v[6];
+                s2f += v[7];
             }
+            const double sc = cl.psc;
+            out[i] = sc * ((double)px.h + (double)px.l);
+            out[(size_t)n_total + i] = sc * ((double)py.h + (double)py.l);
+            out[2 * (size_t)n_total + i] = sc * ((double)pz.h + (double)pz.l);
+            // |P|^2 in frame units (a threshold test: FP32)
+            const float pf2 = fmaf(px.h, px.h, fmaf(py.h, py.h, pz.h * pz.h));
+            // the far threshold: the prior of the frame set-up, or the measured one
+            const float kf2 = chk ? fminf(cl.kfar2, chk[rb.cloud].kfar2) : cl.kfar2;
+            const float kap2 = cl.npad <= kSmallRow ? kKappa2Small : kKappa2;
+            kind = (s2 > kap2 * pf2 ? kFixNear : 0) | (s2f > kf2 * pf2 ? kFixFar : 0);
+            if (risk != nullptr) {
+                const float pf = sqrtf(pf2);
+                risk[i] = kind ? -1.f : sqrtf(s2f) / pf;
+                risk[(size_t)n_total + i] = kind ? -1.f : sqrtf(s2) / pf;
+            }
+        }
+    } else {
+        __shared__ SlotShared64 ss;
+        double px = 0.0, py = 0.0, pz = 0.0;
+        if (row < rb.n) {
+            const int ns = cl.sym_k ? sg_sym_slots(cl, ig - cl.poff) : cl.nslots;
+            const double* P = part + ig;
+#pragma unroll 4
+            for (int sl = g; sl < ns; sl += G) {
+                const double* Q = P + (size_t)sl * 3 * NP;
+                px += Q[0];
+                py += Q[NP];
+                pz += Q[2 * NP];
+            }
+        }
+        // pairwise over the G parts: log2(G) dependent FP64 additions
+        for (int h = G / 2; h > 0; h /= 2) {
+            if (g >= h && g < 2 * h) {
+                ss.v[li][0] = px;
+                ss.v[li][1] = py;
+                ss.v[li][2] = pz;
+            }
+            __syncthreads();
+            if (g < h) {
+                px += ss.v[li + h * R][0];
+                py += ss.v[li + h * R][1];
+                pz += ss.v[li + h * R][2];
+            }
+        }
+        if (li < rb.n) {
+            out[i] = px;
+            out[(size_t)n_total + i] = py;
+            out[2 * (size_t)n_total + i] = pz;
         }
     }
     if (F32 && ran != nullptr && li == 0) ran[rb.cloud] = 1;
@@ -1273,28 +1373,35 @@ cudaError_t sg_launch_coulomb_fp32c(const SgCoulombArgs& a, cudaStream_t s) {
 
 cudaError_t sg_launch_coulomb_fp64(const SgCoulombArgs& a, cudaStream_t s) {
     if (a.n_items <= 0) return cudaSuccess;
+    if (a.sym) {
+        sg_launch(coulomb_fp64_sym_kernel, a.n_items, SG_SYM_IB, 0, s, a.c64, a.items, a.clouds,
+                  a.ctrl, a.part, a.npad_total);
+        return cudaGetLastError();
+    }
     sg_launch(coulomb_fp64_kernel<SG_C64_THREADS, SG_C64_IPT>, a.n_items, SG_C64_THREADS, 0, s, 
         a.c64, a.items, a.ctrl, a.part, a.npad_total);
     return cudaGetLastError();
 }
 
 cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* rows, int n_rows,
-                                     int fp32c, double* out, int n_total, int* counters,
-                                     cudaStream_t s) {
+                                     int row_cap, int fp32c, double* out, int n_total,
+                                     int* counters, cudaStream_t s) {
     if (n_rows <= 0) return cudaSuccess;
+    const int take = n_total <= kInBlockFixupMax ? 16 : 64;
+    const int split = std::max(1, row_cap / take);
     if (fp32c) {
         const float* bbox = sg_variant_sorted(a.variant) ? a.bbox : nullptr;
         if (n_total <= kInBlockFixupMax) {
-            sg_launch(coulomb_reduce_kernel<true, true>, n_rows, SG_ROWS, 0, s, 
+            sg_launch(coulomb_reduce_kernel<true, true>, n_rows * split, SG_ROWS, 0, s, 
                 rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, nullptr,
-                a.c32, a.c64, bbox, a.risk, a.ran, a.chk);
+                a.c32, a.c64, bbox, a.risk, a.ran, a.chk, split);
             return cudaGetLastError();
         }
         cudaError_t e = cudaMemsetAsync(a.fix_list, 0, 2 * sizeof(int), s);
         if (e != cudaSuccess) return e;
-        coulomb_reduce_kernel<true, false><<<n_rows, SG_ROWS, 0, s>>>(
+        coulomb_reduce_kernel<true, false><<<n_rows * split, SG_ROWS, 0, s>>>(
             rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, a.fix_list,
-            nullptr, nullptr, nullptr, a.risk, a.ran, a.chk);
+            nullptr, nullptr, nullptr, a.risk, a.ran, a.chk, split);
         // a fixed grid that strides over however many work units there are (a batch of
         // small clouds can flag a few percent of its ions; unused blocks exit at once)
         const int grid = kFixupBlocks;
@@ -1302,9 +1409,9 @@ cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* r
             a.clouds, a.c32, a.c64, a.npad_total, out, n_total, a.fix_list, bbox,
             a.fix_part, a.fix_done);
     } else {
-        sg_launch(coulomb_reduce_kernel<false, false>, n_rows, SG_ROWS, 0, s, 
+        sg_launch(coulomb_reduce_kernel<false, false>, n_rows * split, SG_ROWS, 0, s, 
             rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, nullptr,
-            nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+            nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, split);
     }
     return cudaGetLastError();
 }

@@ -2,7 +2,7 @@
 // by the tiled kernels (coulomb.cu) and the fused small-cloud kernel (fused.cu) so that
 // both take their pair terms, compensated sums and FP64 re-evaluations with the same
 // operations: the SFU reciprocal square root, packed FP32x2 arithmetic, the float-float
-// pair term, Kahan summation, and the refined FP64 reciprocal square root.
+// pair term, Kahan summation, float-float close-pair terms, and the FP64 1/r^3.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -78,13 +78,86 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
 }
 
 
-__device__ __forceinline__ double rsqrt_fp64(double r2) {
-    // FP32 SFU seed, then y = y0 (1 + e/2 + 3 e^2/8), e = 1 - r2 y0^2 (binomial series of
-    // (1-e)^(-1/2)); the truncation error is ~(5/16) e^3 with |e| < 2^-22.
-    const double y0 = (double)rsqrt_approx(__double2float_rn(r2));
-    const double e = fma(-r2 * y0, y0, 1.0);
-    const double p = fma(e, 0.375, 0.5);
-    return fma(y0 * e, p, y0);
+// r2^(-3/2) in FP64: the SFU's FP64 reciprocal square root y0 (rsqrt.approx.ftz.f64,
+// measured |1 - r2 y0^2| <= 1.9e-6), then y0^3 (1 + 3e/2 + 15 e^2/8), the binomial series
+// of (1-e)^(-3/2) with e = 1 - r2 y0^2; the truncation error is 35/16 e^3 < 1.5e-17.
+// GB300 runs every FP64 warp instruction, conversions to and from FP32 included, in 64
+// cycles of its SM sub-partition and the SFU's FP64 seed in 8: this is 6 such
+// instructions, where an FP32 seed with its two conversions, a refined 1/r and its cube
+// were 9.
+__device__ __forceinline__ double inv_r3_fp64(double r2) {
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(r2));
+    const double t = y0 * y0;
+    const double e = fma(-r2, t, 1.0);
+    const double y3 = t * y0;
+    return fma(y3 * e, fma(e, 1.875, 1.5), y3);
+}
+
+// ---- float-float (unevaluated sums hi + lo of two floats, ~48 bits) ------------------
+struct ff {
+    float h, l;
+};
+__device__ __forceinline__ ff ff_fast_two_sum(float a, float b) {  // |a| >= |b| or a == 0
+    const float s = __fadd_rn(a, b);
+    return {s, __fsub_rn(b, __fsub_rn(s, a))};
+}
+__device__ __forceinline__ ff ff_two_sum(float a, float b) {
+    const float s = __fadd_rn(a, b);
+    const float t = __fsub_rn(s, a);
+    return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+}
+__device__ __forceinline__ ff ff_two_prod(float a, float b) {
+    const float p = __fmul_rn(a, b);
+    return {p, __fmaf_rn(a, b, -p)};
+}
+__device__ __forceinline__ ff ff_add(ff a, ff b) {
+    const ff s = ff_two_sum(a.h, b.h);
+    return ff_fast_two_sum(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
+}
+// (ah + al) - (bh + bl) of two float-float coordinates
+__device__ __forceinline__ ff ff_diff(float ah, float al, float bh, float bl) {
+    const ff s = ff_two_sum(ah, -bh);
+    return ff_fast_two_sum(s.h, __fadd_rn(s.l, __fsub_rn(al, bl)));
+}
+__device__ __forceinline__ ff ff_sqr(ff a) {
+    const ff p = ff_two_prod(a.h, a.h);
+    return {p.h, __fmaf_rn(__fmul_rn(2.0f, a.h), a.l, p.l)};
+}
+__device__ __forceinline__ ff ff_mul(ff a, ff b) {
+    const ff p = ff_two_prod(a.h, b.h);
+    return {p.h, __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, p.l))};
+}
+
+// Beyond this 1/r^3 (frame units: closer than 1e-5 of the cloud's spread) a close pair's
+// distance is taken from the SI coordinates in FP64; float-float frame coordinates
+// (absolute error ~1e-14) give the others to better than ~1e-9.
+constexpr float kVeryClose = 1e15f;
+
+// A close pair's exact term q u / |u|^3 (u = u_j - u_i in float-float; q the normalized
+// charge) minus the capped FP32 term wf d the main loop has summed, per component, in
+// frame units.  FP32 instructions only: in FP64 (64 cycles each whatever the active
+// lanes) the ~30 operations of one close pair cost its warp ~2,500 cycles, which on
+// clouds of a few thousand ions was half of the pair kernel.
+__device__ __forceinline__ void close_term_ff(ff ux, ff uy, ff uz, float q, float wf,
+                                              const PairF& p, ff& cx, ff& cy, ff& cz) {
+    const ff r2 = ff_add(ff_add(ff_sqr(ux), ff_sqr(uy)), ff_sqr(uz));
+    const float y = rsqrt_approx(r2.h);
+    const ff y2 = ff_two_prod(y, y);
+    const ff t = ff_two_prod(r2.h, y2.h);
+    // e = 1 - r2 y^2, |e| ~ 2^-22
+    float e = __fsub_rn(__fsub_rn(1.0f, t.h), t.l);
+    e = __fmaf_rn(-r2.h, y2.l, e);
+    e = __fmaf_rn(-r2.l, y2.h, e);
+    const ff y3 = ff_two_prod(y2.h, y);
+    // y^3 (1-e)^(-3/2), then the charge
+    const float c = __fmul_rn(e, __fmaf_rn(e, 1.875f, 1.5f));
+    ff w = ff_fast_two_sum(y3.h, __fmaf_rn(y3.h, c, __fmaf_rn(y2.l, y, y3.l)));
+    w = ff_mul(w, {q, 0.f});
+    const ff dx = ff_two_prod(wf, p.dx), dy = ff_two_prod(wf, p.dy), dz = ff_two_prod(wf, p.dz);
+    cx = ff_add(ff_mul(w, ux), {-dx.h, -dx.l});
+    cy = ff_add(ff_mul(w, uy), {-dy.h, -dy.l});
+    cz = ff_add(ff_mul(w, uz), {-dz.h, -dz.l});
 }
 
 // The conditioning estimate of an ion: the sum of squares of its FP32 partial sums, or,

@@ -41,14 +41,11 @@ namespace {
 constexpr int kThreads = SG_FUSED_THREADS;
 constexpr int kMaxIons = SG_FUSED_MAX_IONS;
 constexpr int kFlush = 16;        // j-ions per FP32 partial sum before the Kahan fold
-constexpr double kKappa2 = 2.25;  // FP64 row when s2 > 2.25 |P|^2 (the tiled reduction's for large clouds)
+constexpr float kKappa2 = 2.25f;  // FP64 row when s2 > 2.25 |P|^2 (the tiled reduction's for large clouds)
 
 struct FusedShared {
-    double part[kThreads][3];  // per thread: its part of P x, y, z (FP64)
-    float s2[kThreads];        // per thread: its conditioning estimate
     int nflag;
-    int flag_il[kThreads];     // flagged ions (local index) ...
-    double flag_corr[kThreads][3];  // ... and their FP64 rows
+    int flag_il[kThreads];  // flagged ions (local index)
 };
 
 __device__ __forceinline__ int ldcg_int(const int* p) { return __ldcg(p); }
@@ -195,10 +192,8 @@ __device__ void coulomb_phase(const SgFusedArgs& f, const SgCloud& cl, int lo, i
     while (2 * G * m <= kThreads && 2 * G <= 32) G *= 2;
     const int il = tid / G, q = tid - (tid / G) * G;
     const int npair = npc / 2;
-    const double invL2 = cl.invL * cl.invL;
-    const double qscale = cl.qscale;
     const float wc = cl.wc;
-    double px = 0.0, py = 0.0, pz = 0.0;
+    ff px{0.f, 0.f}, py{0.f, 0.f}, pz{0.f, 0.f};
     float ps2 = 0.f;
     if (il < m) {
         const int i = lo + il;
@@ -209,7 +204,7 @@ __device__ void coulomb_phase(const SgFusedArgs& f, const SgCloud& cl, int lo, i
         const f2 xl = pk(xil, xil), yl = pk(yil, yil), zl = pk(zil, zil);
         const f2 tiny2 = pk(kTiny, kTiny);
         float ks[3] = {0.f, 0.f, 0.f}, kc[3] = {0.f, 0.f, 0.f}, s2 = 0.f, fmx = 0.f;
-        double cx = 0.0, cy = 0.0, cz = 0.0;
+        ff cx{0.f, 0.f}, cy{0.f, 0.f}, cz{0.f, 0.f};
         for (int p0 = q; p0 < npair; p0 += kFlush / 2 * G) {
             f2 ax = 0ull, ay = 0ull, az = 0ull;
             float y3max = 0.f;
@@ -257,68 +252,84 @@ __device__ void coulomb_phase(const SgFusedArgs& f, const SgCloud& cl, int lo, i
             s2 = fmaf(tx, tx, fmaf(ty, ty, fmaf(tz, tz, s2)));
             if (y3max <= wc) fmx = fmaxf(fmx, y3max);  // blocks without a close pair
             if (y3max > wc) {
-                // close pairs of this partial: the exact FP64 term, minus the capped FP32 term;
-                // the block's strongest FP32 term (below the cap, or capped) for fmx
-                const double xi = SX[li], yi = SY[li], zi = SZ[li];
+                // close pairs of this partial: the exact term minus the capped FP32 one
+                // (close_term_ff; the closest in FP64 from the SI coordinates); the
+                // block's strongest FP32 term (below the cap, or capped) for fmx
                 for (int u = 0; u < kFlush; u++) {
                     const int p = p0 + (u >> 1) * G;
                     if (p >= npair) break;
                     const int jj = 2 * p + (u & 1);
                     const PairF pr = pair_f32(X[jj], Y[jj], Z[jj], XL[jj], YL[jj], ZL[jj], xih,
                                               yih, zih, xil, yil, zil);
-                    if (jj != li && Q[jj] != 0.f)
-                        fmx = fmaxf(fmx, pr.y3 > wc ? capped_term_y3(pr.y3, wc) : pr.y3);
-                    if (pr.y3 > wc && jj != li) {
-                        const float wf = __fmul_rn(Q[jj], wc);
-                        const double rx = xi - SX[jj];
-                        const double ry = yi - SY[jj];
-                        const double rz = zi - SZ[jj];
-                        const double inv = rsqrt_fp64(rx * rx + ry * ry + rz * rz);
-                        const double wq = SQ[jj] * inv * inv * inv;
-                        const double wsc = invL2 * qscale * (double)wf;
-                        cx += wq * rx + wsc * (double)pr.dx;
-                        cy += wq * ry + wsc * (double)pr.dy;
-                        cz += wq * rz + wsc * (double)pr.dz;
+                    if (jj == li || Q[jj] == 0.f) continue;
+                    fmx = fmaxf(fmx, pr.y3 > wc ? capped_term_y3(pr.y3, wc) : pr.y3);
+                    if (!(pr.y3 > wc)) continue;
+                    const float wf = __fmul_rn(Q[jj], wc);
+                    ff dx, dy, dz;
+                    if (pr.y3 <= kVeryClose) {
+                        close_term_ff(ff_diff(X[jj], XL[jj], xih, xil),
+                                      ff_diff(Y[jj], YL[jj], yih, yil),
+                                      ff_diff(Z[jj], ZL[jj], zih, zil), Q[jj], wf, pr, dx, dy, dz);
+                    } else {
+                        const double rx = SX[li] - SX[jj], ry = SY[li] - SY[jj],
+                                     rz = SZ[li] - SZ[jj];
+                        const double w = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz) / cl.psc;
+                        const double c0 = w * rx - (double)wf * (double)pr.dx,
+                                     c1 = w * ry - (double)wf * (double)pr.dy,
+                                     c2 = w * rz - (double)wf * (double)pr.dz;
+                        dx.h = (float)c0;
+                        dx.l = (float)(c0 - (double)dx.h);
+                        dy.h = (float)c1;
+                        dy.l = (float)(c1 - (double)dy.h);
+                        dz.h = (float)c2;
+                        dz.l = (float)(c2 - (double)dz.h);
                     }
+                    cx = ff_add(cx, dx);
+                    cy = ff_add(cy, dy);
+                    cz = ff_add(cz, dz);
                 }
             }
         }
-        // P_i = -invL^2 qscale sum w (u_j - u_i) + close-pair terms (w carries q_j/qscale)
-        const double s = -invL2 * qscale;
-        px = s * ((double)ks[0] - (double)kc[0]) + cx;
-        py = s * ((double)ks[1] - (double)kc[1]) + cy;
-        pz = s * ((double)ks[2] - (double)kc[2]) + cz;
+        px = ff_add({ks[0], -kc[0]}, cx);
+        py = ff_add({ks[1], -kc[1]}, cy);
+        pz = ff_add({ks[2], -kc[2]}, cz);
         ps2 = conditioning_s2(s2, fmx);
     }
-    sh.part[tid][0] = px;
-    sh.part[tid][1] = py;
-    sh.part[tid][2] = pz;
-    sh.s2[tid] = ps2;
+    // the G parts of each ion (G consecutive lanes of one warp), in a fixed order, still in
+    // float-float; lane 0 of the G holds the ion
+    for (int o = G / 2; o > 0; o >>= 1) {
+        ff v;
+        v.h = __shfl_down_sync(0xffffffffu, px.h, o);
+        v.l = __shfl_down_sync(0xffffffffu, px.l, o);
+        px = ff_add(px, v);
+        v.h = __shfl_down_sync(0xffffffffu, py.h, o);
+        v.l = __shfl_down_sync(0xffffffffu, py.l, o);
+        py = ff_add(py, v);
+        v.h = __shfl_down_sync(0xffffffffu, pz.h, o);
+        v.l = __shfl_down_sync(0xffffffffu, pz.l, o);
+        pz = ff_add(pz, v);
+        ps2 += __shfl_down_sync(0xffffffffu, ps2, o);
+    }
     if (tid == 0) sh.nflag = 0;
     __syncthreads();
-    // the G parts of each ion, in a fixed order; the conditioning test (in FP32, frame
-    // units for a unit charge: a threshold test)
-    double P[3] = {0.0, 0.0, 0.0};
-    const int i = lo + tid;
-    if (tid < m) {
-        float s2 = 0.f;
-        for (int g = 0; g < G; g++) {
-            const double* pp = sh.part[tid * G + g];
-            P[0] += pp[0];
-            P[1] += pp[1];
-            P[2] += pp[2];
-            s2 += sh.s2[tid * G + g];
-        }
-        const float sc2 = (float)(cl.L * cl.L / qscale);  // SI sums -> frame units
-        const float pf = sqrtf((float)(P[0] * P[0] + P[1] * P[1] + P[2] * P[2])) * sc2;
-        const bool flagged = s2 > (float)kKappa2 * pf * pf;
+    // the conditioning test (frame units for a unit charge)
+    const int i = lo + il;
+    const bool owner = il < m && q == 0;
+    if (owner) {
+        const double sc_ = cl.psc;  // frame-unit sums -> SI
+        const size_t N = (size_t)f.n;
+        f.coulS[i] = sc_ * ((double)px.h + (double)px.l);
+        f.coulS[N + i] = sc_ * ((double)py.h + (double)py.l);
+        f.coulS[2 * N + i] = sc_ * ((double)pz.h + (double)pz.l);
+        const float pf2 = fmaf(px.h, px.h, fmaf(py.h, py.h, pz.h * pz.h));
+        const bool flagged = ps2 > kKappa2 * pf2;
         if (flagged) {
             const int at = atomicAdd(&sh.nflag, 1);
-            sh.flag_il[at] = tid;
+            sh.flag_il[at] = il;
         }
         if (f.risk != nullptr) {
             f.risk[i] = flagged ? -1.f : 0.f;
-            f.risk[(size_t)f.n + i] = flagged ? -1.f : sqrtf(s2) / pf;
+            f.risk[N + i] = flagged ? -1.f : sqrtf(ps2 / pf2);
         }
     }
     __syncthreads();
@@ -334,8 +345,7 @@ __device__ void coulomb_phase(const SgFusedArgs& f, const SgCloud& cl, int lo, i
         for (int jj = lane; jj < npc; jj += 32) {
             if (jj == li) continue;
             const double rx = xi - SX[jj], ry = yi - SY[jj], rz = zi - SZ[jj];
-            const double inv = rsqrt_fp64(rx * rx + ry * ry + rz * rz);
-            const double wq = SQ[jj] * inv * inv * inv;
+            const double wq = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz);
             ax = fma(wq, rx, ax);
             ay = fma(wq, ry, ay);
             az = fma(wq, rz, az);
@@ -346,23 +356,12 @@ __device__ void coulomb_phase(const SgFusedArgs& f, const SgCloud& cl, int lo, i
             az += __shfl_down_sync(0xffffffffu, az, o);
         }
         if (lane == 0) {
-            sh.flag_corr[k][0] = ax;
-            sh.flag_corr[k][1] = ay;
-            sh.flag_corr[k][2] = az;
+            const int i = lo + sh.flag_il[k];
+            const size_t N = (size_t)f.n;
+            f.coulS[i] = ax;
+            f.coulS[N + i] = ay;
+            f.coulS[2 * N + i] = az;
         }
-    }
-    __syncthreads();
-    for (int k = 0; k < nf; k++)
-        if (sh.flag_il[k] == tid) {
-            P[0] = sh.flag_corr[k][0];
-            P[1] = sh.flag_corr[k][1];
-            P[2] = sh.flag_corr[k][2];
-        }
-    if (tid < m) {
-        const size_t N = (size_t)f.n;
-        f.coulS[i] = P[0];
-        f.coulS[N + i] = P[1];
-        f.coulS[2 * N + i] = P[2];
     }
 }
 

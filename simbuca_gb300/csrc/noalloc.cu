@@ -5,14 +5,18 @@
 // all its device allocation up front and forbids it afterwards (real-time or
 // memory-budgeted loops), or a plug-in that runs inside another framework's device
 // memory pool and is only handed device pointers.  This entry point takes the
-// caller's device buffers for inputs and outputs and keeps its own scratch -- the
-// structure-of-arrays copy of the positions and the per-j-chunk partial sums -- in
-// one file-scope device array of fixed size, so it creates no context, allocates
-// nothing and frees nothing, and it copies nothing from host memory: each block
-// derives its rows and its j-chunk from its block index.
+// caller's device buffers for inputs and outputs and keeps its own scratch -- the partial
+// sums of the pair kernel -- in one file-scope device array of fixed size, so it creates
+// no context, allocates nothing and frees nothing, and it copies nothing from host
+// memory: each block derives its work item from its block index.
+//
+// Two launches: the pairs, each unordered pair once (fp64_pairs.cuh), straight from the
+// caller's arrays, and the sums of the slots.  FP64-bound: 2,048 ions take 100 us, where
+// the ordered pairs over 32 blocks of 128 threads (a fifth of the SMs) with a launch to
+// transpose the positions took 705.
 //
 // Capacity: at most kNaMaxIons ions per call (larger n returns SG_TOO_LARGE before
-// any work is queued).  The array is 1.8 MB and every GPU that loads this library
+// any work is queued).  The array is 13 MB and every GPU that loads this library
 // holds it until the process exits.  All calls on a device share it and it keeps
 // the last call's contents: every scratch entry a call reads is written earlier in
 // the same call, so nothing has to start at zero, but calls that overlap on the GPU
@@ -29,133 +33,31 @@
 #include <algorithm>
 #include <mutex>
 
+#include "fp64_pairs.cuh"
 #include "sg_internal.cuh"
 
 namespace {
 
 constexpr int kNaMaxIons = 8192;
-constexpr int kNaMaxSlots = 8;
-constexpr int kNaThreads = 128;
-constexpr int kNaIpt = 2;
-constexpr int kNaIb = kNaThreads * kNaIpt;
 constexpr int kNaMaxContexts = 64;
+constexpr int kNaSms = 152;  // GB300
 
-// byte offsets inside the scratch array (each a multiple of 256)
-constexpr size_t kOffC64 = 0;
-constexpr size_t kOffPart = kOffC64 + 4 * (size_t)kNaMaxIons * sizeof(double);
-constexpr size_t kScratchBytes = kOffPart + (size_t)kNaMaxSlots * 3 * kNaMaxIons * sizeof(double);
-static_assert(kOffPart % 256 == 0, "scratch regions must stay aligned");
+// the partial-sum slots: 66 at the largest size (64 i-blocks, 128 ions each, on the j
+// side of the last one), more for smaller sets
+constexpr size_t kNaSlotDoubles = (size_t)66 * 3 * kNaMaxIons;
+constexpr size_t kScratchBytes = kNaSlotDoubles * sizeof(double);
 
 static __device__ __align__(256) unsigned char g_na_scratch[kScratchBytes];
 
-__device__ __forceinline__ double* na_c64(unsigned char* scratch) {
-    return reinterpret_cast<double*>(scratch + kOffC64);
-}
-__device__ __forceinline__ double* na_part(unsigned char* scratch) {
-    return reinterpret_cast<double*>(scratch + kOffPart);
-}
-
-// positions [n][3] (caller's device buffer) -> SoA x, y, z, q in the scratch; the
-// padding ions up to npad sit far away with no charge.
-__global__ void na_coords_kernel(unsigned char* scratch, const double* __restrict__ pos,
-                                 const double* __restrict__ q, int n, int npad) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npad) return;
-    double* c = na_c64(scratch);
-    if (i < n) {
-        c[i] = pos[3 * (size_t)i];
-        c[npad + i] = pos[3 * (size_t)i + 1];
-        c[2 * npad + i] = pos[3 * (size_t)i + 2];
-        c[3 * npad + i] = q[i];
-    } else {
-        const double far = 1.0e3 + 1.0e-3 * i;
-        c[i] = far;
-        c[npad + i] = far;
-        c[2 * npad + i] = far;
-        c[3 * npad + i] = 0.0;
+// The caller's device buffers; the padding ions past n sit far away with no charge.
+struct NaLoad {
+    const double *pos, *q;
+    int n;
+    __device__ __forceinline__ double operator()(int a, int k) const {
+        if (k < n) return a < 3 ? pos[3 * (size_t)k + a] : q[k];
+        return a < 3 ? 1.0e3 + 1.0e-3 * k : 0.0;
     }
-}
-
-__device__ __forceinline__ double na_rsqrt(double r2) {
-    float y0f;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0f) : "f"(__double2float_rn(r2)));
-    const double y0 = (double)y0f;
-    const double e = fma(-r2 * y0, y0, 1.0);
-    const double p = fma(e, 0.375, 0.5);
-    return fma(y0 * e, p, y0);
-}
-
-// The FP64 tile kernel of coulomb.cu.  Block b covers rows [ib*kNaIb, +kNaIb) of
-// j-chunk s = b / nib, i.e. columns [s*jc, s*jc + jc) cut at npad, and writes that
-// chunk's partial sums to slot s of the scratch.
-__global__ void __launch_bounds__(kNaThreads) na_coulomb_kernel(unsigned char* scratch, int n,
-                                                               int npad, int nib, int jc) {
-    __shared__ double tile[4][kNaThreads];
-    const int s = blockIdx.x / nib;
-    const int i0 = (blockIdx.x - s * nib) * kNaIb;
-    const int ni = min(kNaIb, n - i0);
-    const int jb = s * jc;
-    const int je = min(jb + jc, npad);
-    const double* c = na_c64(scratch);
-    const int tid = threadIdx.x;
-    int ipad[kNaIpt];
-    double xi[kNaIpt], yi[kNaIpt], zi[kNaIpt], ax[kNaIpt], ay[kNaIpt], az[kNaIpt];
-#pragma unroll
-    for (int k = 0; k < kNaIpt; k++) {
-        const int li = tid + k * kNaThreads;
-        const int ii = i0 + (li < ni ? li : 0);
-        ipad[k] = li < ni ? ii : -1;
-        xi[k] = c[ii];
-        yi[k] = c[npad + ii];
-        zi[k] = c[2 * npad + ii];
-        ax[k] = ay[k] = az[k] = 0.0;
-    }
-    for (int j0 = jb; j0 < je; j0 += kNaThreads) {
-        const int len = min(kNaThreads, je - j0);
-        __syncthreads();
-        if (tid < len) {
-            tile[0][tid] = c[j0 + tid];
-            tile[1][tid] = c[npad + j0 + tid];
-            tile[2][tid] = c[2 * npad + j0 + tid];
-            tile[3][tid] = c[3 * npad + j0 + tid];
-        }
-        __syncthreads();
-        for (int jj = 0; jj < len; jj++) {
-            const double xj = tile[0][jj], yj = tile[1][jj], zj = tile[2][jj], qj = tile[3][jj];
-            const int jg = j0 + jj;
-#pragma unroll
-            for (int k = 0; k < kNaIpt; k++) {
-                const double rx = xi[k] - xj, ry = yi[k] - yj, rz = zi[k] - zj;
-                const double y = na_rsqrt(rx * rx + ry * ry + rz * rz);
-                double w = qj * (y * y * y);
-                w = (jg == ipad[k]) ? 0.0 : w;
-                ax[k] = fma(w, rx, ax[k]);
-                ay[k] = fma(w, ry, ay[k]);
-                az[k] = fma(w, rz, az[k]);
-            }
-        }
-    }
-    double* P = na_part(scratch) + (size_t)s * 3 * npad;
-#pragma unroll
-    for (int k = 0; k < kNaIpt; k++) {
-        if (ipad[k] < 0) continue;
-        P[ipad[k]] = ax[k];
-        P[npad + ipad[k]] = ay[k];
-        P[2 * (size_t)npad + ipad[k]] = az[k];
-    }
-}
-
-// acc[i][c] = kq[i] * sum over the j-chunks of the partial sums (caller's buffers).
-__global__ void na_finish_kernel(unsigned char* scratch, const double* __restrict__ kq,
-                                 double* __restrict__ acc, int n, int npad, int nslots) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double* part = na_part(scratch);
-    double s[3] = {0.0, 0.0, 0.0};
-    for (int sl = 0; sl < nslots; sl++)
-        for (int c = 0; c < 3; c++) s[c] += part[((size_t)sl * 3 + c) * npad + i];
-    for (int c = 0; c < 3; c++) acc[3 * (size_t)i + c] = kq[i] * s[c];
-}
+};
 
 // The current context's unique id, through the driver entry points the runtime hands
 // out (no link against the driver library).
@@ -233,27 +135,21 @@ extern "C" int sg_coulomb_accel_noalloc(int n, const double* pos, const double* 
     if (!scratch) return SG_CUDA_ERR;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int npad = (n + SG_PAD - 1) / SG_PAD * SG_PAD;
-    // blocks: i-blocks of kNaIb ions x up to kNaMaxSlots j-chunks (multiples of 128)
-    const int nib = (n + kNaIb - 1) / kNaIb;
-    int slots = std::max(1, std::min(kNaMaxSlots, npad / 512));
-    const int jc = ((npad + slots - 1) / slots + 127) / 128 * 128;
-    slots = (npad + jc - 1) / jc;
+    const SymPlan plan = sym_plan(npad, kNaSms, kNaSlotDoubles);
+    double* part = reinterpret_cast<double*>(scratch);
     // Each launch's own return value: an error an earlier call left in the runtime's
     // last-error slot neither fails this call nor gets cleared by it.
     cudaLaunchConfig_t cfg = {};
     cfg.stream = st;
-    cfg.gridDim = dim3((npad + 255) / 256);
-    cfg.blockDim = dim3(256);
-    if (cudaLaunchKernelEx(&cfg, na_coords_kernel, scratch, pos, q, n, npad) != cudaSuccess)
+    cfg.gridDim = dim3(plan.items);
+    cfg.blockDim = dim3(SG_SYM_IB);
+    if (cudaLaunchKernelEx(&cfg, sym_set_kernel<false, NaLoad>, NaLoad{pos, q, n}, n, npad, plan,
+                           false, 1.0, 0.0, part) != cudaSuccess)
         return SG_CUDA_ERR;
-    cfg.gridDim = dim3(slots * nib);
-    cfg.blockDim = dim3(kNaThreads);
-    if (cudaLaunchKernelEx(&cfg, na_coulomb_kernel, scratch, n, npad, nib, jc) != cudaSuccess)
-        return SG_CUDA_ERR;
-    cfg.gridDim = dim3((n + 255) / 256);
+    cfg.gridDim = dim3((n + 15) / 16);
     cfg.blockDim = dim3(256);
-    if (cudaLaunchKernelEx(&cfg, na_finish_kernel, scratch, kq, acc, n, npad, slots) !=
-        cudaSuccess)
+    if (cudaLaunchKernelEx(&cfg, sym_sum_kernel<16>, (const double*)part, n, npad, plan, kq, 1.0,
+                           acc) != cudaSuccess)
         return SG_CUDA_ERR;
     return SG_OK;
 }

@@ -63,9 +63,17 @@ inline cudaError_t sg_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 #define SG_PAD 32
 // O(N) kernels: ions per block.
 #define SG_ROWS 256
-// Arrays of a Coulomb partial-sum slot: x, y, z, and the FP32c conditioning estimates
-// of the near tiles and of the far tiles (sums of squared 32-ion partial sums).
-#define SG_PART_ARRAYS 5
+// Arrays of a Coulomb partial-sum slot.  FP32c: eight floats per ion -- the float-float
+// sums hi x, y, z, lo x, y, z in frame units, and the conditioning estimates of the near
+// tiles and of the far tiles (sums of squared partial sums).  FP64: three doubles (SI).
+#define SG_PART_F32 8
+#define SG_PART_DOUBLES 4  // allocated per ion and slot: the larger of the two
+// FP64 Coulomb, each unordered pair once (fp64_pairs.cuh): ions per i-block, ions per
+// j-tile, and the largest cloud it takes (its j-side partial sums need a slot per i-block:
+// 3 GB there; larger clouds sum ordered pairs).
+#define SG_SYM_IB 128
+#define SG_SYM_JT 32
+#define SG_SYM_MAX_IONS 131072
 // FP32c fix-up kernel: work units per listed ion, and the listed ions that get them
 #define SG_FIX_UNITS 16
 #define SG_FIX_CHUNKED_CAP 4096
@@ -92,15 +100,15 @@ struct SgWorkItem {
     int32_t i0, ni;
     int32_t j0, nj;
     int32_t slot;
-    int32_t pad0, pad1;
+    int32_t jslot, s01;  // FP64 symmetric items: j-side slot, rotation steps s0 | s1 << 16
 };
 
 // Rows of one cloud handled by one block of the O(N) kernels.
 struct SgRowBlock {
     int32_t cloud;
     int32_t i0;     // first ion (unpadded global index)
-    int32_t n;      // ions in this block (<= SG_ROWS)
-    int32_t pad;
+    int32_t n;      // ions in this block (<= cap)
+    int32_t cap;    // rows a block of this batch takes at most (a power of two <= SG_ROWS)
 };
 
 // Device description of a cloud.
@@ -127,8 +135,20 @@ struct SgCloud {
     // FP32c charges: the FP32 coordinate array holds q / qscale; with all ions of the cloud
     // at one charge q, qscale = q (quniform = 1) and the normalized charges are 1
     double qscale;
-    int32_t quniform, pad4;
+    double psc;  // frame-unit sums -> SI: -qscale / L^2
+    int32_t quniform;
+    int32_t sym_k, sym_bands;  // FP64 symmetric items: j-tiles per item (0: ordered pairs), bands
+    int32_t pad4;
 };
+
+// Partial-sum slots of the FP64 symmetric form that hold a part of local padded ion p: one
+// per i-block up to its own (j-side) and band, one per j-chunk of its own i-block (i-side)
+// and band.
+__host__ __device__ inline int sg_sym_slots(const SgCloud& cl, int p) {
+    const int b = p / SG_SYM_IB;
+    const int tiles = cl.npad / SG_SYM_JT - b * (SG_SYM_IB / SG_SYM_JT);
+    return (b + 1 + (tiles + cl.sym_k - 1) / cl.sym_k) * cl.sym_bands;
+}
 
 // Per-cloud Dormand-Prince controller (the scalar part of _ode_vars, bin/ode.h:58-97).
 struct SgCtrl {
@@ -460,8 +480,12 @@ cudaError_t sg_soa_to_aos(const double* y, const int* perm, double* pos, double*
 cudaError_t sg_gather(const double* src, const int* perm, double* dst, int n, cudaStream_t st);
 cudaError_t sg_moments(const SgDpArgs& a, const double* mass, double* out, int n_rows,
                        cudaStream_t st);
+// same: xi is the set xj itself (ni = nj); uniform: every mass is m0; part: at least
+// sg_cunbody_scratch doubles
+size_t sg_cunbody_scratch(int ni, int nj, int same, int n_sm);
 cudaError_t sg_cunbody_launch(const double* xj, const double* mj, const double* xi, double eps2,
-                              double* ai, int ni, int nj, cudaStream_t st);
+                              double* ai, int ni, int nj, int same, int uniform, double m0,
+                              double* part, int n_sm, cudaStream_t st);
 cudaError_t sg_probe_launch(int which, int blocks, int threads, float* sink, cudaStream_t st);
 cudaError_t sg_proposer_launch(const SgCloud* clouds, SgCtrl* ctrl, const double* mom,
                                SgProposerState* pst, const void* wbf, float* log_feat,
@@ -485,7 +509,8 @@ struct SgCoulombArgs {
     int n_items;
     const SgCloud* clouds;
     const SgCtrl* ctrl;      // may be null (stand-alone calls)
-    double* part;            // [slots][SG_PART_ARRAYS][Npad]: x, y, z sums, FP32c s2, s2f
+    double* part;            // partial-sum slots (SG_PART_F32 floats or 3 doubles per ion)
+    int sym = 0;             // FP64: the items are symmetric ones (fp64_pairs.cuh)
     int npad_total;
     int* errword;
     int variant;             // FP32c launch shape (sg_coulomb_fp32c_ib)
@@ -543,5 +568,5 @@ int sg_coulomb_fp32c_ib(int variant);
 cudaError_t sg_launch_coulomb_fp32c(const SgCoulombArgs& a, cudaStream_t s);
 cudaError_t sg_launch_coulomb_fp64(const SgCoulombArgs& a, cudaStream_t s);
 cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* rows, int n_rows,
-                                     int fp32c, double* out, int n_total, int* counters,
-                                     cudaStream_t s);
+                                     int row_cap, int fp32c, double* out, int n_total,
+                                     int* counters, cudaStream_t s);

@@ -188,3 +188,52 @@ def test_1m_spheroid_rows_and_momentum(ctx):
     e = rel_err_per_ion(a[rows], ref)
     print(summary(e))
     assert e.max() <= 1e-6, summary(e)
+
+
+@pytest.mark.parametrize("n", [1, 5, 64, 128, 160, 161, 257, 385, 1025, 2050, 6001])
+def test_fp64_unordered_pairs_mixed_charges(ctx, n):
+    """The FP64 form takes each unordered pair once, 128-ion i-blocks against 32-ion
+    j-tiles in bands of rotation steps or runs of tiles: tile and block edges with charges
+    of both signs, one neutral ion, and factors that differ per ion."""
+    rng = np.random.default_rng(n)
+    pos = rng.normal(0, 4e-4, (n, 3)) * np.array([1.0, 0.2, 3.0])
+    q = rng.choice([1.0, 2.0, -1.0], n)
+    q[n // 2] = 0.0 if n > 5 else 1.0
+    kq = kq_of(np.full(n, 132.905 * oracle.AMU), np.where(q == 0.0, 1.0, q))
+    ref = oracle.coulomb_kq(pos, q, kq)
+    a = ctx.coulomb_accel(pos, q, kq, SG_PREC_FP64)
+    if n == 1:
+        assert np.all(a == 0.0)
+        return
+    scale = np.linalg.norm(ref, axis=1)
+    e = np.linalg.norm(a - ref, axis=1) / scale
+    # signed charges cancel: the bound is on the sum of the terms' magnitudes
+    d = np.linalg.norm(pos[:, None] - pos[None], axis=2) if n <= 2050 else None
+    if d is not None:
+        np.fill_diagonal(d, np.inf)
+        e *= scale / (np.abs(kq) * (np.abs(q)[None] / d ** 2).sum(1))
+        assert e.max() <= TOL[SG_PREC_FP64], e.max()
+    else:
+        assert np.percentile(e, 99) <= TOL[SG_PREC_FP64]
+
+
+@pytest.mark.parametrize("n,variant", [(300, -1), (1000, -1), (4000, 5), (20000, 9), (20000, 14)])
+@pytest.mark.parametrize("sep", [1e-5, 1e-8, 1e-12])
+def test_very_close_pairs(ctx, n, variant, sep):
+    """Close pairs are taken in float-float from the frame coordinates, or, closer than 1e-5
+    of the spread, in FP64 from the SI coordinates: pairs on both sides of that line."""
+    rng = np.random.default_rng(n)
+    pos = rng.normal(0, 5e-4, (n, 3))
+    for k in range(0, 20, 2):
+        u = rng.normal(0, 1, 3)
+        pos[k + 1] = pos[k] + sep * u / np.linalg.norm(u)
+    q = np.ones(n)
+    kq = kq_of(np.full(n, 132.905 * oracle.AMU), q)
+    try:
+        ctx.set_coulomb_variant(variant)
+        a = ctx.coulomb_accel(pos, q, kq, SG_PREC_FP32C)
+    finally:
+        ctx.set_coulomb_variant(-1)
+    ref = ctx.coulomb_accel(pos, q, kq, SG_PREC_FP64)
+    e = rel_err_per_ion(a, ref)
+    assert e.max() <= TOL[SG_PREC_FP32C], summary(e)

@@ -48,3 +48,24 @@ def test_begin_end_distinct_sets():
     L.cunbody1_force_end(*args)
     ref = reference_sum(xj, mj, xi, 1e-12)
     np.testing.assert_allclose(ai, ref, rtol=1e-11, atol=1e-11 * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("ni,nj", [(1, 1), (33, 33), (128, 128), (129, 129), (1000, 1000),
+                                   (1, 700), (129, 3000), (5, 128)])
+@pytest.mark.parametrize("eps2", [0.0, 1e-12])
+def test_set_sizes_and_coincident_pairs(ni, nj, eps2):
+    """One array as both sets takes each unordered pair once, different sets take j-chunks:
+    tile edges of both, with two ions at one place (no contribution without softening) and
+    with equal and unequal masses.  The slot's tolerance, as above."""
+    rng = np.random.default_rng(ni + nj)
+    xj = rng.normal(0, 1e-3, (nj, 3))
+    if nj > 2:
+        xj[nj // 2] = xj[0]
+    same = ni == nj
+    xi = xj.copy() if same else rng.normal(0, 1e-3, (ni, 3))
+    if not same:
+        xi[0] = xj[1]
+    for mj in (np.full(nj, 1.5), rng.uniform(0.5, 2.0, nj)):
+        ai = call("cunbody1_force", xj, mj, xi, eps2)
+        ref = reference_sum(xj, mj, xi, eps2)
+        np.testing.assert_allclose(ai, ref, rtol=1e-11, atol=1e-11 * np.abs(ref).max())
