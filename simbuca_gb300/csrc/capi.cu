@@ -24,6 +24,11 @@ struct Problem {
     int n_clouds = 0, n = 0, npad = 0, precision = 0, n_rows = 0, n_items = 0, max_slots = 0;
     int variant = 0;  // FP32c launch shape the items were planned for
     int method = 5;   // 5 Dormand-Prince, 4 Cash-Karp (every cloud of a batch)
+    int row_cap = SG_ROWS;  // rows of a row block at most
+    // small Dormand-Prince batches (finish.cu): two sets of Coulomb coordinates, stage S
+    // reads set S mod 2; last_set: the one the last sum of an attempt was taken at
+    bool finish = false;
+    int last_set = 0;
     bool any_coulomb = false;
     bool sym = false;  // FP64: items take each unordered pair once
     bool uploaded = false;
@@ -40,6 +45,7 @@ struct Problem {
            *coul7 = nullptr, *coulS = nullptr, *kq = nullptr, *qm = nullptr, *qd = nullptr, *mass = nullptr,
            *c64 = nullptr, *err_part = nullptr, *mom = nullptr, *stage = nullptr;
     float* c32 = nullptr;
+    SgFieldCoef* fcoef = nullptr;  // per cloud and stage of the attempt
     int* flags = nullptr;  // [0] error word, [1] hold-on-accept, [2] FP32c fix-up count
     SgCtrl* hctrl = nullptr;  // pinned mirror of dctrl
     double interactions = 0.0;  // per Coulomb evaluation, all clouds
@@ -187,6 +193,7 @@ void free_problem(Problem& P) {
                     P.qd, P.mass, P.c64, P.err_part, P.mom, P.stage};
     for (double* d : ds) cudaFree(d);
     cudaFree(P.c32);
+    cudaFree(P.fcoef);
     cudaFree(P.flags);
     cudaFree(P.pst);
     cudaFree(P.wbf);
@@ -308,13 +315,15 @@ void plan(Problem& P, int n_sm) {
     P.sorted = P.precision == SG_PREC_FP32C && sg_variant_sorted(P.variant);
     // Row blocks of SG_ROWS ions, or fewer for small batches: the stage, control and
     // reduction kernels are FP64 work, which GB300 runs at a small fraction of its FP32
-    // rate per SM, so a 1,000-ion cloud is spread over 32 SMs rather than 4.  The k-d
-    // ordered shapes keep full blocks (each covers two 128-ion tiles for the tile bounds).
+    // rate per SM, so a 1,000-ion cloud is spread over 63 SMs in blocks of 16 rows rather
+    // than 4.  The k-d ordered shapes keep full blocks (each covers two 128-ion tiles).
     long long total_ions = 0;
     for (int c = 0; c < C; c++) total_ions += P.counts[c];
     int rows = SG_ROWS;
-    if (!P.sorted)
+    if (!P.sorted) {
         while (rows > 32 && total_ions / rows < 2LL * n_sm) rows /= 2;
+        if (total_ions <= SG_FINISH_MAX_IONS) rows = 16;
+    }
     for (int c = 0; c < C; c++) {
         SgCloud& cl = P.hc[c];
         memset(&cl, 0, sizeof cl);
@@ -343,6 +352,7 @@ void plan(Problem& P, int n_sm) {
     P.npad = poff;
     P.ntiles = tiles;
     P.n_rows = (int)P.hrows.size();
+    P.row_cap = rows;
 
     const bool f32 = P.precision == SG_PREC_FP32C;
     P.sym = false;
@@ -516,9 +526,10 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     CK(dalloc(&P.qm, N));
     CK(dalloc(&P.qd, N));
     CK(dalloc(&P.mass, N));
-    CK(dalloc(&P.c64, 4 * NP));
-    CK(dalloc(&P.c32, 7 * NP));
-    CK(dalloc(&P.err_part, (size_t)std::max(P.n_rows, 1)));
+    CK(dalloc(&P.c64, (P.finish ? 8 : 4) * NP));
+    CK(dalloc(&P.c32, (P.finish ? 14 : 7) * NP));
+    CK(dalloc(&P.err_part, (size_t)std::max(P.n_rows, 1) * sg_stage_split(P.row_cap)));
+    CK(dalloc(&P.fcoef, (size_t)std::max(P.n_clouds, 1) * SG_MAX_STAGES));
     CK(dalloc(&P.mom, (size_t)std::max(P.n_rows, 1) * 11));
     CK(dalloc(&P.stage, 6 * N));
     CK(dalloc(&P.flags, SG_NFLAGS));
@@ -596,6 +607,8 @@ SgDpArgs dp_args(Problem& P) {
     a.c64 = P.c64;
     a.c32 = P.c32;
     a.err_part = P.err_part;
+    a.fcoef = P.fcoef;
+    a.split = sg_stage_split(P.row_cap);
     a.bbox = P.sorted ? P.bbox : nullptr;
     a.n = P.n;
     a.npad = P.npad;
@@ -740,12 +753,14 @@ void flush_timing(sg_ctx* ctx) {
 // Coulomb sum of an attempt and every stand-alone one); later stages of the attempt
 // reuse it -- the ions barely move within a step, and only the choice of which ions to
 // fix up depends on it.
+// set: the coordinate set of a finish batch to read; out null: the pair kernel alone (the
+// finish kernel sums its slots).
 int launch_coulomb(sg_ctx* ctx, Problem& P, bool with_ctrl, double inter, double* out,
-                   bool far_estimate = true) {
+                   bool far_estimate = true, int set = 0) {
     if (!P.any_coulomb || P.n_items == 0) return SG_OK;
     SgCoulombArgs ca;
-    ca.c32 = P.c32;
-    ca.c64 = P.c64;
+    ca.c32 = P.c32 + (size_t)set * 7 * P.npad;
+    ca.c64 = P.c64 + (size_t)set * 4 * P.npad;
     ca.items = P.ditems;
     ca.n_items = P.n_items;
     ca.clouds = P.dc;
@@ -754,6 +769,7 @@ int launch_coulomb(sg_ctx* ctx, Problem& P, bool with_ctrl, double inter, double
     ca.npad_total = P.npad;
     ca.errword = P.flags;
     ca.variant = P.variant;
+    ca.max_slots = P.max_slots;
     ca.sym = P.sym ? 1 : 0;
     ca.bbox = P.bbox;
     ca.fix_list = P.fix_list;
@@ -789,7 +805,8 @@ int launch_coulomb(sg_ctx* ctx, Problem& P, bool with_ctrl, double inter, double
         CK(cudaEventRecord(tl.b, ctx->stream));
         ctx->pending.push_back(tl);
     }
-    CK(sg_launch_coulomb_reduce(ca, P.drows, P.n_rows, P.hrows[0].cap, f32 ? 1 : 0, out, P.n,
+    if (!out) return SG_OK;
+    CK(sg_launch_coulomb_reduce(ca, P.drows, P.n_rows, P.row_cap, f32 ? 1 : 0, out, P.n,
                                 P.flags + 2, ctx->stream));
     return SG_OK;
 }
@@ -838,18 +855,38 @@ int enqueue_attempt(sg_ctx* ctx, Problem& P) {
         for (int s = 1; s <= 6; s++) {
             int st = launch_coulomb(ctx, P, true, inter, P.coulS, s == 1);
             if (st != SG_OK) return st;
-            STAGE_TIMED(sg_ck_stage(a, s, P.n_rows, ctx->stream));
+            STAGE_TIMED(sg_ck_stage(a, s, P.n_rows, P.row_cap, ctx->stream));
+        }
+    } else if (P.finish) {
+        // stage S writes coordinate set (S + 1) mod 2, the one sum S + 1 reads
+        SgFinishArgs f;
+        f.dp = a;
+        f.part = P.part;
+        f.coulS = P.coulS;
+        f.counters = P.flags + 2;
+        f.risk = P.risk;
+        f.ran = P.ran;
+        f.n_rows = P.n_rows;
+        STAGE_TIMED(sg_dp_stage(a, 1, P.n_rows, P.row_cap, ctx->stream));
+        for (int s = 2; s <= 7; s++) {
+            int st = launch_coulomb(ctx, P, true, inter, nullptr, s == 2, s & 1);
+            if (st != SG_OK) return st;
+            f.c64r = P.c64 + (size_t)(s & 1) * 4 * P.npad;
+            f.dp.c64 = P.c64 + (size_t)((s + 1) & 1) * 4 * P.npad;
+            f.dp.c32 = P.c32 + (size_t)((s + 1) & 1) * 7 * P.npad;
+            STAGE_TIMED(sg_dp_finish(f, s, P.precision == SG_PREC_FP32C ? 1 : 0, ctx->stream));
         }
     } else {
-        STAGE_TIMED(sg_dp_stage(a, 1, P.n_rows, ctx->stream));
+        STAGE_TIMED(sg_dp_stage(a, 1, P.n_rows, P.row_cap, ctx->stream));
         for (int s = 2; s <= 7; s++) {
             int st = launch_coulomb(ctx, P, true, inter, P.coulS, s == 2);
             if (st != SG_OK) return st;
-            STAGE_TIMED(sg_dp_stage(a, s, P.n_rows, ctx->stream));
+            STAGE_TIMED(sg_dp_stage(a, s, P.n_rows, P.row_cap, ctx->stream));
         }
     }
-    STAGE_TIMED(sg_dp_control(P.dc, P.dctrl, P.err_part, P.y, P.n_clouds, P.flags, P.dops,
-                              ctx->stream));
+    // the Gear corrector leaves one error partial per row block
+    STAGE_TIMED(sg_dp_control(P.dc, P.dctrl, P.err_part, P.method == 1 ? 1 : a.split, P.y,
+                              P.n_clouds, P.flags, P.dops, ctx->stream));
     STAGE_TIMED(sg_dp_commit(a, P.n_rows, ctx->stream));
     if (P.rec_cap > 0) CK(sg_record(rec_args(P), P.n_rows, P.n_clouds, ctx->stream));
     if (P.n_dis > 0)
@@ -924,8 +961,8 @@ int maybe_check(sg_ctx* ctx, Problem& P, int attempts = 1) {
     const long long before = P.attempt_count;
     P.attempt_count += attempts;
     if (P.attempt_count / P.check_every == before / P.check_every) return SG_OK;
-    CK(sg_force_check(P.dc, P.n_clouds, P.ran, P.risk, P.c64, P.npad, P.coulS, P.n, P.dchk,
-                      ctx->stream));
+    CK(sg_force_check(P.dc, P.n_clouds, P.ran, P.risk, P.c64 + (size_t)P.last_set * 4 * P.npad,
+                      P.npad, P.coulS, P.n, P.dchk, ctx->stream));
     return SG_OK;
 }
 
@@ -984,6 +1021,7 @@ int run_fused(sg_ctx* ctx, Problem& P, int n, int counted) {
         CK(cudaEventRecord(tl.a, ctx->stream));
     }
     CK(sg_fused_attempts(f, P.fused_cluster, P.max_npad, ctx->stream));
+    P.last_set = 0;
     if (ctx->timing) {
         CK(cudaEventRecord(tl.b, ctx->stream));
         ctx->pending.push_back(tl);
@@ -993,6 +1031,7 @@ int run_fused(sg_ctx* ctx, Problem& P, int n, int counted) {
 
 int run_attempts(sg_ctx* ctx, Problem& P, int n) {
     if (fused_eligible(ctx, P)) return run_fused(ctx, P, n, n);
+    P.last_set = P.finish ? 1 : 0;  // sum 7 of a finish batch
     if (ctx->use_graph && ctx->timing) {
         // graph replays one at a time, reading the Coulomb event pairs after each
         if (!ctx->graph_timed) {
@@ -1168,6 +1207,13 @@ int upload_state(sg_ctx* ctx, Problem& P, const double* pos, const double* vel,
                        ctx->stream));
     SgDpArgs a = dp_args(P);
     CK(sg_coords_from_state(a, P.qd, P.n_rows, ctx->stream));
+    if (P.finish) {  // charges and padding ions of the second coordinate set
+        const size_t NP = (size_t)P.npad;
+        CK(cudaMemcpyAsync(P.c64 + 4 * NP, P.c64, 4 * NP * sizeof(double), cudaMemcpyDeviceToDevice,
+                           ctx->stream));
+        CK(cudaMemcpyAsync(P.c32 + 7 * NP, P.c32, 7 * NP * sizeof(float), cudaMemcpyDeviceToDevice,
+                           ctx->stream));
+    }
     // a new state restarts the Gear history
     if (P.method == 1) CK(sg_gear_init(a, P.dperm, P.n_rows, ctx->stream));
     // the host vectors above are read by queued copies: finish before they go away
@@ -1392,6 +1438,7 @@ int sg_batch_create(sg_ctx* ctx, int n_clouds, const int* counts, const sg_field
     for (int c = 0; c < n_clouds; c++) P.hc[c].fp = fp[c];
     P.fp0.assign(fp, fp + n_clouds);
     plan(P, ctx->n_sm);
+    P.finish = P.method == 5 && P.row_cap == 16;
     P.hctrl0.assign(n_clouds, SgCtrl());
     for (int c = 0; c < n_clouds; c++) {
         SgCtrl& s = P.hctrl0[c];

@@ -829,13 +829,6 @@ __global__ void __launch_bounds__(NT) coulomb_fp64_kernel(const double* __restri
 // s2f > SgCloud::kfar2 |P_i|^2 gets the exact first-order correction of every far pair
 // term (fixup_ion), which leaves it at the near tiles' FP32 accuracy.
 // ---------------------------------------------------------------------------
-constexpr float kKappa2 = 2.25f;
-// Clouds of up to kSmallRow padded ions flag at sqrt(s2) > |P| instead: their FP64 row
-// is cheap, and with few terms per ion the error per unit of sqrt(s2)/|P| ran up to
-// ~9e-7 (an unflagged ion at 1.37 measured 1.2e-6 in the 512-cloud scan's small clouds;
-// 2.5e-7 at most on the 65,536-ion cloud).  Their flagged rows are one work unit each.
-constexpr float kKappa2Small = 1.0f;
-constexpr int kSmallRow = 4096;
 // kinds of fix-up of a flagged ion
 constexpr int kFixNear = 1, kFixFar = 2;
 
@@ -845,7 +838,7 @@ constexpr int kFixupBlocks = 512;
 constexpr int kFarChunks = SG_FIX_UNITS;
 constexpr int kChunkedCap = SG_FIX_CHUNKED_CAP;
 // batches up to this many ions fix their flagged ions inside the reduction's blocks
-constexpr int kInBlockFixupMax = 8192;
+constexpr int kInBlockFixupMax = SG_FINISH_MAX_IONS;
 
 // Error-free difference: a - b = s + err exactly, s = fl(a - b) (Knuth's two-sum).
 __device__ __forceinline__ float two_diff_err(float a, float b, float s) {
@@ -1018,7 +1011,7 @@ struct SlotShared64 {
 //
 // FP32c: the slots hold float-float sums in frame units (store_partial); they are added
 // in float-float and converted once.  An ion whose near terms cancel strongly
-// (sqrt(s2) > 1.5 |P|, > |P| in clouds of up to kSmallRow ions) or whose far terms are
+// (sqrt(s2) > 1.5 |P|, > |P| in clouds of up to SG_SMALL_ROW ions) or whose far terms are
 // large next to |P| (s2f > SgCloud::kfar2 |P|^2) is fixed up (fixup_ion): INBLOCK, by this
 // block right away (small batches, where a second launch costs more than the work);
 // otherwise it is put on a work list of coulomb_fixup_kernel (ion index; cloud | kind <<
@@ -1026,8 +1019,8 @@ struct SlotShared64 {
 //
 // Latency-bound for small clouds: an FP64 addition takes a warp 64 cycles, so one thread
 // per row over 32 slots of five FP64 values spent ~5 us on additions alone.  Batches of
-// up to kInBlockFixupMax ions take 16 rows a block, 16 threads each (and the flagged rows
-// of more ions in parallel); larger ones 64 rows of 4 threads.
+// up to kInBlockFixupMax ions, and those with more than 24 slots, take 16 rows a block, 16
+// threads each; the others 64 rows of 4 threads.
 template <bool F32, bool INBLOCK>
 __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
     const SgRowBlock* __restrict__ rows, const SgCloud* __restrict__ clouds,
@@ -1100,7 +1093,7 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
             const float pf2 = fmaf(px.h, px.h, fmaf(py.h, py.h, pz.h * pz.h));
             // the far threshold: the prior of the frame set-up, or the measured one
             const float kf2 = chk ? fminf(cl.kfar2, chk[rb.cloud].kfar2) : cl.kfar2;
-            const float kap2 = cl.npad <= kSmallRow ? kKappa2Small : kKappa2;
+            const float kap2 = sg_kappa2(cl.npad);
             kind = (s2 > kap2 * pf2 ? kFixNear : 0) | (s2f > kf2 * pf2 ? kFixFar : 0);
             if (risk != nullptr) {
                 const float pf = sqrtf(pf2);
@@ -1215,7 +1208,7 @@ __global__ void __launch_bounds__(kFixupThreads, 3) coulomb_fixup_kernel(
         const int k = v % nc, c = v / nc;
         const int i = list[2 * k];
         const SgCloud& cl = clouds[list[2 * k + 1] & 0x0FFFFFFF];
-        if (row && cl.npad <= kSmallRow) {  // a small cloud's row: unit 0 alone, whole
+        if (row && cl.npad <= SG_SMALL_ROW) {  // a small cloud's row: unit 0 alone, whole
             if (c == 0)
                 fixup_ion<kFixupThreads>(cl, i, kFixNear, c32, c64, npad_total, out, n_total,
                                          bbox, sh);
@@ -1387,7 +1380,7 @@ cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* r
                                      int row_cap, int fp32c, double* out, int n_total,
                                      int* counters, cudaStream_t s) {
     if (n_rows <= 0) return cudaSuccess;
-    const int take = n_total <= kInBlockFixupMax ? 16 : 64;
+    const int take = n_total <= kInBlockFixupMax || a.max_slots > 24 ? 16 : 64;
     const int split = std::max(1, row_cap / take);
     if (fp32c) {
         const float* bbox = sg_variant_sorted(a.variant) ? a.bbox : nullptr;

@@ -15,12 +15,11 @@
 // The force count still follows the reference (7 per attempt, bin/ode.cpp:101-175).
 #include <math.h>
 
-#include "dp_tableau.cuh"
-#include "sg_internal.cuh"
+#include <algorithm>
+
+#include "dp_stage.cuh"
 
 namespace {
-
-typedef SgDpArgs DpArgs;
 
 __device__ __forceinline__ void write_coords(const DpArgs& a, const SgCloud& cl, int ig,
                                              double x, double y, double z, float* hu = nullptr) {
@@ -79,214 +78,149 @@ __device__ __forceinline__ void tile_bounds(const DpArgs& a, const SgCloud& cl,
     }
 }
 
-// Stage S (1..7) evaluated: finish its force, store k_S, build stage S+1 (or, for
-// S = 7, the embedded error of the attempt).
-template <int S>
-__global__ void __launch_bounds__(SG_ROWS) dp_stage_kernel(DpArgs a) {
+// ---- stage kernels -------------------------------------------------------------------
+// A thread per ion and component: component slots of R threads each, R the rows of the
+// block (a power of two >= 16); at R = 16 the slots are laid out so that the four warps,
+// one per SM sub-partition, hold x and y, z, a_x and a_y, a_z.
+//
+// GB300 takes 64 cycles for every FP64 warp instruction, so a stage costs the FP64
+// instructions of its longest warp, times the warps per sub-partition.  A thread per ion
+// ran all six components' ~100 instructions on one warp of a block, behind one thread's
+// drive cosines and divisions (a 1,000-ion stage: 8.4 - 15.1 us, 32 busy sub-partitions of
+// 608); per component the longest chain is ~20 instructions (7.3 us), and the first
+// stage computes every stage's field coefficients, a lane each.
+// Field coefficients of stage S for the whole block.  The first stage of an attempt takes
+// all of them, lane s - 1 of the first warp stage s, and leaves the others' in a.fcoef
+// (`publish`: the cloud's first block).  Every thread of the block must call this.
+template <int S, class M>
+__device__ __forceinline__ SgFieldCoef stage_coef(const DpArgs& a, const SgCloud& cl,
+                                                  const SgCtrl& cs, int cloud, bool publish) {
+    if constexpr (S == 1) {
+        __shared__ SgFieldCoef sk;
+        if (threadIdx.x < M::stages) {
+            const int s = threadIdx.x + 1;
+            const bool frozen = (cl.fp.flags & SG_F_FROZEN_T) != 0;
+            const SgFieldCoef k = sg_field_coef(cl.fp, frozen ? cs.t : cs.t + M::c(s) * cs.h);
+            if (s == 1) sk = k;
+            if (publish) a.fcoef[cloud * SG_MAX_STAGES + s] = k;
+        }
+        __syncthreads();
+        return sk;
+    } else {
+        return a.fcoef[cloud * SG_MAX_STAGES + S];
+    }
+}
+
+// Large batches: a thread per ion, all six components, R = 128 rows a block (one 128-ion
+// tile of the k-d order).  Throughput-bound by the FP64 pipe, where a thread per component
+// only adds barriers and loads (65,536 ions: 24 - 28 us a stage; this form 17 - 20 us).
+template <int S, class M>
+__global__ void __launch_bounds__(128) stage_wide_kernel(DpArgs a) {
     sg_griddep_wait();
-    __shared__ double red[SG_ROWS / 32];
-    const SgRowBlock rb = a.rows[blockIdx.x];
+    constexpr bool last = S == M::stages;
+    SgRowBlock rb = a.rows[blockIdx.x / a.split];
+    const int sub = blockIdx.x % a.split;
+    rb.i0 += sub * 128;
+    rb.n = min(rb.n - sub * 128, 128);
     const SgCtrl& cs = a.ctrl[rb.cloud];
     if (cs.done || cs.hold || cs.status != SG_OK) return;
     const SgCloud& cl = a.clouds[rb.cloud];
-    const int li = threadIdx.x;
-    const bool active = li < rb.n;
-    const int i = rb.i0 + (active ? li : 0);
-    const int ig = cl.poff + (i - cl.off);
+    const SgFieldCoef fk = stage_coef<S, M>(a, cl, cs, rb.cloud, rb.i0 == cl.off);
+    const int row = threadIdx.x, i = rb.i0 + row;
+    const bool active = row < rb.n;
     const size_t N = (size_t)a.n;
-    const double h = cs.h;
-    const bool frozen = (cl.fp.flags & SG_F_FROZEN_T) != 0;
-    const double ts = frozen ? cs.t : cs.t + c_c[S] * h;
-    const SgFieldCoef fk = sg_field_coef_block(cl.fp, ts);
-
-    double acc2 = 0.0;
+    double v[6], acc2 = 0.0;
     float hu[3] = {0.f, 0.f, 0.f};
     if (active) {
-        const double* st = (S == 1) ? a.y : a.ys;
-        const double px = st[i], py = st[N + i], pz = st[2 * N + i];
-        const double vx = st[3 * N + i], vy = st[4 * N + i], vz = st[5 * N + i];
-        double cx = 0.0, cy = 0.0, cz = 0.0;
+        double P[3] = {0.0, 0.0, 0.0};
         if (cl.fp.flags & SG_F_COULOMB) {
-            if (S == 1) {
-                cx = a.coul1[i];
-                cy = a.coul1[N + i];
-                cz = a.coul1[2 * N + i];
-            } else {
-                cx = a.coulS[i];
-                cy = a.coulS[N + i];
-                cz = a.coulS[2 * N + i];
-                if (S == 7) {
-                    a.coul7[i] = cx;
-                    a.coul7[N + i] = cy;
-                    a.coul7[2 * N + i] = cz;
-                }
+            const double* co = M::stages == 7 && S == 1 ? a.coul1 : a.coulS;
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                P[c] = co[c * N + i];
+                if (M::stages == 7 && last) a.coul7[c * N + i] = P[c];
             }
         }
-        double fx, fy, fz;
-        sg_field_apply(cl.fp, fk, a.qm[i], px, py, pz, vx, vy, vz, fx, fy, fz);
-        const double kqi = a.kq[i];
-        double* kS = a.k + (size_t)(S - 1) * 6 * N;
-        kS[i] = vx;
-        kS[N + i] = vy;
-        kS[2 * N + i] = vz;
-        kS[3 * N + i] = fx + kqi * cx;
-        kS[4 * N + i] = fy + kqi * cy;
-        kS[5 * N + i] = fz + kqi * cz;
-
-        if (S < 7) {
-            // stage S+1: y + h * sum_j a[S+1][j] k_j   (bin/ode.cpp:107-173)
-            double out[6];
 #pragma unroll
-            for (int c = 0; c < 6; c++) {
-                double s = 0.0;
-#pragma unroll
-                for (int j = 1; j <= S; j++) s += c_a[S + 1][j - 1] * a.k[((size_t)(j - 1) * 6 + c) * N + i];
-                out[c] = a.y[c * N + i] + h * s;
-            }
-#pragma unroll
-            for (int c = 0; c < 6; c++) a.ys[c * N + i] = out[c];
-            write_coords(a, cl, ig, out[0], out[1], out[2], hu);
-        } else {
-            // embedded error of the attempt (bin/ode.cpp:189-205); y5 = stage-7 state
-            const double rtol = cs.rtol, atol = cs.atol;
-#pragma unroll
-            for (int c = 0; c < 6; c++) {
-                double e = 0.0;
-#pragma unroll
-                for (int j = 1; j <= 7; j++)
-                    if (j != 2) e += c_e[j] * a.k[((size_t)(j - 1) * 6 + c) * N + i];
-                const double yerr = h * e;
-                const double y0 = fabs(a.y[c * N + i]), y1 = fabs(a.ys[c * N + i]);
-                const double sk = atol + rtol * ((y0 < y1) ? y1 : y0);
-                const double r = yerr / sk;
-                acc2 += r * r;
-            }
+        for (int c = 0; c < 6; c++) {
+            double sol = 0.0;
+            v[c] = stage_one<S, M>(a, cl, cs, fk, c, i, c < 3 ? 0.0 : P[c - 3], sol);
+            if (last) acc2 += v[c];
+            if (last && M::stages == 6) v[c] = sol;
         }
+        if (!last || M::stages == 6)
+#pragma unroll
+            for (int c = 0; c < 6; c++) {
+                a.ys[c * N + i] = v[c];
+                if (!last && c < 3) hu[c] = write_coord(a, cl, c, cl.poff + (i - cl.off), v[c]);
+            }
     }
-    if (S < 7 && a.fp32c && a.bbox) tile_bounds(a, cl, rb, active, hu[0], hu[1], hu[2]);
-    if (S == 7) {
-        // deterministic block reduction -> one partial per row block
-        for (int o = 16; o > 0; o >>= 1) acc2 += __shfl_down_sync(0xffffffffu, acc2, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc2;
+    if constexpr (last) {
+        acc2 = stage_block_sum(acc2);
+        if (threadIdx.x == 0) a.err_part[blockIdx.x] = acc2;
+    } else if (a.fp32c && a.bbox) {
+        __shared__ float sb[4][6];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            float lo = active ? hu[c] : INFINITY, hi = active ? hu[c] : -INFINITY;
+            for (int o = 16; o > 0; o >>= 1) {
+                lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            }
+            if ((threadIdx.x & 31) == 0) {
+                sb[threadIdx.x >> 5][c] = lo;
+                sb[threadIdx.x >> 5][3 + c] = hi;
+            }
+        }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            double s = 0.0;
-            for (int w = 0; w < SG_ROWS / 32; w++) s += red[w];
-            a.err_part[blockIdx.x] = s;
+        if (threadIdx.x < 6 && rb.n > 0) {
+            const int q = threadIdx.x;
+            a.bbox[8 * (size_t)(cl.tile0 + (rb.i0 - cl.off) / 128) + q] =
+                q < 3 ? fminf(fminf(sb[0][q], sb[1][q]), fminf(sb[2][q], sb[3][q]))
+                      : fmaxf(fmaxf(sb[0][q], sb[1][q]), fmaxf(sb[2][q], sb[3][q]));
         }
     }
 }
 
-
-// ---- Cash-Karp 5(4), the reference's "RungaKutta4" (bin/ode.cpp:220-345) ----------
-__constant__ double c_ck_a[7][6] = {
-    {0, 0, 0, 0, 0, 0},
-    {0, 0, 0, 0, 0, 0},
-    {0.2, 0, 0, 0, 0, 0},
-    {3.0 / 40.0, 9.0 / 40.0, 0, 0, 0, 0},
-    {0.3, -0.9, 1.2, 0, 0, 0},
-    {-11.0 / 54.0, 2.5, -70.0 / 27.0, 35.0 / 27.0, 0, 0},
-    {1631.0 / 55296.0, 175.0 / 512.0, 575.0 / 13824.0, 44275.0 / 110592.0, 253.0 / 4096.0, 0}};
-__constant__ double c_ck_c[7] = {0, 0.0, 0.2, 0.3, 0.6, 1.0, 0.875};
-__constant__ double c_ck_b[7] = {0, 37.0 / 378.0, 0.0, 250.0 / 621.0, 125.0 / 594.0, 0.0,
-                                 512.0 / 1771.0};
-__constant__ double c_ck_e[7] = {0,
-                                 37.0 / 378.0 - 2825.0 / 27648.0,
-                                 0.0,
-                                 250.0 / 621.0 - 18575.0 / 48384.0,
-                                 125.0 / 594.0 - 13525.0 / 55296.0,
-                                 -277.00 / 14336.0,
-                                 512.0 / 1771.0 - 0.25};
-
-// Stage S (1..6) of Cash-Karp: finish its force (the Coulomb sum of every stage comes
-// from coulS: no stage coincides with the next step's start), store k_S, build stage
-// S+1, or for S = 6 the 5th-order solution (into ys) and the embedded error.
-template <int S>
-__global__ void __launch_bounds__(SG_ROWS) ck_stage_kernel(DpArgs a) {
+// Stage S of a block's rows, the Coulomb sums in coul1 (Dormand-Prince's first stage) or
+// coulS.
+template <int S, class M>
+__global__ void __launch_bounds__(6 * 32) stage_kernel(DpArgs a) {
     sg_griddep_wait();
-    __shared__ double red[SG_ROWS / 32];
-    const SgRowBlock rb = a.rows[blockIdx.x];
+    constexpr bool last = S == M::stages;
+    SgRowBlock rb = a.rows[blockIdx.x / a.split];
+    const int R = rb.cap / a.split, sub = blockIdx.x % a.split;
+    rb.i0 += sub * R;
+    rb.n = min(rb.n - sub * R, R);
     const SgCtrl& cs = a.ctrl[rb.cloud];
     if (cs.done || cs.hold || cs.status != SG_OK) return;
     const SgCloud& cl = a.clouds[rb.cloud];
-    const int li = threadIdx.x;
-    const bool active = li < rb.n;
-    const int i = rb.i0 + (active ? li : 0);
-    const int ig = cl.poff + (i - cl.off);
+    const SgFieldCoef fk = stage_coef<S, M>(a, cl, cs, rb.cloud, rb.i0 == cl.off);
+    const int row = threadIdx.x & (R - 1), c = stage_component(threadIdx.x / R, R);
+    const bool active = row < rb.n && c >= 0;
     const size_t N = (size_t)a.n;
-    const double h = cs.h;
-    const bool frozen = (cl.fp.flags & SG_F_FROZEN_T) != 0;
-    const double ts = frozen ? cs.t : cs.t + c_ck_c[S] * h;
-    const SgFieldCoef fk = sg_field_coef_block(cl.fp, ts);
-    double acc2 = 0.0;
-    float hu[3] = {0.f, 0.f, 0.f};
+    const int i = rb.i0 + row;
+    double v = 0.0, sol = 0.0;
     if (active) {
-        const double* st = (S == 1) ? a.y : a.ys;
-        const double px = st[i], py = st[N + i], pz = st[2 * N + i];
-        const double vx = st[3 * N + i], vy = st[4 * N + i], vz = st[5 * N + i];
-        double cx = 0.0, cy = 0.0, cz = 0.0;
-        if (cl.fp.flags & SG_F_COULOMB) {
-            cx = a.coulS[i];
-            cy = a.coulS[N + i];
-            cz = a.coulS[2 * N + i];
+        double P = 0.0;
+        if (c >= 3 && (cl.fp.flags & SG_F_COULOMB)) {
+            P = (M::stages == 7 && S == 1 ? a.coul1 : a.coulS)[(c - 3) * N + i];
+            if (M::stages == 7 && last) a.coul7[(c - 3) * N + i] = P;
         }
-        double fx, fy, fz;
-        sg_field_apply(cl.fp, fk, a.qm[i], px, py, pz, vx, vy, vz, fx, fy, fz);
-        const double kqi = a.kq[i];
-        double* kS = a.k + (size_t)(S - 1) * 6 * N;
-        kS[i] = vx;
-        kS[N + i] = vy;
-        kS[2 * N + i] = vz;
-        kS[3 * N + i] = fx + kqi * cx;
-        kS[4 * N + i] = fy + kqi * cy;
-        kS[5 * N + i] = fz + kqi * cz;
-        if (S < 6) {
-            double out[6];
-#pragma unroll
-            for (int c = 0; c < 6; c++) {
-                double sum = 0.0;
-#pragma unroll
-                for (int j = 1; j <= S; j++) sum += c_ck_a[S + 1][j - 1] * a.k[((size_t)(j - 1) * 6 + c) * N + i];
-                out[c] = a.y[c * N + i] + h * sum;
-            }
-#pragma unroll
-            for (int c = 0; c < 6; c++) a.ys[c * N + i] = out[c];
-            write_coords(a, cl, ig, out[0], out[1], out[2], hu);
-        } else {
-            const double rtol = cs.rtol, atol = cs.atol;
-#pragma unroll
-            for (int c = 0; c < 6; c++) {
-                double b = 0.0, e = 0.0;
-#pragma unroll
-                for (int j = 1; j <= 6; j++) {
-                    const double kj = a.k[((size_t)(j - 1) * 6 + c) * N + i];
-                    b += c_ck_b[j] * kj;
-                    e += c_ck_e[j] * kj;
-                }
-                const double y0 = a.y[c * N + i];
-                const double y5 = y0 + h * b;
-                a.ys[c * N + i] = y5;
-                const double yerr = h * e;
-                const double m0 = fabs(y0), m1 = fabs(y5);
-                const double sk = atol + rtol * ((m0 < m1) ? m1 : m0);
-                const double r = yerr / sk;
-                acc2 += r * r;
-            }
+        v = stage_one<S, M>(a, cl, cs, fk, c, i, P, sol);
+    }
+    if (!last || M::stages == 6) {
+        __syncthreads();  // this stage's state has been read
+        if (active) {
+            a.ys[c * N + i] = last ? sol : v;
+            if (!last && c < 3) write_coord(a, cl, c, cl.poff + (i - cl.off), v);
         }
     }
-    if (S < 6 && a.fp32c && a.bbox) tile_bounds(a, cl, rb, active, hu[0], hu[1], hu[2]);
-    if (S == 6) {
-        for (int o = 16; o > 0; o >>= 1) acc2 += __shfl_down_sync(0xffffffffu, acc2, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc2;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double sum = 0.0;
-            for (int w = 0; w < SG_ROWS / 32; w++) sum += red[w];
-            a.err_part[blockIdx.x] = sum;
-        }
+    if constexpr (last) {
+        v = stage_block_sum(active ? v : 0.0);
+        if (threadIdx.x == 0) a.err_part[blockIdx.x] = v;
     }
 }
-
 
 // ---- Gear predictor-corrector, the reference's GearMethod (bin/ode.cpp:347-424) ----
 // Fifth-order Nordsieck form with one force evaluation per step and a fixed step.
@@ -391,28 +325,33 @@ __global__ void __launch_bounds__(SG_ROWS) gear_kernel(DpArgs a) {
     }
 }
 
-// error_succes + step bookkeeping (bin/ode.cpp:426-494), one thread per cloud.
+// error_succes + step bookkeeping (bin/ode.cpp:426-494), one warp per cloud: its lanes
+// sum the error partials, lane 0 decides.
 // With flags[SG_FLAG_HOLD] set, a cloud that accepts holds (skips further attempts) until
 // the host clears the hold: used to take exactly one step per cloud.
 __global__ void dp_control_kernel(SgCloud* __restrict__ clouds, SgCtrl* __restrict__ ctrl,
-                                  const double* __restrict__ err_part, const double* __restrict__ y,
-                                  int n_clouds, const int* __restrict__ flags,
-                                  const SgOp* __restrict__ ops) {
+                                  const double* __restrict__ err_part, int split,
+                                  const double* __restrict__ y, int n_clouds,
+                                  const int* __restrict__ flags, const SgOp* __restrict__ ops) {
     sg_griddep_wait();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (c >= n_clouds) return;
+    const SgCloud& cl = clouds[c];
+    const int nb = cl.nrb * split;
+    const double* ep = err_part + (size_t)cl.rb0 * split;
+    double s = 0.0;
+    for (int b = lane; b < nb; b += 32) s += ep[b];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane != 0) return;
     SgCtrl cs = ctrl[c];
-    const SgCloud cl = clouds[c];
     if (cs.done || cs.hold || cs.status != SG_OK) {
         ctrl[c].accepted = 0;
         ctrl[c].print_due = 0;
         return;
     }
     cs.print_due = 0;
-    double s = 0.0;
     // Cash-Karp: the reference adds to the previous norm, odev.err is never reset there
-    if (cs.method == 4) s = cs.err;
-    for (int b = 0; b < cl.nrb; b++) s += err_part[cl.rb0 + b];
+    if (cs.method == 4) s += cs.err;
     const double err = sqrt(s / (6 * cl.n));
     cs.err = err;
     cs.force_evals += (cs.method == 4) ? 6 : (cs.method == 1 ? 1 : 7);
@@ -638,33 +577,43 @@ __global__ void __launch_bounds__(SG_ROWS) moments_kernel(DpArgs a, const double
 
 // ---- host-side launchers (called from capi.cu) ------------------------------------
 
-cudaError_t sg_dp_stage(const SgDpArgs& a, int stage, int n_rows, cudaStream_t st) {
+// Blocks per row block: row blocks of 256 (large batches) take two of 128 rows, a thread
+// per ion; the others blocks of 32 (a warp per component) or 16 rows.
+int sg_stage_split(int cap) { return cap >= 256 ? 2 : std::max(1, cap / 32); }
+
+template <int S, class M>
+static void launch_stage_s(const SgDpArgs& a, int n_rows, int cap, cudaStream_t st) {
+    const int R = cap / a.split;
+    if (cap >= 256)
+        sg_launch(stage_wide_kernel<S, M>, n_rows * a.split, 128, 0, st, a);
+    else
+        sg_launch(stage_kernel<S, M>, n_rows * a.split, R > 16 ? 6 * R : 8 * R, 0, st, a);
+}
+
+template <class M>
+static cudaError_t launch_stage(const SgDpArgs& a, int stage, int n_rows, int cap, cudaStream_t st) {
     if (n_rows <= 0) return cudaSuccess;
     switch (stage) {
-        case 1: sg_launch(dp_stage_kernel<1>, n_rows, SG_ROWS, 0, st, a); break;
-        case 2: sg_launch(dp_stage_kernel<2>, n_rows, SG_ROWS, 0, st, a); break;
-        case 3: sg_launch(dp_stage_kernel<3>, n_rows, SG_ROWS, 0, st, a); break;
-        case 4: sg_launch(dp_stage_kernel<4>, n_rows, SG_ROWS, 0, st, a); break;
-        case 5: sg_launch(dp_stage_kernel<5>, n_rows, SG_ROWS, 0, st, a); break;
-        case 6: sg_launch(dp_stage_kernel<6>, n_rows, SG_ROWS, 0, st, a); break;
-        case 7: sg_launch(dp_stage_kernel<7>, n_rows, SG_ROWS, 0, st, a); break;
+        case 1: launch_stage_s<1, M>(a, n_rows, cap, st); break;
+        case 2: launch_stage_s<2, M>(a, n_rows, cap, st); break;
+        case 3: launch_stage_s<3, M>(a, n_rows, cap, st); break;
+        case 4: launch_stage_s<4, M>(a, n_rows, cap, st); break;
+        case 5: launch_stage_s<5, M>(a, n_rows, cap, st); break;
+        case 6: launch_stage_s<6, M>(a, n_rows, cap, st); break;
+        case 7:
+            if constexpr (M::stages == 7) launch_stage_s<7, M>(a, n_rows, cap, st);
+            break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
-cudaError_t sg_ck_stage(const SgDpArgs& a, int stage, int n_rows, cudaStream_t st) {
-    if (n_rows <= 0) return cudaSuccess;
-    switch (stage) {
-        case 1: sg_launch(ck_stage_kernel<1>, n_rows, SG_ROWS, 0, st, a); break;
-        case 2: sg_launch(ck_stage_kernel<2>, n_rows, SG_ROWS, 0, st, a); break;
-        case 3: sg_launch(ck_stage_kernel<3>, n_rows, SG_ROWS, 0, st, a); break;
-        case 4: sg_launch(ck_stage_kernel<4>, n_rows, SG_ROWS, 0, st, a); break;
-        case 5: sg_launch(ck_stage_kernel<5>, n_rows, SG_ROWS, 0, st, a); break;
-        case 6: sg_launch(ck_stage_kernel<6>, n_rows, SG_ROWS, 0, st, a); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+cudaError_t sg_dp_stage(const SgDpArgs& a, int stage, int n_rows, int cap, cudaStream_t st) {
+    return launch_stage<MethodDP>(a, stage, n_rows, cap, st);
+}
+
+cudaError_t sg_ck_stage(const SgDpArgs& a, int stage, int n_rows, int cap, cudaStream_t st) {
+    return launch_stage<MethodCK>(a, stage, n_rows, cap, st);
 }
 
 cudaError_t sg_gear_stage(const SgDpArgs& a, int phase, int n_rows, cudaStream_t st) {
@@ -683,10 +632,10 @@ cudaError_t sg_gear_init(const SgDpArgs& a, const int* perm, int n_rows, cudaStr
 }
 
 cudaError_t sg_dp_control(SgCloud* clouds, SgCtrl* ctrl, const double* err_part,
-                          const double* y, int n_clouds, const int* flags,
+                          int split, const double* y, int n_clouds, const int* flags,
                           const SgOp* ops, cudaStream_t st) {
-    sg_launch(dp_control_kernel, (n_clouds + 127) / 128, 128, 0, st, clouds, ctrl, err_part, y, n_clouds,
-                                                              flags, ops);
+    sg_launch(dp_control_kernel, (n_clouds + 3) / 4, 128, 0, st, clouds, ctrl, err_part, split, y,
+              n_clouds, flags, ops);
     return cudaGetLastError();
 }
 

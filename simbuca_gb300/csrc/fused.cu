@@ -30,9 +30,8 @@
 #include <cooperative_groups.h>
 #include <math.h>
 
-#include "dp_tableau.cuh"
+#include "dp_stage.cuh"
 #include "fp32c_math.cuh"
-#include "sg_internal.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -51,84 +50,30 @@ struct FusedShared {
 __device__ __forceinline__ int ldcg_int(const int* p) { return __ldcg(p); }
 
 // Stage S of the CTA's ions [lo, hi): k_S, then the state and Coulomb inputs of stage
-// S+1, or (S = 7) the CTA's sum of squared scaled errors, returned on thread 0.
+// S+1, or (S = 7) the CTA's sum of squared scaled errors, returned on thread 0.  A thread
+// per ion and component, components in warps of their own: the FP64 instructions of a
+// stage (64 cycles each) are spread over the SM's four sub-partitions.
 template <int S>
-__device__ double stage_phase(const SgFusedArgs& f, const SgCloud& cl, const SgCtrl& cs, int lo,
-                              int hi) {
-    const size_t N = (size_t)f.n;
-    const double h = cs.h;
-    const bool frozen = (cl.fp.flags & SG_F_FROZEN_T) != 0;
-    const double ts = frozen ? cs.t : cs.t + c_c[S] * h;
-    const SgFieldCoef fk = sg_field_coef_block(cl.fp, ts);
-    const int i = lo + (int)threadIdx.x;
-    double acc2 = 0.0;
-    if (i < hi) {
-        const double* st = (S == 1) ? f.y : f.ys;
-        const double px = st[i], py = st[N + i], pz = st[2 * N + i];
-        const double vx = st[3 * N + i], vy = st[4 * N + i], vz = st[5 * N + i];
-        double cx = 0.0, cy = 0.0, cz = 0.0;
-        if (cl.fp.flags & SG_F_COULOMB) {
-            const double* cs_ = (S == 1) ? f.coul1 : f.coulS;
-            cx = cs_[i];
-            cy = cs_[N + i];
-            cz = cs_[2 * N + i];
-            if (S == 7) {
-                f.coul7[i] = cx;
-                f.coul7[N + i] = cy;
-                f.coul7[2 * N + i] = cz;
+__device__ double stage_phase(const DpArgs& a, const SgCloud& cl, const SgCtrl& cs,
+                              const SgFieldCoef& fk, int lo, int hi) {
+    constexpr int kPasses = 6;  // up to kThreads ions of the CTA
+    const size_t N = (size_t)a.n;
+    const int m = hi - lo, mp = (m + 31) & ~31;
+    double out[kPasses], acc2 = 0.0, sol = 0.0;
+#pragma unroll
+    for (int u = 0; u < kPasses; u++) {
+        const int t = (int)threadIdx.x + u * kThreads;
+        const int c = mp ? t / mp : 6, row = t - c * mp;
+        out[u] = 0.0;
+        if (u * kThreads < 6 * mp && c < 6 && row < m) {
+            const int i = lo + row;
+            double P = 0.0;
+            if (c >= 3 && (cl.fp.flags & SG_F_COULOMB)) {
+                P = (S == 1 ? a.coul1 : a.coulS)[(c - 3) * N + i];
+                if (S == 7) a.coul7[(c - 3) * N + i] = P;
             }
-        }
-        double fx, fy, fz;
-        sg_field_apply(cl.fp, fk, f.qm[i], px, py, pz, vx, vy, vz, fx, fy, fz);
-        const double kqi = f.kq[i];
-        double* kS = f.k + (size_t)(S - 1) * 6 * N;
-        kS[i] = vx;
-        kS[N + i] = vy;
-        kS[2 * N + i] = vz;
-        kS[3 * N + i] = fx + kqi * cx;
-        kS[4 * N + i] = fy + kqi * cy;
-        kS[5 * N + i] = fz + kqi * cz;
-        if (S < 7) {
-            double out[6];
-#pragma unroll
-            for (int c = 0; c < 6; c++) {
-                double s = 0.0;
-#pragma unroll
-                for (int j = 1; j <= S; j++) s += c_a[S + 1][j - 1] * f.k[((size_t)(j - 1) * 6 + c) * N + i];
-                out[c] = f.y[c * N + i] + h * s;
-            }
-#pragma unroll
-            for (int c = 0; c < 6; c++) f.ys[c * N + i] = out[c];
-            // Coulomb inputs of stage S+1 (SI and FP32 frame coordinates)
-            const int ig = cl.poff + (i - cl.off);
-            const size_t NP = (size_t)f.npad;
-            f.c64[ig] = out[0];
-            f.c64[NP + ig] = out[1];
-            f.c64[2 * NP + ig] = out[2];
-            const double u = (out[0] - cl.cx) * cl.invL, v = (out[1] - cl.cy) * cl.invL,
-                         w = (out[2] - cl.cz) * cl.invL;
-            const float uh = __double2float_rn(u), vh = __double2float_rn(v),
-                        wh = __double2float_rn(w);
-            f.c32[ig] = uh;
-            f.c32[NP + ig] = vh;
-            f.c32[2 * NP + ig] = wh;
-            f.c32[4 * NP + ig] = __double2float_rn(u - (double)uh);
-            f.c32[5 * NP + ig] = __double2float_rn(v - (double)vh);
-            f.c32[6 * NP + ig] = __double2float_rn(w - (double)wh);
-        } else {
-            const double rtol = cs.rtol, atol = cs.atol;
-#pragma unroll
-            for (int c = 0; c < 6; c++) {
-                double e = 0.0;
-#pragma unroll
-                for (int j = 1; j <= 7; j++)
-                    if (j != 2) e += c_e[j] * f.k[((size_t)(j - 1) * 6 + c) * N + i];
-                const double yerr = h * e;
-                const double y0 = fabs(f.y[c * N + i]), y1 = fabs(f.ys[c * N + i]);
-                const double sk = atol + rtol * ((y0 < y1) ? y1 : y0);
-                const double r = yerr / sk;
-                acc2 += r * r;
-            }
+            out[u] = stage_one<S, MethodDP>(a, cl, cs, fk, c, i, P, sol);
+            if (S == 7) acc2 += out[u];
         }
     }
     if constexpr (S == 7) {
@@ -137,11 +82,24 @@ __device__ double stage_phase(const SgFusedArgs& f, const SgCloud& cl, const SgC
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc2;
         __syncthreads();
         double s = 0.0;
-        if (threadIdx.x == 0)
-            for (int w = 0; w < kThreads / 32; w++) s += red[w];
+        if (threadIdx.x < 32) {
+            s = threadIdx.x < kThreads / 32 ? red[threadIdx.x] : 0.0;
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        }
         __syncthreads();
         return s;
     } else {
+        __syncthreads();  // this stage's state has been read
+#pragma unroll
+        for (int u = 0; u < kPasses; u++) {
+            const int t = (int)threadIdx.x + u * kThreads;
+            const int c = mp ? t / mp : 6, row = t - c * mp;
+            if (u * kThreads < 6 * mp && c < 6 && row < m) {
+                const int i = lo + row;
+                a.ys[c * N + i] = out[u];
+                if (c < 3) write_coord(a, cl, c, cl.poff + (i - cl.off), out[u]);
+            }
+        }
         return 0.0;
     }
 }
@@ -410,6 +368,21 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
     const int m = (cl.n + R - 1) / R;
     const int lo = cl.off + min(cl.n, r * m), hi = cl.off + min(cl.n, (r + 1) * m);
     const bool coul = (cl.fp.flags & SG_F_COULOMB) != 0;
+    __shared__ SgFieldCoef fk[SG_MAX_STAGES];
+    DpArgs a = {};
+    a.y = f.y;
+    a.ys = f.ys;
+    a.k = f.k;
+    a.coulS = f.coulS;
+    a.coul1 = f.coul1;
+    a.coul7 = f.coul7;
+    a.kq = f.kq;
+    a.qm = f.qm;
+    a.c64 = f.c64;
+    a.c32 = f.c32;
+    a.n = f.n;
+    a.npad = f.npad;
+    a.fp32c = 1;
     for (int att = 0; att < f.max_attempts; att++) {
         {
             // every CTA reads the control block after the previous cluster barrier
@@ -423,7 +396,14 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
         cs.h = __ldcg(&f.ctrl[c].h);
         cs.rtol = __ldcg(&f.ctrl[c].rtol);
         cs.atol = __ldcg(&f.ctrl[c].atol);
-        stage_phase<1>(f, cl, cs, lo, hi);
+        // every stage's field coefficients, a lane each
+        if (threadIdx.x < MethodDP::stages) {
+            const int st = threadIdx.x + 1;
+            const bool frozen = (cl.fp.flags & SG_F_FROZEN_T) != 0;
+            fk[st] = sg_field_coef(cl.fp, frozen ? cs.t : cs.t + MethodDP::c(st) * cs.h);
+        }
+        __syncthreads();
+        stage_phase<1>(a, cl, cs, fk[1], lo, hi);
         cluster.sync();
 #define SG_FUSED_STAGE(S)                                      \
     if (coul) {                                                \
@@ -431,7 +411,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
         cluster.sync();                                        \
     }                                                          \
     {                                                          \
-        const double e = stage_phase<S>(f, cl, cs, lo, hi);    \
+        const double e = stage_phase<S>(a, cl, cs, fk[S], lo, hi);    \
         if (S == 7 && threadIdx.x == 0)                        \
             f.errp[(size_t)c * SG_FUSED_MAX_CTAS + r] = e;     \
     }                                                          \
@@ -448,12 +428,12 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
         if (ldcg_int(&f.ctrl[c].accepted)) {
             // commit: pos <- pos2, vel <- vel2; the stage-7 sum is the next stage-1 sum
             const size_t N = (size_t)f.n;
-            const int i = lo + (int)threadIdx.x;
-            if (i < hi) {
-#pragma unroll
-                for (int q = 0; q < 6; q++) f.y[q * N + i] = f.ys[q * N + i];
-#pragma unroll
-                for (int q = 0; q < 3; q++) f.coul1[q * N + i] = f.coul7[q * N + i];
+            for (int t = threadIdx.x; t < 9 * (hi - lo); t += kThreads) {
+                const int q = t / (hi - lo), i = lo + t - q * (hi - lo);
+                if (q < 6)
+                    f.y[q * N + i] = f.ys[q * N + i];
+                else
+                    f.coul1[(q - 6) * N + i] = f.coul7[(q - 6) * N + i];
             }
         }
         if (f.ran != nullptr && coul && r == 0 && threadIdx.x == 0) f.ran[c] = 1;

@@ -171,6 +171,21 @@ struct SgCtrl {
     double beta;  // PI term of error_succes (0: the reference's I-controller)
 };
 
+// x^(-1/5) for a positive finite x: an FP32 estimate and two Newton steps
+// y <- y + y (1 - x y^5) / 5, each squaring the relative error (times 3): below the
+// rounding of the last one.  ~15 FP64 operations where pow takes ~100, 64 cycles each, on
+// the one lane that every block of the next attempt waits for.
+__device__ inline double sg_inv_fifth_root(double x) {
+    if (!(x > 1e-30 && x < 1e30)) return pow(x, -0.2);
+    double y = (double)exp2f(-0.2f * log2f((float)x));
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const double y2 = y * y;
+        y = fma(y * 0.2, fma(-x * y, y2 * y2, 1.0), y);
+    }
+    return y;
+}
+
 // error_succes and the retry bookkeeping of step() (bin/ode.cpp:426-494) for one attempt
 // of one cloud with error norm err: returns 1 if the attempt is accepted.  A non-finite
 // norm stops the cloud (SG_NONFINITE); a reject shrinks h and checks the underflow
@@ -191,7 +206,8 @@ __device__ inline int sg_error_succes(SgCtrl& cs, double err, const double* x0) 
         if (err == 0.0)
             scale = maxscale;
         else {
-            scale = safe * pow(err, -alpha) * pow(cs.errold, beta);
+            scale = beta == 0.0 ? safe * sg_inv_fifth_root(err)
+                                : safe * pow(err, -alpha) * pow(cs.errold, beta);
             if (scale < minscale) scale = minscale;
             if (scale > maxscale) scale = maxscale;
         }
@@ -200,7 +216,7 @@ __device__ inline int sg_error_succes(SgCtrl& cs, double err, const double* x0) 
         cs.reject = 0;
         return 1;
     }
-    double scale = safe * pow(err, -alpha);
+    double scale = safe * (beta == 0.0 ? sg_inv_fifth_root(err) : pow(err, -alpha));
     scale = (scale < minscale) ? minscale : scale;
     cs.h *= scale;
     cs.reject = 1;
@@ -363,14 +379,33 @@ __device__ __forceinline__ void sg_field_accel(const sg_field_params& fp, double
     sg_field_apply(fp, sg_field_coef(fp, t), qm, x, y, z, vx, vy, vz, ax, ay, az);
 }
 
-// The block's field coefficients at time t, computed by thread 0 (every thread of the
-// block must call this: it synchronises the block).
-__device__ __forceinline__ SgFieldCoef sg_field_coef_block(const sg_field_params& fp, double t) {
-    __shared__ SgFieldCoef sk;
-    if (threadIdx.x == 0) sk = sg_field_coef(fp, t);
-    __syncthreads();
-    return sk;
+// Acceleration along axis c (0..2) of one ion: sg_field_apply's operations in its order
+// for that axis (p, v: position and velocity along c; po, vo: along the other transverse
+// axis, anything finite for z).  The axes differ in operands, not in operations, so the
+// lanes of a warp may hold different axes without diverging; where sg_field_apply has no
+// term an axis adds an exact zero.
+__device__ __forceinline__ double sg_field_axis(const sg_field_params& fp, const SgFieldCoef& k,
+                                                double qm, int c, double p, double v, double po,
+                                                double vo) {
+    const uint32_t f = fp.flags;
+    double a = 0.0;
+    if (f & SG_F_PAUL)
+        a = __dmul_rn(__dmul_rn(qm, c == 0 ? k.paul_x : c == 1 ? k.paul_y : k.paul_z), p);
+    if (f & SG_F_TOF) a = __dadd_rn(a, c == 0 ? __dmul_rn(qm, fp.E_kick) : 0.0);
+    if (f & (SG_F_PENNING | SG_F_QUAD | SG_F_DIPOLE)) {
+        double e = 0.0;
+        if (f & SG_F_PENNING)
+            e = __dadd_rn(__dmul_rn(c == 2 ? -2.0 * k.kp : k.kp, p),
+                          __dmul_rn(c == 0 ? fp.B : c == 1 ? -fp.B : 0.0, vo));
+        e = __dadd_rn(e, __dadd_rn(__dmul_rn(c == 2 ? 0.0 : k.gq, po), c == 0 ? k.gd : 0.0));
+        a = __dadd_rn(a, __dmul_rn(qm, e));
+    }
+    if (f & SG_F_FRICTION) a = __dsub_rn(a, __dmul_rn(fp.delta, v));
+    return a;
 }
+
+// Stages a method's attempt takes at most, and its field coefficients per cloud.
+#define SG_MAX_STAGES 8
 
 // ---- Dormand-Prince 5(4) tableau (bin/ode.cpp:76-86) ------------------------------
 #define DP_C2 (1.0 / 5.0)
@@ -393,12 +428,39 @@ struct SgDpArgs {
     const double* qm;     // [N]
     double* c64;          // [4][Npad]
     float* c32;           // [7][Npad]
-    double* err_part;     // [rows]
+    double* err_part;     // [row blocks x split]
+    SgFieldCoef* fcoef;   // [clouds][SG_MAX_STAGES] written by an attempt's first stage
     float* bbox;          // [tiles][8] frame-unit bounds of each 128-ion tile (FP32c)
     int n;                // ions (unpadded)
     int npad;             // padded ions
     int fp32c;            // write the FP32 frame coordinates
+    int split;            // blocks of the stage kernels per row block
 };
+
+// ---- conditioning test of the FP32c sums ----------------------------------------------
+// An ion's sum is replaced by its FP64 row when s2 > kappa2 |P|^2: sqrt(s2) > 1.5 |P|, or
+// > |P| in clouds of up to SG_SMALL_ROW padded ions, whose FP64 row is cheap and whose
+// error per unit of sqrt(s2)/|P| ran up to ~9e-7 with their few terms per ion (an
+// unflagged ion at 1.37 measured 1.2e-6 in the 512-cloud scan's small clouds; 2.5e-7 at
+// most on the 65,536-ion cloud).  Their flagged rows are one work unit each.
+#define SG_SMALL_ROW 4096
+__device__ __forceinline__ float sg_kappa2(int npad) { return npad <= SG_SMALL_ROW ? 1.0f : 2.25f; }
+
+// ---- small batches: slot sums, flagged rows and stage in one launch (finish.cu) -------
+// Batches of up to this many ions in the plain order; larger ones have enough rows to
+// fill the device with a launch each, and long flagged rows (coulomb_fixup_kernel).
+#define SG_FINISH_MAX_IONS 8192
+struct SgFinishArgs {
+    SgDpArgs dp;            // c64, c32: the coordinates the stage writes
+    const double* part;     // partial-sum slots
+    const double* c64r;     // the coordinates the sums were taken at
+    double* coulS;          // [3][N] stage-7 sums
+    int* counters;
+    float* risk;            // in-run force check inputs (null: not written)
+    int* ran;
+    int n_rows;
+};
+cudaError_t sg_dp_finish(const SgFinishArgs& f, int stage, int fp32c, cudaStream_t st);
 
 // ---- fused small-cloud attempts (fused.cu) -----------------------------------------
 // One thread-block cluster per cloud runs whole Dormand-Prince attempts (FP32c, no
@@ -458,13 +520,15 @@ cudaError_t sg_record_now(SgCtrl* ctrl, int n_clouds, cudaStream_t st);
 cudaError_t sg_gather_int(const int* src, const int* perm, int* dst, int n, cudaStream_t st);
 
 // ---- launchers implemented in the .cu files ------------------------------------
-cudaError_t sg_dp_stage(const SgDpArgs& a, int stage, int n_rows, cudaStream_t st);
-cudaError_t sg_ck_stage(const SgDpArgs& a, int stage, int n_rows, cudaStream_t st);
+// blocks the stage kernels split a row block into (cap: its rows at most)
+int sg_stage_split(int cap);
+cudaError_t sg_dp_stage(const SgDpArgs& a, int stage, int n_rows, int cap, cudaStream_t st);
+cudaError_t sg_ck_stage(const SgDpArgs& a, int stage, int n_rows, int cap, cudaStream_t st);
 // Gear: phase 0 predicts, phase 1 corrects; sg_gear_init seeds the Gear state in k
 cudaError_t sg_gear_stage(const SgDpArgs& a, int phase, int n_rows, cudaStream_t st);
 cudaError_t sg_gear_init(const SgDpArgs& a, const int* perm, int n_rows, cudaStream_t st);
 cudaError_t sg_dp_control(SgCloud* clouds, SgCtrl* ctrl, const double* err_part,
-                          const double* y, int n_clouds, const int* flags,
+                          int split, const double* y, int n_clouds, const int* flags,
                           const SgOp* ops, cudaStream_t st);
 cudaError_t sg_clear_hold(SgCtrl* ctrl, int n_clouds, cudaStream_t st);
 int sg_probe_iters(int which);
@@ -510,6 +574,7 @@ struct SgCoulombArgs {
     const SgCloud* clouds;
     const SgCtrl* ctrl;      // may be null (stand-alone calls)
     double* part;            // partial-sum slots (SG_PART_F32 floats or 3 doubles per ion)
+    int max_slots = 0;       // of any cloud
     int sym = 0;             // FP64: the items are symmetric ones (fp64_pairs.cuh)
     int npad_total;
     int* errword;
