@@ -54,7 +54,7 @@ def parse():
     ap.add_argument("--no-sequential", action="store_true",
                     help="batched workloads: skip the one-cloud-at-a-time comparison pass")
     ap.add_argument("--variant", type=int, default=-1,
-                    help="FP32c Coulomb launch shape (-1 automatic, 0..16 fixed: sg_set_coulomb_variant)")
+                    help="FP32c Coulomb launch shape (-1 automatic, 0..17 fixed: sg_set_coulomb_variant)")
     ap.add_argument("--method", type=int, default=5, choices=[4, 5],
                     help="5 Dormand-Prince, 4 Cash-Karp")
     ap.add_argument("--proposer", default="off", choices=["on", "off"],
@@ -181,9 +181,25 @@ def l2_flush():
 def coulomb_kernel_name(prec, variant):
     from simbuca_gb300 import abi
     if prec != abi.SG_PREC_FP32C:
-        return "coulomb_fp64_kernel"
+        return "coulomb_fp64_sym_kernel"
+    if variant == 17:
+        return "coulomb_leaf_kernel"
     sorted_shapes = (4, 7, 8, 9, 12, 13, 14, 15, 16)
     return "coulomb_fp32c_sorted_kernel" if variant in sorted_shapes else "coulomb_fp32c_kernel"
+
+
+def launches_per_attempt(prec, n_total, variant):
+    """Our kernel launches of one Dormand-Prince attempt: stage 1, then per Coulomb sum
+    the pair kernel and, up to 8,192 ions in the plain order, the finish kernel (slot sums,
+    flagged rows, stage), else the reduction, with FP32c the fix-up, and the stage; shape
+    17 lists its near leaves before each pair kernel.  Control and commit."""
+    from simbuca_gb300 import abi
+    fp32c = prec == abi.SG_PREC_FP32C
+    plain = not fp32c or variant < 4 or variant in (5, 6, 10, 11)
+    if n_total <= 8192 and plain:
+        return 1 + 6 * 2 + 2
+    per_sum = 3 + (1 if fp32c and n_total > 8192 else 0) + (1 if fp32c and variant == 17 else 0)
+    return 1 + 6 * per_sum + 2
 
 
 # Algorithmic HBM traffic of one Dormand-Prince attempt per ion in the O(N) kernels:
@@ -434,14 +450,11 @@ def run_ours(args, dist: Dist):
                 "mean_h": sum(a["t"] - b["t"] for a, b in zip(e_after, e_before)) /
                 max(1, sum(a["steps"] - b["steps"] for a, b in zip(e_after, e_before)))},
         "mean_h": sim_us * 1e-6 / max(1, sum(a["steps"] - b["steps"] for a, b in zip(s_after, s_before))),
-        # per attempt: 7 stages, 6 Coulomb sums, 6 reductions, control, commit, and with
-        # FP32c on batches over 8,192 ions the 6 fix-up launches of the conditioning work
-        # list (smaller batches fix up inside the reduction); per step one hold reset
-        # (+2 per attempt with the proposer: cloud moments and the MLP)
-        # fused small-cloud path: one launch per step (its attempts inside it)
+        # per step one hold reset (+2 per attempt with the proposer: cloud moments and the
+        # MLP); fused small-cloud path: one launch per step (its attempts inside it)
         "gpu_launches": int((args.steps if fused_cluster else
-                             attempts * ((27 if prec == abi.SG_PREC_FP32C and w.n_total > 8192
-                                          else 21) + (2 if args.proposer == "on" else 0)))
+                             attempts * (launches_per_attempt(prec, w.n_total, batch.variant())
+                                         + (2 if args.proposer == "on" else 0)))
                             + args.steps
                             + (3 * (attempts // CHECK_EVERY) if prec == abi.SG_PREC_FP32C else 0)),
         "fixup_ions_per_coulomb_call": fixups / max(1, 6 * attempts),
@@ -609,7 +622,7 @@ def run_batched(args, dist: Dist):
                    "step_control": step_control,
                    "parallelism": f"replicas x{dist.world}",
                    "l2": "flushed (256 MB write) between timed steps"},
-        "gpu_launches": int(((27 if args.precision == "fp32c" else 21)
+        "gpu_launches": int((launches_per_attempt(prec, w.n_total, batch.variant())
                              + (2 if args.proposer == "on" else 0)) * per_step * args.steps
                             + (3 * (per_step * args.steps // CHECK_EVERY)
                                if args.precision == "fp32c" else 0)),

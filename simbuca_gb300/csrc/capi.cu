@@ -36,6 +36,14 @@ struct Problem {
     std::vector<SgCtrl> hctrl0;
     std::vector<SgRowBlock> hrows;
     std::vector<SgWorkItem> hitems;
+    std::vector<SgFarItem> hfar;   // shape 17
+    SgFarItem* dfar = nullptr;
+    std::vector<int> hleaf;        // cloud of each leaf
+    int near_cap = 0;              // leaves of the largest cloud
+    int *leaf_cloud = nullptr, *near_count = nullptr;
+    unsigned short* near_list = nullptr;
+    unsigned long long* far_acc = nullptr;
+    float* far_s2f = nullptr;
     std::vector<int> counts;
     SgCloud* dc = nullptr;
     SgCtrl* dctrl = nullptr;
@@ -194,6 +202,12 @@ void free_problem(Problem& P) {
     for (double* d : ds) cudaFree(d);
     cudaFree(P.c32);
     cudaFree(P.fcoef);
+    cudaFree(P.dfar);
+    cudaFree(P.leaf_cloud);
+    cudaFree(P.near_count);
+    cudaFree(P.near_list);
+    cudaFree(P.far_acc);
+    cudaFree(P.far_s2f);
     cudaFree(P.flags);
     cudaFree(P.pst);
     cudaFree(P.wbf);
@@ -226,23 +240,26 @@ void free_problem(Problem& P) {
 
 inline int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
-// Thresholds from the launch-shape tuner (simbuca_gb300/tune.py) on GB300: one cloud of
-// up to ~6k ions is latency-bound and runs best as one-warp blocks of 32 ions (11);
-// 64 x 2 blocks (5) to ~24k; the k-d ordered shapes beyond (9; 14 from ~48k).  A batch
-// whose pair work fills the GPU on its own (the 512-cloud scan: 3.5e9 pairs per call)
-// takes the k-d ordered leaf shape whatever its largest cloud.
-int auto_variant(const std::vector<int>& counts, int requested) {
-    if (requested >= 0) return requested;
+// Largest cloud shape 17 takes: its leaf indices are 16 bits and its near lists n / 128
+// entries per leaf (0.5 GB there); beyond, shape 14.
+constexpr int kFarOnceMax = 1 << 21;
+
+// Measured on GB300 (us per Coulomb call, shapes 5 / 9 / 14 / 17): 8,000 ions 56 / 52 / 61 /
+// 50, 20,001 ions 250 / 192 / 204 / 162, 65,536 ions 2,482 / 1,755 / 1,761 / 1,316, 524,288
+// ions - / - / 106,900 / 76,000.  Up to SG_FINISH_MAX_IONS the plain shapes keep the one
+// launch of finish.cu per stage, worth more than the pair kernel's last 10 %: one-warp
+// blocks of 32 ions (11) to ~6k, 64 x 2 (5) beyond.  Batches of such clouds keep them too:
+// the k-d order flags 3 % of a small cloud's ions for their FP64 row where the plain order
+// flags 0.6 % (512 clouds of 64 to 8,192 ions, us per attempt: 15,171 / 18,919 / - / 18,128).
+// A stand-alone call pays for the k-d order of its ions on the host each time (1 ms at
+// 20,000): plain shapes to 24,000 ions there.
+int auto_variant(const std::vector<int>& counts, int requested, bool resident) {
     int big = 0;
-    double pairs = 0.0;
-    for (int n : counts) {
-        big = std::max(big, n);
-        pairs += (double)n * (double)n;
-    }
-    if (big >= 48000) return 14;
-    if (pairs >= 2e9) return 9;
-    if (big <= 6000) return 11;
-    return big < 24000 ? 5 : 9;
+    for (int n : counts) big = std::max(big, n);
+    if (requested >= 0) return requested == SG_C32_FAR_ONCE && big > kFarOnceMax ? 14 : requested;
+    if (big > kFarOnceMax) return 14;
+    if (big > (resident ? SG_FINISH_MAX_IONS : 24000)) return SG_C32_FAR_ONCE;
+    return big <= 6000 ? 11 : 5;
 }
 
 // FP64 items that take each unordered pair once: i-block b (128 ions) against the j-tiles
@@ -297,6 +314,65 @@ void plan_sym(Problem& P, int n_sm) {
         return (a.j0 >= a.i0 + SG_SYM_IB) > (b.j0 >= b.i0 + SG_SYM_IB);
     });
     P.n_items = (int)P.hitems.size();
+}
+
+// Shape 17: near items (leaf, one in C of its near leaves: slot c) and far items (leaf
+// against up to 32 later leaves).  C so that there are ~16 near blocks per SM; far runs so
+// that a warp slot of the device (18 warps per SM) gets at least ~8 items, unless the
+// cloud is large enough for whole runs of 32.
+void plan_far_once(Problem& P, int n_sm) {
+    double leaves = 0.0, pairs = 0.0;
+    for (int c = 0; c < P.n_clouds; c++) {
+        if (!(P.hc[c].fp.flags & SG_F_COULOMB)) continue;
+        const double nt = (P.hc[c].npad + 127) / 128;
+        leaves += nt;
+        pairs += 0.5 * nt * (nt - 1.0);
+    }
+    const int C = (int)std::min(8.0, std::max(1.0, std::ceil(16.0 * n_sm / std::max(leaves, 1.0))));
+    const int K = (int)std::min(32.0, std::max(1.0, std::floor(pairs / (18.0 * n_sm * 8.0))));
+    P.max_slots = 0;
+    P.hfar.clear();
+    P.hleaf.clear();
+    P.near_cap = 0;
+    for (int c = 0; c < P.n_clouds; c++) {
+        SgCloud& cl = P.hc[c];
+        cl.nslots = 0;
+        P.hleaf.insert(P.hleaf.end(), (cl.npad + 127) / 128, c);
+        P.near_cap = std::max(P.near_cap, (cl.npad + 127) / 128);
+        if (!(cl.fp.flags & SG_F_COULOMB) || cl.n == 0) continue;
+        P.any_coulomb = true;
+        const int nt = (cl.npad + 127) / 128;
+        const int Cc = std::min(C, nt);
+        cl.nslots = Cc;
+        P.max_slots = std::max(P.max_slots, Cc);
+        P.cloud_inter[c] = (double)cl.n * (cl.n - 1);
+        for (int l = 0; l < nt; l++) {
+            for (int q = 0; q < Cc; q++) {
+                SgWorkItem it;
+                memset(&it, 0, sizeof it);
+                it.cloud = c;
+                it.i0 = cl.poff + 128 * l;
+                it.ni = std::min(128, cl.n - 128 * l);
+                it.j0 = q;   // entries q, q + Cc, ... of the leaf's near list
+                it.nj = Cc;
+                it.slot = q;
+                P.hitems.push_back(it);
+            }
+            for (int j = l + 1; j < nt; j += K)
+                P.hfar.push_back(SgFarItem{c, l, j, std::min(K, nt - j)});
+        }
+    }
+    P.n_items = (int)P.hitems.size();
+}
+
+// Fixed-point scales of a cloud's far sums: a far pair is farther apart than d_far, so
+// |sum| <= B = sum |q| / d_far^2 and a 32-term partial is <= 32 q_max / d_far^2; the
+// scales put those bounds at 2^54 (far_fixed's range), a quantum of B 2^-54.
+void far_scale(SgCloud& cl, double q_abs, double q_max) {
+    const double w = 1.0 / ((double)cl.dfar * cl.dfar);
+    const double B = std::max(q_abs * w, 1.0), B2 = B * std::max(32.0 * q_max * w, 1.0);
+    cl.far_fs = (float)std::ldexp(1.0, 53 - (int)std::ceil(std::log2(B)));
+    cl.far_fs2 = (float)std::ldexp(1.0, 53 - (int)std::ceil(std::log2(B2)));
 }
 
 // Partition clouds into row blocks and Coulomb work items.  Items are sized so that
@@ -363,6 +439,10 @@ void plan(Problem& P, int n_sm) {
     }
     if (P.sym) {
         plan_sym(P, n_sm);
+        return;
+    }
+    if (f32 && P.variant == SG_C32_FAR_ONCE) {
+        plan_far_once(P, n_sm);
         return;
     }
     const int ib = f32 ? sg_coulomb_fp32c_ib(P.variant) : SG_C64_IB;
@@ -479,10 +559,20 @@ void set_frame(SgCloud& cl, const double* pos_aos, int off) {
 }
 
 // k-d tree order of one cloud: recursive median splits along the widest axis, the
-// lower part always a multiple of 128 ions, so that every 128-ion tile is a leaf.
+// lower part always a multiple of 128 ions, so that every 128-ion tile is a leaf.  The
+// coordinates travel with their index: selecting on indices into the caller's array took
+// about twice as long (65,536 ions: 7.9 ms, 6.3 ms so; 500,009: 88 ms, 63 ms).
+struct KdIon {
+    double x[3];
+    int i;
+};
+
 void kd_order(const double* pos, int off, int n, int* out) {
-    std::vector<int> idx(n);
-    for (int i = 0; i < n; i++) idx[i] = off + i;
+    std::vector<KdIon> p(n);
+    for (int i = 0; i < n; i++) {
+        for (int c = 0; c < 3; c++) p[i].x[c] = pos[3 * (size_t)(off + i) + c];
+        p[i].i = off + i;
+    }
     std::vector<std::pair<int, int>> stack;
     stack.push_back(std::make_pair(0, n));
     while (!stack.empty()) {
@@ -493,20 +583,19 @@ void kd_order(const double* pos, int off, int n, int* out) {
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
         for (int i = b; i < e; i++)
             for (int c = 0; c < 3; c++) {
-                const double v = pos[3 * (size_t)idx[i] + c];
-                lo[c] = std::min(lo[c], v);
-                hi[c] = std::max(hi[c], v);
+                lo[c] = std::min(lo[c], p[i].x[c]);
+                hi[c] = std::max(hi[c], p[i].x[c]);
             }
         int ax = 0;
         for (int c = 1; c < 3; c++)
             if (hi[c] - lo[c] > hi[ax] - lo[ax]) ax = c;
         const int m = std::min(len - 1, (len / 2 + 127) / 128 * 128);
-        std::nth_element(idx.begin() + b, idx.begin() + b + m, idx.begin() + e,
-                         [pos, ax](int p, int q) { return pos[3 * (size_t)p + ax] < pos[3 * (size_t)q + ax]; });
+        std::nth_element(p.begin() + b, p.begin() + b + m, p.begin() + e,
+                         [ax](const KdIon& u, const KdIon& v) { return u.x[ax] < v.x[ax]; });
         stack.push_back(std::make_pair(b + m, e));
         stack.push_back(std::make_pair(b, b + m));
     }
-    for (int i = 0; i < n; i++) out[i] = idx[i];
+    for (int i = 0; i < n; i++) out[i] = p[i].i;
 }
 
 int alloc_problem(sg_ctx* ctx, Problem& P) {
@@ -585,6 +674,23 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     CK(cudaMallocHost((void**)&P.hctrl, sizeof(SgCtrl) * (size_t)std::max(P.n_clouds, 1)));
     CK(cudaMemcpy(P.drows, P.hrows.data(), sizeof(SgRowBlock) * P.hrows.size(),
                   cudaMemcpyHostToDevice));
+    if (!P.hfar.empty()) {
+        CK(dalloc(&P.dfar, P.hfar.size()));
+        CK(cudaMemcpy(P.dfar, P.hfar.data(), sizeof(SgFarItem) * P.hfar.size(),
+                      cudaMemcpyHostToDevice));
+    }
+    if (P.precision == SG_PREC_FP32C && P.variant == SG_C32_FAR_ONCE) {
+        CK(dalloc(&P.leaf_cloud, P.hleaf.size()));
+        CK(dalloc(&P.near_count, P.hleaf.size()));
+        CK(dalloc(&P.near_list, P.hleaf.size() * P.near_cap));
+        CK(cudaMemset(P.near_count, 0, P.hleaf.size() * sizeof(int)));
+        CK(cudaMemcpy(P.leaf_cloud, P.hleaf.data(), sizeof(int) * P.hleaf.size(),
+                      cudaMemcpyHostToDevice));
+        CK(dalloc(&P.far_acc, 4 * NP));
+        CK(dalloc(&P.far_s2f, NP));
+        CK(cudaMemset(P.far_acc, 0, 4 * NP * sizeof(unsigned long long)));
+        CK(cudaMemset(P.far_s2f, 0, NP * sizeof(float)));
+    }
     if (P.n_items)
         CK(cudaMemcpy(P.ditems, P.hitems.data(), sizeof(SgWorkItem) * P.hitems.size(),
                       cudaMemcpyHostToDevice));
@@ -772,6 +878,15 @@ int launch_coulomb(sg_ctx* ctx, Problem& P, bool with_ctrl, double inter, double
     ca.max_slots = P.max_slots;
     ca.sym = P.sym ? 1 : 0;
     ca.bbox = P.bbox;
+    ca.leaf_cloud = P.leaf_cloud;
+    ca.n_leaves = (int)P.hleaf.size();
+    ca.near_cap = P.near_cap;
+    ca.near_count = P.near_count;
+    ca.near_list = P.near_list;
+    ca.far_items = P.dfar;
+    ca.n_far = (int)P.hfar.size();
+    ca.far_acc = P.far_acc;
+    ca.far_s2f = P.far_s2f;
     ca.fix_list = P.fix_list;
     ca.fix_part = P.fix_part;
     ca.fix_done = P.fix_done;
@@ -1132,6 +1247,12 @@ void set_charge_scale(Problem& P, const double* q) {
         for (int i = cl.off + 1; uni && i < cl.off + cl.n; i++) uni = q[i] == q[cl.off];
         cl.quniform = uni ? 1 : 0;
         cl.qscale = uni ? q[cl.off] : 1.0;
+        cl.qabs = uni ? cl.n : 0.0;
+        cl.qmax = uni ? 1.0 : 0.0;
+        for (int i = cl.off; !uni && i < cl.off + cl.n; i++) {
+            cl.qabs += std::fabs(q[i]);
+            cl.qmax = std::max(cl.qmax, std::fabs(q[i]));
+        }
     }
 }
 
@@ -1195,6 +1316,7 @@ int upload_state(sg_ctx* ctx, Problem& P, const double* pos, const double* vel,
     }
     for (int c = 0; c < P.n_clouds; c++) {
         set_frame(P.hc[c], pos, P.hc[c].off);
+        far_scale(P.hc[c], P.hc[c].qabs, P.hc[c].qmax);
         P.hc[c].psc = -(P.hc[c].invL * P.hc[c].invL) * P.hc[c].qscale;
         if (P.kfar_prior > 0.0) P.hc[c].kfar2 = (float)(P.kfar_prior * P.kfar_prior);
         double v2 = 0.0;
@@ -1233,14 +1355,14 @@ int check_fp(const sg_field_params* fp) {
 int solo_prepare(sg_ctx* ctx, int n, int precision, const sg_field_params& fp) {
     Problem& P = ctx->solo;
     const bool same = P.n_clouds == 1 && P.n == n && P.precision == precision &&
-                      P.variant == auto_variant(std::vector<int>(1, n), ctx->c32_variant) &&
+                      P.variant == auto_variant(std::vector<int>(1, n), ctx->c32_variant, false) &&
                       ((P.hc[0].fp.flags & SG_F_COULOMB) == (fp.flags & SG_F_COULOMB));
     if (!same) {
         free_problem(P);
         P.n_clouds = 1;
         P.counts.assign(1, n);
         P.precision = precision;
-        P.variant = auto_variant(P.counts, ctx->c32_variant);
+        P.variant = auto_variant(P.counts, ctx->c32_variant, false);
         P.hc.assign(1, SgCloud());
         P.hc[0].fp = fp;
         plan(P, ctx->n_sm);
@@ -1432,7 +1554,7 @@ int sg_batch_create(sg_ctx* ctx, int n_clouds, const int* counts, const sg_field
     P.n_clouds = n_clouds;
     P.counts.assign(counts, counts + n_clouds);
     P.precision = precision;
-    P.variant = auto_variant(P.counts, ctx->c32_variant);
+    P.variant = auto_variant(P.counts, ctx->c32_variant, true);
     P.method = op[0].method == 0 ? 5 : op[0].method;
     P.hc.assign(n_clouds, SgCloud());
     for (int c = 0; c < n_clouds; c++) P.hc[c].fp = fp[c];

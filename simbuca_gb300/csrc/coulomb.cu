@@ -532,6 +532,478 @@ __device__ __forceinline__ void fold_partials(const f2* ax, const f2* ay, const 
     }
 }
 
+// ---- k-d ordered clouds, far leaf pairs once (shape 17) -------------------------------
+// A leaf pair farther apart than d_far is summed from the high parts for both leaves at
+// once (far_warp); the near ones, 5 % of the pairs of a 65,536-ion cloud, keep
+// the float-float differences, close pairs and conditioning of the kernels above, every
+// ordered pair (near_block).
+
+// The near leaves of every leaf, in order: one warp per leaf of the batch; lists[leaf]
+// holds cap entries, counts[leaf] of them used.
+__global__ void __launch_bounds__(128) near_list_kernel(const SgCloud* __restrict__ clouds,
+                                                        const SgCtrl* __restrict__ ctrl,
+                                                        const int* __restrict__ leaf_cloud,
+                                                        int n_leaves, int cap,
+                                                        const float* __restrict__ bbox,
+                                                        int* __restrict__ counts,
+                                                        unsigned short* __restrict__ lists) {
+    sg_griddep_wait();
+    const int leaf = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (leaf >= n_leaves) return;
+    const int c = leaf_cloud[leaf];
+    if (ctrl != nullptr && (ctrl[c].done || ctrl[c].hold || ctrl[c].status != SG_OK)) return;
+    const SgCloud& cl = clouds[c];
+    const int nt = (cl.npad + SG_TILE - 1) / SG_TILE, own = leaf - cl.tile0;
+    const float dfar2 = cl.dfar * cl.dfar;
+    float ib[6];
+    for (int q = 0; q < 6; q++) ib[q] = bbox[8 * (size_t)leaf + q];
+    unsigned short* L = lists + (size_t)leaf * cap;
+    int m = 0;
+    for (int j0 = 0; j0 < nt; j0 += 32) {
+        // past the end: the last leaf again, not listed (every lane takes the same path)
+        const int J = min(j0 + lane, nt - 1);
+        float jb[6];
+#pragma unroll
+        for (int q = 0; q < 6; q++) jb[q] = bbox[8 * (size_t)(cl.tile0 + J) + q];
+        const bool near = j0 + lane < nt && (J == own || !(box_dist2(ib, jb) > dfar2));
+        const unsigned b = __ballot_sync(0xffffffffu, near);
+        if (near) L[m + __popc(b & ((1u << lane) - 1u))] = (unsigned short)J;
+        __syncwarp();
+        m += __popc(b);
+    }
+    if (lane == 0) counts[leaf] = m;
+}
+
+template <int NT, int IPT, int STAGES>
+struct NearShared {
+    float tile[STAGES][7][SG_TILE];
+    uint64_t full[STAGES];
+    uint64_t never;  // the wait test's barrier
+    float corr[6][NT * IPT];
+};
+
+// Near leaves of leaf it.i0, entries it.j0, it.j0 + it.nj, ... of its list, by a block: as
+// the sorted kernel, with the list's leaves as its j-tiles.
+template <int NT, int IPT, int STAGES>
+__device__ __forceinline__ void near_block(const float* __restrict__ c32,
+                                           const double* __restrict__ c64, const SgWorkItem& it,
+                                           const SgCloud& cl, double* __restrict__ part,
+                                           int npad_total, int* errword,
+                                           const int* __restrict__ counts,
+                                           const unsigned short* __restrict__ lists, int cap,
+                                           NearShared<NT, IPT, STAGES>& sh) {
+    constexpr int T = SG_TILE;
+    constexpr int NU = IPT == 1 ? 4 : 2;
+    float(*tile)[7][T] = sh.tile;
+    uint64_t* full = sh.full;
+    float(*corr)[NT * IPT] = sh.corr;
+    const int wtest = errword ? errword[SG_FLAG_WAIT_TILE] : 0;
+    const float wc = cl.wc;
+    const double sc = cl.psc;
+    const int j_real_end = cl.poff + cl.n, j_end = cl.poff + cl.npad;
+    const int tid = threadIdx.x;
+    const size_t NP = (size_t)npad_total;
+    const int leaf = (it.i0 - cl.poff) / T;
+    const unsigned short* L = lists + (size_t)(cl.tile0 + leaf) * cap + it.j0;
+    // entries of this item: it.j0 + t it.nj < counts
+    const int left = counts[cl.tile0 + leaf] - it.j0;
+    const int ntiles = left > 0 ? (left + it.nj - 1) / it.nj : 0;
+
+    int ipad[IPT];
+    f2 xh[IPT], yh[IPT], zh[IPT], xl[IPT], yl[IPT], zl[IPT];
+#pragma unroll
+    for (int k = 0; k < IPT; k++) {
+        const int li = IPT * tid + k;
+        const int ii = it.i0 + (li < it.ni ? li : 0);
+        ipad[k] = li < it.ni ? ii : -1;
+        const float a = c32[ii], b = c32[NP + ii], c = c32[2 * NP + ii], d = c32[4 * NP + ii],
+                    e = c32[5 * NP + ii], f = c32[6 * NP + ii];
+        xh[k] = pk(a, a);
+        yh[k] = pk(b, b);
+        zh[k] = pk(c, c);
+        xl[k] = pk(d, d);
+        yl[k] = pk(e, e);
+        zl[k] = pk(f, f);
+#pragma unroll
+        for (int q = 0; q < 6; q++) corr[q][li] = 0.f;
+    }
+    float ks[IPT][3], kc[IPT][3], s2[IPT], s2f[IPT], fmx[IPT];
+#pragma unroll
+    for (int k = 0; k < IPT; k++) {
+        s2[k] = s2f[k] = fmx[k] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 3; c++) ks[k][c] = kc[k][c] = 0.f;
+    }
+    bool ok = true;
+    if (tid == 0) {
+        for (int s = 0; s < STAGES; s++) mbar_init(&full[s], 1);
+        mbar_init(&sh.never, 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    // prologue: fill the ring
+    if (tid == 0) {
+        for (int s = 0; s < STAGES && s < ntiles; s++) {
+            const int j0 = cl.poff + (int)L[s * it.nj] * T;
+            const uint32_t bytes = (uint32_t)min(T, j_end - j0) * 4u;
+            mbar_arrive_tx(&full[s], 7u * bytes);
+            for (int a = 0; a < 7; a++)
+                bulk_g2s(&tile[s][a][0], c32 + a * NP + j0, bytes, &full[s]);
+        }
+    }
+    __syncwarp();
+    const f2 tiny2 = pk(kTiny, kTiny);
+    const int flush_len = (cl.npad <= 2048) ? 16 : 32;
+    for (int t = 0; t < ntiles; t++) {
+        const int s = t % STAGES;
+        const int J = L[t * it.nj];
+        const int j0 = cl.poff + J * T;
+        const int len = min(T, j_end - j0);
+        bool arrived = mbar_wait(&full[s], (uint32_t)((t / STAGES) & 1));
+        if (t + 1 == wtest) arrived = wait_test(&sh.never, errword) && arrived;
+        if (!__syncthreads_and(arrived)) {  // block-uniform decision
+            ok = false;
+            if (tid == 0) {
+                atomicExch(errword, SG_TIMEOUT);
+                // drain the copies still in flight (tiles t .. t+STAGES-1), bounded
+                for (int u = t; u < ntiles && u < t + STAGES; u++)
+                    (void)mbar_wait(&full[u % STAGES], (uint32_t)((u / STAGES) & 1));
+            }
+            __syncthreads();
+            break;
+        }
+        float y3max[IPT];
+#pragma unroll
+        for (int k = 0; k < IPT; k++) y3max[k] = 0.f;
+        const float* tx = tile[s][0];
+        const float* ty = tile[s][1];
+        const float* tz = tile[s][2];
+        const float* tq = tile[s][3];
+        const float* txl = tile[s][4];
+        const float* tyl = tile[s][5];
+        const float* tzl = tile[s][6];
+        const bool diag = J == leaf;
+        const bool noq = cl.quniform && j0 + len <= j_real_end;
+        for (int jb = 0; jb < len; jb += flush_len) {
+            const int je = min(len, jb + flush_len);
+            f2 ax[IPT], ay[IPT], az[IPT];
+#pragma unroll
+            for (int k = 0; k < IPT; k++) ax[k] = ay[k] = az[k] = 0ull;
+            if (!diag && noq)
+                tile_pairs<IPT, false, true, NU>(tx, ty, tz, tq, txl, tyl, tzl, jb, je, j0, ipad, xh,
+                                             yh, zh, xl, yl, zl, tiny2, wc, ax, ay, az, y3max);
+            else if (!diag)
+                tile_pairs<IPT, false, false, NU>(tx, ty, tz, tq, txl, tyl, tzl, jb, je, j0, ipad, xh, yh,
+                                       zh, xl, yl, zl, tiny2, wc, ax, ay, az, y3max);
+            else
+                tile_pairs<IPT, true, false, NU>(tx, ty, tz, tq, txl, tyl, tzl, jb, je, j0, ipad, xh, yh,
+                                      zh, xl, yl, zl, tiny2, wc, ax, ay, az, y3max);
+            fold_partials<IPT, false>(ax, ay, az, ks, kc, s2, s2f, true);
+            fold_close<IPT>(tile[s], jb, je, j0, ipad, xh, yh, zh, xl, yl, zl, wc, sc, c64,
+                            npad_total, corr, y3max, fmx, [tid](int k) { return IPT * tid + k; });
+        }
+        __syncthreads();  // every thread is done with ring slot s
+        if (tid == 0 && t + STAGES < ntiles) {
+            fence_proxy_async();
+            const int jn = cl.poff + (int)L[(t + STAGES) * it.nj] * T;
+            const uint32_t bytes = (uint32_t)min(T, j_end - jn) * 4u;
+            mbar_arrive_tx(&full[s], 7u * bytes);
+            for (int a = 0; a < 7; a++)
+                bulk_g2s(&tile[s][a][0], c32 + a * NP + jn, bytes, &full[s]);
+        }
+        __syncwarp();
+    }
+    if (!ok) return;
+    float* P = reinterpret_cast<float*>(part) + (size_t)it.slot * SG_PART_F32 * NP;
+#pragma unroll
+    for (int k = 0; k < IPT; k++) {
+        if (ipad[k] < 0) continue;
+        store_partial(P, NP, ipad[k], ks[k], kc[k], corr, IPT * tid + k, s2[k], fmx[k]);
+        P[7 * NP + ipad[k]] = 0.f;  // the far estimate is kept apart
+    }
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ f2 shfl2(f2 v, int src) {
+    return __shfl_sync(0xffffffffu, v, src);
+}
+
+// v (a float-float far sum in frame units) in the cloud's fixed point: round(v fs).  The
+// bound on the far sums keeps |v fs| below 2^54 (far_scale in capi.cu), so the high part
+// splits exactly at 2^30 and both halves are 32-bit conversions.
+__device__ __forceinline__ long long far_fixed(float h, float l, float fs) {
+    const float a = __fmul_rn(h, fs);                        // exact: a power of two
+    const int hi = __float2int_rn(__fmul_rn(a, 9.31322574615478515625e-10f));  // a / 2^30
+    const float rem = __fmaf_rn(-(float)hi, 1073741824.0f, a);  // exact
+    const int lo = __float2int_rn(__fmaf_rn(l, fs, rem));
+    return ((long long)hi << 30) + lo;
+}
+
+// Far pairs of leaf I against up to 32 leaves J > I, by one warp, each unordered pair
+// once, from the high parts.  Bound by the FMA pipe: 8 packed FP32x2 operations shared by
+// the two ions and 3 for each, 7 lane operations per ordered pair where summing each
+// ordered pair takes 11.
+//
+// Lane l keeps four ions of I (4 l ...) in registers with their sums; the ions of J
+// pass through the lanes as packed pairs: at step s lane l meets j-pair (l + s) mod 32 of a
+// 64-ion half-leaf, whose running sum it takes from lane l + 1, so no two lanes ever add
+// to one j-ion.  Both sides' FP32 sums are folded into Kahan pairs in shared memory after
+// chains of 32 terms.  The leaf sums of both
+// sides are added to the cloud's far accumulators as 64-bit fixed point: integer
+// additions commute, so the result does not depend on the order the warps run in, and
+// there are no partial-sum slots to store and add up.
+//
+// Register reads bound it before the FMA pipe: a packed FMA of three distinct operands
+// takes 3.1 - 3.6 cycles of its SM sub-partition, one of two 2.0 (measured), which makes
+// the pair 17 cycles, not 14.  Near and far leaves of a 65,536-ion cloud: 1,316 us per
+// call, 1,755 with the ordered pairs of shape 9; 524,288 ions 76.0 ms, 106.9.
+constexpr int kFarWarps = 4;
+constexpr int kFarFold = 8;  // steps between j-side folds
+template <bool S2F>
+struct __align__(16) FarWarpShared {
+    float j[2][4][SG_TILE];   // x, y, z, q of leaf J, two in flight
+    float S[3][SG_TILE], C[3][SG_TILE];    // leaf J's Kahan pairs
+    float IS[3][SG_TILE], IC[3][SG_TILE];  // leaf I's
+    float s2[S2F ? SG_TILE : 4];
+};
+
+template <bool NOQ, bool S2F>
+__device__ __forceinline__ void far_leaf(const float (*tj)[SG_TILE], FarWarpShared<S2F>& sh,
+                                         const f2 (*xi)[4], const float* __restrict__ qg,
+                                         float* s2i) {
+    const int lane = threadIdx.x & 31, next = (lane + 1) & 31;
+    const f2 tiny2 = pk(kTiny, kTiny);
+    f2 qi[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float q = NOQ ? 0.f : qg[4 * lane + k];
+        qi[k] = pk(q, q);
+    }
+#pragma unroll 1
+    for (int half = 0; half < 4; half++) {  // sixteen steps of a 64-ion half-leaf
+        const int sub = half >> 1, r0 = (half & 1) * 16;
+        f2 a[3][4];
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) a[c][k] = 0ull;
+#pragma unroll 1
+        for (int s8 = r0; s8 < r0 + 16; s8 += kFarFold) {
+            f2 b[3];
+#pragma unroll
+            for (int u = 0; u < kFarFold; u++) {
+                const int p = 64 * sub + 2 * ((lane + s8 + u) & 31);
+                const f2 X = *reinterpret_cast<const f2*>(&tj[0][p]);
+                const f2 Y = *reinterpret_cast<const f2*>(&tj[1][p]);
+                const f2 Z = *reinterpret_cast<const f2*>(&tj[2][p]);
+                const f2 Q = NOQ ? 0ull : *reinterpret_cast<const f2*>(&tj[3][p]);
+                if (u > 0) {
+#pragma unroll
+                    for (int c = 0; c < 3; c++) b[c] = shfl2(b[c], next);
+                }
+                // the step's four j-side terms are summed first: chains of 4 and 8
+                // additions instead of one of 32, and the shuffles off the critical path
+                f2 t[3];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const f2 dx = sub2(X, xi[0][k]), dy = sub2(Y, xi[1][k]), dz = sub2(Z, xi[2][k]);
+                    f2 r2 = fma2(dx, dx, tiny2);
+                    r2 = fma2(dy, dy, r2);
+                    r2 = fma2(dz, dz, r2);
+                    float ra, rb;
+                    upk(r2, ra, rb);
+                    const f2 y = pk(rsqrt_approx(ra), rsqrt_approx(rb));
+                    const f2 y3 = mul2(mul2(y, y), y);
+                    const f2 w = NOQ ? y3 : mul2(Q, y3);
+                    a[0][k] = fma2(w, dx, a[0][k]);
+                    a[1][k] = fma2(w, dy, a[1][k]);
+                    a[2][k] = fma2(w, dz, a[2][k]);
+                    const f2 v = NOQ ? y3 : mul2(qi[k], y3);
+                    t[0] = k ? fma2(v, dx, t[0]) : mul2(v, dx);
+                    t[1] = k ? fma2(v, dy, t[1]) : mul2(v, dy);
+                    t[2] = k ? fma2(v, dz, t[2]) : mul2(v, dz);
+                }
+#pragma unroll
+                for (int c = 0; c < 3; c++) b[c] = u ? add2(b[c], t[c]) : t[c];  // subtracted in the end
+            }
+            // j-side fold: the pair this lane has now
+            const int p = 64 * sub + 2 * ((lane + s8 + kFarFold - 1) & 31);
+            if (S2F) {
+                f2 e = s8 ? *reinterpret_cast<f2*>(&sh.s2[p]) : 0ull;
+                e = fma2(b[0], b[0], fma2(b[1], b[1], fma2(b[2], b[2], e)));
+                *reinterpret_cast<f2*>(&sh.s2[p]) = e;
+            }
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                f2* S = reinterpret_cast<f2*>(&sh.S[c][p]);
+                f2* C = reinterpret_cast<f2*>(&sh.C[c][p]);
+                if (s8 == 0) {  // every pair's first fold
+                    *S = b[c];
+                    *C = 0ull;
+                } else {
+                    const f2 s = *S, y = sub2(b[c], *C), t = add2(s, y);
+                    *C = sub2(sub2(t, s), y);
+                    *S = t;
+                }
+            }
+            __syncwarp();  // the pair moves on to another lane
+        }
+        // i-side fold: two chains of 16 terms per component and ion
+        float t[3][4];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            float4* S = reinterpret_cast<float4*>(sh.IS[c]) + lane;
+            float4* C = reinterpret_cast<float4*>(sh.IC[c]) + lane;
+            float4 s4 = *S, c4 = *C;
+            float* sp = &s4.x;
+            float* cp = &c4.x;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                float lo, hi;
+                upk(a[c][k], lo, hi);
+                t[c][k] = __fadd_rn(lo, hi);
+                kahan_add(sp[k], cp[k], t[c][k]);
+            }
+            *S = s4;
+            *C = c4;
+        }
+        if (S2F)
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                s2i[k] = fmaf(t[0][k], t[0][k], fmaf(t[1][k], t[1][k], fmaf(t[2][k], t[2][k], s2i[k])));
+    }
+}
+
+template <bool S2F>
+__device__ __forceinline__ void far_warp(const float* __restrict__ c32, const SgFarItem& it,
+                                         const SgCloud& cl, unsigned long long* __restrict__ acc,
+                                         int npad_total, const float* __restrict__ bbox,
+                                         FarWarpShared<S2F>& sh) {
+    const int lane = threadIdx.x & 31;
+    const size_t NP = (size_t)npad_total;
+    // far leaves of the item: a lane each
+    unsigned m;
+    {
+        float ib[6], jb[6];
+        const int J = it.j0 + (lane < it.n ? lane : 0);
+        for (int q = 0; q < 6; q++) ib[q] = bbox[8 * (size_t)(cl.tile0 + it.leaf) + q];
+        for (int q = 0; q < 6; q++) jb[q] = bbox[8 * (size_t)(cl.tile0 + J) + q];
+        m = __ballot_sync(0xffffffffu, lane < it.n && box_dist2(ib, jb) > cl.dfar * cl.dfar);
+    }
+    if (m == 0) return;
+    // leaf I is whole: only the last leaf of a cloud may not be, and I < J
+    const int i0 = cl.poff + it.leaf * SG_TILE;
+    f2 xi[3][4];
+    float s2i[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const float x = c32[c * NP + i0 + 4 * lane + k];
+            xi[c][k] = pk(x, x);
+            sh.IS[c][lane + 32 * k] = sh.IC[c][lane + 32 * k] = 0.f;
+        }
+        s2i[k] = 0.f;
+    }
+    const float* qg = c32 + 3 * NP + i0;
+    const float fs = cl.far_fs, fs2 = cl.far_fs2;
+    auto fetch = [&](int J, int slot) {
+        const int j0 = cl.poff + J * SG_TILE, len = min(SG_TILE, cl.poff + cl.npad - j0);
+        float(*t)[SG_TILE] = sh.j[slot];
+#pragma unroll
+        for (int a = 0; a < 4; a++) {
+            if (4 * lane < len)
+                cp_async16(&t[a][4 * lane], c32 + a * NP + j0 + 4 * lane);
+            else  // a cloud's last leaf: far away, no charge
+#pragma unroll
+                for (int q = 0; q < 4; q++) t[a][4 * lane + q] = a < 3 ? 2.0e4f : 0.f;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int slot = 0;
+    __syncwarp();
+    fetch(it.j0 + __ffs(m) - 1, 0);
+    while (m) {
+        const int J = it.j0 + __ffs(m) - 1;
+        m &= m - 1;
+        if (m) {
+            fetch(it.j0 + __ffs(m) - 1, slot ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncwarp();
+        const int j0 = cl.poff + J * SG_TILE;
+        if (cl.quniform && j0 + SG_TILE <= cl.poff + cl.n)
+            far_leaf<true, S2F>(sh.j[slot], sh, xi, qg, s2i);
+        else
+            far_leaf<false, S2F>(sh.j[slot], sh, xi, qg, s2i);
+        // leaf J's sums, their sign the pair's other side's
+#pragma unroll 1
+        for (int k = 0; k < 4; k++) {
+            const int p = lane + 32 * k, jg = j0 + p;
+            if (jg >= cl.poff + cl.n) continue;
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                atomicAdd(acc + c * NP + jg,
+                          (unsigned long long)far_fixed(-sh.S[c][p], sh.C[c][p], fs));
+            if (S2F) atomicAdd(acc + 3 * NP + jg, (unsigned long long)far_fixed(sh.s2[p], 0.f, fs2));
+        }
+        __syncwarp();
+        slot ^= 1;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int p = lane + 32 * k;
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+            atomicAdd(acc + c * NP + i0 + p,
+                      (unsigned long long)far_fixed(sh.IS[c][p], -sh.IC[c][p], fs));
+        if (S2F)
+            atomicAdd(acc + 3 * NP + i0 + 4 * lane + k, (unsigned long long)far_fixed(s2i[k], 0.f, fs2));
+    }
+}
+
+// Near blocks [0, n_near), then blocks of four far warps: one launch, so that the far
+// warps fill the SMs as the near blocks run out.
+constexpr int kLeafThreads = 32 * kFarWarps;
+template <bool S2F>
+__global__ void __launch_bounds__(kLeafThreads, 5) coulomb_leaf_kernel(
+    const float* __restrict__ c32, const double* __restrict__ c64,
+    const SgWorkItem* __restrict__ items, int n_near, const SgFarItem* __restrict__ far_items,
+    int n_far, const SgCloud* __restrict__ clouds, const SgCtrl* __restrict__ ctrl,
+    double* __restrict__ part, unsigned long long* __restrict__ acc, int npad_total, int* errword,
+    const float* __restrict__ bbox, const int* __restrict__ counts,
+    const unsigned short* __restrict__ lists, int cap) {
+    sg_griddep_wait();
+    typedef NearShared<kLeafThreads, 1, 3> Near;
+    typedef FarWarpShared<S2F> Far;
+    constexpr size_t kBytes = sizeof(Near) > kFarWarps * sizeof(Far) ? sizeof(Near)
+                                                                      : kFarWarps * sizeof(Far);
+    __shared__ __align__(128) unsigned char raw[kBytes];
+    if ((int)blockIdx.x < n_near) {
+        const SgWorkItem it = items[blockIdx.x];
+        if (ctrl != nullptr &&
+            (ctrl[it.cloud].done || ctrl[it.cloud].hold || ctrl[it.cloud].status != SG_OK))
+            return;
+        near_block<kLeafThreads, 1, 3>(c32, c64, it, clouds[it.cloud], part, npad_total, errword,
+                                       counts, lists, cap, *reinterpret_cast<Near*>(raw));
+        return;
+    }
+    const int warp = threadIdx.x >> 5;
+    const int item = ((int)blockIdx.x - n_near) * kFarWarps + warp;
+    if (item >= n_far) return;  // warps are independent here
+    const SgFarItem it = far_items[item];
+    if (ctrl != nullptr &&
+        (ctrl[it.cloud].done || ctrl[it.cloud].hold || ctrl[it.cloud].status != SG_OK))
+        return;
+    far_warp<S2F>(c32, it, clouds[it.cloud], acc, npad_total, bbox,
+                  reinterpret_cast<Far*>(raw)[warp]);
+}
+
 template <int NT, int IPT, int MINB, int STAGES, int TJ = SG_TILE, int FU = 0, bool S2F = true>
 __global__ void __launch_bounds__(NT, MINB) coulomb_fp32c_sorted_kernel(const float* __restrict__ c32,
                                                             const double* __restrict__ c64,
@@ -997,6 +1469,25 @@ __device__ void fixup_ion(const SgCloud& cl, int i, int kind, const float* __res
     __syncthreads();
 }
 
+// Far accumulators of shape 17 (null for the others): [4][Npad] fixed-point sums x, y, z
+// and s2f, and the s2f of the last call that estimated it.
+struct FarSums {
+    unsigned long long* acc;
+    float* s2f;
+    int estimate;
+};
+
+// A fixed-point sum in units of 1 / fs as a float-float, by 24-bit pieces.
+__device__ __forceinline__ ff far_value(long long v, float fs) {
+    const float inv = 1.0f / fs;  // a power of two
+    const float h = (float)(int)(v >> 30);            // up to 2^25 or so: may round
+    const long long r = v - ((long long)(int)h << 30);
+    const int r1 = (int)(r >> 8);                      // |r| <= 2^31
+    const float m = (float)(r1 >> 8), l = (float)(int)(r - ((long long)(r1 >> 8) << 16));
+    const ff a = ff_two_sum(__fmul_rn(h, 1073741824.0f * inv), __fmul_rn(m, 65536.0f * inv));
+    return ff_add(a, {__fmul_rn(l, inv), 0.f});
+}
+
 // The G threads of a row (thread li sums slots li / R, li / R + G, ... of row li % R, R
 // rows in the block): their parts combined in a fixed order by the row's first thread.
 struct SlotShared {
@@ -1028,7 +1519,7 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
     double* __restrict__ out, int n_total, int* __restrict__ counters,
     int* __restrict__ fix_list, const float* __restrict__ c32,
     const double* __restrict__ c64, const float* __restrict__ bbox, float* __restrict__ risk,
-    int* __restrict__ ran, const SgCheck* __restrict__ chk, int split) {
+    int* __restrict__ ran, const SgCheck* __restrict__ chk, int split, FarSums far) {
     sg_griddep_wait();
     // this block's share of its row block: cap / split rows
     SgRowBlock rb = rows[blockIdx.x / split];
@@ -1086,6 +1577,23 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
                 s2f += v[7];
             }
             const double sc = cl.psc;
+            if (far.acc != nullptr) {
+                // the far leaves' sums: taken and cleared for the next call
+                unsigned long long* A = far.acc + ig;
+                const ff fx = far_value((long long)A[0], cl.far_fs),
+                         fy = far_value((long long)A[NP], cl.far_fs),
+                         fz = far_value((long long)A[2 * NP], cl.far_fs);
+                A[0] = A[NP] = A[2 * NP] = 0ull;
+                px = ff_add(px, fx);
+                py = ff_add(py, fy);
+                pz = ff_add(pz, fz);
+                if (far.estimate) {
+                    const ff e = far_value((long long)A[3 * NP], cl.far_fs2);
+                    A[3 * NP] = 0ull;
+                    far.s2f[ig] = e.h;
+                }
+                s2f = far.s2f[ig];
+            }
             out[i] = sc * ((double)px.h + (double)px.l);
             out[(size_t)n_total + i] = sc * ((double)py.h + (double)py.l);
             out[2 * (size_t)n_total + i] = sc * ((double)pz.h + (double)pz.l);
@@ -1261,7 +1769,7 @@ static const int kC32Shapes[SG_C32_VARIANTS][2] = {{128, 4}, {128, 2}, {256, 2},
                                                    {128, 4}, {64, 2}, {32, 4}, {32, 4},
                                                    {64, 2}, {128, 1}, {32, 2}, {32, 1},
                                                    {128, 1}, {64, 2}, {64, 2}, {32, 4},
-                                                   {64, 2}};
+                                                   {64, 2}, {128, 1}};
 
 int sg_coulomb_fp32c_ib(int variant) {
     if (variant < 0 || variant >= SG_C32_VARIANTS) variant = 0;
@@ -1349,6 +1857,18 @@ cudaError_t sg_launch_coulomb_fp32c(const SgCoulombArgs& a, cudaStream_t s) {
             sg_launch(coulomb_fp32c_sorted_kernel<64, 2, 8, 4, 256>, a.n_items, 64, 0, s, 
                 a.c32, a.c64, a.items, a.clouds, a.ctrl, a.part, a.npad_total, a.errword, a.bbox);
             break;
+        case SG_C32_FAR_ONCE:
+            sg_launch(near_list_kernel, (a.n_leaves + 3) / 4, 128, 0, s, a.clouds, a.ctrl, a.leaf_cloud,
+                      a.n_leaves, a.near_cap, a.bbox, a.near_count, a.near_list);
+            {
+                const int grid = a.n_items + (a.n_far + kFarWarps - 1) / kFarWarps;
+                sg_launch(a.far_estimate ? coulomb_leaf_kernel<true> : coulomb_leaf_kernel<false>,
+                          grid, kLeafThreads, 0, s, a.c32, a.c64, a.items, a.n_items, a.far_items,
+                          a.n_far, a.clouds, a.ctrl, a.part, a.far_acc, a.npad_total, a.errword,
+                          a.bbox, (const int*)a.near_count, (const unsigned short*)a.near_list,
+                          a.near_cap);
+            }
+            break;
         case 10:
             sg_launch(coulomb_fp32c_kernel<32, 2>, a.n_items, 32, 0, s, 
                 a.c32, a.c64, a.items, a.clouds, a.ctrl, a.part, a.npad_total, a.errword);
@@ -1384,17 +1904,19 @@ cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* r
     const int split = std::max(1, row_cap / take);
     if (fp32c) {
         const float* bbox = sg_variant_sorted(a.variant) ? a.bbox : nullptr;
+        FarSums far{};
+        if (a.variant == SG_C32_FAR_ONCE) far = FarSums{a.far_acc, a.far_s2f, a.far_estimate};
         if (n_total <= kInBlockFixupMax) {
             sg_launch(coulomb_reduce_kernel<true, true>, n_rows * split, SG_ROWS, 0, s, 
                 rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, nullptr,
-                a.c32, a.c64, bbox, a.risk, a.ran, a.chk, split);
+                a.c32, a.c64, bbox, a.risk, a.ran, a.chk, split, far);
             return cudaGetLastError();
         }
         cudaError_t e = cudaMemsetAsync(a.fix_list, 0, 2 * sizeof(int), s);
         if (e != cudaSuccess) return e;
         coulomb_reduce_kernel<true, false><<<n_rows * split, SG_ROWS, 0, s>>>(
             rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, a.fix_list,
-            nullptr, nullptr, nullptr, a.risk, a.ran, a.chk, split);
+            nullptr, nullptr, nullptr, a.risk, a.ran, a.chk, split, far);
         // a fixed grid that strides over however many work units there are (a batch of
         // small clouds can flag a few percent of its ions; unused blocks exit at once)
         const int grid = kFixupBlocks;
@@ -1404,7 +1926,7 @@ cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* r
     } else {
         sg_launch(coulomb_reduce_kernel<false, false>, n_rows * split, SG_ROWS, 0, s, 
             rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, nullptr,
-            nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, split);
+            nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, split, FarSums{});
     }
     return cudaGetLastError();
 }

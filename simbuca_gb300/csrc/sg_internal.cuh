@@ -103,6 +103,12 @@ struct SgWorkItem {
     int32_t jslot, s01;  // FP64 symmetric items: j-side slot, rotation steps s0 | s1 << 16
 };
 
+// Far leaf pairs of shape 17: leaf `leaf` of the cloud against its leaves [j0, j0 + n),
+// n <= 32, j0 > leaf.
+struct SgFarItem {
+    int32_t cloud, leaf, j0, n;
+};
+
 // Rows of one cloud handled by one block of the O(N) kernels.
 struct SgRowBlock {
     int32_t cloud;
@@ -136,7 +142,10 @@ struct SgCloud {
     // at one charge q, qscale = q (quniform = 1) and the normalized charges are 1
     double qscale;
     double psc;  // frame-unit sums -> SI: -qscale / L^2
+    double qabs, qmax;  // sum and largest of |q / qscale|
     int32_t quniform;
+    // shape 17: fixed-point scales (powers of two) of the far sums and their estimate
+    float far_fs, far_fs2;
     int32_t sym_k, sym_bands;  // FP64 symmetric items: j-tiles per item (0: ordered pairs), bands
     int32_t pad4;
 };
@@ -580,6 +589,15 @@ struct SgCoulombArgs {
     int* errword;
     int variant;             // FP32c launch shape (sg_coulomb_fp32c_ib)
     const float* bbox;       // [tiles][8] tile bounds (sorted variant)
+    // shape 17: the near leaves of each leaf (near_cap entries), the far items and sums
+    const int* leaf_cloud = nullptr;  // [leaves] the leaf's cloud
+    int n_leaves = 0, near_cap = 0;
+    int* near_count = nullptr;
+    unsigned short* near_list = nullptr;
+    const SgFarItem* far_items = nullptr;
+    int n_far = 0;
+    unsigned long long* far_acc = nullptr;  // [4][Npad], zero between calls
+    float* far_s2f = nullptr;               // [Npad]
     // FP32c conditioning fix-up work list, filled by the reduction: [0] count, then
     // per flagged ion its global index and cloud (ints) and |P| in frame units
     int* fix_list;
@@ -621,13 +639,15 @@ cudaError_t sg_force_check(const SgCloud* clouds, int n_clouds, int* ran, const 
                            const double* c64, int npad_total, const double* out, int n_total,
                            SgCheck* chk, cudaStream_t st);
 
-#define SG_C32_VARIANTS 17
+#define SG_C32_VARIANTS 18
+// shape 17: k-d order, far leaf pairs evaluated once for both leaves
+#define SG_C32_FAR_ONCE 17
 // variant 4: ions in k-d tree order, far tile pairs from the high parts only
 #define SG_C32_SORTED 4
 #define SG_C32_SORTED_LEAF 7
 // launch shapes that keep ions in k-d tree order
 __host__ __device__ inline bool sg_variant_sorted(int v) {
-    return v == SG_C32_SORTED || (v >= SG_C32_SORTED_LEAF && v <= 9) || (v >= 12 && v <= 16);
+    return v == SG_C32_SORTED || (v >= SG_C32_SORTED_LEAF && v <= 9) || (v >= 12 && v <= SG_C32_FAR_ONCE);
 }
 int sg_coulomb_fp32c_ib(int variant);
 cudaError_t sg_launch_coulomb_fp32c(const SgCoulombArgs& a, cudaStream_t s);

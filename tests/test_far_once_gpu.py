@@ -1,0 +1,78 @@
+"""Launch shape 17: k-d ordered clouds whose far leaf pairs are evaluated once for both
+leaves, their sums kept in 64-bit fixed point.  Against the FP64 form: leaf edges, equal
+and mixed charges, batches of uneven clouds, and repeated calls (integer sums: the same
+bits whatever the order the warps ran in)."""
+import numpy as np
+import pytest
+
+import oracle
+from simbuca_gb300 import configs
+from simbuca_gb300.abi import SG_PREC_FP32C, SG_PREC_FP64
+from simbuca_gb300.api import Batch
+from helpers import kq_of, rel_err_per_ion, summary
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-6  # the FP32c form's per-ion bound
+
+
+@pytest.fixture()
+def far_once(ctx):
+    ctx.set_coulomb_variant(17)
+    ctx.set_fused(False)
+    yield ctx
+    ctx.set_coulomb_variant(-1)
+    ctx.set_fused(True)
+
+
+def cloud(n, kind):
+    rng = np.random.default_rng(n)
+    pos = rng.normal(0, 5e-4, (n, 3))
+    q = np.ones(n)
+    if kind == "mixed":
+        q = rng.choice([1.0, 2.0, 7.0], n)
+    if kind == "elongated":  # most leaf pairs far
+        pos *= np.array([0.1, 0.1, 10.0])
+        q *= 3.0
+    return pos, q
+
+
+@pytest.mark.parametrize("kind", ["equal", "mixed", "elongated"])
+@pytest.mark.parametrize("n", [2, 100, 128, 129, 257, 384, 1000, 4100, 20003])
+def test_sums_at_leaf_edges(far_once, n, kind):
+    pos, q = cloud(n, kind)
+    kq = kq_of(np.full(n, 132.905 * oracle.AMU), q)
+    a = far_once.coulomb_accel(pos, q, kq, SG_PREC_FP32C)
+    ref = far_once.coulomb_accel(pos, q, kq, SG_PREC_FP64)
+    e = rel_err_per_ion(a, ref)
+    assert e.max() <= TOL, (n, kind, summary(e))
+    again = far_once.coulomb_accel(pos, q, kq, SG_PREC_FP32C)
+    assert np.array_equal(a, again)
+
+
+def test_batch_of_uneven_clouds(far_once):
+    """Clouds below one leaf, of whole leaves and ragged, in one batch: each ends where it
+    ends alone (fixed steps; the batch's own far runs and near items differ)."""
+    counts = [40, 128, 700, 3001, 9000]
+    rng = configs.rng_for(17)
+    clouds = [configs.gaussian_cloud(rng, n, 5e-4, 300.0, np.full(n, configs.M_CS)) for n in counts]
+    fp = configs.penning_field(quad=(0.5, configs.nu_c(configs.M_CS), 0.0, 0.0, 1.0), delta=1e3)
+    op = configs.ode(1e-9, 1e-15, 2e-9, 1.0, adaptive=False)
+
+    def run(sel):
+        cs = [clouds[k] for k in sel]
+        b = Batch(far_once, [counts[k] for k in sel], [fp] * len(sel), [op] * len(sel), SG_PREC_FP32C)
+        assert b.variant() == 17
+        b.upload(np.concatenate([c.pos for c in cs]), np.concatenate([c.vel for c in cs]),
+                 np.concatenate([c.mass for c in cs]),
+                 np.concatenate([c.charge for c in cs]).astype(np.int32))
+        b.attempts(3)
+        return b.download()
+
+    p, v = run(range(len(counts)))
+    at = 0
+    for k, n in enumerate(counts):
+        ps, vs = run([k])
+        # the state's forces agree to the FP32c bound; three 2 ns steps dilute it
+        assert np.abs(p[at:at + n] - ps).max() <= 1e-9 * np.abs(ps).max()
+        assert np.abs(v[at:at + n] - vs).max() <= 1e-9 * np.abs(vs).max()
+        at += n
