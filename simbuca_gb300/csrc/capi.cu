@@ -103,8 +103,8 @@ struct Problem {
     long long attempt_count = 0;
     double kfar_prior = 0.0;  // > 0: the far fix-up threshold's prior of every cloud
     // fused small-cloud attempts (fused.cu)
-    double* errp = nullptr;   // [clouds][SG_FUSED_MAX_CTAS]
-    int fused_cluster = -1;   // cluster size for this batch (0: not launchable), -1 unknown
+bool fused_known = false, fused_resident = false;
+    int fused_cluster = 0;    // cluster size for this batch (0: none can be launched)
     int max_npad = 0;         // largest padded cloud
 };
 
@@ -140,7 +140,7 @@ struct sg_ctx {
     long long coul_launches = 0;
     double fused_ms = 0.0;
     long long fused_launches = 0;
-    int use_fused = 1;  // 0 off, 1 clouds up to SG_FUSED_AUTO_IONS, 2 up to SG_FUSED_MAX_IONS
+    int use_fused = 1;  // 0 off, 1 where it is the faster one, 2 clouds up to SG_FUSED_MAX_IONS
     bool use_graph = true;
     cudaGraphExec_t graph = nullptr;
     // timed graph: the same attempt with an event pair around each Coulomb launch
@@ -233,7 +233,6 @@ void free_problem(Problem& P) {
     cudaFree(P.risk);
     cudaFree(P.ran);
     cudaFree(P.dchk);
-    cudaFree(P.errp);
     if (P.hctrl) cudaFreeHost(P.hctrl);
     P = Problem();
 }
@@ -623,7 +622,6 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     CK(dalloc(&P.stage, 6 * N));
     CK(dalloc(&P.flags, SG_NFLAGS));
     CK(cudaMemset(P.flags, 0, SG_NFLAGS * sizeof(int)));
-    CK(dalloc(&P.errp, (size_t)std::max(P.n_clouds, 1) * SG_FUSED_MAX_CTAS));
     P.max_npad = 0;
     for (int c = 0; c < P.n_clouds; c++) P.max_npad = std::max(P.max_npad, P.hc[c].npad);
     if (P.precision == SG_PREC_FP32C) {
@@ -1082,27 +1080,30 @@ int maybe_check(sg_ctx* ctx, Problem& P, int attempts = 1) {
 }
 
 // The fused small-cloud path (fused.cu) applies to FP32c Dormand-Prince batches of
-// clouds of at most SG_FUSED_AUTO_IONS ions (SG_FUSED_MAX_IONS when forced) in the plain
-// ion order, without a recorder,
-// operations, dissociation, step log or proposer, when the device can launch a cluster
-// with at most SG_FUSED_THREADS ions per CTA.
+// clouds in the plain ion order, without a recorder, operations, dissociation, step log or
+// proposer.  Automatic: clouds of at most SG_FUSED_AUTO_PAIRS pairs per CTA, while every
+// cloud's cluster fits on the device at once; a larger batch of small clouds keeps the
+// SMs busy in the tiled kernels too.  Forced: clouds of up to SG_FUSED_MAX_IONS ions.
 bool fused_eligible(sg_ctx* ctx, Problem& P) {
     if (!ctx->use_fused || P.precision != SG_PREC_FP32C || P.method != 5 || P.sorted ||
         P.rec_cap > 0 || !P.hops.empty() || P.n_dis > 0 || P.use_mlp || P.log_cap > 0 ||
         P.n_clouds == 0)
         return false;
     int big = 0;
-    const int limit = ctx->use_fused == 2 ? SG_FUSED_MAX_IONS : SG_FUSED_AUTO_IONS;
     for (int c = 0; c < P.n_clouds; c++) {
-        if (P.hc[c].n < 1 || P.hc[c].n > limit) return false;
+        if (P.hc[c].n < 1 || P.hc[c].n > SG_FUSED_MAX_IONS) return false;
         big = std::max(big, P.hc[c].n);
     }
-    if (P.fused_cluster < 0) P.fused_cluster = sg_fused_cluster_size(P.max_npad);
-    if (P.fused_cluster <= 0 || big > P.fused_cluster * SG_FUSED_THREADS) return false;
-    // automatic: only while every cloud's cluster fits on the device at once; a larger
-    // batch of small clouds runs faster through the batched tiled kernels (167 clouds of
-    // <= 300 ions: 4.6x)
-    return ctx->use_fused == 2 || (long long)P.n_clouds * P.fused_cluster <= ctx->n_sm;
+    if (!P.fused_known) {
+        const int R = sg_fused_cluster_size(P.max_npad, P.n_clouds);
+        P.fused_cluster = std::abs(R);
+        P.fused_resident = R > 0;
+        P.fused_known = true;
+    }
+    if (P.fused_cluster == 0) return false;
+    if (ctx->use_fused == 2) return true;
+    const int own = (big + P.fused_cluster - 1) / P.fused_cluster;
+    return P.fused_resident && (long long)own * big <= SG_FUSED_AUTO_PAIRS;
 }
 
 // n attempts of every active cloud at most (a cloud stops early once done or held);
@@ -1112,16 +1113,12 @@ int run_fused(sg_ctx* ctx, Problem& P, int n, int counted) {
     f.clouds = P.dc;
     f.ctrl = P.dctrl;
     f.y = P.y;
-    f.ys = P.ys;
-    f.k = P.k;
     f.coul1 = P.coul1;
-    f.coul7 = P.coul7;
     f.coulS = P.coulS;
     f.kq = P.kq;
     f.qm = P.qm;
     f.c64 = P.c64;
     f.c32 = P.c32;
-    f.errp = P.errp;
     f.flags = P.flags;
     f.risk = P.risk;
     f.ran = P.ran;

@@ -1,32 +1,34 @@
 // fused.cu -- the small-cloud path: whole Dormand-Prince attempts of a cloud in one kernel.
 //
-// A cloud of a few thousand ions is latency-bound in every kernel of the tiled path: an
-// attempt is 21 launches (stage 1, then for s = 2..7 the pair kernel, the reduction and
-// stage s, then control and commit), each a few microseconds of dependent work on a
-// handful of SMs, plus the launch gaps between them.  Here one thread-block cluster of
-// up to 16 CTAs holds one cloud and runs its attempts back to back inside one launch,
-// the phases separated by cluster barriers (hardware barriers of co-scheduled CTAs: no
-// flag is spun on).  CTA r of the cluster owns the cloud's ions [r m, (r+1) m),
-// m = ceil(n / R), in every phase:
-//   * stage S (bin/ode.cpp:101-175): k_S from the field terms at t + c_S h and the
-//     Coulomb sum, the next stage state y + h sum a_Sj k_j and its Coulomb inputs (SI and
-//     FP32 frame coordinates), or for S = 7 the CTA's part of the error norm
-//     (bin/ode.cpp:189-205);
-//   * the Coulomb sum of stage S (bin/force.cpp:147-174): every CTA copies the cloud's
-//     FP32 frame coordinates into shared memory and G threads sum each of its ions
-//     against interleaved G-ths of the cloud, in the FP32-compensated form of the tiled kernel
-//     (float-float differences, SFU 1/r, 1/r^3 capped with FP64 close pairs, partial sums
-//     folded into Kahan accumulators every 16 j-ions); the G parts are added in FP64 in a
-//     fixed order, and an ion whose terms cancel strongly (sqrt(s2) > 1.5 |P|) gets its
-//     whole row in FP64 instead, as the tiled reduction does;
-//   * control (CTA 0): error_succes and step() (sg_error_succes), then the commit
-//     pos <- pos2, vel <- vel2 of accepted attempts (bin/ode.cpp:488-489).
-// The cloud's coordinates, FP32 frame and SI, sit in shared memory during a Coulomb phase
-// (close pairs and fix-ups read their SI coordinates there), which bounds the path to
-// clouds of 2,048 ions.  Per-ion state stays in the batch's global arrays, so every other entry point (upload,
-// download, moments, the tiled path itself) sees the same state.  Data a CTA wrote for
-// its own ions it reads back itself; what other CTAs wrote (coordinates, the control
-// block, error partials) is read with L2-only loads after the cluster barrier.
+// A cloud of a few hundred ions waits for latencies: launches, memory round trips, barriers
+// and chains of FP64 instructions (64 cycles of their sub-partition each).  Here one
+// thread-block cluster of up to 16 CTAs holds one cloud and runs its attempts back to back
+// inside one launch.  CTA r owns the cloud's ions [r m, (r+1) m) in every phase:
+//   * stage S (bin/ode.cpp:101-175): a thread per ion and component keeps y, the k_j and
+//     the stage state in registers; the components of an ion meet in shared memory;
+//   * exchange: each CTA stores its ions' new coordinates (SI and FP32 frame) into the
+//     shared memory of every CTA of the cluster, then one cluster barrier (hardware
+//     barriers of co-scheduled CTAs: no flag is spun on).  Two coordinate sets alternate
+//     by stage, so a CTA may write stage S+1's while another still reads stage S's;
+//   * between arriving at the barrier and waiting for it: the part of the next stage that
+//     needs no Coulomb sum (field terms, the sum over earlier k_j);
+//   * the Coulomb sum (bin/force.cpp:147-174): G threads sum each ion of the CTA against
+//     interleaved G-ths of the cloud, in the FP32-compensated form of the tiled kernels
+//     (float-float differences, SFU 1/r, 1/r^3 capped with float-float close pairs, partial
+//     sums folded into Kahan accumulators every 16 j-ions, the G parts added in
+//     float-float); an ion whose terms cancel strongly (sqrt(s2) > 1.5 |P|) gets its whole
+//     row in FP64 instead, spread over the CTA's warps;
+//   * control: error partials go to every CTA, and every CTA decides alike
+//     (error_succes and step(), sg_error_succes; bin/ode.cpp:426-494), so the commit
+//     pos <- pos2, vel <- vel2 (bin/ode.cpp:488-489) needs no second barrier.
+// Seven cluster barriers per attempt.  State returns to the batch's global arrays when the
+// launch ends, so every other entry point (upload, download, moments, the tiled path
+// itself) sees it.
+//
+// Measured, one cloud, us per attempt (state, coordinates and sums through global memory
+// with 15 barriers, close pairs found by a second scan, a flagged row per warp -> this
+// form): 64 ions 70 -> 34, 300 131 -> 60, 512 155 -> 72.  What is left is the
+// chain stage - barrier - pairs of dependent instructions.
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -38,124 +40,218 @@ namespace cg = cooperative_groups;
 namespace {
 
 constexpr int kThreads = SG_FUSED_THREADS;
-constexpr int kMaxIons = SG_FUSED_MAX_IONS;
-constexpr int kFlush = 16;        // j-ions per FP32 partial sum before the Kahan fold
+constexpr int kWarps = kThreads / 32;
+constexpr int kFold = 8;          // packed j-pairs per FP32 partial sum before the Kahan fold
 constexpr float kKappa2 = 2.25f;  // FP64 row when s2 > 2.25 |P|^2 (the tiled reduction's for large clouds)
 
-struct FusedShared {
-    int nflag;
-    int flag_il[kThreads];  // flagged ions (local index)
+// What the CTAs of a cluster tell each other at the end of an attempt, two attempts in
+// turn: a CTA may be one barrier ahead of another's reads.
+struct FusedNote {
+    double err[SG_FUSED_MAX_CTAS];  // error partials
+    double x0;                      // x of the caller's first ion
+    int ew, hold;                   // the context's error word and hold switch
 };
 
-__device__ __forceinline__ int ldcg_int(const int* p) { return __ldcg(p); }
+struct FusedShared {
+    SgCtrl cs;
+    SgFieldCoef fk[SG_MAX_STAGES];
+    FusedNote note[2];
+    double red[2][kWarps][3];  // parts of a flagged row; [0][w][0]: error partials
+    double x0;
+    int ew, hold;  // at the launch
+    int nflag;
+};
 
-// Stage S of the CTA's ions [lo, hi): k_S, then the state and Coulomb inputs of stage
-// S+1, or (S = 7) the CTA's sum of squared scaled errors, returned on thread 0.  A thread
-// per ion and component, components in warps of their own: the FP64 instructions of a
-// stage (64 cycles each) are spread over the SM's four sub-partitions.
-template <int S>
-__device__ double stage_phase(const DpArgs& a, const SgCloud& cl, const SgCtrl& cs,
-                              const SgFieldCoef& fk, int lo, int hi) {
-    constexpr int kPasses = 6;  // up to kThreads ions of the CTA
-    const size_t N = (size_t)a.n;
-    const int m = hi - lo, mp = (m + 31) & ~31;
-    double out[kPasses], acc2 = 0.0, sol = 0.0;
+// Dynamic shared memory: the cloud's coordinates in two sets, its normalized charges, and
+// the CTA's own ions (mc of them at most): state, Coulomb sums, flagged ions.
+struct FusedArrays {
+    double* D;    // [2][3][npc] SI coordinates
+    float* C;     // [2][6][npc] frame coordinates: high parts x, y, z, low parts x, y, z
+    float* Q;     // [npc]
+    double* ST;   // [6][mc]
+    float2* P;    // [3][mc] sums in frame units (float-float), or of a flagged ion SI (double)
+    int* list;    // [mc] flagged ions
+    int* flag;    // [mc]
+    int npc, mc;
+};
+constexpr size_t smem_bytes(int npc, int mc) {
+    return (12 * sizeof(float) + 6 * sizeof(double) + sizeof(float)) * (size_t)npc +
+           (6 * sizeof(double) + 3 * sizeof(float2) + 2 * sizeof(int)) * (size_t)mc;
+}
+__device__ __forceinline__ FusedArrays carve(unsigned char* p, int npc, int mc) {
+    FusedArrays s;
+    s.D = reinterpret_cast<double*>(p);
+    s.C = reinterpret_cast<float*>(s.D + 6 * npc);
+    s.Q = s.C + 12 * npc;
+    s.ST = reinterpret_cast<double*>(s.Q + npc);  // npc is a multiple of 4: 16-byte aligned
+    s.P = reinterpret_cast<float2*>(s.ST + 6 * mc);
+    s.list = reinterpret_cast<int*>(s.P + 3 * mc);
+    s.flag = s.list + mc;
+    s.npc = npc;
+    s.mc = mc;
+    return s;
+}
+// Ions of a CTA: a multiple of 4, so that a CTA's rows of the coordinate arrays are whole
+// 16-byte words.
+__host__ __device__ constexpr int own_ions(int n, int ctas) {
+    return ((n + ctas - 1) / ctas + 3) / 4 * 4;
+}
+
+// A thread's ions and components of the CTA's 6 m: slot t = thread + u kThreads is row
+// t mod m of component t / m (packed: a stage costs an FP64 instruction per warp, whatever
+// its lanes hold).
+template <int PASSES>
+struct Slots {
+    int c[PASSES], row[PASSES];  // c = -1: none
+    double y[PASSES];            // the step's initial value
+    double st[PASSES];           // the stage's
+    double k[PASSES][6];
+    double p1[PASSES], p7[PASSES];  // Coulomb sums of stages 1 and 7 (acceleration components)
+    double base[PASSES], part[PASSES];
+    double qm[PASSES], kq[PASSES];
+};
+
+// What stage S needs besides its Coulomb sum: k_S of a coordinate or the field terms, and
+// the sum over the earlier k_j for the next state or the error.
+template <int S, int PASSES>
+__device__ __forceinline__ void stage_before(const FusedArrays& s, const SgCloud& cl,
+                                             const SgFieldCoef& fk, Slots<PASSES>& w) {
 #pragma unroll
-    for (int u = 0; u < kPasses; u++) {
-        const int t = (int)threadIdx.x + u * kThreads;
-        const int c = mp ? t / mp : 6, row = t - c * mp;
-        out[u] = 0.0;
-        if (u * kThreads < 6 * mp && c < 6 && row < m) {
-            const int i = lo + row;
-            double P = 0.0;
-            if (c >= 3 && (cl.fp.flags & SG_F_COULOMB)) {
-                P = (S == 1 ? a.coul1 : a.coulS)[(c - 3) * N + i];
-                if (S == 7) a.coul7[(c - 3) * N + i] = P;
-            }
-            out[u] = stage_one<S, MethodDP>(a, cl, cs, fk, c, i, P, sol);
-            if (S == 7) acc2 += out[u];
+    for (int u = 0; u < PASSES; u++) {
+        const int c = w.c[u];
+        if (c < 0) continue;
+        const double* st = s.ST + w.row[u];
+        if (c < 3) {
+            w.base[u] = st[(3 + c) * s.mc];
+        } else {
+            const int ax = c - 3, o = ax == 0 ? 1 : 0;
+            w.base[u] = sg_field_axis(cl.fp, fk, w.qm[u], ax, st[ax * s.mc], st[c * s.mc],
+                                      st[o * s.mc], st[(3 + o) * s.mc]);
         }
-    }
-    if constexpr (S == 7) {
-        __shared__ double red[kThreads / 32];
-        for (int o = 16; o > 0; o >>= 1) acc2 += __shfl_down_sync(0xffffffffu, acc2, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc2;
-        __syncthreads();
-        double s = 0.0;
-        if (threadIdx.x < 32) {
-            s = threadIdx.x < kThreads / 32 ? red[threadIdx.x] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        }
-        __syncthreads();
-        return s;
-    } else {
-        __syncthreads();  // this stage's state has been read
+        double a = 0.0;
 #pragma unroll
-        for (int u = 0; u < kPasses; u++) {
-            const int t = (int)threadIdx.x + u * kThreads;
-            const int c = mp ? t / mp : 6, row = t - c * mp;
-            if (u * kThreads < 6 * mp && c < 6 && row < m) {
-                const int i = lo + row;
-                a.ys[c * N + i] = out[u];
-                if (c < 3) write_coord(a, cl, c, cl.poff + (i - cl.off), out[u]);
-            }
+        for (int j = 1; j < S; j++) {
+            if (S < 7)
+                a += MethodDP::a(S + 1, j - 1) * w.k[u][j - 1];
+            else if (j != 2)
+                a += MethodDP::e(j) * w.k[u][j - 1];
         }
-        return 0.0;
+        w.part[u] = a;
     }
 }
 
-// The Coulomb sums of the CTA's ions [lo, hi) at the current Coulomb inputs, into coulS
-// (SI, m^-2), in the FP32-compensated form.  sc: the cloud's FP32 frame coordinates
-// (7 x npad floats) and then its SI coordinates and charges (4 x npad doubles, 16-byte
-// aligned) in shared memory.
-__device__ void coulomb_phase(const SgFusedArgs& f, const SgCloud& cl, int lo, int hi, float* sc,
-                              FusedShared& sh) {
-    const int tid = threadIdx.x;
-    const int npc = cl.npad;
-    const size_t NP = (size_t)f.npad;
-    double* sd = reinterpret_cast<double*>(sc + 7 * npc);  // 7 npc floats: a multiple of 16 B
-    // the cloud's coordinates (written by every CTA of the cluster) through L2
-    {
-        const int nv = npc / 4;
-        for (int q = tid; q < 7 * nv; q += kThreads) {
-            const int a = q / nv, v = q - a * nv;
-            const float4* src = reinterpret_cast<const float4*>(f.c32 + a * NP + cl.poff);
-            reinterpret_cast<float4*>(sc + a * npc)[v] = __ldcg(src + v);
+// k_S with the Coulomb sum of the ion, and the next stage's state; at S = 7 the squared
+// scaled error (bin/ode.cpp:107-205).
+template <int S, int PASSES>
+__device__ __forceinline__ double stage_after(const FusedArrays& s, const SgCloud& cl, double h,
+                                              double atol, double rtol, bool coul,
+                                              Slots<PASSES>& w) {
+    double acc2 = 0.0;
+#pragma unroll
+    for (int u = 0; u < PASSES; u++) {
+        const int c = w.c[u];
+        if (c < 0) continue;
+        double kS = w.base[u];
+        if (c >= 3) {
+            double P = 0.0;
+            if (S == 1) {
+                P = w.p1[u];
+            } else if (coul) {
+                const float2* p = s.P + (c - 3) * s.mc + w.row[u];
+                P = s.flag[w.row[u]] ? *reinterpret_cast<const double*>(p)
+                                     : cl.psc * ((double)p->x + (double)p->y);
+            }
+            if (S == 7) w.p7[u] = P;
+            kS = kS + w.kq[u] * P;
         }
-        const int nd = npc / 2;
-        for (int q = tid; q < 4 * nd; q += kThreads) {
-            const int a = q / nd, v = q - a * nd;
-            const double2* src = reinterpret_cast<const double2*>(f.c64 + a * NP + cl.poff);
-            reinterpret_cast<double2*>(sd + a * npc)[v] = __ldcg(src + v);
+        if constexpr (S < 7) {
+            w.k[u][S - 1] = kS;
+            w.st[u] = w.y[u] + h * (w.part[u] + MethodDP::a(S + 1, S - 1) * kS);
+        } else {
+            const double e = w.part[u] + MethodDP::e(7) * kS;
+            const double m0 = fabs(w.y[u]), m1 = fabs(w.st[u]);
+            const double sk = atol + rtol * ((m0 < m1) ? m1 : m0);
+            const double r = h * e * stage_rcp(sk);
+            acc2 += r * r;
         }
     }
-    __syncthreads();
-    const double* SX = sd;
-    const double* SY = sd + npc;
-    const double* SZ = sd + 2 * npc;
-    const double* SQ = sd + 3 * npc;
-    const float* X = sc;
-    const float* Y = sc + npc;
-    const float* Z = sc + 2 * npc;
-    const float* Q = sc + 3 * npc;
-    const float* XL = sc + 4 * npc;
-    const float* YL = sc + 5 * npc;
-    const float* ZL = sc + 6 * npc;
-    const int m = hi - lo;
+    return acc2;
+}
+
+// The new state into shared memory, its coordinates into set `set` of this CTA.
+template <int PASSES>
+__device__ __forceinline__ void store_state(const FusedArrays& s, const SgCloud& cl, int lo,
+                                            int set, const Slots<PASSES>& w) {
+#pragma unroll
+    for (int u = 0; u < PASSES; u++) {
+        const int c = w.c[u];
+        if (c < 0) continue;
+        s.ST[c * s.mc + w.row[u]] = w.st[u];
+        if (c < 3) {
+            const int li = lo + w.row[u];
+            const double v = (w.st[u] - (c == 0 ? cl.cx : c == 1 ? cl.cy : cl.cz)) * cl.invL;
+            const float hi = __double2float_rn(v);
+            float* C = s.C + set * 6 * s.npc + li;
+            C[c * s.npc] = hi;
+            C[(3 + c) * s.npc] = __double2float_rn(v - (double)hi);
+            s.D[(set * 3 + c) * s.npc + li] = w.st[u];
+        }
+    }
+}
+
+// This CTA's rows [lo, lo + m) of set `set` into the other CTAs' shared memory, 16 bytes a
+// store: 6 m / 4 words of frame coordinates and 3 m / 2 of SI ones for each.
+__device__ __forceinline__ void push_coords(cg::cluster_group& cluster, const FusedArrays& s,
+                                            int lo, int m, int set, int ctas, int r) {
+    const int m4 = min(m, s.npc - lo) / 4, nv = 12 * m4;  // past the last ion: padding
+    for (int q = threadIdx.x; q < nv * ctas; q += kThreads) {
+        const int to = q / nv, v = q - to * nv;
+        if (to == r) continue;
+        float4* src;
+        if (v < 6 * m4) {
+            const int a = v / m4;
+            src = reinterpret_cast<float4*>(s.C + (set * 6 + a) * s.npc + lo) + (v - a * m4);
+        } else {
+            const int a = (v - 6 * m4) / (2 * m4);
+            src = reinterpret_cast<float4*>(s.D + (set * 3 + a) * s.npc + lo) +
+                  (v - 6 * m4 - a * 2 * m4);
+        }
+        *cluster.map_shared_rank(src, to) = *src;
+    }
+}
+
+// Coulomb sums of the CTA's mo ions (cloud indices lo ...) at coordinate set `set` into
+// s.P, in the FP32-compensated form; risk: where the in-run check's inputs go (null: not
+// written).
+__device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedArrays& s,
+                                              const SgCloud& cl, int lo, int mo, int set,
+                                              float* risk, FusedShared& sh) {
+    const int tid = threadIdx.x;
+    const int npc = s.npc;
+    const float* X = s.C + set * 6 * npc;
+    const float* Y = X + npc;
+    const float* Z = X + 2 * npc;
+    const float* XL = X + 3 * npc;
+    const float* YL = X + 4 * npc;
+    const float* ZL = X + 5 * npc;
+    const float* Q = s.Q;
+    const double* SX = s.D + set * 3 * npc;
+    const double* SY = SX + npc;
+    const double* SZ = SX + 2 * npc;
+    const double* SQ = f.c64 + 3 * (size_t)f.npad + cl.poff;  // charges: never rewritten here
     // G threads per ion.  Thread q of an ion takes the packed j-pairs q, q + G, q + 2G, ...
     // (j = 2p, 2p + 1), so the G threads of an ion read consecutive 8-byte words of
     // shared memory (no bank conflicts; the ions of a warp read the same words); every 8
     // pairs (16 j-ions) its FP32 partial sums are folded into the Kahan accumulators.
     int G = 1;
-    while (2 * G * m <= kThreads && 2 * G <= 32) G *= 2;
-    const int il = tid / G, q = tid - (tid / G) * G;
+    while (2 * G * mo <= kThreads && 2 * G <= 32) G *= 2;
+    const int il = tid / G, q = tid - il * G;
     const int npair = npc / 2;
     const float wc = cl.wc;
     ff px{0.f, 0.f}, py{0.f, 0.f}, pz{0.f, 0.f};
     float ps2 = 0.f;
-    if (il < m) {
-        const int i = lo + il;
-        const int li = i - cl.off;  // index in the cloud's coordinate arrays
+    const int li = lo + il;  // index in the cloud's coordinate arrays
+    if (il < mo) {
         const float xih = X[li], yih = Y[li], zih = Z[li];
         const float xil = XL[li], yil = YL[li], zil = ZL[li];
         const f2 xh = pk(xih, xih), yh = pk(yih, yih), zh = pk(zih, zih);
@@ -163,89 +259,95 @@ __device__ void coulomb_phase(const SgFusedArgs& f, const SgCloud& cl, int lo, i
         const f2 tiny2 = pk(kTiny, kTiny);
         float ks[3] = {0.f, 0.f, 0.f}, kc[3] = {0.f, 0.f, 0.f}, s2 = 0.f, fmx = 0.f;
         ff cx{0.f, 0.f}, cy{0.f, 0.f}, cz{0.f, 0.f};
-        for (int p0 = q; p0 < npair; p0 += kFlush / 2 * G) {
-            f2 ax = 0ull, ay = 0ull, az = 0ull;
-            float y3max = 0.f;
+        for (int b0 = q; b0 < npair; b0 += 2 * kFold * G) {
+            // close pairs of these 32 j-ions, a bit each (the self pair, dx = 0, with them)
+            unsigned close = 0u;
 #pragma unroll
-            for (int u = 0; u < kFlush / 2; u++) {
-                // past the cloud's last pair (ragged tail): pair 0 again, with no weight
-                const bool ok = p0 + u * G < npair;
-                const int jj = ok ? 2 * (p0 + u * G) : 0;
-                const f2 Xj = *reinterpret_cast<const f2*>(X + jj);
-                const f2 Yj = *reinterpret_cast<const f2*>(Y + jj);
-                const f2 Zj = *reinterpret_cast<const f2*>(Z + jj);
-                const f2 Qj = *reinterpret_cast<const f2*>(Q + jj);
-                const f2 XLj = *reinterpret_cast<const f2*>(XL + jj);
-                const f2 YLj = *reinterpret_cast<const f2*>(YL + jj);
-                const f2 ZLj = *reinterpret_cast<const f2*>(ZL + jj);
-                const f2 dx = add2(sub2(Xj, xh), sub2(XLj, xl));
-                const f2 dy = add2(sub2(Yj, yh), sub2(YLj, yl));
-                const f2 dz = add2(sub2(Zj, zh), sub2(ZLj, zl));
-                f2 r2 = fma2(dx, dx, tiny2);
-                r2 = fma2(dy, dy, r2);
-                r2 = fma2(dz, dz, r2);
-                float ra, rb;
-                upk(r2, ra, rb);
-                const f2 yv = pk(rsqrt_approx(ra), rsqrt_approx(rb));
-                const f2 y3 = mul2(mul2(yv, yv), yv);
-                float ua, ub;
-                upk(y3, ua, ub);
-                // the self pair (dx = 0, no contribution) stays out of the close-pair flag
-                y3max = fmaxf(y3max, ok ? fmaxf(jj == li ? 0.f : ua, jj + 1 == li ? 0.f : ub) : 0.f);
-                const f2 w = mul2(ok ? Qj : 0ull, pk(fminf(ua, wc), fminf(ub, wc)));
-                ax = fma2(w, dx, ax);
-                ay = fma2(w, dy, ay);
-                az = fma2(w, dz, az);
-            }
-            float a, bb;
-            upk(ax, a, bb);
-            const float tx = __fadd_rn(a, bb);
-            upk(ay, a, bb);
-            const float ty = __fadd_rn(a, bb);
-            upk(az, a, bb);
-            const float tz = __fadd_rn(a, bb);
-            kahan_add(ks[0], kc[0], tx);
-            kahan_add(ks[1], kc[1], ty);
-            kahan_add(ks[2], kc[2], tz);
-            s2 = fmaf(tx, tx, fmaf(ty, ty, fmaf(tz, tz, s2)));
-            if (y3max <= wc) fmx = fmaxf(fmx, y3max);  // blocks without a close pair
-            if (y3max > wc) {
-                // close pairs of this partial: the exact term minus the capped FP32 one
-                // (close_term_ff; the closest in FP64 from the SI coordinates); the
-                // block's strongest FP32 term (below the cap, or capped) for fmx
-                for (int u = 0; u < kFlush; u++) {
-                    const int p = p0 + (u >> 1) * G;
-                    if (p >= npair) break;
-                    const int jj = 2 * p + (u & 1);
-                    const PairF pr = pair_f32(X[jj], Y[jj], Z[jj], XL[jj], YL[jj], ZL[jj], xih,
-                                              yih, zih, xil, yil, zil);
-                    if (jj == li || Q[jj] == 0.f) continue;
-                    fmx = fmaxf(fmx, pr.y3 > wc ? capped_term_y3(pr.y3, wc) : pr.y3);
-                    if (!(pr.y3 > wc)) continue;
-                    const float wf = __fmul_rn(Q[jj], wc);
-                    ff dx, dy, dz;
-                    if (pr.y3 <= kVeryClose) {
-                        close_term_ff(ff_diff(X[jj], XL[jj], xih, xil),
-                                      ff_diff(Y[jj], YL[jj], yih, yil),
-                                      ff_diff(Z[jj], ZL[jj], zih, zil), Q[jj], wf, pr, dx, dy, dz);
-                    } else {
-                        const double rx = SX[li] - SX[jj], ry = SY[li] - SY[jj],
-                                     rz = SZ[li] - SZ[jj];
-                        const double w = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz) / cl.psc;
-                        const double c0 = w * rx - (double)wf * (double)pr.dx,
-                                     c1 = w * ry - (double)wf * (double)pr.dy,
-                                     c2 = w * rz - (double)wf * (double)pr.dz;
-                        dx.h = (float)c0;
-                        dx.l = (float)(c0 - (double)dx.h);
-                        dy.h = (float)c1;
-                        dy.l = (float)(c1 - (double)dy.h);
-                        dz.h = (float)c2;
-                        dz.l = (float)(c2 - (double)dz.h);
+            for (int hb = 0; hb < 2; hb++) {
+                f2 ax = 0ull, ay = 0ull, az = 0ull;
+#pragma unroll
+                for (int u0 = 0; u0 < kFold; u0 += 4) {
+                    if (b0 + (hb * kFold + u0) * G >= npair) break;
+#pragma unroll
+                    for (int u = u0; u < u0 + 4; u++) {
+                        // past the cloud's last pair: pair 0 again, with no weight
+                        const int p = b0 + (hb * kFold + u) * G;
+                        const bool ok = p < npair;
+                        const int jj = ok ? 2 * p : 0;
+                        const f2 Xj = *reinterpret_cast<const f2*>(X + jj);
+                        const f2 Yj = *reinterpret_cast<const f2*>(Y + jj);
+                        const f2 Zj = *reinterpret_cast<const f2*>(Z + jj);
+                        const f2 Qj = *reinterpret_cast<const f2*>(Q + jj);
+                        const f2 XLj = *reinterpret_cast<const f2*>(XL + jj);
+                        const f2 YLj = *reinterpret_cast<const f2*>(YL + jj);
+                        const f2 ZLj = *reinterpret_cast<const f2*>(ZL + jj);
+                        const f2 dx = add2(sub2(Xj, xh), sub2(XLj, xl));
+                        const f2 dy = add2(sub2(Yj, yh), sub2(YLj, yl));
+                        const f2 dz = add2(sub2(Zj, zh), sub2(ZLj, zl));
+                        f2 r2 = fma2(dx, dx, tiny2);
+                        r2 = fma2(dy, dy, r2);
+                        r2 = fma2(dz, dz, r2);
+                        float ra, rb;
+                        upk(r2, ra, rb);
+                        const f2 yv = pk(rsqrt_approx(ra), rsqrt_approx(rb));
+                        const f2 y3 = mul2(mul2(yv, yv), yv);
+                        float ua, ub;
+                        upk(y3, ua, ub);
+                        // the strongest term below the cap; a capped one counts below
+                        const bool ca = ua > wc, cb = ub > wc;
+                        fmx = fmaxf(fmx, ok ? fmaxf(ca ? 0.f : ua, cb ? 0.f : ub) : 0.f);
+                        if (ok && ca) close |= 1u << (2 * (hb * kFold + u));
+                        if (ok && cb) close |= 2u << (2 * (hb * kFold + u));
+                        const f2 w = mul2(ok ? Qj : 0ull, pk(fminf(ua, wc), fminf(ub, wc)));
+                        ax = fma2(w, dx, ax);
+                        ay = fma2(w, dy, ay);
+                        az = fma2(w, dz, az);
                     }
-                    cx = ff_add(cx, dx);
-                    cy = ff_add(cy, dy);
-                    cz = ff_add(cz, dz);
                 }
+                float a, b;
+                upk(ax, a, b);
+                const float tx = __fadd_rn(a, b);
+                upk(ay, a, b);
+                const float ty = __fadd_rn(a, b);
+                upk(az, a, b);
+                const float tz = __fadd_rn(a, b);
+                kahan_add(ks[0], kc[0], tx);
+                kahan_add(ks[1], kc[1], ty);
+                kahan_add(ks[2], kc[2], tz);
+                s2 = fmaf(tx, tx, fmaf(ty, ty, fmaf(tz, tz, s2)));
+            }
+            // close pairs: the exact term minus the capped FP32 one (close_term_ff; the
+            // closest in FP64 from the SI coordinates); a capped term is a candidate for
+            // the strongest
+            while (close) {
+                const int bit = __ffs(close) - 1;
+                close &= close - 1u;
+                const int jj = 2 * (b0 + (bit >> 1) * G) + (bit & 1);
+                if (jj == li || Q[jj] == 0.f) continue;
+                const PairF pr = pair_f32(X[jj], Y[jj], Z[jj], XL[jj], YL[jj], ZL[jj], xih, yih,
+                                          zih, xil, yil, zil);
+                fmx = fmaxf(fmx, capped_term_y3(pr.y3, wc));
+                const float wf = __fmul_rn(Q[jj], wc);
+                ff dx, dy, dz;
+                if (pr.y3 <= kVeryClose) {
+                    close_term_ff(ff_diff(X[jj], XL[jj], xih, xil), ff_diff(Y[jj], YL[jj], yih, yil),
+                                  ff_diff(Z[jj], ZL[jj], zih, zil), Q[jj], wf, pr, dx, dy, dz);
+                } else {
+                    const double rx = SX[li] - SX[jj], ry = SY[li] - SY[jj], rz = SZ[li] - SZ[jj];
+                    const double w = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz) / cl.psc;
+                    const double c0 = w * rx - (double)wf * (double)pr.dx,
+                                 c1 = w * ry - (double)wf * (double)pr.dy,
+                                 c2 = w * rz - (double)wf * (double)pr.dz;
+                    dx.h = (float)c0;
+                    dx.l = (float)(c0 - (double)dx.h);
+                    dy.h = (float)c1;
+                    dy.l = (float)(c1 - (double)dy.h);
+                    dz.h = (float)c2;
+                    dz.l = (float)(c2 - (double)dz.h);
+                }
+                cx = ff_add(cx, dx);
+                cy = ff_add(cy, dy);
+                cz = ff_add(cz, dz);
             }
         }
         px = ff_add({ks[0], -kc[0]}, cx);
@@ -268,80 +370,87 @@ __device__ void coulomb_phase(const SgFusedArgs& f, const SgCloud& cl, int lo, i
         pz = ff_add(pz, v);
         ps2 += __shfl_down_sync(0xffffffffu, ps2, o);
     }
-    if (tid == 0) sh.nflag = 0;
-    __syncthreads();
     // the conditioning test (frame units for a unit charge)
-    const int i = lo + il;
-    const bool owner = il < m && q == 0;
-    if (owner) {
-        const double sc_ = cl.psc;  // frame-unit sums -> SI
-        const size_t N = (size_t)f.n;
-        f.coulS[i] = sc_ * ((double)px.h + (double)px.l);
-        f.coulS[N + i] = sc_ * ((double)py.h + (double)py.l);
-        f.coulS[2 * N + i] = sc_ * ((double)pz.h + (double)pz.l);
+    if (il < mo && q == 0) {
         const float pf2 = fmaf(px.h, px.h, fmaf(py.h, py.h, pz.h * pz.h));
         const bool flagged = ps2 > kKappa2 * pf2;
+        s.flag[il] = flagged;
         if (flagged) {
-            const int at = atomicAdd(&sh.nflag, 1);
-            sh.flag_il[at] = il;
+            s.list[atomicAdd(&sh.nflag, 1)] = il;
+        } else {
+            s.P[il] = make_float2(px.h, px.l);
+            s.P[s.mc + il] = make_float2(py.h, py.l);
+            s.P[2 * s.mc + il] = make_float2(pz.h, pz.l);
         }
-        if (f.risk != nullptr) {
-            f.risk[i] = flagged ? -1.f : 0.f;
-            f.risk[N + i] = flagged ? -1.f : sqrtf(ps2 / pf2);
+        if (risk != nullptr) {
+            const size_t i = (size_t)cl.off + li;
+            risk[i] = flagged ? -1.f : 0.f;
+            risk[(size_t)f.n + i] = flagged ? -1.f : sqrtf(ps2 / pf2);
         }
     }
     __syncthreads();
-    // fix-up of the flagged ions, one warp per ion: the whole row in FP64 from the SI
-    // coordinates, which replaces the ion's sum (re-evaluating only its dominant pairs
-    // would keep the rounding of the FP32 additions made while they were in a partial sum)
+    // Flagged ions: the whole row in FP64 from the SI coordinates, which replaces the ion's
+    // sum (re-evaluating only its dominant pairs would keep the rounding of the FP32
+    // additions made while they were in a partial sum).  The CTA's warps share a row by 32
+    // j-ions: a row of 300 in one warp held up the whole cluster for 11,700 cycles.
     const int nf = sh.nflag;
     const int warp = tid >> 5, lane = tid & 31;
-    for (int k = warp; k < nf; k += kThreads / 32) {
-        const int li = lo + sh.flag_il[k] - cl.off;
-        double ax = 0.0, ay = 0.0, az = 0.0;
-        const double xi = SX[li], yi = SY[li], zi = SZ[li];
-        for (int jj = lane; jj < npc; jj += 32) {
-            if (jj == li) continue;
-            const double rx = xi - SX[jj], ry = yi - SY[jj], rz = zi - SZ[jj];
-            const double wq = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz);
-            ax = fma(wq, rx, ax);
-            ay = fma(wq, ry, ay);
-            az = fma(wq, rz, az);
+    for (int k = 0; k < nf; k++) {
+        const int fi = s.list[k], lf = lo + fi;
+        double(*red)[3] = sh.red[k & 1];
+        if (32 * warp < npc) {
+            double ax = 0.0, ay = 0.0, az = 0.0;
+            const double xi = SX[lf], yi = SY[lf], zi = SZ[lf];
+            for (int jj = 32 * warp + lane; jj < npc; jj += kThreads) {
+                if (jj == lf) continue;
+                const double rx = xi - SX[jj], ry = yi - SY[jj], rz = zi - SZ[jj];
+                const double wq = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz);
+                ax = fma(wq, rx, ax);
+                ay = fma(wq, ry, ay);
+                az = fma(wq, rz, az);
+            }
+            __syncwarp();
+            // 32 lanes x 3 components in six additions: the upper half-warp takes y while
+            // the lower sums x, then every other 8 lanes z
+            const bool up = lane & 16;
+            double a = up ? ay : ax;
+            a += __shfl_xor_sync(0xffffffffu, up ? ax : ay, 16);
+            az += __shfl_xor_sync(0xffffffffu, az, 16);
+            const bool odd = lane & 8;
+            double v = odd ? az : a;
+            v += __shfl_xor_sync(0xffffffffu, odd ? a : az, 8);
+            for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) red[warp][0] = v;
+            if (lane == 16) red[warp][1] = v;
+            if (lane == 8) red[warp][2] = v;
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            ax += __shfl_down_sync(0xffffffffu, ax, o);
-            ay += __shfl_down_sync(0xffffffffu, ay, o);
-            az += __shfl_down_sync(0xffffffffu, az, o);
-        }
-        if (lane == 0) {
-            const int i = lo + sh.flag_il[k];
-            const size_t N = (size_t)f.n;
-            f.coulS[i] = ax;
-            f.coulS[N + i] = ay;
-            f.coulS[2 * N + i] = az;
+        __syncthreads();
+        if (tid < 96) {
+            const int c = warp;
+            double v = lane < kWarps && 32 * lane < npc ? red[lane][c] : 0.0;
+            for (int o = kWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) *reinterpret_cast<double*>(s.P + c * s.mc + fi) = v;
         }
     }
+    if (nf > 0) __syncthreads();
 }
 
-// One attempt's worth of control for cloud c (CTA 0, thread 0): error_succes, step()
-// and the bookkeeping of dp_control_kernel for clouds without a recorder or operations.
-__device__ void control_phase(const SgFusedArgs& f, const SgCloud& cl, int c, int nctas) {
-    SgCtrl cs = f.ctrl[c];
-    double s = 0.0;
-    for (int r = 0; r < nctas; r++) s += __ldcg(f.errp + (size_t)c * SG_FUSED_MAX_CTAS + r);
-    const double err = sqrt(s / (6 * cl.n));
+// Control of an attempt with error norm err (thread 0 of every CTA alike): error_succes,
+// step() and the bookkeeping of dp_control_kernel for clouds without a recorder or
+// operations.
+__device__ __forceinline__ void control_phase(SgCtrl& cs, const SgCloud& cl, const FusedNote& nt,
+                                              double err) {
     cs.err = err;
     cs.print_due = 0;
     cs.force_evals += 7;
     cs.coulomb_evals += (cl.fp.flags & SG_F_COULOMB) ? 6 : 0;
     int accepted;
-    const int ew = ldcg_int(f.flags + SG_FLAG_ERR);
-    if (ew != 0) {
-        cs.status = ew;
+    if (nt.ew != 0) {
+        cs.status = nt.ew;
         cs.done = 1;
         accepted = 0;
     } else {
-        accepted = sg_error_succes(cs, err, f.y + cl.ion0);
+        accepted = sg_error_succes(cs, err, &nt.x0);
     }
     if (accepted) {
         cs.h_last = cs.h;
@@ -350,143 +459,243 @@ __device__ void control_phase(const SgFusedArgs& f, const SgCloud& cl, int c, in
         cs.steps++;
         cs.rejects_here = 0;
         if (cs.t >= cs.t_end) cs.done = 1;
-        if (f.flags[SG_FLAG_HOLD]) cs.hold |= 1;
+        if (nt.hold) cs.hold |= 1;
     }
     cs.accepted = accepted;
-    f.ctrl[c] = cs;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs f) {
-    extern __shared__ __align__(16) float sc[];  // 7 x npad floats + 4 x npad doubles
+template <int PASSES>
+__global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs f, int mc) {
+    extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ FusedShared sh;
     cg::cluster_group cluster = cg::this_cluster();
     const int R = (int)cluster.num_blocks();
     const int r = (int)cluster.block_rank();
     const int c = blockIdx.x / R;
-    if (c >= f.n_clouds) return;  // whole clusters only: uniform
+    const int tid = threadIdx.x;
     const SgCloud& cl = f.clouds[c];
-    const int m = (cl.n + R - 1) / R;
-    const int lo = cl.off + min(cl.n, r * m), hi = cl.off + min(cl.n, (r + 1) * m);
+    const FusedArrays s = carve(dyn, cl.npad, mc);
+    const int n = cl.n, npc = cl.npad;
+    const int m = own_ions(n, R);
+    const int lo = min(n, r * m), mo = min(n, (r + 1) * m) - lo;
+    const int ctas = (n + m - 1) / m;  // CTAs with ions
     const bool coul = (cl.fp.flags & SG_F_COULOMB) != 0;
-    __shared__ SgFieldCoef fk[SG_MAX_STAGES];
-    DpArgs a = {};
-    a.y = f.y;
-    a.ys = f.ys;
-    a.k = f.k;
-    a.coulS = f.coulS;
-    a.coul1 = f.coul1;
-    a.coul7 = f.coul7;
-    a.kq = f.kq;
-    a.qm = f.qm;
-    a.c64 = f.c64;
-    a.c32 = f.c32;
-    a.n = f.n;
-    a.npad = f.npad;
-    a.fp32c = 1;
-    for (int att = 0; att < f.max_attempts; att++) {
-        {
-            // every CTA reads the control block after the previous cluster barrier
-            const SgCtrl* cp = f.ctrl + c;
-            if (ldcg_int(&cp->done) || ldcg_int(&cp->hold) || ldcg_int(&cp->status) != SG_OK ||
-                ldcg_int(f.flags + SG_FLAG_ERR) != 0)
-                break;
+    const bool frozen = (cl.fp.flags & SG_F_FROZEN_T) != 0;
+    const size_t N = (size_t)f.n, NP = (size_t)f.npad;
+    if (tid == 0) {
+        sh.cs = f.ctrl[c];
+        sh.ew = f.flags[SG_FLAG_ERR];
+        sh.hold = f.flags[SG_FLAG_HOLD];
+    }
+    // charges; the padding's coordinates, and for whole 16-byte words of the last CTA's rows
+    // they are in both sets of every CTA
+    for (int j = tid; j < npc; j += kThreads) s.Q[j] = f.c32[3 * NP + cl.poff + j];
+    for (int j = n + tid; j < npc; j += kThreads)
+        for (int set = 0; set < 2; set++)
+            for (int a = 0; a < 3; a++) {
+                float* C = s.C + (set * 6 + a) * npc + j;
+                C[0] = f.c32[a * NP + cl.poff + j];
+                C[3 * npc] = f.c32[(4 + a) * NP + cl.poff + j];
+                s.D[(set * 3 + a) * npc + j] = f.c64[a * NP + cl.poff + j];
+            }
+    Slots<PASSES> w;
+#pragma unroll
+    for (int u = 0; u < PASSES; u++) {
+        const int t = tid + u * kThreads;
+        w.c[u] = t < 6 * mo ? t / mo : -1;
+        w.row[u] = 0;
+        w.y[u] = w.p1[u] = w.p7[u] = w.qm[u] = w.kq[u] = w.st[u] = 0.0;
+        if (w.c[u] < 0) continue;
+        w.row[u] = t - w.c[u] * mo;
+        const size_t i = (size_t)cl.off + lo + w.row[u];
+        w.y[u] = f.y[w.c[u] * N + i];
+        if (w.c[u] >= 3) {
+            w.qm[u] = f.qm[i];
+            w.kq[u] = f.kq[i];
+            if (coul) w.p1[u] = f.coul1[(w.c[u] - 3) * N + i];
         }
-        SgCtrl cs;
-        cs.t = __ldcg(&f.ctrl[c].t);
-        cs.h = __ldcg(&f.ctrl[c].h);
-        cs.rtol = __ldcg(&f.ctrl[c].rtol);
-        cs.atol = __ldcg(&f.ctrl[c].atol);
+    }
+    cluster.sync();  // every CTA runs, and has read the control block
+    int att = 0;
+    for (; att < f.max_attempts; att++) {
+        if (sh.cs.done || sh.cs.hold || sh.cs.status != SG_OK || sh.ew != 0) break;
+        const double t0 = sh.cs.t, h = sh.cs.h, atol = sh.cs.atol, rtol = sh.cs.rtol;
         // every stage's field coefficients, a lane each
-        if (threadIdx.x < MethodDP::stages) {
-            const int st = threadIdx.x + 1;
-            const bool frozen = (cl.fp.flags & SG_F_FROZEN_T) != 0;
-            fk[st] = sg_field_coef(cl.fp, frozen ? cs.t : cs.t + MethodDP::c(st) * cs.h);
+        if (tid < MethodDP::stages) {
+            const int st = tid + 1;
+            sh.fk[st] = sg_field_coef(cl.fp, frozen ? t0 : t0 + MethodDP::c(st) * h);
         }
+#pragma unroll
+        for (int u = 0; u < PASSES; u++)
+            if (w.c[u] >= 0) {
+                w.st[u] = w.y[u];
+                s.ST[w.c[u] * mc + w.row[u]] = w.y[u];
+            }
         __syncthreads();
-        stage_phase<1>(a, cl, cs, fk[1], lo, hi);
-        cluster.sync();
-#define SG_FUSED_STAGE(S)                                      \
-    if (coul) {                                                \
-        coulomb_phase(f, cl, lo, hi, sc, sh);                  \
-        cluster.sync();                                        \
-    }                                                          \
-    {                                                          \
-        const double e = stage_phase<S>(a, cl, cs, fk[S], lo, hi);    \
-        if (S == 7 && threadIdx.x == 0)                        \
-            f.errp[(size_t)c * SG_FUSED_MAX_CTAS + r] = e;     \
-    }                                                          \
-    cluster.sync();
+        stage_before<1>(s, cl, sh.fk[1], w);
+        stage_after<1>(s, cl, h, atol, rtol, coul, w);
+        __syncthreads();  // the step's initial state has been read
+        // the state of stage S+1 is in w: its Coulomb sum, then k_{S+1}
+#define SG_FUSED_STAGE(S)                                                          \
+    store_state(s, cl, lo, (S) & 1, w);                                            \
+    if (tid == 0) sh.nflag = 0;                                                    \
+    __syncthreads();                                                               \
+    if (coul) {                                                                    \
+        if (mo > 0) push_coords(cluster, s, lo, m, (S) & 1, ctas, r);              \
+        auto token = cluster.barrier_arrive();                                     \
+        stage_before<S>(s, cl, sh.fk[S], w);                                       \
+        cluster.barrier_wait(std::move(token));                                    \
+        coulomb_phase(f, s, cl, lo, mo, (S) & 1, (S) == 7 ? f.risk : nullptr, sh); \
+    } else {                                                                       \
+        stage_before<S>(s, cl, sh.fk[S], w);                                       \
+        __syncthreads();                                                           \
+    }
         SG_FUSED_STAGE(2)
+        stage_after<2>(s, cl, h, atol, rtol, coul, w);
         SG_FUSED_STAGE(3)
+        stage_after<3>(s, cl, h, atol, rtol, coul, w);
         SG_FUSED_STAGE(4)
+        stage_after<4>(s, cl, h, atol, rtol, coul, w);
         SG_FUSED_STAGE(5)
+        stage_after<5>(s, cl, h, atol, rtol, coul, w);
         SG_FUSED_STAGE(6)
+        stage_after<6>(s, cl, h, atol, rtol, coul, w);
         SG_FUSED_STAGE(7)
+        double e = stage_after<7>(s, cl, h, atol, rtol, coul, w);
 #undef SG_FUSED_STAGE
-        if (r == 0 && threadIdx.x == 0) control_phase(f, cl, c, R);
-        cluster.sync();
-        if (ldcg_int(&f.ctrl[c].accepted)) {
-            // commit: pos <- pos2, vel <- vel2; the stage-7 sum is the next stage-1 sum
-            const size_t N = (size_t)f.n;
-            for (int t = threadIdx.x; t < 9 * (hi - lo); t += kThreads) {
-                const int q = t / (hi - lo), i = lo + t - q * (hi - lo);
-                if (q < 6)
-                    f.y[q * N + i] = f.ys[q * N + i];
-                else
-                    f.coul1[(q - 6) * N + i] = f.coul7[(q - 6) * N + i];
+        // the CTA's error partial (warps without a component add nothing), to every CTA
+        const int warp = tid >> 5, lane = tid & 31;
+        const int nw = min(kWarps, (6 * mo + 31) / 32);  // warps with a component
+        if (warp < nw) {
+            for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+            if (lane == 0) sh.red[0][warp][0] = e;
+        }
+#pragma unroll
+        for (int u = 0; u < PASSES; u++)
+            if (w.c[u] == 0 && cl.off + lo + w.row[u] == cl.ion0) sh.x0 = w.y[u];
+        __syncthreads();
+        FusedNote& nt = sh.note[att & 1];
+        if (tid < 32) {
+            double v = lane < nw ? sh.red[0][lane][0] : 0.0;
+            for (int o = kWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane < R) {
+                FusedNote* to = cluster.map_shared_rank(&nt, lane);
+                to->err[r] = v;
+                if (cl.ion0 >= cl.off + lo && cl.ion0 < cl.off + lo + mo) to->x0 = sh.x0;
+                if (r == 0) {
+                    to->ew = sh.ew;
+                    to->hold = sh.hold;
+                }
             }
         }
-        if (f.ran != nullptr && coul && r == 0 && threadIdx.x == 0) f.ran[c] = 1;
         cluster.sync();
+        if (tid < 32) {
+            double v = lane < R ? nt.err[lane] : 0.0;
+            for (int o = SG_FUSED_MAX_CTAS / 2; o > 0; o >>= 1)
+                v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) control_phase(sh.cs, cl, nt, sqrt(v / (6 * n)));
+        }
+        __syncthreads();
+        if (sh.cs.accepted) {
+            // commit: pos <- pos2, vel <- vel2; the stage-7 sum is the next stage-1 sum
+#pragma unroll
+            for (int u = 0; u < PASSES; u++) {
+                w.y[u] = w.st[u];
+                w.p1[u] = w.p7[u];
+            }
+        }
     }
+    if (att == 0) return;
+    // state, stage sums and the last evaluation's coordinates back to the batch's arrays
+    DpArgs a = {};
+    a.c64 = f.c64;
+    a.c32 = f.c32;
+    a.npad = f.npad;
+    a.fp32c = 1;
+#pragma unroll
+    for (int u = 0; u < PASSES; u++) {
+        const int q = w.c[u];
+        if (q < 0) continue;
+        const int li = lo + w.row[u];
+        const size_t i = (size_t)cl.off + li;
+        f.y[q * N + i] = w.y[u];
+        if (q < 3)
+            write_coord(a, cl, q, cl.poff + li, w.st[u]);
+        else if (coul) {
+            f.coul1[(q - 3) * N + i] = w.p1[u];
+            f.coulS[(q - 3) * N + i] = w.p7[u];
+        }
+    }
+    if (r == 0 && tid == 0) {
+        f.ctrl[c] = sh.cs;
+        if (f.ran != nullptr && coul) f.ran[c] = 1;
+    }
+}
+
+// Slots per thread for mc own ions.  One covers clouds of up to 1,344 ions on 16 CTAs; the
+// others keep more of them in registers (six: the largest clouds on 4 CTAs).
+template <typename F>
+auto by_passes(int mc, F&& f) {
+    if (6 * mc <= kThreads) return f(fused_attempts_kernel<1>);
+    if (6 * mc <= 2 * kThreads) return f(fused_attempts_kernel<2>);
+    return f(fused_attempts_kernel<6>);
 }
 
 }  // namespace
 
-constexpr size_t smem_bytes(int npad) {
-    return (7 * sizeof(float) + 4 * sizeof(double)) * (size_t)npad;
+// Dynamic shared memory any launch asks for at most (2,048 ions on 8 CTAs).  Every kernel
+// is allowed it once and for all: a launch of one thread cannot lower another's.
+constexpr size_t kMaxSmem = smem_bytes(SG_FUSED_MAX_IONS, SG_FUSED_MAX_IONS / 8);
+
+int sg_fused_cluster_size(int max_npad, int n_clouds) {
+    int found = 0;
+    for (int R = SG_FUSED_MAX_CTAS; R >= 2; R /= 2) {
+        const int mc = own_ions(max_npad, R);
+        const size_t smem = smem_bytes(max_npad, mc);
+        if (mc > kThreads || smem > kMaxSmem) continue;
+        const int active = by_passes(mc, [&](auto* kernel) {
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                    cudaSuccess ||
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kMaxSmem) != cudaSuccess)
+                return 0;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(R);
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = smem;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = R;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int n = 0;
+            return cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess ? n : 0;
+        });
+        if (active > 0) found = R;
+        if (active >= n_clouds) return R;
+    }
+    cudaGetLastError();
+    return -found;
 }
 
-int sg_fused_cluster_size(int max_npad) {
-    const size_t smem = smem_bytes(max_npad);
-    if (cudaFuncSetAttribute(fused_attempts_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                             1) != cudaSuccess)
-        return 0;
-    if (cudaFuncSetAttribute(fused_attempts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_bytes(kMaxIons)) != cudaSuccess)
-        return 0;
-    for (int R = SG_FUSED_MAX_CTAS; R >= 4; R /= 2) {
+cudaError_t sg_fused_attempts(const SgFusedArgs& f, int cluster, int max_npad, cudaStream_t st) {
+    const int mc = own_ions(max_npad, cluster);
+    const size_t smem = smem_bytes(max_npad, mc);
+    return by_passes(mc, [&](auto* kernel) {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(R);
+        cfg.gridDim = dim3(f.n_clouds * cluster);
         cfg.blockDim = dim3(kThreads);
         cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = R;
+        at[0].val.clusterDim.x = cluster;
         at[0].val.clusterDim.y = 1;
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, fused_attempts_kernel, &cfg) == cudaSuccess && n > 0)
-            return R;
-    }
-    cudaGetLastError();
-    return 0;
-}
-
-cudaError_t sg_fused_attempts(const SgFusedArgs& f, int cluster, int max_npad, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(f.n_clouds * cluster);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem_bytes(max_npad);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cluster;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, fused_attempts_kernel, f);
+        return cudaLaunchKernelEx(&cfg, kernel, f, mc);
+    });
 }

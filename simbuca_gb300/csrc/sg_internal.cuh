@@ -478,27 +478,31 @@ cudaError_t sg_dp_finish(const SgFinishArgs& f, int stage, int fp32c, cudaStream
 #define SG_FUSED_THREADS 512
 #define SG_FUSED_MAX_CTAS 16
 #define SG_FUSED_MAX_IONS 2048
-// Clouds the fused path takes by default (sg_set_fused mode 1): measured on GB300 it
-// needs ~180 us per attempt at 256 ions against ~245 us for the tiled kernels, breaks
-// even near 1,000 ions and loses beyond; mode 2 takes it up to SG_FUSED_MAX_IONS.
-#define SG_FUSED_AUTO_IONS 512
+// Ordered pairs per CTA (its ions times the cloud's) up to which the fused path is taken by
+// default (sg_set_fused mode 1); mode 2 takes it up to SG_FUSED_MAX_IONS.  Measured on
+// GB300, us per attempt, fused / tiled kernels: one cloud on 16 CTAs of 300 ions 60 / 143,
+// 512 71 / 131, 700 (31,000 pairs) 93 / 119, 850 (48,000) 125 / 136, 1,000 124 / 120, 1,500
+// 294 / 154; 32 clouds of 300 on 4 CTAs each (23,000) 101 / 278, 16 of 512 (66,000) 168 / 194;
+// 70 of 100 on 2 (5,000) 67 / 223.
+#define SG_FUSED_AUTO_PAIRS 40000
 struct SgFusedArgs {
     const SgCloud* clouds;
     SgCtrl* ctrl;
-    double *y, *ys, *k, *coul1, *coul7, *coulS;
+    double *y, *coul1, *coulS;
     const double *kq, *qm;
     double* c64;
     float* c32;
-    double* errp;    // [clouds][SG_FUSED_MAX_CTAS] error partials of an attempt
     int* flags;      // the context's flag words (error word, hold on accept)
     float* risk;     // in-run force check inputs (null: not written)
     int* ran;
     int n, npad, n_clouds;
     int max_attempts;  // attempts per launch at most
 };
-// The cluster size the fused kernel can be launched with on this device for clouds of
-// up to max_npad padded ions (16, 8 or 4), or 0 if none.
-int sg_fused_cluster_size(int max_npad);
+// The cluster size (16, 8, 4 or 2) for n_clouds clouds of up to max_npad padded ions: the
+// largest with which all of them are on the device at once (clusters of 16 take the SMs of
+// a GPC: 8 clouds of 64 ions took 76 us per attempt on 16 CTAs each and 43 on 8).  If there
+// is none, minus the smallest that can be launched (0: no cluster can).
+int sg_fused_cluster_size(int max_npad, int n_clouds);
 cudaError_t sg_fused_attempts(const SgFusedArgs& f, int cluster, int max_npad, cudaStream_t st);
 
 // ---- device-side observables (observe.cu) -------------------------------------------
