@@ -36,13 +36,15 @@ struct Problem {
     std::vector<SgCtrl> hctrl0;
     std::vector<SgRowBlock> hrows;
     std::vector<SgWorkItem> hitems;
-    std::vector<SgFarItem> hfar;   // shape 17
-    SgFarItem* dfar = nullptr;
+    std::vector<SgFarItem> hfar, hnear;   // shape 17
+    int leaf_min = 0;              // ... its clouds of more ions; smaller ones are plain
+    SgFarItem *dfar = nullptr, *dnear = nullptr;
     std::vector<int> hleaf;        // cloud of each leaf
     int near_cap = 0;              // leaves of the largest cloud
     int *leaf_cloud = nullptr, *near_count = nullptr;
     unsigned short* near_list = nullptr;
-    unsigned long long* far_acc = nullptr;
+    unsigned long long* leaf_sum = nullptr;
+    int *leaf_fmx = nullptr, *leaf_n_close = nullptr, *leaf_close = nullptr;
     float* far_s2f = nullptr;
     std::vector<int> counts;
     SgCloud* dc = nullptr;
@@ -203,10 +205,14 @@ void free_problem(Problem& P) {
     cudaFree(P.c32);
     cudaFree(P.fcoef);
     cudaFree(P.dfar);
+    cudaFree(P.dnear);
     cudaFree(P.leaf_cloud);
     cudaFree(P.near_count);
     cudaFree(P.near_list);
-    cudaFree(P.far_acc);
+    cudaFree(P.leaf_sum);
+    cudaFree(P.leaf_fmx);
+    cudaFree(P.leaf_n_close);
+    cudaFree(P.leaf_close);
     cudaFree(P.far_s2f);
     cudaFree(P.flags);
     cudaFree(P.pst);
@@ -242,23 +248,33 @@ inline int round_up(int a, int b) { return (a + b - 1) / b * b; }
 // Largest cloud shape 17 takes: its leaf indices are 16 bits and its near lists n / 128
 // entries per leaf (0.5 GB there); beyond, shape 14.
 constexpr int kFarOnceMax = 1 << 21;
+// Clouds of at most this many ions keep the plain kernel in an automatic batch of shape 17:
+// us per attempt, all plain / all leaves: 40 of 1,500 ions 776 / 837, 40 of 2,000 1,126 /
+// 1,101, 20 of 3,000 1,156 / 994, 10 of 4,096 1,009 / 812; below ~3,000 ions the leaves' errors
+// are 4 % larger (RMS), above smaller.
+constexpr int kLeafMin = 2500;
 
-// Measured on GB300 (us per Coulomb call, shapes 5 / 9 / 14 / 17): 8,000 ions 56 / 52 / 61 /
-// 50, 20,001 ions 250 / 192 / 204 / 162, 65,536 ions 2,482 / 1,755 / 1,761 / 1,316, 524,288
-// ions - / - / 106,900 / 76,000.  Up to SG_FINISH_MAX_IONS the plain shapes keep the one
-// launch of finish.cu per stage, worth more than the pair kernel's last 10 %: one-warp
-// blocks of 32 ions (11) to ~6k, 64 x 2 (5) beyond.  Batches of such clouds keep them too:
-// the k-d order flags 3 % of a small cloud's ions for their FP64 row where the plain order
-// flags 0.6 % (512 clouds of 64 to 8,192 ions, us per attempt: 15,171 / 18,919 / - / 18,128).
-// A stand-alone call pays for the k-d order of its ions on the host each time (1 ms at
-// 20,000): plain shapes to 24,000 ions there.
+// Measured on GB300 (us per Coulomb call, shapes 5 / 9 / 14 / 17): 8,000 ions 57 / 52 / 62 /
+// 53, 20,001 ions 250 / 195 / 203 / 151, 65,536 ions 2,483 / 1,755 / 1,756 / 1,245.  One
+// cloud, or a batch, of up to SG_FINISH_MAX_IONS ions keeps the plain shapes and with them
+// the one launch of finish.cu per stage: one-warp blocks of 32 ions (11) to ~6k, 64 x 2 (5)
+// beyond.  A larger batch takes shape 17 if it has clouds of more than kLeafMin ions (128
+// clouds of 64 to 8,192 ions: 5,190 us per attempt plain, 4,030 so; 3 of 8,000 993 / 769),
+// otherwise plain blocks, 64 x 2 from ~32k ions (100 clouds of 1,000: 953 us, 1,004 with
+// one-warp blocks; 167 of <= 300: 416 / 335).  A stand-alone call pays for the k-d order of
+// its ions on the host each time (1 ms at 20,000): plain shapes to 24,000 ions there.
 int auto_variant(const std::vector<int>& counts, int requested, bool resident) {
     int big = 0;
-    for (int n : counts) big = std::max(big, n);
+    long long total = 0;
+    for (int n : counts) {
+        big = std::max(big, n);
+        total += n;
+    }
     if (requested >= 0) return requested == SG_C32_FAR_ONCE && big > kFarOnceMax ? 14 : requested;
     if (big > kFarOnceMax) return 14;
     if (big > (resident ? SG_FINISH_MAX_IONS : 24000)) return SG_C32_FAR_ONCE;
-    return big <= 6000 ? 11 : 5;
+    if (resident && total > SG_FINISH_MAX_IONS && big > kLeafMin) return SG_C32_FAR_ONCE;
+    return big <= 6000 && total <= 32768 ? 11 : 5;
 }
 
 // FP64 items that take each unordered pair once: i-block b (128 ions) against the j-tiles
@@ -315,63 +331,57 @@ void plan_sym(Problem& P, int n_sm) {
     P.n_items = (int)P.hitems.size();
 }
 
-// Shape 17: near items (leaf, one in C of its near leaves: slot c) and far items (leaf
-// against up to 32 later leaves).  C so that there are ~16 near blocks per SM; far runs so
-// that a warp slot of the device (18 warps per SM) gets at least ~8 items, unless the
+// Shape 17: near items (half a leaf, one in C of its near leaves) and far items (leaf
+// against up to 32 later leaves).  C so that a warp slot of the device (18 warps per SM)
+// gets at least ~8 near items, far runs so that it gets at least ~8 far ones, unless the
 // cloud is large enough for whole runs of 32.
 void plan_far_once(Problem& P, int n_sm) {
     double leaves = 0.0, pairs = 0.0;
     for (int c = 0; c < P.n_clouds; c++) {
-        if (!(P.hc[c].fp.flags & SG_F_COULOMB)) continue;
+        if (!P.hc[c].leafs) continue;
         const double nt = (P.hc[c].npad + 127) / 128;
         leaves += nt;
         pairs += 0.5 * nt * (nt - 1.0);
     }
-    const int C = (int)std::min(8.0, std::max(1.0, std::ceil(16.0 * n_sm / std::max(leaves, 1.0))));
-    const int K = (int)std::min(32.0, std::max(1.0, std::floor(pairs / (18.0 * n_sm * 8.0))));
-    P.max_slots = 0;
+    if (leaves == 0.0) pairs = 1.0;
+    const double slots = 18.0 * n_sm * 8.0;
+    const int C = (int)std::min(8.0, std::max(1.0, std::ceil(0.5 * slots / std::max(leaves, 1.0))));
+    const int K = (int)std::min(32.0, std::max(1.0, std::floor(pairs / slots)));
     P.hfar.clear();
+    P.hnear.clear();
     P.hleaf.clear();
     P.near_cap = 0;
     for (int c = 0; c < P.n_clouds; c++) {
         SgCloud& cl = P.hc[c];
-        cl.nslots = 0;
-        P.hleaf.insert(P.hleaf.end(), (cl.npad + 127) / 128, c);
+        P.hleaf.insert(P.hleaf.end(), (cl.npad + 127) / 128, cl.leafs ? c : -1);
+        if (!cl.leafs) continue;
         P.near_cap = std::max(P.near_cap, (cl.npad + 127) / 128);
-        if (!(cl.fp.flags & SG_F_COULOMB) || cl.n == 0) continue;
         P.any_coulomb = true;
         const int nt = (cl.npad + 127) / 128;
-        const int Cc = std::min(C, nt);
-        cl.nslots = Cc;
-        P.max_slots = std::max(P.max_slots, Cc);
         P.cloud_inter[c] = (double)cl.n * (cl.n - 1);
         for (int l = 0; l < nt; l++) {
-            for (int q = 0; q < Cc; q++) {
-                SgWorkItem it;
-                memset(&it, 0, sizeof it);
-                it.cloud = c;
-                it.i0 = cl.poff + 128 * l;
-                it.ni = std::min(128, cl.n - 128 * l);
-                it.j0 = q;   // entries q, q + Cc, ... of the leaf's near list
-                it.nj = Cc;
-                it.slot = q;
-                P.hitems.push_back(it);
-            }
+            for (int h = 0; h < 2 && 128 * l + 64 * h < cl.n; h++)
+                for (int q = 0; q < std::min(C, nt - l); q++)
+                    P.hnear.push_back(SgFarItem{c, 2 * l + h, q, C});
             for (int j = l + 1; j < nt; j += K)
                 P.hfar.push_back(SgFarItem{c, l, j, std::min(K, nt - j)});
         }
     }
-    P.n_items = (int)P.hitems.size();
 }
 
-// Fixed-point scales of a cloud's far sums: a far pair is farther apart than d_far, so
-// |sum| <= B = sum |q| / d_far^2 and a 32-term partial is <= 32 q_max / d_far^2; the
-// scales put those bounds at 2^54 (far_fixed's range), a quantum of B 2^-54.
+// Fixed-point scales of a cloud's leaf sums.  A capped term is at most q / r_c^2 (r_c the
+// close-pair radius, 1 / r_c^3 = wc) and a far one q / d_far^2, so |sum| <= B = sum |q| / r^2
+// and a 32-term partial is <= 32 q_max / r^2; the scales put those bounds at 2^54
+// (far_fixed's range), a quantum of B 2^-54 at most (65,536 ions: 1e-13 of a typical sum).
 void far_scale(SgCloud& cl, double q_abs, double q_max) {
-    const double w = 1.0 / ((double)cl.dfar * cl.dfar);
-    const double B = std::max(q_abs * w, 1.0), B2 = B * std::max(32.0 * q_max * w, 1.0);
-    cl.far_fs = (float)std::ldexp(1.0, 53 - (int)std::ceil(std::log2(B)));
-    cl.far_fs2 = (float)std::ldexp(1.0, 53 - (int)std::ceil(std::log2(B2)));
+    const double wf = 1.0 / ((double)cl.dfar * cl.dfar), wn = std::max(std::pow(cl.wc, 2.0 / 3.0), wf);
+    auto scale = [&](double w, bool squares) {
+        const double B = std::max(q_abs * w, 1.0) * (squares ? std::max(32.0 * q_max * w, 1.0) : 1.0);
+        return (float)std::ldexp(1.0, 53 - (int)std::ceil(std::log2(B)));
+    };
+    cl.far_fs = scale(wn, false);
+    cl.near_fs2 = scale(wn, true);
+    cl.far_fs2 = scale(wf, true);
 }
 
 // Partition clouds into row blocks and Coulomb work items.  Items are sized so that
@@ -441,21 +451,23 @@ void plan(Problem& P, int n_sm) {
         return;
     }
     if (f32 && P.variant == SG_C32_FAR_ONCE) {
+        for (int c = 0; c < C; c++)
+            P.hc[c].leafs = (P.hc[c].fp.flags & SG_F_COULOMB) && P.hc[c].n > P.leaf_min;
         plan_far_once(P, n_sm);
-        return;
     }
-    const int ib = f32 ? sg_coulomb_fp32c_ib(P.variant) : SG_C64_IB;
+    const int ib = f32 ? sg_coulomb_fp32c_ib(P.variant == SG_C32_FAR_ONCE ? SG_C32_PLAIN : P.variant)
+                       : SG_C64_IB;
     const int per_sm = f32 ? std::max(1, 2048 / ib) : 4;
     const double conc = (double)n_sm * per_sm;
     double total = 0.0;
     for (int c = 0; c < C; c++)
-        if (P.hc[c].fp.flags & SG_F_COULOMB) total += (double)P.hc[c].n * P.hc[c].npad;
+        if ((P.hc[c].fp.flags & SG_F_COULOMB) && !P.hc[c].leafs) total += (double)P.hc[c].n * P.hc[c].npad;
     std::vector<int> S(C, 0);
     long long items = 0;
     const double cap = std::max(total / (conc * 2.0), 512.0 * 512.0);
     for (int c = 0; c < C; c++) {
         const SgCloud& cl = P.hc[c];
-        if (!(cl.fp.flags & SG_F_COULOMB) || cl.n == 0) continue;
+        if (!(cl.fp.flags & SG_F_COULOMB) || cl.n == 0 || cl.leafs) continue;
         const double jmax = std::max(128.0, std::floor(cap / std::min(ib, cl.n) / 128.0) * 128.0);
         S[c] = std::max(1, (int)std::ceil(cl.npad / jmax));
         items += (long long)((cl.n + ib - 1) / ib) * S[c];
@@ -648,8 +660,8 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     CK(dalloc(&P.pmass, N));
     CK(dalloc(&P.pmass0, N));
     // two lists (near-only ions; ions with a far fix-up): counts, then N pairs each
-    CK(dalloc(&P.fix_list, 2 + 4 * N));
-    CK(cudaMemset(P.fix_list, 0, 2 * sizeof(int)));
+    CK(dalloc(&P.fix_list, 4 + 6 * N));
+    CK(cudaMemset(P.fix_list, 0, 4 * sizeof(int)));
     // two lists (row re-evaluations, far corrections) of up to SG_FIX_CHUNKED_CAP ions
     CK(dalloc(&P.fix_part, (size_t)2 * SG_FIX_CHUNKED_CAP * SG_FIX_UNITS * 3));
     CK(dalloc(&P.fix_done, 2 * SG_FIX_CHUNKED_CAP));
@@ -684,9 +696,17 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
         CK(cudaMemset(P.near_count, 0, P.hleaf.size() * sizeof(int)));
         CK(cudaMemcpy(P.leaf_cloud, P.hleaf.data(), sizeof(int) * P.hleaf.size(),
                       cudaMemcpyHostToDevice));
-        CK(dalloc(&P.far_acc, 4 * NP));
+        CK(dalloc(&P.dnear, std::max(P.hnear.size(), (size_t)1)));
+        CK(cudaMemcpy(P.dnear, P.hnear.data(), sizeof(SgFarItem) * P.hnear.size(),
+                      cudaMemcpyHostToDevice));
+        CK(dalloc(&P.leaf_sum, 5 * NP));
+        CK(dalloc(&P.leaf_fmx, NP));
+        CK(dalloc(&P.leaf_n_close, NP));
+        CK(dalloc(&P.leaf_close, SG_CLOSE_CAP * NP));
         CK(dalloc(&P.far_s2f, NP));
-        CK(cudaMemset(P.far_acc, 0, 4 * NP * sizeof(unsigned long long)));
+        CK(cudaMemset(P.leaf_sum, 0, 5 * NP * sizeof(unsigned long long)));
+        CK(cudaMemset(P.leaf_fmx, 0, NP * sizeof(int)));
+        CK(cudaMemset(P.leaf_n_close, 0, NP * sizeof(int)));
         CK(cudaMemset(P.far_s2f, 0, NP * sizeof(float)));
     }
     if (P.n_items)
@@ -861,7 +881,7 @@ void flush_timing(sg_ctx* ctx) {
 // finish kernel sums its slots).
 int launch_coulomb(sg_ctx* ctx, Problem& P, bool with_ctrl, double inter, double* out,
                    bool far_estimate = true, int set = 0) {
-    if (!P.any_coulomb || P.n_items == 0) return SG_OK;
+    if (!P.any_coulomb || (P.n_items == 0 && P.hnear.empty())) return SG_OK;
     SgCoulombArgs ca;
     ca.c32 = P.c32 + (size_t)set * 7 * P.npad;
     ca.c64 = P.c64 + (size_t)set * 4 * P.npad;
@@ -883,7 +903,12 @@ int launch_coulomb(sg_ctx* ctx, Problem& P, bool with_ctrl, double inter, double
     ca.near_list = P.near_list;
     ca.far_items = P.dfar;
     ca.n_far = (int)P.hfar.size();
-    ca.far_acc = P.far_acc;
+    ca.near_items = P.dnear;
+    ca.n_near = (int)P.hnear.size();
+    ca.leaf_sum = P.leaf_sum;
+    ca.leaf_fmx = P.leaf_fmx;
+    ca.leaf_n_close = P.leaf_n_close;
+    ca.leaf_close = P.leaf_close;
     ca.far_s2f = P.far_s2f;
     ca.fix_list = P.fix_list;
     ca.fix_part = P.fix_part;
@@ -1285,7 +1310,8 @@ int upload_state(sg_ctx* ctx, Problem& P, const double* pos, const double* vel,
         CK(cudaMemsetAsync(P.ran, 0, sizeof(int) * (size_t)std::max(P.n_clouds, 1), ctx->stream));
     if (P.sorted && resort) {
         for (int c = 0; c < P.n_clouds; c++)
-            kd_order(pos, P.hc[c].off, P.hc[c].n, P.perm.data() + P.hc[c].off);
+            if (P.variant != SG_C32_FAR_ONCE || P.hc[c].leafs)
+                kd_order(pos, P.hc[c].off, P.hc[c].n, P.perm.data() + P.hc[c].off);
         CK(cudaMemcpyAsync(P.dperm, P.perm.data(), sizeof(int) * N, cudaMemcpyHostToDevice,
                            ctx->stream));
     }
@@ -1360,6 +1386,7 @@ int solo_prepare(sg_ctx* ctx, int n, int precision, const sg_field_params& fp) {
         P.counts.assign(1, n);
         P.precision = precision;
         P.variant = auto_variant(P.counts, ctx->c32_variant, false);
+        P.leaf_min = ctx->c32_variant == SG_C32_FAR_ONCE ? 0 : kLeafMin;
         P.hc.assign(1, SgCloud());
         P.hc[0].fp = fp;
         plan(P, ctx->n_sm);
@@ -1552,6 +1579,7 @@ int sg_batch_create(sg_ctx* ctx, int n_clouds, const int* counts, const sg_field
     P.counts.assign(counts, counts + n_clouds);
     P.precision = precision;
     P.variant = auto_variant(P.counts, ctx->c32_variant, true);
+    P.leaf_min = ctx->c32_variant == SG_C32_FAR_ONCE ? 0 : kLeafMin;
     P.method = op[0].method == 0 ? 5 : op[0].method;
     P.hc.assign(n_clouds, SgCloud());
     for (int c = 0; c < n_clouds; c++) P.hc[c].fp = fp[c];

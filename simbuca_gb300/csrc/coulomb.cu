@@ -532,14 +532,15 @@ __device__ __forceinline__ void fold_partials(const f2* ax, const f2* ay, const 
     }
 }
 
-// ---- k-d ordered clouds, far leaf pairs once (shape 17) -------------------------------
-// A leaf pair farther apart than d_far is summed from the high parts for both leaves at
-// once (far_warp); the near ones, 5 % of the pairs of a 65,536-ion cloud, keep
-// the float-float differences, close pairs and conditioning of the kernels above, every
-// ordered pair (near_block).
+// ---- k-d ordered clouds, leaf pairs once (shape 17) -----------------------------------
+// Every unordered pair of 128-ion leaves is evaluated once, for both leaves, by one warp.
+// A pair of leaves farther apart than d_far is summed from the high parts (far_warp); a near
+// one, 5 % of the pairs of a 65,536-ion cloud and 36 % of a 4,000-ion one, keeps the
+// float-float differences, the capped close pairs and the conditioning of the kernels
+// above (near_warp).  Both sides' sums go to 64-bit fixed-point accumulators.
 
-// The near leaves of every leaf, in order: one warp per leaf of the batch; lists[leaf]
-// holds cap entries, counts[leaf] of them used.
+// The near leaves J >= I of every leaf I, in order (I itself first): one warp per leaf of
+// the batch; lists[leaf] holds cap entries, counts[leaf] of them used.
 __global__ void __launch_bounds__(128) near_list_kernel(const SgCloud* __restrict__ clouds,
                                                         const SgCtrl* __restrict__ ctrl,
                                                         const int* __restrict__ leaf_cloud,
@@ -551,6 +552,7 @@ __global__ void __launch_bounds__(128) near_list_kernel(const SgCloud* __restric
     const int leaf = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (leaf >= n_leaves) return;
     const int c = leaf_cloud[leaf];
+    if (c < 0) return;
     if (ctrl != nullptr && (ctrl[c].done || ctrl[c].hold || ctrl[c].status != SG_OK)) return;
     const SgCloud& cl = clouds[c];
     const int nt = (cl.npad + SG_TILE - 1) / SG_TILE, own = leaf - cl.tile0;
@@ -559,7 +561,7 @@ __global__ void __launch_bounds__(128) near_list_kernel(const SgCloud* __restric
     for (int q = 0; q < 6; q++) ib[q] = bbox[8 * (size_t)leaf + q];
     unsigned short* L = lists + (size_t)leaf * cap;
     int m = 0;
-    for (int j0 = 0; j0 < nt; j0 += 32) {
+    for (int j0 = own; j0 < nt; j0 += 32) {
         // past the end: the last leaf again, not listed (every lane takes the same path)
         const int J = min(j0 + lane, nt - 1);
         float jb[6];
@@ -572,155 +574,6 @@ __global__ void __launch_bounds__(128) near_list_kernel(const SgCloud* __restric
         m += __popc(b);
     }
     if (lane == 0) counts[leaf] = m;
-}
-
-template <int NT, int IPT, int STAGES>
-struct NearShared {
-    float tile[STAGES][7][SG_TILE];
-    uint64_t full[STAGES];
-    uint64_t never;  // the wait test's barrier
-    float corr[6][NT * IPT];
-};
-
-// Near leaves of leaf it.i0, entries it.j0, it.j0 + it.nj, ... of its list, by a block: as
-// the sorted kernel, with the list's leaves as its j-tiles.
-template <int NT, int IPT, int STAGES>
-__device__ __forceinline__ void near_block(const float* __restrict__ c32,
-                                           const double* __restrict__ c64, const SgWorkItem& it,
-                                           const SgCloud& cl, double* __restrict__ part,
-                                           int npad_total, int* errword,
-                                           const int* __restrict__ counts,
-                                           const unsigned short* __restrict__ lists, int cap,
-                                           NearShared<NT, IPT, STAGES>& sh) {
-    constexpr int T = SG_TILE;
-    constexpr int NU = IPT == 1 ? 4 : 2;
-    float(*tile)[7][T] = sh.tile;
-    uint64_t* full = sh.full;
-    float(*corr)[NT * IPT] = sh.corr;
-    const int wtest = errword ? errword[SG_FLAG_WAIT_TILE] : 0;
-    const float wc = cl.wc;
-    const double sc = cl.psc;
-    const int j_real_end = cl.poff + cl.n, j_end = cl.poff + cl.npad;
-    const int tid = threadIdx.x;
-    const size_t NP = (size_t)npad_total;
-    const int leaf = (it.i0 - cl.poff) / T;
-    const unsigned short* L = lists + (size_t)(cl.tile0 + leaf) * cap + it.j0;
-    // entries of this item: it.j0 + t it.nj < counts
-    const int left = counts[cl.tile0 + leaf] - it.j0;
-    const int ntiles = left > 0 ? (left + it.nj - 1) / it.nj : 0;
-
-    int ipad[IPT];
-    f2 xh[IPT], yh[IPT], zh[IPT], xl[IPT], yl[IPT], zl[IPT];
-#pragma unroll
-    for (int k = 0; k < IPT; k++) {
-        const int li = IPT * tid + k;
-        const int ii = it.i0 + (li < it.ni ? li : 0);
-        ipad[k] = li < it.ni ? ii : -1;
-        const float a = c32[ii], b = c32[NP + ii], c = c32[2 * NP + ii], d = c32[4 * NP + ii],
-                    e = c32[5 * NP + ii], f = c32[6 * NP + ii];
-        xh[k] = pk(a, a);
-        yh[k] = pk(b, b);
-        zh[k] = pk(c, c);
-        xl[k] = pk(d, d);
-        yl[k] = pk(e, e);
-        zl[k] = pk(f, f);
-#pragma unroll
-        for (int q = 0; q < 6; q++) corr[q][li] = 0.f;
-    }
-    float ks[IPT][3], kc[IPT][3], s2[IPT], s2f[IPT], fmx[IPT];
-#pragma unroll
-    for (int k = 0; k < IPT; k++) {
-        s2[k] = s2f[k] = fmx[k] = 0.f;
-#pragma unroll
-        for (int c = 0; c < 3; c++) ks[k][c] = kc[k][c] = 0.f;
-    }
-    bool ok = true;
-    if (tid == 0) {
-        for (int s = 0; s < STAGES; s++) mbar_init(&full[s], 1);
-        mbar_init(&sh.never, 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    // prologue: fill the ring
-    if (tid == 0) {
-        for (int s = 0; s < STAGES && s < ntiles; s++) {
-            const int j0 = cl.poff + (int)L[s * it.nj] * T;
-            const uint32_t bytes = (uint32_t)min(T, j_end - j0) * 4u;
-            mbar_arrive_tx(&full[s], 7u * bytes);
-            for (int a = 0; a < 7; a++)
-                bulk_g2s(&tile[s][a][0], c32 + a * NP + j0, bytes, &full[s]);
-        }
-    }
-    __syncwarp();
-    const f2 tiny2 = pk(kTiny, kTiny);
-    const int flush_len = (cl.npad <= 2048) ? 16 : 32;
-    for (int t = 0; t < ntiles; t++) {
-        const int s = t % STAGES;
-        const int J = L[t * it.nj];
-        const int j0 = cl.poff + J * T;
-        const int len = min(T, j_end - j0);
-        bool arrived = mbar_wait(&full[s], (uint32_t)((t / STAGES) & 1));
-        if (t + 1 == wtest) arrived = wait_test(&sh.never, errword) && arrived;
-        if (!__syncthreads_and(arrived)) {  // block-uniform decision
-            ok = false;
-            if (tid == 0) {
-                atomicExch(errword, SG_TIMEOUT);
-                // drain the copies still in flight (tiles t .. t+STAGES-1), bounded
-                for (int u = t; u < ntiles && u < t + STAGES; u++)
-                    (void)mbar_wait(&full[u % STAGES], (uint32_t)((u / STAGES) & 1));
-            }
-            __syncthreads();
-            break;
-        }
-        float y3max[IPT];
-#pragma unroll
-        for (int k = 0; k < IPT; k++) y3max[k] = 0.f;
-        const float* tx = tile[s][0];
-        const float* ty = tile[s][1];
-        const float* tz = tile[s][2];
-        const float* tq = tile[s][3];
-        const float* txl = tile[s][4];
-        const float* tyl = tile[s][5];
-        const float* tzl = tile[s][6];
-        const bool diag = J == leaf;
-        const bool noq = cl.quniform && j0 + len <= j_real_end;
-        for (int jb = 0; jb < len; jb += flush_len) {
-            const int je = min(len, jb + flush_len);
-            f2 ax[IPT], ay[IPT], az[IPT];
-#pragma unroll
-            for (int k = 0; k < IPT; k++) ax[k] = ay[k] = az[k] = 0ull;
-            if (!diag && noq)
-                tile_pairs<IPT, false, true, NU>(tx, ty, tz, tq, txl, tyl, tzl, jb, je, j0, ipad, xh,
-                                             yh, zh, xl, yl, zl, tiny2, wc, ax, ay, az, y3max);
-            else if (!diag)
-                tile_pairs<IPT, false, false, NU>(tx, ty, tz, tq, txl, tyl, tzl, jb, je, j0, ipad, xh, yh,
-                                       zh, xl, yl, zl, tiny2, wc, ax, ay, az, y3max);
-            else
-                tile_pairs<IPT, true, false, NU>(tx, ty, tz, tq, txl, tyl, tzl, jb, je, j0, ipad, xh, yh,
-                                      zh, xl, yl, zl, tiny2, wc, ax, ay, az, y3max);
-            fold_partials<IPT, false>(ax, ay, az, ks, kc, s2, s2f, true);
-            fold_close<IPT>(tile[s], jb, je, j0, ipad, xh, yh, zh, xl, yl, zl, wc, sc, c64,
-                            npad_total, corr, y3max, fmx, [tid](int k) { return IPT * tid + k; });
-        }
-        __syncthreads();  // every thread is done with ring slot s
-        if (tid == 0 && t + STAGES < ntiles) {
-            fence_proxy_async();
-            const int jn = cl.poff + (int)L[(t + STAGES) * it.nj] * T;
-            const uint32_t bytes = (uint32_t)min(T, j_end - jn) * 4u;
-            mbar_arrive_tx(&full[s], 7u * bytes);
-            for (int a = 0; a < 7; a++)
-                bulk_g2s(&tile[s][a][0], c32 + a * NP + jn, bytes, &full[s]);
-        }
-        __syncwarp();
-    }
-    if (!ok) return;
-    float* P = reinterpret_cast<float*>(part) + (size_t)it.slot * SG_PART_F32 * NP;
-#pragma unroll
-    for (int k = 0; k < IPT; k++) {
-        if (ipad[k] < 0) continue;
-        store_partial(P, NP, ipad[k], ks[k], kc[k], corr, IPT * tid + k, s2[k], fmx[k]);
-        P[7 * NP + ipad[k]] = 0.f;  // the far estimate is kept apart
-    }
 }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -741,6 +594,23 @@ __device__ __forceinline__ long long far_fixed(float h, float l, float fs) {
     return ((long long)hi << 30) + lo;
 }
 
+// Accumulators of a batch in shape 17, per padded ion; all zero between calls.
+struct LeafAcc {
+    unsigned long long* sum;  // [5][Npad]: x, y, z; s2 of the near leaves; s2f of the far ones
+    int* fmx;                 // strongest near term (1/r^3 below the cap, float bits); kPoison
+    int* n_close;             // close pairs of the ion, and the first kCloseCap partners
+    int* close;               // [Npad][kCloseCap]
+};
+constexpr int kCloseCap = SG_CLOSE_CAP;
+constexpr int kPoison = 0x7fffffff;  // a sum that is not finite: fixed point cannot hold it
+
+// Float-float sum (h, l) of component c of ion ig into the accumulators.
+__device__ __forceinline__ void leaf_add(const LeafAcc& A, size_t NP, int c, int ig, float h,
+                                         float l, float fs) {
+    if (!(fabsf(h) <= 3.402823466e38f)) A.fmx[ig] = kPoison;
+    atomicAdd(A.sum + c * NP + ig, (unsigned long long)far_fixed(h, l, fs));
+}
+
 // Far pairs of leaf I against up to 32 leaves J > I, by one warp, each unordered pair
 // once, from the high parts.  Bound by the FMA pipe: 8 packed FP32x2 operations shared by
 // the two ions and 3 for each, 7 lane operations per ordered pair where summing each
@@ -757,9 +627,8 @@ __device__ __forceinline__ long long far_fixed(float h, float l, float fs) {
 //
 // Register reads bound it before the FMA pipe: a packed FMA of three distinct operands
 // takes 3.1 - 3.6 cycles of its SM sub-partition, one of two 2.0 (measured), which makes
-// the pair 17 cycles, not 14.  Near and far leaves of a 65,536-ion cloud: 1,316 us per
-// call, 1,755 with the ordered pairs of shape 9; 524,288 ions 76.0 ms, 106.9.
-constexpr int kFarWarps = 4;
+// the pair 17 cycles, not 14.  Near and far leaves of a 65,536-ion cloud: 1,245 us per
+// call, 1,755 with the ordered pairs of shape 9; 500,009 ions 67.9 ms, 98.
 constexpr int kFarFold = 8;  // steps between j-side folds
 template <bool S2F>
 struct __align__(16) FarWarpShared {
@@ -878,9 +747,8 @@ __device__ __forceinline__ void far_leaf(const float (*tj)[SG_TILE], FarWarpShar
 
 template <bool S2F>
 __device__ __forceinline__ void far_warp(const float* __restrict__ c32, const SgFarItem& it,
-                                         const SgCloud& cl, unsigned long long* __restrict__ acc,
-                                         int npad_total, const float* __restrict__ bbox,
-                                         FarWarpShared<S2F>& sh) {
+                                         const SgCloud& cl, const LeafAcc& acc, int npad_total,
+                                         const float* __restrict__ bbox, FarWarpShared<S2F>& sh) {
     const int lane = threadIdx.x & 31;
     const size_t NP = (size_t)npad_total;
     // far leaves of the item: a lane each
@@ -946,10 +814,8 @@ __device__ __forceinline__ void far_warp(const float* __restrict__ c32, const Sg
             const int p = lane + 32 * k, jg = j0 + p;
             if (jg >= cl.poff + cl.n) continue;
 #pragma unroll
-            for (int c = 0; c < 3; c++)
-                atomicAdd(acc + c * NP + jg,
-                          (unsigned long long)far_fixed(-sh.S[c][p], sh.C[c][p], fs));
-            if (S2F) atomicAdd(acc + 3 * NP + jg, (unsigned long long)far_fixed(sh.s2[p], 0.f, fs2));
+            for (int c = 0; c < 3; c++) leaf_add(acc, NP, c, jg, -sh.S[c][p], sh.C[c][p], fs);
+            if (S2F) leaf_add(acc, NP, 4, jg, sh.s2[p], 0.f, fs2);
         }
         __syncwarp();
         slot ^= 1;
@@ -959,49 +825,263 @@ __device__ __forceinline__ void far_warp(const float* __restrict__ c32, const Sg
     for (int k = 0; k < 4; k++) {
         const int p = lane + 32 * k;
 #pragma unroll
-        for (int c = 0; c < 3; c++)
-            atomicAdd(acc + c * NP + i0 + p,
-                      (unsigned long long)far_fixed(sh.IS[c][p], -sh.IC[c][p], fs));
-        if (S2F)
-            atomicAdd(acc + 3 * NP + i0 + 4 * lane + k, (unsigned long long)far_fixed(s2i[k], 0.f, fs2));
+        for (int c = 0; c < 3; c++) leaf_add(acc, NP, c, i0 + p, sh.IS[c][p], -sh.IC[c][p], fs);
+        if (S2F) leaf_add(acc, NP, 4, i0 + 4 * lane + k, s2i[k], 0.f, fs2);
     }
 }
 
-// Near blocks [0, n_near), then blocks of four far warps: one launch, so that the far
-// warps fill the SMs as the near blocks run out.
-constexpr int kLeafThreads = 32 * kFarWarps;
-template <bool S2F>
-__global__ void __launch_bounds__(kLeafThreads, 5) coulomb_leaf_kernel(
-    const float* __restrict__ c32, const double* __restrict__ c64,
-    const SgWorkItem* __restrict__ items, int n_near, const SgFarItem* __restrict__ far_items,
-    int n_far, const SgCloud* __restrict__ clouds, const SgCtrl* __restrict__ ctrl,
-    double* __restrict__ part, unsigned long long* __restrict__ acc, int npad_total, int* errword,
-    const float* __restrict__ bbox, const int* __restrict__ counts,
-    const unsigned short* __restrict__ lists, int cap) {
-    sg_griddep_wait();
-    typedef NearShared<kLeafThreads, 1, 3> Near;
-    typedef FarWarpShared<S2F> Far;
-    constexpr size_t kBytes = sizeof(Near) > kFarWarps * sizeof(Far) ? sizeof(Near)
-                                                                      : kFarWarps * sizeof(Far);
-    __shared__ __align__(128) unsigned char raw[kBytes];
-    if ((int)blockIdx.x < n_near) {
-        const SgWorkItem it = items[blockIdx.x];
-        if (ctrl != nullptr &&
-            (ctrl[it.cloud].done || ctrl[it.cloud].hold || ctrl[it.cloud].status != SG_OK))
-            return;
-        near_block<kLeafThreads, 1, 3>(c32, c64, it, clouds[it.cloud], part, npad_total, errword,
-                                       counts, lists, cap, *reinterpret_cast<Near*>(raw));
-        return;
+// Half a near leaf I (64 ions, two per lane) against near leaves J >= I, by one warp, each
+// unordered pair once: the j-pairs pass through the lanes as in far_leaf.  Per packed pair
+// of j-ions and i-ion 14 FP32x2 operations serve both sides and 3 each side, where the
+// ordered pairs of the plain kernels take 17 each.  60 clouds of 4,096 ions (36 % of their
+// pairs near): 485 us with ordered near pairs, 400 so.
+//
+// A close pair enters both sums capped (1/r^3 <= wc) and is noted in the lists of both ions:
+// the sums' reduction adds its exact term minus the capped one, in the order of the
+// partners' indices.  An ion with more close pairs than a list holds gets its FP64 row.
+struct __align__(16) NearWarpShared {
+    float j[2][7][SG_TILE];              // leaf J: x, y, z, q, low parts; two in flight
+    float S[3][SG_TILE], C[3][SG_TILE];  // leaf J's Kahan pairs
+    float s2[SG_TILE], M[SG_TILE];       // ... conditioning: sum of squares, strongest term
+};
+constexpr int kNearStep = 8;  // steps per FP32 partial sum: 16 terms on either side
+
+struct NearSide {
+    f2 x[6][2], q[2];  // the lane's two ions, each value twice
+    float ks[2][3], kc[2][3], s2[2], fmx[2];
+};
+
+template <bool NOQ, bool TWO>
+__device__ __forceinline__ void near_leaf(const float (*tj)[SG_TILE], NearWarpShared& sh,
+                                          NearSide& w, float wc, int i0, int j0,
+                                          const LeafAcc& acc) {
+    const int lane = threadIdx.x & 31, next = (lane + 1) & 31;
+    const f2 tiny2 = pk(kTiny, kTiny);
+#pragma unroll 1
+    for (int g = 0; g < 64; g += kNearStep) {
+        const int sub = g >> 5, s0 = g & 31;  // half-leaf of J, first step in it
+        f2 a[3][2], b[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) a[c][0] = a[c][1] = b[c] = 0ull;
+        float jm0 = 0.f, jm1 = 0.f;
+        unsigned close = 0u;
+#pragma unroll
+        for (int u = 0; u < kNearStep; u++) {
+            const int p = 64 * sub + 2 * ((lane + s0 + u) & 31);
+            const f2 X = *reinterpret_cast<const f2*>(&tj[0][p]);
+            const f2 Y = *reinterpret_cast<const f2*>(&tj[1][p]);
+            const f2 Z = *reinterpret_cast<const f2*>(&tj[2][p]);
+            const f2 Q = NOQ ? 0ull : *reinterpret_cast<const f2*>(&tj[3][p]);
+            const f2 XL = *reinterpret_cast<const f2*>(&tj[4][p]);
+            const f2 YL = *reinterpret_cast<const f2*>(&tj[5][p]);
+            const f2 ZL = *reinterpret_cast<const f2*>(&tj[6][p]);
+            if (TWO && u > 0) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) b[c] = shfl2(b[c], next);
+                jm0 = __shfl_sync(0xffffffffu, jm0, next);
+                jm1 = __shfl_sync(0xffffffffu, jm1, next);
+            }
+            f2 t[3];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const f2 dx = add2(sub2(X, w.x[0][k]), sub2(XL, w.x[3][k]));
+                const f2 dy = add2(sub2(Y, w.x[1][k]), sub2(YL, w.x[4][k]));
+                const f2 dz = add2(sub2(Z, w.x[2][k]), sub2(ZL, w.x[5][k]));
+                f2 r2 = fma2(dx, dx, tiny2);
+                r2 = fma2(dy, dy, r2);
+                r2 = fma2(dz, dz, r2);
+                float ra, rb, ua, ub;
+                upk(r2, ra, rb);
+                const f2 y = pk(rsqrt_approx(ra), rsqrt_approx(rb));
+                upk(mul2(mul2(y, y), y), ua, ub);
+                // the self pair (dx = 0) counts as close: no term, not listed
+                const bool ca = ua > wc, cb = ub > wc;
+                if (ca) close |= 1u << (4 * u + 2 * k);
+                if (cb) close |= 2u << (4 * u + 2 * k);
+                const float m0 = ca ? 0.f : ua, m1 = cb ? 0.f : ub;
+                w.fmx[k] = fmaxf(w.fmx[k], fmaxf(m0, m1));
+                const f2 cap = pk(fminf(ua, wc), fminf(ub, wc));
+                const f2 wi = NOQ ? cap : mul2(Q, cap);
+                a[0][k] = fma2(wi, dx, a[0][k]);
+                a[1][k] = fma2(wi, dy, a[1][k]);
+                a[2][k] = fma2(wi, dz, a[2][k]);
+                if (TWO) {
+                    jm0 = fmaxf(jm0, m0);
+                    jm1 = fmaxf(jm1, m1);
+                    const f2 wj = NOQ ? cap : mul2(w.q[k], cap);
+                    t[0] = k ? fma2(wj, dx, t[0]) : mul2(wj, dx);
+                    t[1] = k ? fma2(wj, dy, t[1]) : mul2(wj, dy);
+                    t[2] = k ? fma2(wj, dz, t[2]) : mul2(wj, dz);
+                }
+            }
+            if (TWO)
+#pragma unroll
+                for (int c = 0; c < 3; c++) b[c] = u ? add2(b[c], t[c]) : t[c];  // subtracted in the end
+        }
+        if (TWO) {  // j-side fold: the pair this lane has now
+            const int p = 64 * sub + 2 * ((lane + s0 + kNearStep - 1) & 31);
+            f2* S2 = reinterpret_cast<f2*>(&sh.s2[p]);
+            *S2 = fma2(b[0], b[0], fma2(b[1], b[1], fma2(b[2], b[2], s0 ? *S2 : 0ull)));
+            sh.M[p] = s0 ? fmaxf(sh.M[p], jm0) : jm0;
+            sh.M[p + 1] = s0 ? fmaxf(sh.M[p + 1], jm1) : jm1;
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                f2* S = reinterpret_cast<f2*>(&sh.S[c][p]);
+                f2* C = reinterpret_cast<f2*>(&sh.C[c][p]);
+                if (s0 == 0) {  // every pair's first fold
+                    *S = b[c];
+                    *C = 0ull;
+                } else {
+                    const f2 s = *S, y = sub2(b[c], *C), t = add2(s, y);
+                    *C = sub2(sub2(t, s), y);
+                    *S = t;
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            float t[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                float lo, hi;
+                upk(a[c][k], lo, hi);
+                t[c] = __fadd_rn(lo, hi);
+                kahan_add(w.ks[k][c], w.kc[k][c], t[c]);
+            }
+            w.s2[k] = fmaf(t[0], t[0], fmaf(t[1], t[1], fmaf(t[2], t[2], w.s2[k])));
+        }
+        while (close) {
+            const int bit = __ffs(close) - 1;
+            close &= close - 1u;
+            const int i = i0 + 2 * lane + ((bit >> 1) & 1);
+            const int j = j0 + 64 * sub + 2 * ((lane + s0 + (bit >> 2)) & 31) + (bit & 1);
+            if (i == j) continue;
+            int at = atomicAdd(acc.n_close + i, 1);
+            if (at < kCloseCap) acc.close[(size_t)i * kCloseCap + at] = j;
+            if (!TWO) continue;
+            at = atomicAdd(acc.n_close + j, 1);
+            if (at < kCloseCap) acc.close[(size_t)j * kCloseCap + at] = i;
+        }
+        __syncwarp();  // the j-pair moves on to another lane
     }
-    const int warp = threadIdx.x >> 5;
-    const int item = ((int)blockIdx.x - n_near) * kFarWarps + warp;
-    if (item >= n_far) return;  // warps are independent here
-    const SgFarItem it = far_items[item];
+}
+
+// Near item: leaf it.leaf >> 1, its half it.leaf & 1, entries it.j0, it.j0 + it.n, ... of the
+// leaf's near list.
+__device__ __forceinline__ void near_warp(const float* __restrict__ c32, const SgFarItem& it,
+                                          const SgCloud& cl, const LeafAcc& acc, int npad_total,
+                                          const int* __restrict__ counts,
+                                          const unsigned short* __restrict__ lists, int cap,
+                                          NearWarpShared& sh) {
+    const int lane = threadIdx.x & 31;
+    const size_t NP = (size_t)npad_total;
+    const int leaf = it.leaf >> 1, i0 = cl.poff + leaf * SG_TILE + (it.leaf & 1) * (SG_TILE / 2);
+    const int end = cl.poff + cl.n, pend = cl.poff + cl.npad;
+    const int count = counts[cl.tile0 + leaf];
+    if (i0 >= end || it.j0 >= count) return;
+    const unsigned short* L = lists + (size_t)(cl.tile0 + leaf) * cap;
+    NearSide w;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = i0 + 2 * lane + k;
+        const bool in = i < pend;  // past a cloud's last leaf: far from everything, no charge
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            const float x = in ? c32[(c < 3 ? c : c + 1) * NP + i] : c < 3 ? 3.0e4f : 0.f;
+            w.x[c][k] = pk(x, x);
+        }
+        const float q = in ? c32[3 * NP + i] : 0.f;
+        w.q[k] = pk(q, q);
+        w.s2[k] = w.fmx[k] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 3; c++) w.ks[k][c] = w.kc[k][c] = 0.f;
+    }
+    auto fetch = [&](int J, int slot) {
+        const int j0 = cl.poff + J * SG_TILE, len = min(SG_TILE, pend - j0);
+        float(*t)[SG_TILE] = sh.j[slot];
+#pragma unroll
+        for (int a = 0; a < 7; a++) {
+            if (4 * lane < len)
+                cp_async16(&t[a][4 * lane], c32 + a * NP + j0 + 4 * lane);
+            else
+#pragma unroll
+                for (int q = 0; q < 4; q++) t[a][4 * lane + q] = a < 3 ? 2.0e4f : 0.f;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int slot = 0;
+    fetch(L[it.j0], 0);
+    for (int e = it.j0; e < count; e += it.n) {
+        const int J = L[e];
+        if (e + it.n < count) {
+            fetch(L[e + it.n], slot ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncwarp();
+        const int j0 = cl.poff + J * SG_TILE;
+        const bool noq = cl.quniform && j0 + SG_TILE <= end;
+        if (J == leaf) {  // every ordered pair of the half, one side
+            if (noq)
+                near_leaf<true, false>(sh.j[slot], sh, w, cl.wc, i0, j0, acc);
+            else
+                near_leaf<false, false>(sh.j[slot], sh, w, cl.wc, i0, j0, acc);
+        } else {
+            if (noq)
+                near_leaf<true, true>(sh.j[slot], sh, w, cl.wc, i0, j0, acc);
+            else
+                near_leaf<false, true>(sh.j[slot], sh, w, cl.wc, i0, j0, acc);
+#pragma unroll 1
+            for (int k = 0; k < 4; k++) {
+                const int p = lane + 32 * k, jg = j0 + p;
+                if (jg >= end) continue;
+#pragma unroll
+                for (int c = 0; c < 3; c++)
+                    leaf_add(acc, NP, c, jg, -sh.S[c][p], sh.C[c][p], cl.far_fs);
+                leaf_add(acc, NP, 3, jg, sh.s2[p], 0.f, cl.near_fs2);
+                atomicMax(acc.fmx + jg, __float_as_int(sh.M[p]));
+            }
+        }
+        __syncwarp();
+        slot ^= 1;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = i0 + 2 * lane + k;
+        if (i >= end) continue;
+#pragma unroll
+        for (int c = 0; c < 3; c++) leaf_add(acc, NP, c, i, w.ks[k][c], -w.kc[k][c], cl.far_fs);
+        leaf_add(acc, NP, 3, i, w.s2[k], 0.f, cl.near_fs2);
+        atomicMax(acc.fmx + i, __float_as_int(w.fmx[k]));
+    }
+}
+
+// A near item or a far item per one-warp block: one launch, so that the far items fill the
+// SMs as the near ones run out.  In blocks of four warps the slots of a block's finished
+// warps waited for its longest item: 20,001 / 65,536 / 200,000 ions 160 / 1,302 / 11,682 us
+// per call with four, 151 / 1,245 / 11,190 with one.
+template <bool S2F>
+__global__ void __launch_bounds__(32, 19) coulomb_leaf_kernel(
+    const float* __restrict__ c32, const SgFarItem* __restrict__ near_items, int n_near,
+    const SgFarItem* __restrict__ far_items, int n_far, const SgCloud* __restrict__ clouds,
+    const SgCtrl* __restrict__ ctrl, LeafAcc acc, int npad_total, const float* __restrict__ bbox,
+    const int* __restrict__ counts, const unsigned short* __restrict__ lists, int cap) {
+    sg_griddep_wait();
+    typedef FarWarpShared<S2F> Far;
+    constexpr size_t kWarp = sizeof(NearWarpShared) > sizeof(Far) ? sizeof(NearWarpShared) : sizeof(Far);
+    __shared__ __align__(16) unsigned char raw[kWarp];
+    const bool near = (int)blockIdx.x < n_near;
+    const SgFarItem it = near ? near_items[blockIdx.x] : far_items[(int)blockIdx.x - n_near];
     if (ctrl != nullptr &&
         (ctrl[it.cloud].done || ctrl[it.cloud].hold || ctrl[it.cloud].status != SG_OK))
         return;
-    far_warp<S2F>(c32, it, clouds[it.cloud], acc, npad_total, bbox,
-                  reinterpret_cast<Far*>(raw)[warp]);
+    if (near)
+        near_warp(c32, it, clouds[it.cloud], acc, npad_total, counts, lists, cap,
+                  *reinterpret_cast<NearWarpShared*>(raw));
+    else
+        far_warp<S2F>(c32, it, clouds[it.cloud], acc, npad_total, bbox,
+                      *reinterpret_cast<Far*>(raw));
 }
 
 template <int NT, int IPT, int MINB, int STAGES, int TJ = SG_TILE, int FU = 0, bool S2F = true>
@@ -1331,25 +1411,30 @@ struct Corr3 {
 // Block-wide sum of one value per thread and component; the result is thread 0's.
 template <int NTH>
 __device__ Corr3 block_sum3(double ax, double ay, double az, FixupShared<NTH>& sh) {
+    // An FP64 addition takes a warp 64 cycles whatever its lanes hold: 32 lanes x 3
+    // components in six (the upper half-warp takes y while the lower sums x, then every other
+    // 8 lanes z), the warps' parts in three.
+    static_assert(NTH == 256, "eight warps");
     const int li = threadIdx.x, warp = li >> 5, lane = li & 31;
-    for (int o = 16; o > 0; o >>= 1) {
-        ax += __shfl_down_sync(0xffffffffu, ax, o);
-        ay += __shfl_down_sync(0xffffffffu, ay, o);
-        az += __shfl_down_sync(0xffffffffu, az, o);
-    }
-    if (lane == 0) {
-        sh.wsum[warp][0] = ax;
-        sh.wsum[warp][1] = ay;
-        sh.wsum[warp][2] = az;
-    }
+    const bool up = lane & 16, odd = lane & 8;
+    double a = up ? ay : ax;
+    a += __shfl_xor_sync(0xffffffffu, up ? ax : ay, 16);
+    az += __shfl_xor_sync(0xffffffffu, az, 16);
+    double v = odd ? az : a;
+    v += __shfl_xor_sync(0xffffffffu, odd ? a : az, 8);
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) sh.wsum[warp][0] = v;
+    if (lane == 16) sh.wsum[warp][1] = v;
+    if (lane == 8) sh.wsum[warp][2] = v;
     __syncthreads();
     Corr3 r{0.0, 0.0, 0.0};
-    if (li == 0)
-        for (int w = 0; w < NTH / 32; w++) {
-            r.x += sh.wsum[w][0];
-            r.y += sh.wsum[w][1];
-            r.z += sh.wsum[w][2];
-        }
+    if (warp == 0) {
+        v = lane < 24 ? sh.wsum[lane & 7][lane >> 3] : 0.0;
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 8);
+        r.x = __shfl_sync(0xffffffffu, v, 0);
+        r.y = __shfl_sync(0xffffffffu, v, 8);
+        r.z = __shfl_sync(0xffffffffu, v, 16);
+    }
     __syncthreads();
     return r;
 }
@@ -1469,10 +1554,10 @@ __device__ void fixup_ion(const SgCloud& cl, int i, int kind, const float* __res
     __syncthreads();
 }
 
-// Far accumulators of shape 17 (null for the others): [4][Npad] fixed-point sums x, y, z
-// and s2f, and the s2f of the last call that estimated it.
-struct FarSums {
-    unsigned long long* acc;
+// Shape 17's accumulators (sum null for the other shapes) and the s2f of the last call that
+// estimated it.
+struct LeafSums {
+    LeafAcc acc;
     float* s2f;
     int estimate;
 };
@@ -1486,6 +1571,54 @@ __device__ __forceinline__ ff far_value(long long v, float fs) {
     const float m = (float)(r1 >> 8), l = (float)(int)(r - ((long long)(r1 >> 8) << 16));
     const ff a = ff_two_sum(__fmul_rn(h, 1073741824.0f * inv), __fmul_rn(m, 65536.0f * inv));
     return ff_add(a, {__fmul_rn(l, inv), 0.f});
+}
+
+// The listed close pairs of ion ig (m of them, at most kCloseCap): the exact term minus the
+// capped FP32 one of each, in the order of the partners (the lists fill in any order);
+// returns the strongest capped term.
+__device__ float close_list_terms(const SgCloud& cl, int ig, int m, const int* __restrict__ list,
+                                  const float* __restrict__ c32, const double* __restrict__ c64,
+                                  size_t NP, ff& px, ff& py, ff& pz) {
+    const float xih = c32[ig], yih = c32[NP + ig], zih = c32[2 * NP + ig];
+    const float xil = c32[4 * NP + ig], yil = c32[5 * NP + ig], zil = c32[6 * NP + ig];
+    float fmx = 0.f;
+    int done = -1;
+    for (int k = 0; k < m; k++) {
+        int j = 0x7fffffff;
+        for (int q = 0; q < m; q++) {
+            const int l = list[q];
+            if (l > done && l < j) j = l;
+        }
+        done = j;
+        const float xjh = c32[j], yjh = c32[NP + j], zjh = c32[2 * NP + j], q = c32[3 * NP + j];
+        const float xjl = c32[4 * NP + j], yjl = c32[5 * NP + j], zjl = c32[6 * NP + j];
+        if (q == 0.f) continue;
+        const PairF pr = pair_f32(xjh, yjh, zjh, xjl, yjl, zjl, xih, yih, zih, xil, yil, zil);
+        fmx = fmaxf(fmx, capped_term_y3(pr.y3, cl.wc));
+        const float wf = __fmul_rn(q, cl.wc);
+        ff dx, dy, dz;
+        if (pr.y3 <= kVeryClose) {
+            close_term_ff(ff_diff(xjh, xjl, xih, xil), ff_diff(yjh, yjl, yih, yil),
+                          ff_diff(zjh, zjl, zih, zil), q, wf, pr, dx, dy, dz);
+        } else {
+            const double rx = c64[ig] - c64[j], ry = c64[NP + ig] - c64[NP + j],
+                         rz = c64[2 * NP + ig] - c64[2 * NP + j];
+            const double w = c64[3 * NP + j] * inv_r3_fp64(rx * rx + ry * ry + rz * rz) / cl.psc;
+            const double c0 = w * rx - (double)wf * (double)pr.dx,
+                         c1 = w * ry - (double)wf * (double)pr.dy,
+                         c2 = w * rz - (double)wf * (double)pr.dz;
+            dx.h = (float)c0;
+            dx.l = (float)(c0 - (double)dx.h);
+            dy.h = (float)c1;
+            dy.l = (float)(c1 - (double)dy.h);
+            dz.h = (float)c2;
+            dz.l = (float)(c2 - (double)dz.h);
+        }
+        px = ff_add(px, dx);
+        py = ff_add(py, dy);
+        pz = ff_add(pz, dz);
+    }
+    return fmx;
 }
 
 // The G threads of a row (thread li sums slots li / R, li / R + G, ... of row li % R, R
@@ -1519,7 +1652,7 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
     double* __restrict__ out, int n_total, int* __restrict__ counters,
     int* __restrict__ fix_list, const float* __restrict__ c32,
     const double* __restrict__ c64, const float* __restrict__ bbox, float* __restrict__ risk,
-    int* __restrict__ ran, const SgCheck* __restrict__ chk, int split, FarSums far) {
+    int* __restrict__ ran, const SgCheck* __restrict__ chk, int split, LeafSums leaf) {
     sg_griddep_wait();
     // this block's share of its row block: cap / split rows
     SgRowBlock rb = rows[blockIdx.x / split];
@@ -1577,22 +1710,31 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
                 s2f += v[7];
             }
             const double sc = cl.psc;
-            if (far.acc != nullptr) {
-                // the far leaves' sums: taken and cleared for the next call
-                unsigned long long* A = far.acc + ig;
-                const ff fx = far_value((long long)A[0], cl.far_fs),
-                         fy = far_value((long long)A[NP], cl.far_fs),
-                         fz = far_value((long long)A[2 * NP], cl.far_fs);
-                A[0] = A[NP] = A[2 * NP] = 0ull;
-                px = ff_add(px, fx);
-                py = ff_add(py, fy);
-                pz = ff_add(pz, fz);
-                if (far.estimate) {
-                    const ff e = far_value((long long)A[3 * NP], cl.far_fs2);
-                    A[3 * NP] = 0ull;
-                    far.s2f[ig] = e.h;
+            bool many = false;
+            if (cl.leafs) {
+                // the leaf pairs' sums: taken and cleared for the next call
+                unsigned long long* A = leaf.acc.sum + ig;
+                px = far_value((long long)A[0], cl.far_fs);
+                py = far_value((long long)A[NP], cl.far_fs);
+                pz = far_value((long long)A[2 * NP], cl.far_fs);
+                s2 = far_value((long long)A[3 * NP], cl.near_fs2).h;
+                A[0] = A[NP] = A[2 * NP] = A[3 * NP] = 0ull;
+                if (leaf.estimate) {
+                    leaf.s2f[ig] = far_value((long long)A[4 * NP], cl.far_fs2).h;
+                    A[4 * NP] = 0ull;
                 }
-                s2f = far.s2f[ig];
+                s2f = leaf.s2f[ig];
+                const int fm = leaf.acc.fmx[ig], m = leaf.acc.n_close[ig];
+                leaf.acc.fmx[ig] = 0;
+                leaf.acc.n_close[ig] = 0;
+                float fmx = __int_as_float(fm);
+                many = m > kCloseCap;
+                if (m > 0)
+                    fmx = fmaxf(fmx, close_list_terms(cl, ig, min(m, kCloseCap),
+                                                      leaf.acc.close + (size_t)ig * kCloseCap, c32,
+                                                      c64, NP, px, py, pz));
+                s2 = conditioning_s2(s2, fmx);
+                if (fm == kPoison) px = py = pz = {__int_as_float(kPoison), 0.f};
             }
             out[i] = sc * ((double)px.h + (double)px.l);
             out[(size_t)n_total + i] = sc * ((double)py.h + (double)py.l);
@@ -1601,8 +1743,8 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
             const float pf2 = fmaf(px.h, px.h, fmaf(py.h, py.h, pz.h * pz.h));
             // the far threshold: the prior of the frame set-up, or the measured one
             const float kf2 = chk ? fminf(cl.kfar2, chk[rb.cloud].kfar2) : cl.kfar2;
-            const float kap2 = sg_kappa2(cl.npad);
-            kind = (s2 > kap2 * pf2 ? kFixNear : 0) | (s2f > kf2 * pf2 ? kFixFar : 0);
+            const float kap2 = cl.leafs ? sg_kappa2_leaf(cl.npad) : sg_kappa2(cl.npad);
+            kind = (many || s2 > kap2 * pf2 ? kFixNear : 0) | (s2f > kf2 * pf2 ? kFixFar : 0);
             if (risk != nullptr) {
                 const float pf = sqrtf(pf2);
                 risk[i] = kind ? -1.f : sqrtf(s2f) / pf;
@@ -1647,11 +1789,11 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
     if (!F32) return;
     if (!INBLOCK) {
         if (kind) {
-            // two lists: ions whose row is re-evaluated (kFixNear) from fix_list[2], the
-            // far-only ones from fix_list[2 + 2N]
-            const bool far = kind == kFixFar;
-            const int at = atomicAdd(fix_list + (far ? 1 : 0), 1);
-            const size_t base = far ? 2 + 2 * (size_t)n_total : 2;
+            // three lists: ions whose row is re-evaluated (kFixNear), the far-only ones, and
+            // the rows of small clouds
+            const int l = kind == kFixFar ? 1 : cl.npad <= SG_SMALL_ROW ? 2 : 0;
+            const int at = atomicAdd(fix_list + l, 1);
+            const size_t base = 4 + 2 * (size_t)n_total * l;
             fix_list[base + 2 * at] = i;
             fix_list[base + 2 * at + 1] = rb.cloud | (kind << 28);
             if (counters != nullptr) atomicAdd(counters, 1);
@@ -1695,13 +1837,20 @@ __global__ void __launch_bounds__(kFixupThreads, 3) coulomb_fixup_kernel(
     __shared__ FixupShared<kFixupThreads> sh;
     __shared__ int last;
     constexpr int U = kFarChunks;
-    const int cn = fix_list[0], cf = fix_list[1];
-    const int* row_list = fix_list + 2;
-    const int* far_list = fix_list + 2 + 2 * (size_t)n_total;
+    const int cn = fix_list[0], cf = fix_list[1], cs = fix_list[2];
+    const int* row_list = fix_list + 4;
+    const int* far_list = row_list + 2 * (size_t)n_total;
+    const int* small_list = far_list + 2 * (size_t)n_total;
     const int cnc = min(cn, kChunkedCap), cfc = min(cf, kChunkedCap);
     const int u_rows = cnc * U + (cn - cnc);
-    const int units = u_rows + cfc * U + (cf - cfc);
+    const int u_all = u_rows + cfc * U + (cf - cfc), units = u_all + cs;
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        if (u >= u_all) {  // a small cloud's row: one unit
+            const int i = small_list[2 * (u - u_all)], ck = small_list[2 * (u - u_all) + 1];
+            fixup_ion<kFixupThreads>(clouds[ck & 0x0FFFFFFF], i, kFixNear, c32, c64, npad_total,
+                                     out, n_total, bbox, sh);
+            continue;
+        }
         const bool row = u < u_rows;
         const int v = row ? u : u - u_rows;
         const int nc = row ? cnc : cfc;
@@ -1716,12 +1865,6 @@ __global__ void __launch_bounds__(kFixupThreads, 3) coulomb_fixup_kernel(
         const int k = v % nc, c = v / nc;
         const int i = list[2 * k];
         const SgCloud& cl = clouds[list[2 * k + 1] & 0x0FFFFFFF];
-        if (row && cl.npad <= SG_SMALL_ROW) {  // a small cloud's row: unit 0 alone, whole
-            if (c == 0)
-                fixup_ion<kFixupThreads>(cl, i, kFixNear, c32, c64, npad_total, out, n_total,
-                                         bbox, sh);
-            continue;
-        }
         Corr3 r{0.0, 0.0, 0.0};
         if (row)
             r = fixup_row<kFixupThreads>(cl, i, c64, npad_total, c, U, sh);
@@ -1777,7 +1920,7 @@ int sg_coulomb_fp32c_ib(int variant) {
 }
 
 cudaError_t sg_launch_coulomb_fp32c(const SgCoulombArgs& a, cudaStream_t s) {
-    if (a.n_items <= 0) return cudaSuccess;
+    if (a.n_items <= 0 && a.n_near <= 0) return cudaSuccess;
     switch (a.variant) {
         case 1:
             sg_launch(coulomb_fp32c_kernel<128, 2>, a.n_items, 128, 0, s, 
@@ -1858,15 +2001,18 @@ cudaError_t sg_launch_coulomb_fp32c(const SgCoulombArgs& a, cudaStream_t s) {
                 a.c32, a.c64, a.items, a.clouds, a.ctrl, a.part, a.npad_total, a.errword, a.bbox);
             break;
         case SG_C32_FAR_ONCE:
+            if (a.n_items > 0)
+                sg_launch(coulomb_fp32c_kernel<64, 2>, a.n_items, 64, 0, s, 
+                    a.c32, a.c64, a.items, a.clouds, a.ctrl, a.part, a.npad_total, a.errword);
+            if (a.n_near <= 0) break;
             sg_launch(near_list_kernel, (a.n_leaves + 3) / 4, 128, 0, s, a.clouds, a.ctrl, a.leaf_cloud,
                       a.n_leaves, a.near_cap, a.bbox, a.near_count, a.near_list);
             {
-                const int grid = a.n_items + (a.n_far + kFarWarps - 1) / kFarWarps;
+                const LeafAcc acc{a.leaf_sum, a.leaf_fmx, a.leaf_n_close, a.leaf_close};
                 sg_launch(a.far_estimate ? coulomb_leaf_kernel<true> : coulomb_leaf_kernel<false>,
-                          grid, kLeafThreads, 0, s, a.c32, a.c64, a.items, a.n_items, a.far_items,
-                          a.n_far, a.clouds, a.ctrl, a.part, a.far_acc, a.npad_total, a.errword,
-                          a.bbox, (const int*)a.near_count, (const unsigned short*)a.near_list,
-                          a.near_cap);
+                          a.n_near + a.n_far, 32, 0, s, a.c32, a.near_items, a.n_near, a.far_items,
+                          a.n_far, a.clouds, a.ctrl, acc, a.npad_total, a.bbox,
+                          (const int*)a.near_count, (const unsigned short*)a.near_list, a.near_cap);
             }
             break;
         case 10:
@@ -1900,23 +2046,26 @@ cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* r
                                      int row_cap, int fp32c, double* out, int n_total,
                                      int* counters, cudaStream_t s) {
     if (n_rows <= 0) return cudaSuccess;
+    // leaf sums have no slots to share: a thread per row
+    const bool whole = fp32c && a.variant == SG_C32_FAR_ONCE && a.n_items <= 0 && n_total > kInBlockFixupMax;
     const int take = n_total <= kInBlockFixupMax || a.max_slots > 24 ? 16 : 64;
-    const int split = std::max(1, row_cap / take);
+    const int split = whole ? 1 : std::max(1, row_cap / take);
     if (fp32c) {
         const float* bbox = sg_variant_sorted(a.variant) ? a.bbox : nullptr;
-        FarSums far{};
-        if (a.variant == SG_C32_FAR_ONCE) far = FarSums{a.far_acc, a.far_s2f, a.far_estimate};
+        LeafSums leaf{};
+        if (a.variant == SG_C32_FAR_ONCE)
+            leaf = LeafSums{{a.leaf_sum, a.leaf_fmx, a.leaf_n_close, a.leaf_close}, a.far_s2f, a.far_estimate};
         if (n_total <= kInBlockFixupMax) {
             sg_launch(coulomb_reduce_kernel<true, true>, n_rows * split, SG_ROWS, 0, s, 
                 rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, nullptr,
-                a.c32, a.c64, bbox, a.risk, a.ran, a.chk, split, far);
+                a.c32, a.c64, bbox, a.risk, a.ran, a.chk, split, leaf);
             return cudaGetLastError();
         }
-        cudaError_t e = cudaMemsetAsync(a.fix_list, 0, 2 * sizeof(int), s);
+        cudaError_t e = cudaMemsetAsync(a.fix_list, 0, 3 * sizeof(int), s);
         if (e != cudaSuccess) return e;
         coulomb_reduce_kernel<true, false><<<n_rows * split, SG_ROWS, 0, s>>>(
             rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, a.fix_list,
-            nullptr, nullptr, nullptr, a.risk, a.ran, a.chk, split, far);
+            a.c32, a.c64, nullptr, a.risk, a.ran, a.chk, split, leaf);
         // a fixed grid that strides over however many work units there are (a batch of
         // small clouds can flag a few percent of its ions; unused blocks exit at once)
         const int grid = kFixupBlocks;
@@ -1926,7 +2075,7 @@ cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* r
     } else {
         sg_launch(coulomb_reduce_kernel<false, false>, n_rows * split, SG_ROWS, 0, s, 
             rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, nullptr,
-            nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, split, FarSums{});
+            nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, split, LeafSums{});
     }
     return cudaGetLastError();
 }

@@ -103,8 +103,9 @@ struct SgWorkItem {
     int32_t jslot, s01;  // FP64 symmetric items: j-side slot, rotation steps s0 | s1 << 16
 };
 
-// Far leaf pairs of shape 17: leaf `leaf` of the cloud against its leaves [j0, j0 + n),
-// n <= 32, j0 > leaf.
+// Leaf pairs of shape 17.  Far: leaf `leaf` of the cloud against its leaves [j0, j0 + n),
+// n <= 32, j0 > leaf.  Near: half `leaf & 1` of leaf `leaf >> 1` against entries j0, j0 + n, ...
+// of that leaf's near list.
 struct SgFarItem {
     int32_t cloud, leaf, j0, n;
 };
@@ -145,7 +146,8 @@ struct SgCloud {
     double qabs, qmax;  // sum and largest of |q / qscale|
     int32_t quniform;
     // shape 17: fixed-point scales (powers of two) of the far sums and their estimate
-    float far_fs, far_fs2;
+    float far_fs, far_fs2, near_fs2;
+    int32_t leafs;  // shape 17: k-d ordered leaf pairs (else the plain kernel)
     int32_t sym_k, sym_bands;  // FP64 symmetric items: j-tiles per item (0: ordered pairs), bands
     int32_t pad4;
 };
@@ -454,6 +456,16 @@ struct SgDpArgs {
 // most on the 65,536-ion cloud).  Their flagged rows are one work unit each.
 #define SG_SMALL_ROW 4096
 __device__ __forceinline__ float sg_kappa2(int npad) { return npad <= SG_SMALL_ROW ? 1.0f : 2.25f; }
+// k-d ordered leaves (shape 17): their partial sums are coherent, so sqrt(s2)/|P| is larger
+// for the same error.  Largest errors over 2 to 40 Gaussian and uniform clouds of a size,
+// plain order at its threshold / leaves at 1.5 / at 2: 1,000 ions 3.3e-7 / 3.6e-7 / 5.2e-7,
+// 2,000 4.0e-7 / 3.7e-7 / 3.7e-7, 4,000 4.8e-7 / 3.3e-7 / 4.0e-7, 8,000 7.1e-7 / 3.4e-7 /
+// 3.9e-7, 20,001 6.8e-7 / 3.2e-7 / 3.7e-7; the larger clouds had k-d order and 1.5 before.
+__device__ __forceinline__ float sg_kappa2_leaf(int npad) {
+    return npad <= 1024 ? 1.5625f : npad <= 24000 ? 4.0f : 2.25f;
+}
+// Close pairs listed per ion (shape 17); an ion with more gets its FP64 row.
+#define SG_CLOSE_CAP 8
 
 // ---- small batches: slot sums, flagged rows and stage in one launch (finish.cu) -------
 // Batches of up to this many ions in the plain order; larger ones have enough rows to
@@ -600,7 +612,10 @@ struct SgCoulombArgs {
     unsigned short* near_list = nullptr;
     const SgFarItem* far_items = nullptr;
     int n_far = 0;
-    unsigned long long* far_acc = nullptr;  // [4][Npad], zero between calls
+    const SgFarItem* near_items = nullptr;
+    int n_near = 0;
+    unsigned long long* leaf_sum = nullptr;  // [5][Npad] (LeafAcc), zero between calls
+    int *leaf_fmx = nullptr, *leaf_n_close = nullptr, *leaf_close = nullptr;
     float* far_s2f = nullptr;               // [Npad]
     // FP32c conditioning fix-up work list, filled by the reduction: [0] count, then
     // per flagged ion its global index and cloud (ints) and |P| in frame units
@@ -646,6 +661,7 @@ cudaError_t sg_force_check(const SgCloud* clouds, int n_clouds, int* ran, const 
 #define SG_C32_VARIANTS 18
 // shape 17: k-d order, far leaf pairs evaluated once for both leaves
 #define SG_C32_FAR_ONCE 17
+#define SG_C32_PLAIN 5  // shape of the small clouds of a batch in shape 17
 // variant 4: ions in k-d tree order, far tile pairs from the high parts only
 #define SG_C32_SORTED 4
 #define SG_C32_SORTED_LEAF 7

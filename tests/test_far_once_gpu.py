@@ -76,3 +76,57 @@ def test_batch_of_uneven_clouds(far_once):
         assert np.abs(p[at:at + n] - ps).max() <= 1e-9 * np.abs(ps).max()
         assert np.abs(v[at:at + n] - vs).max() <= 1e-9 * np.abs(vs).max()
         at += n
+
+
+@pytest.mark.parametrize("partners", [7, 8, 9, 12])
+def test_more_close_pairs_than_an_ion_lists(far_once, partners):
+    """Eight close partners of an ion are listed and re-taken one by one; an ion with more
+    gets its FP64 row, exact to FP64 rounding.  A clump of ions within a fifth of the ion
+    spacing, split over leaves or not by the order of the rest."""
+    n = 3000
+    pos, q = cloud(n, "equal")
+    rng = np.random.default_rng(partners)
+    spacing = np.cbrt((2 * np.pi) ** 1.5 * 5e-4 ** 3 / n)
+    clump = rng.choice(n, partners + 1, replace=False)
+    pos[clump] = pos[clump[0]] + rng.uniform(-0.1, 0.1, (partners + 1, 3)) * spacing
+    kq = kq_of(np.full(n, 132.905 * oracle.AMU), q)
+    a = far_once.coulomb_accel(pos, q, kq, SG_PREC_FP32C)
+    ref = far_once.coulomb_accel(pos, q, kq, SG_PREC_FP64)
+    e = rel_err_per_ion(a, ref)
+    assert e.max() <= TOL, summary(e)
+    if partners > 8:
+        assert e[clump].max() <= 1e-12
+    assert np.array_equal(a, far_once.coulomb_accel(pos, q, kq, SG_PREC_FP32C))
+
+
+def test_a_non_finite_position_is_not_lost_in_fixed_point(far_once):
+    pos, q = cloud(3000, "equal")
+    pos[17, 1] = np.nan
+    kq = kq_of(np.full(3000, 132.905 * oracle.AMU), q)
+    assert np.isnan(far_once.coulomb_accel(pos, q, kq, SG_PREC_FP32C)).all()
+
+
+def test_automatic_batch_of_small_and_large_clouds(ctx):
+    """A batch above 8,192 ions: clouds of up to 2,500 ions take the plain kernel, larger ones
+    the leaf pairs, in the same call; each ends where the FP64 form ends (fixed steps; the
+    FP32c force bound of 1e-6 diluted by three 2 ns steps)."""
+    counts = [64, 2500, 2501, 700, 5003, 128]
+    rng = configs.rng_for(18)
+    clouds = [configs.gaussian_cloud(rng, n, 5e-4, 300.0, np.full(n, configs.M_CS)) for n in counts]
+    fp = configs.penning_field(quad=(0.5, configs.nu_c(configs.M_CS), 0.0, 0.0, 1.0), delta=1e3)
+    op = configs.ode(1e-9, 1e-15, 2e-9, 1.0, adaptive=False)
+    out = []
+    for prec in (SG_PREC_FP32C, SG_PREC_FP64):
+        b = Batch(ctx, counts, [fp] * len(counts), [op] * len(counts), prec)
+        if prec == SG_PREC_FP32C:
+            assert b.variant() == 17
+        b.upload(np.concatenate([c.pos for c in clouds]), np.concatenate([c.vel for c in clouds]),
+                 np.concatenate([c.mass for c in clouds]),
+                 np.concatenate([c.charge for c in clouds]).astype(np.int32))
+        b.attempts(3)
+        out.append(b.download())
+    at = 0
+    for n in counts:
+        for got, ref in zip(out[0], out[1]):
+            assert np.abs(got[at:at + n] - ref[at:at + n]).max() <= 1e-9 * np.abs(ref[at:at + n]).max()
+        at += n
