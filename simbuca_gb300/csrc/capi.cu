@@ -108,7 +108,10 @@ struct Problem {
     long long attempt_count = 0;
     double kfar_prior = 0.0;  // > 0: the far fix-up threshold's prior of every cloud
     // fused small-cloud attempts (fused.cu)
-bool fused_known = false, fused_resident = false;
+    bool fused_known = false, fused_resident = false;
+    int fused_wide = 0;       // CTAs per cloud of the wide form (0: not launchable)
+    int* fused_barrier = nullptr;
+    double* fused_notes = nullptr;
     int fused_cluster = 0;    // cluster size for this batch (0: none can be launched)
     int max_npad = 0;         // largest padded cloud
 };
@@ -212,6 +215,8 @@ void free_problem(Problem& P) {
     cudaFree(P.leaf_cloud);
     cudaFree(P.near_count);
     cudaFree(P.near_list);
+    cudaFree(P.fused_barrier);
+    cudaFree(P.fused_notes);
     cudaFree(P.leaf_sum);
     cudaFree(P.leaf_fmx);
     cudaFree(P.leaf_n_close);
@@ -694,6 +699,11 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     CK(dalloc(&P.qd, N));
     CK(dalloc(&P.mass, N));
     CK(dalloc(&P.c64, (P.finish ? 8 : 4) * NP));
+    if (P.finish && P.precision == SG_PREC_FP32C) {
+        CK(dalloc(&P.fused_barrier, 2 * (size_t)std::max(P.n_clouds, 1)));
+        CK(cudaMemset(P.fused_barrier, 0, 2 * sizeof(int) * (size_t)std::max(P.n_clouds, 1)));
+        CK(dalloc(&P.fused_notes, 2 * (SG_FUSED_MAX_WIDE + 1) * (size_t)std::max(P.n_clouds, 1)));
+    }
     CK(dalloc(&P.c32, (P.finish ? 14 : 7) * NP));
     CK(dalloc(&P.err_part, (size_t)std::max(P.n_rows, 1) * sg_stage_split(P.row_cap)));
     CK(dalloc(&P.fcoef, (size_t)std::max(P.n_clouds, 1) * SG_MAX_STAGES));
@@ -1173,34 +1183,44 @@ int maybe_check(sg_ctx* ctx, Problem& P, int attempts = 1) {
 
 // The fused small-cloud path (fused.cu) applies to FP32c Dormand-Prince batches of
 // clouds in the plain ion order, without a recorder, operations, dissociation, step log or
-// proposer.  Automatic: clouds of at most SG_FUSED_AUTO_PAIRS pairs per CTA, while every
-// cloud's cluster fits on the device at once; a larger batch of small clouds keeps the
-// SMs busy in the tiled kernels too.  Forced: clouds of up to SG_FUSED_MAX_IONS ions.
-bool fused_eligible(sg_ctx* ctx, Problem& P) {
+// proposer.  Automatic: by the pairs per CTA (SG_FUSED_CLUSTER_PAIRS), while every cloud's
+// CTAs fit on the device at once; a larger batch of small clouds keeps the SMs busy in the
+// tiled kernels too.  Forced: clouds of up to SG_FUSED_MAX_IONS ions, or any the wide form
+// takes.
+// 0: the tiled kernels, 1: a cluster per cloud, 2: the wide form.
+int fused_form(sg_ctx* ctx, Problem& P) {
     if (!ctx->use_fused || P.precision != SG_PREC_FP32C || P.method != 5 || P.sorted ||
         P.rec_cap > 0 || !P.hops.empty() || P.n_dis > 0 || P.use_mlp || P.log_cap > 0 ||
         P.n_clouds == 0)
-        return false;
+        return 0;
     int big = 0;
     for (int c = 0; c < P.n_clouds; c++) {
-        if (P.hc[c].n < 1 || P.hc[c].n > SG_FUSED_MAX_IONS) return false;
+        if (P.hc[c].n < 1) return 0;
         big = std::max(big, P.hc[c].n);
     }
     if (!P.fused_known) {
-        const int R = sg_fused_cluster_size(P.max_npad, P.n_clouds);
-        P.fused_cluster = std::abs(R);
-        P.fused_resident = R > 0;
+        if (big <= SG_FUSED_MAX_IONS) {
+            const int R = sg_fused_cluster_size(P.max_npad, P.n_clouds);
+            P.fused_cluster = std::abs(R);
+            P.fused_resident = R > 0;
+        }
+        if (P.finish) P.fused_wide = sg_fused_wide_ctas(P.max_npad, P.n_clouds, ctx->n_sm);
         P.fused_known = true;
     }
-    if (P.fused_cluster == 0) return false;
-    if (ctx->use_fused == 2) return true;
-    const int own = (big + P.fused_cluster - 1) / P.fused_cluster;
-    return P.fused_resident && (long long)own * big <= SG_FUSED_AUTO_PAIRS;
+    // pairs per CTA of either form (0 CTAs: none)
+    auto pairs = [big](int ctas) { return ctas ? (long long)((big + ctas - 1) / ctas) * big : 0; };
+    const int R = P.fused_cluster, W = P.fused_wide;
+    const bool wide = W > 0 && (R == 0 || (W > R && pairs(R) > SG_FUSED_CLUSTER_PAIRS));
+    if (ctx->use_fused == 2) return wide ? 2 : R > 0;
+    if (wide && pairs(W) <= SG_FUSED_WIDE_PAIRS) return 2;
+    return R > 0 && P.fused_resident && pairs(R) <= SG_FUSED_AUTO_PAIRS;
 }
+bool fused_eligible(sg_ctx* ctx, Problem& P) { return fused_form(ctx, P) != 0; }
 
 // n attempts of every active cloud at most (a cloud stops early once done or held);
 // `counted`: attempts counted towards the in-run check's interval.
 int run_fused(sg_ctx* ctx, Problem& P, int n, int counted) {
+    const bool wide = fused_form(ctx, P) == 2;
     SgFusedArgs f;
     f.clouds = P.dc;
     f.ctrl = P.dctrl;
@@ -1218,13 +1238,16 @@ int run_fused(sg_ctx* ctx, Problem& P, int n, int counted) {
     f.npad = P.npad;
     f.n_clouds = P.n_clouds;
     f.max_attempts = n;
+    f.ctas = wide ? P.fused_wide : 0;
+    f.barrier = P.fused_barrier;
+    f.notes = P.fused_notes;
     TimedLaunch tl{nullptr, nullptr, 0.0, 1};
     if (ctx->timing) {
         tl.a = take_event(ctx);
         tl.b = take_event(ctx);
         CK(cudaEventRecord(tl.a, ctx->stream));
     }
-    CK(sg_fused_attempts(f, P.fused_cluster, P.max_npad, ctx->stream));
+    CK(sg_fused_attempts(f, wide ? P.fused_wide : P.fused_cluster, P.max_npad, ctx->stream));
     P.last_set = 0;
     if (ctx->timing) {
         CK(cudaEventRecord(tl.b, ctx->stream));
@@ -2255,7 +2278,8 @@ int sg_batch_fused(sg_ctx* ctx, int* cluster) {
     Problem& P = ctx->batch;
     if (P.n_clouds == 0) return SG_NOT_READY;
     CK(cudaSetDevice(ctx->device));
-    *cluster = fused_eligible(ctx, P) ? P.fused_cluster : 0;
+    const int form = fused_form(ctx, P);
+    *cluster = form == 2 ? P.fused_wide : form == 1 ? P.fused_cluster : 0;
     return SG_OK;
 }
 

@@ -21,9 +21,15 @@
 //   * control: error partials go to every CTA, and every CTA decides alike
 //     (error_succes and step(), sg_error_succes; bin/ode.cpp:426-494), so the commit
 //     pos <- pos2, vel <- vel2 (bin/ode.cpp:488-489) needs no second barrier.
-// Seven cluster barriers per attempt.  State returns to the batch's global arrays when the
+// Seven barriers per attempt.  State returns to the batch's global arrays when the
 // launch ends, so every other entry point (upload, download, moments, the tiled path
 // itself) sees it.
+//
+// A cloud of many hundred ions has more pairs than 16 SMs take quickly: the wide form spreads
+// it over up to all SMs of the device (a cooperative launch).  There the coordinates go
+// through the batch's two global sets and the barrier is a counter in global memory, waited
+// for with a limit (SG_TIMEOUT); the rest is the same.  1,000 ions: 69 us per attempt, 124
+// in a cluster of 16, 121 in the tiled kernels.
 //
 // Measured, one cloud, us per attempt (state, coordinates and sums through global memory
 // with 15 barriers, close pairs found by a second scan, a flagged row per warp -> this
@@ -31,6 +37,10 @@
 // chain stage - barrier - pairs of dependent instructions.
 #include <cooperative_groups.h>
 #include <math.h>
+
+#include <algorithm>
+
+#include <algorithm>
 
 #include "dp_stage.cuh"
 #include "fp32c_math.cuh"
@@ -49,24 +59,24 @@ constexpr float kKappa2 = 2.25f;  // FP64 row when s2 > 2.25 |P|^2 (the tiled re
 struct FusedNote {
     double err[SG_FUSED_MAX_CTAS];  // error partials
     double x0;                      // x of the caller's first ion
-    int ew, hold;                   // the context's error word and hold switch
 };
 
 struct FusedShared {
     SgCtrl cs;
     SgFieldCoef fk[SG_MAX_STAGES];
     FusedNote note[2];
+    int expired;  // wide: a wait ran out
     double red[2][kWarps][3];  // parts of a flagged row; [0][w][0]: error partials
     double x0;
-    int ew, hold;  // at the launch
+    int ew, hold, wtest;  // at the launch
     int nflag;
 };
 
 // Dynamic shared memory: the cloud's coordinates in two sets, its normalized charges, and
 // the CTA's own ions (mc of them at most): state, Coulomb sums, flagged ions.
 struct FusedArrays {
-    double* D;    // [2][3][npc] SI coordinates
-    float* C;     // [2][6][npc] frame coordinates: high parts x, y, z, low parts x, y, z
+    double* D;    // [2][3][npc] SI coordinates (wide: the batch's arrays hold them)
+    float* C;     // [2][6][npc] frame coordinates: high parts x, y, z, low parts x, y, z (wide: [6][npc])
     float* Q;     // [npc]
     double* ST;   // [6][mc]
     float2* P;    // [3][mc] sums in frame units (float-float), or of a flagged ion SI (double)
@@ -74,15 +84,16 @@ struct FusedArrays {
     int* flag;    // [mc]
     int npc, mc;
 };
-constexpr size_t smem_bytes(int npc, int mc) {
-    return (12 * sizeof(float) + 6 * sizeof(double) + sizeof(float)) * (size_t)npc +
+constexpr size_t smem_bytes(int npc, int mc, bool wide) {
+    return (wide ? 7 * sizeof(float) : 13 * sizeof(float) + 6 * sizeof(double)) * (size_t)npc +
            (6 * sizeof(double) + 3 * sizeof(float2) + 2 * sizeof(int)) * (size_t)mc;
 }
+template <bool WIDE>
 __device__ __forceinline__ FusedArrays carve(unsigned char* p, int npc, int mc) {
     FusedArrays s;
     s.D = reinterpret_cast<double*>(p);
-    s.C = reinterpret_cast<float*>(s.D + 6 * npc);
-    s.Q = s.C + 12 * npc;
+    s.C = WIDE ? reinterpret_cast<float*>(p) : reinterpret_cast<float*>(s.D + 6 * npc);
+    s.Q = s.C + (WIDE ? 6 : 12) * npc;
     s.ST = reinterpret_cast<double*>(s.Q + npc);  // npc is a multiple of 4: 16-byte aligned
     s.P = reinterpret_cast<float2*>(s.ST + 6 * mc);
     s.list = reinterpret_cast<int*>(s.P + 3 * mc);
@@ -178,10 +189,13 @@ __device__ __forceinline__ double stage_after(const FusedArrays& s, const SgClou
     return acc2;
 }
 
-// The new state into shared memory, its coordinates into set `set` of this CTA.
-template <int PASSES>
-__device__ __forceinline__ void store_state(const FusedArrays& s, const SgCloud& cl, int lo,
-                                            int set, const Slots<PASSES>& w) {
+// The new state into shared memory, its coordinates into set `set`: of this CTA's shared
+// memory, or (wide) of the batch's arrays.
+template <bool WIDE, int PASSES>
+__device__ __forceinline__ void store_state(const SgFusedArgs& f, const FusedArrays& s,
+                                            const SgCloud& cl, int lo, int set,
+                                            const Slots<PASSES>& w) {
+    const size_t NP = (size_t)f.npad;
 #pragma unroll
     for (int u = 0; u < PASSES; u++) {
         const int c = w.c[u];
@@ -190,13 +204,65 @@ __device__ __forceinline__ void store_state(const FusedArrays& s, const SgCloud&
         if (c < 3) {
             const int li = lo + w.row[u];
             const double v = (w.st[u] - (c == 0 ? cl.cx : c == 1 ? cl.cy : cl.cz)) * cl.invL;
-            const float hi = __double2float_rn(v);
-            float* C = s.C + set * 6 * s.npc + li;
-            C[c * s.npc] = hi;
-            C[(3 + c) * s.npc] = __double2float_rn(v - (double)hi);
-            s.D[(set * 3 + c) * s.npc + li] = w.st[u];
+            const float hi = __double2float_rn(v), low = __double2float_rn(v - (double)hi);
+            if (WIDE) {
+                float* C = f.c32 + set * 7 * NP + cl.poff + li;
+                C[c * NP] = hi;
+                C[(4 + c) * NP] = low;
+                f.c64[(set * 4 + c) * NP + cl.poff + li] = w.st[u];
+            } else {
+                float* C = s.C + set * 6 * s.npc + li;
+                C[c * s.npc] = hi;
+                C[(3 + c) * s.npc] = low;
+                s.D[(set * 3 + c) * s.npc + li] = w.st[u];
+            }
         }
     }
+}
+
+// Wide: the cloud's frame coordinates of set `set`, written by every CTA of the cloud, from
+// the batch's arrays (through L2).
+__device__ __forceinline__ void load_coords(const SgFusedArgs& f, const FusedArrays& s,
+                                            const SgCloud& cl, int set) {
+    const size_t NP = (size_t)f.npad;
+    const int nv = s.npc / 4;
+#pragma unroll 4
+    for (int q = threadIdx.x; q < 6 * nv; q += kThreads) {
+        const int a = q / nv, v = q - a * nv;
+        const float4* src = reinterpret_cast<const float4*>(
+            f.c32 + (set * 7 + (a < 3 ? a : a + 1)) * NP + cl.poff);
+        reinterpret_cast<float4*>(s.C + a * s.npc)[v] = __ldcg(src + v);
+    }
+    __syncthreads();
+}
+
+// Wide: the barrier of a cloud's CTAs, a counter that each raises by one.  All of them are
+// resident (cooperative launch); a wait gives up after SG_WAIT_NS.
+__device__ __forceinline__ void wide_arrive(int* count) {
+    __syncthreads();  // the CTA's stores come before its arrival
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(count, 1);
+    }
+}
+__device__ __forceinline__ bool wide_wait(const int* count, int target, FusedShared& sh,
+                                          unsigned long long limit_ns = SG_WAIT_NS) {
+    if (threadIdx.x == 0) {
+        int seen;
+        unsigned long long t0 = 0, t;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
+            if (seen >= target) break;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (t0 == 0) t0 = t;
+            if (t - t0 > limit_ns) {
+                sh.expired = 1;
+                break;
+            }
+        }
+    }
+    __syncthreads();
+    return sh.expired == 0;
 }
 
 // This CTA's rows [lo, lo + m) of set `set` into the other CTAs' shared memory, 16 bytes a
@@ -223,21 +289,25 @@ __device__ __forceinline__ void push_coords(cg::cluster_group& cluster, const Fu
 // Coulomb sums of the CTA's mo ions (cloud indices lo ...) at coordinate set `set` into
 // s.P, in the FP32-compensated form; risk: where the in-run check's inputs go (null: not
 // written).
+template <bool WIDE>
 __device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedArrays& s,
                                               const SgCloud& cl, int lo, int mo, int set,
                                               float* risk, FusedShared& sh) {
     const int tid = threadIdx.x;
     const int npc = s.npc;
-    const float* X = s.C + set * 6 * npc;
+    const float* X = s.C + (WIDE ? 0 : set * 6 * npc);
     const float* Y = X + npc;
     const float* Z = X + 2 * npc;
     const float* XL = X + 3 * npc;
     const float* YL = X + 4 * npc;
     const float* ZL = X + 5 * npc;
     const float* Q = s.Q;
-    const double* SX = s.D + set * 3 * npc;
-    const double* SY = SX + npc;
-    const double* SZ = SX + 2 * npc;
+    const size_t ND = WIDE ? (size_t)f.npad : (size_t)npc;
+    const double* SX = WIDE ? f.c64 + set * 4 * ND + cl.poff : s.D + set * 3 * npc;
+    const double* SY = SX + ND;
+    const double* SZ = SX + 2 * ND;
+    // other CTAs write the global coordinates: through L2
+    auto ld = [](const double* p) { return WIDE ? __ldcg(p) : *p; };
     const double* SQ = f.c64 + 3 * (size_t)f.npad + cl.poff;  // charges: never rewritten here
     // G threads per ion.  Thread q of an ion takes the packed j-pairs q, q + G, q + 2G, ...
     // (j = 2p, 2p + 1), so the G threads of an ion read consecutive 8-byte words of
@@ -333,7 +403,8 @@ __device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedA
                     close_term_ff(ff_diff(X[jj], XL[jj], xih, xil), ff_diff(Y[jj], YL[jj], yih, yil),
                                   ff_diff(Z[jj], ZL[jj], zih, zil), Q[jj], wf, pr, dx, dy, dz);
                 } else {
-                    const double rx = SX[li] - SX[jj], ry = SY[li] - SY[jj], rz = SZ[li] - SZ[jj];
+                    const double rx = ld(SX + li) - ld(SX + jj), ry = ld(SY + li) - ld(SY + jj),
+                                 rz = ld(SZ + li) - ld(SZ + jj);
                     const double w = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz) / cl.psc;
                     const double c0 = w * rx - (double)wf * (double)pr.dx,
                                  c1 = w * ry - (double)wf * (double)pr.dy,
@@ -400,10 +471,10 @@ __device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedA
         double(*red)[3] = sh.red[k & 1];
         if (32 * warp < npc) {
             double ax = 0.0, ay = 0.0, az = 0.0;
-            const double xi = SX[lf], yi = SY[lf], zi = SZ[lf];
+            const double xi = ld(SX + lf), yi = ld(SY + lf), zi = ld(SZ + lf);
             for (int jj = 32 * warp + lane; jj < npc; jj += kThreads) {
                 if (jj == lf) continue;
-                const double rx = xi - SX[jj], ry = yi - SY[jj], rz = zi - SZ[jj];
+                const double rx = xi - ld(SX + jj), ry = yi - ld(SY + jj), rz = zi - ld(SZ + jj);
                 const double wq = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz);
                 ax = fma(wq, rx, ax);
                 ay = fma(wq, ry, ay);
@@ -438,19 +509,20 @@ __device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedA
 // Control of an attempt with error norm err (thread 0 of every CTA alike): error_succes,
 // step() and the bookkeeping of dp_control_kernel for clouds without a recorder or
 // operations.
-__device__ __forceinline__ void control_phase(SgCtrl& cs, const SgCloud& cl, const FusedNote& nt,
+__device__ __forceinline__ void control_phase(FusedShared& sh, const SgCloud& cl, const double* x0,
                                               double err) {
+    SgCtrl& cs = sh.cs;
     cs.err = err;
     cs.print_due = 0;
     cs.force_evals += 7;
     cs.coulomb_evals += (cl.fp.flags & SG_F_COULOMB) ? 6 : 0;
     int accepted;
-    if (nt.ew != 0) {
-        cs.status = nt.ew;
+    if (sh.ew != 0) {
+        cs.status = sh.ew;
         cs.done = 1;
         accepted = 0;
     } else {
-        accepted = sg_error_succes(cs, err, &nt.x0);
+        accepted = sg_error_succes(cs, err, x0);
     }
     if (accepted) {
         cs.h_last = cs.h;
@@ -459,22 +531,22 @@ __device__ __forceinline__ void control_phase(SgCtrl& cs, const SgCloud& cl, con
         cs.steps++;
         cs.rejects_here = 0;
         if (cs.t >= cs.t_end) cs.done = 1;
-        if (nt.hold) cs.hold |= 1;
+        if (sh.hold) cs.hold |= 1;
     }
     cs.accepted = accepted;
 }
 
-template <int PASSES>
+template <int PASSES, bool WIDE>
 __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs f, int mc) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ FusedShared sh;
     cg::cluster_group cluster = cg::this_cluster();
-    const int R = (int)cluster.num_blocks();
-    const int r = (int)cluster.block_rank();
+    const int R = WIDE ? f.ctas : (int)cluster.num_blocks();
     const int c = blockIdx.x / R;
+    const int r = blockIdx.x - c * R;  // the rank in its cluster
     const int tid = threadIdx.x;
     const SgCloud& cl = f.clouds[c];
-    const FusedArrays s = carve(dyn, cl.npad, mc);
+    const FusedArrays s = carve<WIDE>(dyn, cl.npad, mc);
     const int n = cl.n, npc = cl.npad;
     const int m = own_ions(n, R);
     const int lo = min(n, r * m), mo = min(n, (r + 1) * m) - lo;
@@ -486,11 +558,13 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
         sh.cs = f.ctrl[c];
         sh.ew = f.flags[SG_FLAG_ERR];
         sh.hold = f.flags[SG_FLAG_HOLD];
+        sh.wtest = f.flags[SG_FLAG_WAIT_TILE];
+        sh.expired = 0;
     }
     // charges; the padding's coordinates, and for whole 16-byte words of the last CTA's rows
     // they are in both sets of every CTA
     for (int j = tid; j < npc; j += kThreads) s.Q[j] = f.c32[3 * NP + cl.poff + j];
-    for (int j = n + tid; j < npc; j += kThreads)
+    for (int j = n + tid; !WIDE && j < npc; j += kThreads)
         for (int set = 0; set < 2; set++)
             for (int a = 0; a < 3; a++) {
                 float* C = s.C + (set * 6 + a) * npc + j;
@@ -515,9 +589,22 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
             if (coul) w.p1[u] = f.coul1[(w.c[u] - 3) * N + i];
         }
     }
-    cluster.sync();  // every CTA runs, and has read the control block
+    // wide: the cloud's barrier counter and notes
+    int* count = WIDE ? f.barrier + 2 * c : nullptr;
+    double* notes = WIDE ? f.notes + (size_t)c * 2 * (SG_FUSED_MAX_WIDE + 1) : nullptr;
+    int arrived = 0;
+    bool ok = true;
+    if (WIDE) {
+        wide_arrive(count);
+        arrived += R;
+        ok = sh.wtest != 1 ? wide_wait(count, arrived, sh)
+                           : wide_wait(count, arrived + 1, sh,  // the wait test: never
+                                       1000ull * max(f.flags[SG_FLAG_WAIT_US], 1));
+    } else {
+        cluster.sync();  // every CTA runs, and has read the control block
+    }
     int att = 0;
-    for (; att < f.max_attempts; att++) {
+    for (; ok && att < f.max_attempts; att++) {
         if (sh.cs.done || sh.cs.hold || sh.cs.status != SG_OK || sh.ew != 0) break;
         const double t0 = sh.cs.t, h = sh.cs.h, atol = sh.cs.atol, rtol = sh.cs.rtol;
         // every stage's field coefficients, a lane each
@@ -536,19 +623,27 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
         stage_after<1>(s, cl, h, atol, rtol, coul, w);
         __syncthreads();  // the step's initial state has been read
         // the state of stage S+1 is in w: its Coulomb sum, then k_{S+1}
-#define SG_FUSED_STAGE(S)                                                          \
-    store_state(s, cl, lo, (S) & 1, w);                                            \
-    if (tid == 0) sh.nflag = 0;                                                    \
-    __syncthreads();                                                               \
-    if (coul) {                                                                    \
-        if (mo > 0) push_coords(cluster, s, lo, m, (S) & 1, ctas, r);              \
-        auto token = cluster.barrier_arrive();                                     \
-        stage_before<S>(s, cl, sh.fk[S], w);                                       \
-        cluster.barrier_wait(std::move(token));                                    \
-        coulomb_phase(f, s, cl, lo, mo, (S) & 1, (S) == 7 ? f.risk : nullptr, sh); \
-    } else {                                                                       \
-        stage_before<S>(s, cl, sh.fk[S], w);                                       \
-        __syncthreads();                                                           \
+#define SG_FUSED_STAGE(S)                                                              \
+    store_state<WIDE>(f, s, cl, lo, (S) & 1, w);                                       \
+    if (tid == 0) sh.nflag = 0;                                                        \
+    if (!coul) {                                                                       \
+        __syncthreads();                                                               \
+        stage_before<S>(s, cl, sh.fk[S], w);                                           \
+        __syncthreads();                                                               \
+    } else if (WIDE) {                                                                 \
+        wide_arrive(count);                                                            \
+        stage_before<S>(s, cl, sh.fk[S], w);                                           \
+        ok = wide_wait(count, (arrived += R), sh);                                     \
+        if (!ok) break;                                                                \
+        load_coords(f, s, cl, (S) & 1);                                                \
+        coulomb_phase<WIDE>(f, s, cl, lo, mo, (S) & 1, (S) == 7 ? f.risk : nullptr, sh); \
+    } else {                                                                           \
+        __syncthreads();                                                               \
+        if (mo > 0) push_coords(cluster, s, lo, m, (S) & 1, ctas, r);                  \
+        auto token = cluster.barrier_arrive();                                         \
+        stage_before<S>(s, cl, sh.fk[S], w);                                           \
+        cluster.barrier_wait(std::move(token));                                        \
+        coulomb_phase<WIDE>(f, s, cl, lo, mo, (S) & 1, (S) == 7 ? f.risk : nullptr, sh); \
     }
         SG_FUSED_STAGE(2)
         stage_after<2>(s, cl, h, atol, rtol, coul, w);
@@ -574,26 +669,47 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
         for (int u = 0; u < PASSES; u++)
             if (w.c[u] == 0 && cl.off + lo + w.row[u] == cl.ion0) sh.x0 = w.y[u];
         __syncthreads();
-        FusedNote& nt = sh.note[att & 1];
-        if (tid < 32) {
-            double v = lane < nw ? sh.red[0][lane][0] : 0.0;
-            for (int o = kWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane < R) {
-                FusedNote* to = cluster.map_shared_rank(&nt, lane);
-                to->err[r] = v;
-                if (cl.ion0 >= cl.off + lo && cl.ion0 < cl.off + lo + mo) to->x0 = sh.x0;
-                if (r == 0) {
-                    to->ew = sh.ew;
-                    to->hold = sh.hold;
+        const bool own0 = cl.ion0 >= cl.off + lo && cl.ion0 < cl.off + lo + mo;
+        if constexpr (WIDE) {
+            double* nt = notes + (att & 1) * (SG_FUSED_MAX_WIDE + 1);
+            if (tid < 32) {
+                double v = lane < nw ? sh.red[0][lane][0] : 0.0;
+                for (int o = kWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) {
+                    nt[r] = v;
+                    if (own0) nt[SG_FUSED_MAX_WIDE] = sh.x0;
                 }
             }
-        }
-        cluster.sync();
-        if (tid < 32) {
-            double v = lane < R ? nt.err[lane] : 0.0;
-            for (int o = SG_FUSED_MAX_CTAS / 2; o > 0; o >>= 1)
-                v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) control_phase(sh.cs, cl, nt, sqrt(v / (6 * n)));
+            wide_arrive(count);
+            ok = wide_wait(count, (arrived += R), sh);
+            if (!ok) break;
+            if (tid < 32) {
+                double v = 0.0;
+                for (int q = lane; q < R; q += 32) v += __ldcg(nt + q);
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) {
+                    sh.x0 = __ldcg(nt + SG_FUSED_MAX_WIDE);
+                    control_phase(sh, cl, &sh.x0, sqrt(v / (6 * n)));
+                }
+            }
+        } else {
+            FusedNote& nt = sh.note[att & 1];
+            if (tid < 32) {
+                double v = lane < nw ? sh.red[0][lane][0] : 0.0;
+                for (int o = kWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane < R) {
+                    FusedNote* to = cluster.map_shared_rank(&nt, lane);
+                    to->err[r] = v;
+                    if (own0) to->x0 = sh.x0;
+                }
+            }
+            cluster.sync();
+            if (tid < 32) {
+                double v = lane < R ? nt.err[lane] : 0.0;
+                for (int o = SG_FUSED_MAX_CTAS / 2; o > 0; o >>= 1)
+                    v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) control_phase(sh, cl, &nt.x0, sqrt(v / (6 * n)));
+            }
         }
         __syncthreads();
         if (sh.cs.accepted) {
@@ -604,6 +720,24 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
                 w.p1[u] = w.p7[u];
             }
         }
+    }
+    if constexpr (WIDE) {
+        // the last CTA to leave clears the counters for the next launch; a wait that ran out
+        // stops the batch
+        if (tid == 0) {
+            if (!ok) {
+                atomicExch(f.flags + SG_FLAG_ERR, SG_TIMEOUT);
+                if (r == 0) {
+                    f.ctrl[c].status = SG_TIMEOUT;
+                    f.ctrl[c].done = 1;
+                }
+            }
+            if (atomicAdd(count + 1, 1) == R - 1) {
+                count[0] = 0;
+                count[1] = 0;
+            }
+        }
+        if (!ok) return;
     }
     if (att == 0) return;
     // state, stage sums and the last evaluation's coordinates back to the batch's arrays
@@ -632,70 +766,93 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
     }
 }
 
-// Slots per thread for mc own ions.  One covers clouds of up to 1,344 ions on 16 CTAs; the
-// others keep more of them in registers (six: the largest clouds on 4 CTAs).
-template <typename F>
-auto by_passes(int mc, F&& f) {
-    if (6 * mc <= kThreads) return f(fused_attempts_kernel<1>);
-    if (6 * mc <= 2 * kThreads) return f(fused_attempts_kernel<2>);
-    return f(fused_attempts_kernel<6>);
+// The kernel with enough slots per thread for mc own ions.  Clusters: one slot covers clouds
+// of up to 1,344 ions on 16 CTAs; the others keep more of them in registers (six: the
+// largest clouds on 4 CTAs).
+typedef void (*FusedKernel)(SgFusedArgs, int);
+FusedKernel cluster_kernel(int mc) {
+    return 6 * mc <= kThreads       ? fused_attempts_kernel<1, false>
+           : 6 * mc <= 2 * kThreads ? fused_attempts_kernel<2, false>
+                                    : fused_attempts_kernel<6, false>;
 }
 
-}  // namespace
+// Dynamic shared memory any launch asks for at most (clusters: 2,048 ions on 8 CTAs; wide:
+// SG_FUSED_WIDE_IONS).  Every kernel is allowed it once and for all: a launch of one thread
+// cannot lower another's.
+constexpr size_t kMaxSmem = smem_bytes(SG_FUSED_MAX_IONS, SG_FUSED_MAX_IONS / 8, false);
+constexpr size_t kMaxWide = smem_bytes(SG_FUSED_WIDE_IONS, kThreads / 6 / 4 * 4, true);
 
-// Dynamic shared memory any launch asks for at most (2,048 ions on 8 CTAs).  Every kernel
-// is allowed it once and for all: a launch of one thread cannot lower another's.
-constexpr size_t kMaxSmem = smem_bytes(SG_FUSED_MAX_IONS, SG_FUSED_MAX_IONS / 8);
+}  // namespace
 
 int sg_fused_cluster_size(int max_npad, int n_clouds) {
     int found = 0;
     for (int R = SG_FUSED_MAX_CTAS; R >= 2; R /= 2) {
         const int mc = own_ions(max_npad, R);
-        const size_t smem = smem_bytes(max_npad, mc);
+        const size_t smem = smem_bytes(max_npad, mc, false);
         if (mc > kThreads || smem > kMaxSmem) continue;
-        const int active = by_passes(mc, [&](auto* kernel) {
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                    cudaSuccess ||
-                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kMaxSmem) != cudaSuccess)
-                return 0;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(R);
-            cfg.blockDim = dim3(kThreads);
-            cfg.dynamicSmemBytes = smem;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = R;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int n = 0;
-            return cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess ? n : 0;
-        });
-        if (active > 0) found = R;
+        const FusedKernel kernel = cluster_kernel(mc);
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kMaxSmem) != cudaSuccess)
+            continue;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(R);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = R;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int active = 0;
+        if (cudaOccupancyMaxActiveClusters(&active, kernel, &cfg) != cudaSuccess || active <= 0)
+            continue;
+        found = R;
         if (active >= n_clouds) return R;
     }
     cudaGetLastError();
     return -found;
 }
 
-cudaError_t sg_fused_attempts(const SgFusedArgs& f, int cluster, int max_npad, cudaStream_t st) {
-    const int mc = own_ions(max_npad, cluster);
-    const size_t smem = smem_bytes(max_npad, mc);
-    return by_passes(mc, [&](auto* kernel) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(f.n_clouds * cluster);
-        cfg.blockDim = dim3(kThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
+int sg_fused_wide_ctas(int max_npad, int n_clouds, int n_sm) {
+    if (max_npad > SG_FUSED_WIDE_IONS) return 0;
+    // no more CTAs than groups of four ions
+    const int R = std::min({n_sm / n_clouds, max_npad / 4, SG_FUSED_MAX_WIDE});
+    if (R < 1 || 6 * own_ions(max_npad, R) > kThreads) return 0;
+    const size_t smem = smem_bytes(max_npad, own_ions(max_npad, R), true);
+    int per_sm = 0;
+    if (cudaFuncSetAttribute(fused_attempts_kernel<1, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxWide) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_attempts_kernel<1, true>,
+                                                      kThreads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return per_sm > 0 ? R : 0;
+}
+
+cudaError_t sg_fused_attempts(const SgFusedArgs& f, int ctas, int max_npad, cudaStream_t st) {
+    const bool wide = f.ctas > 0;
+    const int mc = own_ions(max_npad, ctas);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(f.n_clouds * ctas);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem_bytes(max_npad, mc, wide);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    if (wide) {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    } else {
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cluster;
+        at[0].val.clusterDim.x = ctas;
         at[0].val.clusterDim.y = 1;
         at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kernel, f, mc);
-    });
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, wide ? fused_attempts_kernel<1, true> : cluster_kernel(mc), f, mc);
 }

@@ -490,12 +490,18 @@ cudaError_t sg_dp_finish(const SgFinishArgs& f, int stage, int fp32c, cudaStream
 #define SG_FUSED_THREADS 512
 #define SG_FUSED_MAX_CTAS 16
 #define SG_FUSED_MAX_IONS 2048
-// Ordered pairs per CTA (its ions times the cloud's) up to which the fused path is taken by
-// default (sg_set_fused mode 1); mode 2 takes it up to SG_FUSED_MAX_IONS.  Measured on
-// GB300, us per attempt, fused / tiled kernels: one cloud on 16 CTAs of 300 ions 60 / 143,
-// 512 71 / 131, 700 (31,000 pairs) 93 / 119, 850 (48,000) 125 / 136, 1,000 124 / 120, 1,500
-// 294 / 154; 32 clouds of 300 on 4 CTAs each (23,000) 101 / 278, 16 of 512 (66,000) 168 / 194;
-// 70 of 100 on 2 (5,000) 67 / 223.
+#define SG_FUSED_MAX_WIDE 160    // CTAs of a cloud in the wide form
+#define SG_FUSED_WIDE_IONS 4096  // ions of a cloud in the wide form
+// Ordered pairs per CTA (its ions times the cloud's).  Up to SG_FUSED_CLUSTER_PAIRS a cluster
+// is faster than the wide form with more CTAs; the wide form is taken by default (sg_set_fused
+// mode 1) up to SG_FUSED_WIDE_PAIRS, clusters up to SG_FUSED_AUTO_PAIRS.  Measured on GB300, us
+// per attempt (pairs per CTA), cluster / wide / tiled kernels: one cloud of 300 ions 60 (6,000)
+// / 62 / 142, 512 71 (16,000) / 69 (2,000) / 131, 1,000 125 / 69 (8,000) / 121, 1,344 225 / 108
+// (16,000) / 156, 2,048 400 / 126 to 214 (33,000) / 150, 3,000 - / 205 (60,000) / 182; 8 of
+// 300 77 (12,000) / 60 (5,000) / 166, 16 of 300 101 (23,000) / 82 / 227, 4 of 1,000 139 / 108
+// (28,000) / 154; 70 of 100 on 2 CTAs each 67 (5,000) / 76 / 224.
+#define SG_FUSED_CLUSTER_PAIRS 8000
+#define SG_FUSED_WIDE_PAIRS 30000
 #define SG_FUSED_AUTO_PAIRS 40000
 struct SgFusedArgs {
     const SgCloud* clouds;
@@ -509,13 +515,19 @@ struct SgFusedArgs {
     int* ran;
     int n, npad, n_clouds;
     int max_attempts;  // attempts per launch at most
+    // wide form: CTAs per cloud (0: clusters), c64 and c32 hold two coordinate sets
+    int ctas;
+    int* barrier;   // [clouds][2] arrivals, departures; zero between launches
+    double* notes;  // [clouds][2][SG_FUSED_MAX_WIDE + 1] error partials, x of the first ion
 };
 // The cluster size (16, 8, 4 or 2) for n_clouds clouds of up to max_npad padded ions: the
 // largest with which all of them are on the device at once (clusters of 16 take the SMs of
 // a GPC: 8 clouds of 64 ions took 76 us per attempt on 16 CTAs each and 43 on 8).  If there
 // is none, minus the smallest that can be launched (0: no cluster can).
 int sg_fused_cluster_size(int max_npad, int n_clouds);
-cudaError_t sg_fused_attempts(const SgFusedArgs& f, int cluster, int max_npad, cudaStream_t st);
+// CTAs per cloud of the wide form (0: it cannot be launched).
+int sg_fused_wide_ctas(int max_npad, int n_clouds, int n_sm);
+cudaError_t sg_fused_attempts(const SgFusedArgs& f, int ctas, int max_npad, cudaStream_t st);
 
 // ---- device-side observables (observe.cu) -------------------------------------------
 // A record of a cloud: [0] t, then per species s < n_species the PrintCloud statistics

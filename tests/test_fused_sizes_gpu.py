@@ -1,11 +1,11 @@
-"""The fused small-cloud kernel at the sizes where its layout changes: clouds of fewer ions
+"""The fused small-cloud kernels at the sizes where their layout changes: clouds of fewer ions
 than CTAs take, the CTA's rows whole 16-byte words or not, one and two slots per thread
 (1,344 ions on 16 CTAs), each with an ion at the centre whose terms cancel (its row comes
 from the FP64 loop) and a close pair."""
 import numpy as np
 import pytest
 
-from simbuca_gb300 import configs
+from simbuca_gb300 import abi, configs
 from simbuca_gb300.abi import SG_PREC_FP32C, SG_PREC_FP64
 from simbuca_gb300.api import Batch
 
@@ -45,3 +45,80 @@ def test_sizes_against_fp64(ctx, n, charges):
     ev = np.abs(out[0][1] - out[1][1]).max() / np.abs(out[1][1]).max()
     print(n, charges, ep, ev)
     assert ep <= 1e-9 and ev <= 1e-8
+
+
+def test_clusters_with_several_slots_per_thread(ctx):
+    """A batch above 8,192 ions, forced: clusters, two to six slots per thread; fixed steps
+    against the FP64 form, bounds as above."""
+    counts = [1344, 1345, 2048, 2048, 2047]
+    clouds = [configs.gaussian_cloud(configs.rng_for(90 + k), n, 0.5e-3, 300.0, np.full(n, configs.M_CS))
+              for k, n in enumerate(counts)]
+    fp = configs.penning_field(quad=(0.5, configs.nu_c(132.905), 0.0, 0.0, 1.0), delta=1e3)
+    op = configs.ode(1e-9, 1e-15, 2e-9, 1.0, adaptive=False)
+    out = []
+    for prec in (SG_PREC_FP32C, SG_PREC_FP64):
+        ctx.set_fused(2)
+        try:
+            b = Batch(ctx, counts, [fp] * 5, [op] * 5, prec)
+            assert (2 <= b.fused() <= 16) == (prec == SG_PREC_FP32C)
+            b.upload(np.concatenate([c.pos for c in clouds]), np.concatenate([c.vel for c in clouds]),
+                     np.concatenate([c.mass for c in clouds]),
+                     np.concatenate([c.charge for c in clouds]).astype(np.int32))
+            b.run(max_attempts=4)
+            out.append(b.download())
+        finally:
+            ctx.set_fused(1)
+    for got, ref, tol in zip(out[0], out[1], (1e-9, 1e-8)):
+        assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("counts", [[500], [1000], [1825], [1826], [300] * 8, [1000, 16, 999, 64]])
+def test_wide_form_against_fp64(ctx, counts):
+    """The form that spreads a cloud over many CTAs: sizes of its automatic range and its
+    edges, equal and uneven batches, with a close pair in every cloud; bounds as above."""
+    clouds = []
+    for k, n in enumerate(counts):
+        c = configs.gaussian_cloud(configs.rng_for(120 + k), n, 0.5e-3, 300.0, np.full(n, configs.M_CS))
+        c.pos[2] = c.pos[1] + [4e-7, 0.0, 2e-7]
+        c.pos[0] = c.pos.mean(0)
+        clouds.append(c)
+    fp = configs.penning_field(quad=(0.5, configs.nu_c(132.905), 0.0, 0.0, 1.0), delta=1e3)
+    op = configs.ode(1e-9, 1e-15, 2e-9, 1.0, adaptive=False)
+    out = []
+    for prec in (SG_PREC_FP32C, SG_PREC_FP64):
+        b = Batch(ctx, counts, [fp] * len(counts), [op] * len(counts), prec)
+        if prec == SG_PREC_FP32C and counts[0] <= 1824:
+            assert b.fused() > 16
+        b.upload(np.concatenate([c.pos for c in clouds]), np.concatenate([c.vel for c in clouds]),
+                 np.concatenate([c.mass for c in clouds]),
+                 np.concatenate([c.charge for c in clouds]).astype(np.int32))
+        b.run(max_attempts=8)
+        out.append(b.download())
+    for got, ref, tol in zip(out[0], out[1], (1e-9, 1e-8)):
+        assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+
+
+def test_wide_wait_runs_out_and_context_recovers(ctx):
+    """The barrier's wait is bounded: with the wait test on, the first one runs out after
+    1 ms, the call returns SG_TIMEOUT, nothing is committed, and a new upload integrates."""
+    c = configs.penning_1k(n=1000, seed=5).clouds[0]
+    fp = configs.penning_field(quad=(0.5, configs.nu_c(132.905), 0.0, 0.0, 1.0), delta=1e3)
+    b = Batch(ctx, [1000], [fp], [configs.ode(1e-9, 1e-15, 1e-9, 1e-6)], SG_PREC_FP32C)
+    assert b.fused() > 16
+    b.upload(c.pos, c.vel, c.mass, c.charge)
+    ref_info, st = b.step()
+    assert st == abi.SG_OK
+    ref_p, ref_v = b.download()
+    b.upload(c.pos, c.vel, c.mass, c.charge)
+    ctx.set_wait_test(0, 1000)
+    info, st = b.step(raise_on_error=False)
+    assert st == abi.SG_TIMEOUT
+    assert info[0]["status"] == abi.SG_TIMEOUT and info[0]["steps"] == 0 and info[0]["t"] == 0.0
+    p, v = b.download()
+    assert np.array_equal(p, c.pos) and np.array_equal(v, c.vel)
+    ctx.set_wait_test(-1)
+    b.upload(c.pos, c.vel, c.mass, c.charge)
+    info, st = b.step()
+    assert st == abi.SG_OK and info[0]["steps"] == ref_info[0]["steps"] == 1
+    p, v = b.download()
+    assert np.array_equal(p, ref_p) and np.array_equal(v, ref_v)
