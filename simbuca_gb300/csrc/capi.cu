@@ -15,6 +15,7 @@
 #include <utility>
 #include <vector>
 
+#include "fp64_pairs.cuh"
 #include "sg_internal.cuh"
 #include "sg_mt19937.h"
 
@@ -286,55 +287,56 @@ int auto_variant(const std::vector<int>& counts, int requested, bool resident) {
 }
 
 // FP64 items that take each unordered pair once: i-block b (128 ions) against the j-tiles
-// (32 ions) from its own diagonal up, K tiles per item, or 1/bands of the rotation steps
-// of one tile when that leaves the device short of items.  A block keeps all four FP64
-// pipes of an SM busy whatever else it does, so the items only have to be small against
-// one SM's share of the work (at least 4 items per SM) and large against the ~1 us it
-// takes to start one (a tile is 20 us of FP64).
+// (32 ions) from its own diagonal up, K tiles per item, or pairs of 32-ion tiles when that
+// leaves the device short of items.  A block keeps all four FP64 pipes of an SM busy
+// whatever else it does, so the items only have to be small against one SM's share of
+// the work and large against the ~1 us it takes to start one (a 128 x 32 tile is 20 us of
+// FP64).
 void plan_sym(Problem& P, int n_sm) {
     const int TB = SG_SYM_IB / SG_SYM_JT;
-    double tiles = 0.0;
+    double tiles = 0.0, tile_pairs = 0.0;
     for (int c = 0; c < P.n_clouds; c++) {
         if (!(P.hc[c].fp.flags & SG_F_COULOMB)) continue;
         const int nj = P.hc[c].npad / SG_SYM_JT;
         for (int b = 0; b * TB < nj; b++) tiles += nj - b * TB;
+        tile_pairs += 0.5 * nj * (nj + 1.0);
     }
-    int bands = 1, K = 1;
-    while (bands < 8 && tiles * bands < 4.0 * n_sm) bands *= 2;
-    if (bands == 1) K = (int)std::min(64.0, std::max(1.0, std::floor(tiles / (16.0 * n_sm))));
+    const bool pairs = tiles < kSymTilePairs * n_sm;
+    const int parts = pairs ? sym_parts(tile_pairs, n_sm) : 1;
+    const int K = (int)std::min(64.0, std::max(1.0, std::floor(tiles / (16.0 * n_sm))));
     P.max_slots = 0;
     for (int c = 0; c < P.n_clouds; c++) {
         SgCloud& cl = P.hc[c];
         cl.nslots = 0;
         if (!(cl.fp.flags & SG_F_COULOMB) || cl.n == 0) continue;
         P.any_coulomb = true;
-        cl.sym_k = K;
-        cl.sym_bands = bands;
+        cl.sym_k = pairs ? 0 : K;
         const int nj = cl.npad / SG_SYM_JT;
-        for (int b = 0; b * TB < nj; b++)
-            for (int t = b * TB, q = 0; t < nj; t += K, q++)
-                for (int band = 0; band < bands; band++) {
+        const int ti = pairs ? 1 : TB, tj = pairs ? 1 : K;  // tiles of an item
+        for (int b = 0; b * ti < nj; b++)
+            for (int t = b * ti, q = 0; t < nj; t += tj, q++)
+                for (int part = 0; part < parts; part++) {
                     SgWorkItem it;
                     memset(&it, 0, sizeof it);
                     it.cloud = c;
-                    it.i0 = cl.poff + b * SG_SYM_IB;
-                    it.ni = std::min(SG_SYM_IB, cl.npad - b * SG_SYM_IB);
+                    it.i0 = cl.poff + b * ti * SG_SYM_JT;
+                    it.ni = std::min(ti * SG_SYM_JT, cl.npad - b * ti * SG_SYM_JT);
                     it.j0 = cl.poff + t * SG_SYM_JT;
-                    it.nj = std::min(K, nj - t) * SG_SYM_JT;
-                    it.slot = (b + 1 + q) * bands + band;
-                    it.jslot = b * bands + band;
-                    const int step = SG_SYM_JT / bands;
-                    it.s01 = band * step | (band + 1) * step << 16;
+                    it.nj = std::min(tj, nj - t) * SG_SYM_JT;
+                    // slots of an ion: as a j-ion of the blocks up to its own, then as an i-ion
+                    // (tile pairs: by the j-tile, so that every ion has them all)
+                    it.slot = (pairs ? t + 1 : b + 1 + q) * parts + part;
+                    it.jslot = b * parts + part;
+                    it.tile_pair = pairs ? parts << 8 | part : 0;
+                    cl.nslots = std::max(cl.nslots, it.slot + 1);
                     P.hitems.push_back(it);
                 }
-        for (int p = 0; p < cl.npad; p += SG_SYM_IB)
-            cl.nslots = std::max(cl.nslots, sg_sym_slots(cl, p));
         P.max_slots = std::max(P.max_slots, cl.nslots);
         P.cloud_inter[c] = (double)cl.n * (cl.n - 1);
     }
     // diagonal items (about half a tile's work each) last
     std::stable_sort(P.hitems.begin(), P.hitems.end(), [](const SgWorkItem& a, const SgWorkItem& b) {
-        return (a.j0 >= a.i0 + SG_SYM_IB) > (b.j0 >= b.i0 + SG_SYM_IB);
+        return (a.j0 >= a.i0 + a.ni) > (b.j0 >= b.i0 + b.ni);
     });
     P.n_items = (int)P.hitems.size();
 }

@@ -1289,13 +1289,16 @@ __global__ void __launch_bounds__(SG_SYM_IB) coulomb_fp64_sym_kernel(
     const SgWorkItem it = items[blockIdx.x];
     if (ctrl != nullptr && (ctrl[it.cloud].done || ctrl[it.cloud].hold || ctrl[it.cloud].status != SG_OK)) return;
     const SgCloud& cl = clouds[it.cloud];
-    const int s0 = it.s01 & 0xffff, s1 = it.s01 >> 16;
     const size_t NP = (size_t)npad_total;
     const double* c = c64 + cl.poff;
-    fp64_sym_block<false>([c, NP](int a, int k) { return c[a * NP + k]; }, cl.n, cl.npad,
-                          it.i0 - cl.poff, it.j0 - cl.poff, it.nj, s0, s1, cl.quniform != 0,
-                          cl.qscale, 0.0, part + (size_t)it.slot * 3 * NP + cl.poff,
-                          part + (size_t)it.jslot * 3 * NP + cl.poff, NP, sh);
+    const auto ld = [c, NP](int a, int k) { return c[a * NP + k]; };
+    double *pi = part + (size_t)it.slot * 3 * NP + cl.poff, *pj = part + (size_t)it.jslot * 3 * NP + cl.poff;
+    if (it.tile_pair)
+        fp64_sym_tile_block<false>(ld, cl.n, it.i0 - cl.poff, it.j0 - cl.poff, it.tile_pair & 255,
+                                   it.tile_pair >> 8, cl.quniform != 0, cl.qscale, 0.0, pi, pj, NP, sh);
+    else
+        fp64_sym_block<false>(ld, cl.n, cl.npad, it.i0 - cl.poff, it.j0 - cl.poff, it.nj,
+                              cl.quniform != 0, cl.qscale, 0.0, pi, pj, NP, sh);
 }
 
 // Every ordered pair, for clouds whose symmetric partial sums would not fit

@@ -18,6 +18,12 @@
 // in registers over the item's j-tiles.
 //
 // Measured: 1,000 ions 26.1 us (ordered pairs: 47.3), 5,003 ions 499 us (1,029).
+//
+// Small sets have too few such items for the device.  There a block takes one pair of
+// 32-ion tiles, a quarter of the rotation steps in each warp, and adds the warps' parts
+// before it stores them: an ion has npad / 32 + 1 slots (1,000 ions: 33, where eighths of a
+// 128 x 32 item's steps as items of their own left it 264 slots to sum).  The smallest sets
+// share a pair's steps between two or four blocks.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -32,6 +38,7 @@ namespace {
 struct Fp64SymShared {
     double tj[4][32];      // x, y, z, charge weight of the j-tile
     double sj[4][3][32];   // per warp: its sums for the j-tile's ions
+    double si[4][3][32];   // (tile pairs) ... for the i-tile's
 };
 
 // One step's pair: i-side sums a, j-side sums b (subtracted: the pair's force changes
@@ -92,8 +99,7 @@ __device__ __forceinline__ void sym_tile(const double (*tj)[32], int s0, int s1,
 // [3][ps] from the cloud's first padded ion.
 template <bool SOFT, class Load>
 __device__ __forceinline__ void fp64_sym_block(const Load& ld, int n, int npad, int i0, int j0,
-                                               int nj, int s0, int s1, bool uniform, double qs,
-                                               double eps2, double* __restrict__ pi,
+                                               int nj, bool uniform, double qs, double eps2, double* __restrict__ pi,
                                                double* __restrict__ pj, size_t ps,
                                                Fp64SymShared& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -122,13 +128,13 @@ __device__ __forceinline__ void fp64_sym_block(const Load& ld, int n, int npad, 
         if (!mine || jt < iw) {
             sj[0][lane] = sj[1][lane] = sj[2][lane] = 0.0;
         } else if (jt == iw) {
-            sym_tile<false, SOFT, true>(sh.tj, s0, s1, xi, yi, zi, qi, eps2, ax, ay, az, sj[0],
+            sym_tile<false, SOFT, true>(sh.tj, 0, 32, xi, yi, zi, qi, eps2, ax, ay, az, sj[0],
                                         sj[1], sj[2]);
         } else if (noq) {
-            sym_tile<true, SOFT, false>(sh.tj, s0, s1, xi, yi, zi, qi, eps2, ax, ay, az, sj[0],
+            sym_tile<true, SOFT, false>(sh.tj, 0, 32, xi, yi, zi, qi, eps2, ax, ay, az, sj[0],
                                         sj[1], sj[2]);
         } else {
-            sym_tile<false, SOFT, false>(sh.tj, s0, s1, xi, yi, zi, qi, eps2, ax, ay, az, sj[0],
+            sym_tile<false, SOFT, false>(sh.tj, 0, 32, xi, yi, zi, qi, eps2, ax, ay, az, sj[0],
                                          sj[1], sj[2]);
         }
         __syncthreads();
@@ -147,11 +153,66 @@ __device__ __forceinline__ void fp64_sym_block(const Load& ld, int n, int npad, 
     }
 }
 
+// Part `part` of `parts` (a power of two up to 4) of one pair of 32-ion tiles, i0 <= j0, by
+// a block of 128 threads; arguments as above.
+template <bool SOFT, class Load>
+__device__ __forceinline__ void fp64_sym_tile_block(const Load& ld, int n, int i0, int j0,
+                                                    int part, int parts, bool uniform, double qs, double eps2,
+                                                    double* __restrict__ pi,
+                                                    double* __restrict__ pj, size_t ps,
+                                                    Fp64SymShared& sh) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double xi = ld(0, i0 + lane), yi = ld(1, i0 + lane), zi = ld(2, i0 + lane);
+    double qi = ld(3, i0 + lane), ax = 0.0, ay = 0.0, az = 0.0;
+    if (uniform) qi = qi != 0.0 ? 1.0 : 0.0;
+    {
+        double v = ld(warp, j0 + lane);
+        if (warp == 3 && uniform) v = v != 0.0 ? 1.0 : 0.0;
+        sh.tj[warp][lane] = v;
+    }
+    __syncthreads();
+    double(*sj)[32] = sh.sj[warp];
+    const int steps = 8 / parts, s0 = steps * (4 * part + warp), s1 = s0 + steps;
+    if (j0 == i0)
+        sym_tile<false, SOFT, true>(sh.tj, s0, s1, xi, yi, zi, qi, eps2, ax, ay, az, sj[0], sj[1],
+                                    sj[2]);
+    else if (uniform && j0 + 32 <= n)  // all weights 1
+        sym_tile<true, SOFT, false>(sh.tj, s0, s1, xi, yi, zi, qi, eps2, ax, ay, az, sj[0], sj[1],
+                                    sj[2]);
+    else
+        sym_tile<false, SOFT, false>(sh.tj, s0, s1, xi, yi, zi, qi, eps2, ax, ay, az, sj[0], sj[1],
+                                     sj[2]);
+    sh.si[warp][0][lane] = ax;
+    sh.si[warp][1][lane] = ay;
+    sh.si[warp][2][lane] = az;
+    __syncthreads();
+    if (warp < 3) {
+        double v = (sh.si[0][warp][lane] + sh.si[1][warp][lane]) +
+                   (sh.si[2][warp][lane] + sh.si[3][warp][lane]);
+        double u = (sh.sj[0][warp][lane] + sh.sj[1][warp][lane]) +
+                   (sh.sj[2][warp][lane] + sh.sj[3][warp][lane]);
+        pi[warp * ps + (size_t)(i0 + lane)] = uniform ? v * qs : v;
+        pj[warp * ps + (size_t)(j0 + lane)] = uniform ? u * qs : u;
+    }
+}
+
+// Sets with fewer 128 x 32 blocks than this per SM take tile pairs, and share each between
+// up to four blocks while those find an SM each.  A Dormand-Prince attempt, us, 128 x 32
+// items (in eighths where there are few) / tile pairs: 64 ions 78 / 65, 300 92 / 83, 1,000
+// 231 / 196, 1,500 323 / 320, 2,000 567 / 503, 3,000 1,036 / 1,015, 4,000 1,749 / 1,707, 5,003
+// 2,615 / 2,670.
+constexpr double kSymTilePairs = 16.0;
+inline int sym_parts(double tile_pairs, int n_sm) {
+    int parts = 1;
+    while (parts < 4 && 2 * parts * tile_pairs <= n_sm) parts *= 2;
+    return parts;
+}
+
 // ---- one set of ions on its own (allocation-free entry point, CUNBODY slot) -----------
 // Work items of one set of npad ions, in the order of their i-blocks: K j-tiles each, or
-// 1/bands of the rotation steps of one tile.
+// (K = 0) pairs of 32-ion tiles in `parts` parts.
 struct SymPlan {
-    int K, bands, items, slots;
+    int K, parts, items, slots;
 };
 
 __host__ __device__ inline int sym_chunks(int npad, int b, int K) {
@@ -161,24 +222,22 @@ __host__ __device__ inline int sym_chunks(int npad, int b, int K) {
 // The plan for a device of n_sm SMs whose slots hold at most cap doubles: at least 4
 // items per SM (as plan_sym in capi.cu), more j-tiles per item until the slots fit.
 inline SymPlan sym_plan(int npad, int n_sm, size_t cap) {
-    const int nb = (npad + SG_SYM_IB - 1) / SG_SYM_IB;
+    const int nb = (npad + SG_SYM_IB - 1) / SG_SYM_IB, nt = npad / SG_SYM_JT;
     double tiles = 0.0;
     for (int b = 0; b < nb; b++) tiles += sym_chunks(npad, b, 1);
-    SymPlan p{1, 1, 0, 0};
-    while (p.bands < 8 && tiles * p.bands < 4.0 * n_sm) p.bands *= 2;
-    if (p.bands == 1) p.K = std::max(1, (int)(tiles / (16.0 * n_sm)));
+    const int parts = sym_parts(0.5 * nt * (nt + 1), n_sm);
+    if (tiles < kSymTilePairs * n_sm && (size_t)(nt + 1) * parts * 3 * npad <= cap)
+        return SymPlan{0, parts, nt * (nt + 1) / 2 * parts, (nt + 1) * parts};
+    SymPlan p{std::max(1, (int)(tiles / (16.0 * n_sm))), 1, 0, 0};
     for (;;) {
         p.items = p.slots = 0;
         for (int b = 0; b < nb; b++) {
             const int q = sym_chunks(npad, b, p.K);
-            p.items += q * p.bands;
-            if ((b + 1 + q) * p.bands > p.slots) p.slots = (b + 1 + q) * p.bands;
+            p.items += q;
+            p.slots = std::max(p.slots, b + 1 + q);
         }
-        if ((size_t)p.slots * 3 * npad <= cap || (p.bands == 1 && p.K >= npad / SG_SYM_JT)) return p;
-        if (p.bands > 1)
-            p.bands /= 2;
-        else
-            p.K++;
+        if ((size_t)p.slots * 3 * npad <= cap || p.K >= nt) return p;
+        p.K++;
     }
 }
 
@@ -187,17 +246,29 @@ __global__ void __launch_bounds__(SG_SYM_IB) sym_set_kernel(Load ld, int n, int 
                                                             bool uniform, double qs, double eps2,
                                                             double* part) {
     __shared__ Fp64SymShared sh;
-    int it = blockIdx.x, b = 0, q = sym_chunks(npad, 0, p.K);
-    while (it >= q * p.bands) {
-        it -= q * p.bands;
+    const size_t slot = (size_t)3 * npad;
+    int it = blockIdx.x, b = 0;
+    if (p.K == 0) {
+        const int band = it % p.parts;
+        it /= p.parts;
+        int q = npad / SG_SYM_JT;
+        while (it >= q) {
+            it -= q--;
+            b++;
+        }
+        fp64_sym_tile_block<SOFT>(ld, n, 32 * b, 32 * (b + it), band, p.parts, uniform, qs, eps2,
+                                  part + ((b + it + 1) * p.parts + band) * slot,
+                                  part + (b * p.parts + band) * slot, (size_t)npad, sh);
+        return;
+    }
+    int q = sym_chunks(npad, 0, p.K);
+    while (it >= q) {
+        it -= q;
         q = sym_chunks(npad, ++b, p.K);
     }
-    const int c = it / p.bands, band = it % p.bands, step = SG_SYM_JT / p.bands;
-    const int j0 = b * SG_SYM_IB + c * p.K * SG_SYM_JT;
-    fp64_sym_block<SOFT>(ld, n, npad, b * SG_SYM_IB, j0, min(p.K * SG_SYM_JT, npad - j0),
-                         band * step, (band + 1) * step, uniform, qs, eps2,
-                         part + (size_t)((b + 1 + c) * p.bands + band) * 3 * npad,
-                         part + (size_t)(b * p.bands + band) * 3 * npad, (size_t)npad, sh);
+    const int j0 = b * SG_SYM_IB + it * p.K * SG_SYM_JT;
+    fp64_sym_block<SOFT>(ld, n, npad, b * SG_SYM_IB, j0, min(p.K * SG_SYM_JT, npad - j0), uniform,
+                         qs, eps2, part + (b + 1 + it) * slot, part + b * slot, (size_t)npad, sh);
 }
 
 // out[i][c] = scale[i] (or f) times the sum of ion i's slots, [slot][3][npad]: R ions a
@@ -215,7 +286,7 @@ __global__ void __launch_bounds__(256) sym_sum_kernel(const double* __restrict__
     double s[3] = {0.0, 0.0, 0.0};
     if (i < n) {
         const int b = i / SG_SYM_IB;
-        const int ns = p.K ? (b + 1 + sym_chunks(npad, b, p.K)) * p.bands : p.slots;
+        const int ns = p.K ? b + 1 + sym_chunks(npad, b, p.K) : p.slots;
 #pragma unroll 4
         for (int sl = g; sl < ns; sl += G)
 #pragma unroll

@@ -100,7 +100,7 @@ struct SgWorkItem {
     int32_t i0, ni;
     int32_t j0, nj;
     int32_t slot;
-    int32_t jslot, s01;  // FP64 symmetric items: j-side slot, rotation steps s0 | s1 << 16
+    int32_t jslot, tile_pair;  // FP64 unordered items: j-side slot; parts << 8 | part of a tile pair
 };
 
 // Leaf pairs of shape 17.  Far: leaf `leaf` of the cloud against its leaves [j0, j0 + n),
@@ -148,7 +148,7 @@ struct SgCloud {
     // shape 17: fixed-point scales (powers of two) of the far sums and their estimate
     float far_fs, far_fs2, near_fs2;
     int32_t leafs;  // shape 17: k-d ordered leaf pairs (else the plain kernel)
-    int32_t sym_k, sym_bands;  // FP64 symmetric items: j-tiles per item (0: ordered pairs), bands
+    int32_t sym_k;  // FP64 unordered items of K j-tiles (0: every ion has nslots slots)
     int32_t pad4;
 };
 
@@ -158,7 +158,7 @@ struct SgCloud {
 __host__ __device__ inline int sg_sym_slots(const SgCloud& cl, int p) {
     const int b = p / SG_SYM_IB;
     const int tiles = cl.npad / SG_SYM_JT - b * (SG_SYM_IB / SG_SYM_JT);
-    return (b + 1 + (tiles + cl.sym_k - 1) / cl.sym_k) * cl.sym_bands;
+    return b + 1 + (tiles + cl.sym_k - 1) / cl.sym_k;
 }
 
 // Per-cloud Dormand-Prince controller (the scalar part of _ode_vars, bin/ode.h:58-97).
