@@ -91,9 +91,9 @@ struct Problem {
     std::vector<int> hspec0;
     std::vector<double> hmass0;
     double *pmass = nullptr, *pmass0 = nullptr;  // print masses (dissociation), both orders
-    int* fix_list = nullptr;   // FP32c fix-up work lists: counts, then (ion, cloud) pairs
-    double* fix_part = nullptr;  // fix-up work units' corrections [listed][units][3]
-    int* fix_done = nullptr;     // finished units per listed ion (zero between calls)
+    int* fix_list = nullptr;   // FP32c fix-up work list: counts, units, ions past its end
+    double* fix_part = nullptr;  // fix-up work units' parts [SG_FIX_CAP][3]
+    int* fix_done = nullptr;     // finished units by an ion's first (zero between calls)
     // operation sequence
     std::vector<sg_field_params> fp0;  // field parameters as created / set by the caller
     std::vector<SgOp> hops;
@@ -739,12 +739,11 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     CK(dalloc(&P.pmass, N));
     CK(dalloc(&P.pmass0, N));
     // two lists (near-only ions; ions with a far fix-up): counts, then N pairs each
-    CK(dalloc(&P.fix_list, 4 + 6 * N));
+    CK(dalloc(&P.fix_list, 4 + 4 * SG_FIX_CAP + 2 * N));
     CK(cudaMemset(P.fix_list, 0, 4 * sizeof(int)));
-    // two lists (row re-evaluations, far corrections) of up to SG_FIX_CHUNKED_CAP ions
-    CK(dalloc(&P.fix_part, (size_t)2 * SG_FIX_CHUNKED_CAP * SG_FIX_UNITS * 3));
-    CK(dalloc(&P.fix_done, 2 * SG_FIX_CHUNKED_CAP));
-    CK(cudaMemset(P.fix_done, 0, sizeof(int) * 2 * SG_FIX_CHUNKED_CAP));
+    CK(dalloc(&P.fix_part, (size_t)3 * SG_FIX_CAP));
+    CK(dalloc(&P.fix_done, SG_FIX_CAP));
+    CK(cudaMemset(P.fix_done, 0, sizeof(int) * SG_FIX_CAP));
     CK(cudaMemset(P.pmass, 0, N * sizeof(double)));
     CK(cudaMemset(P.pmass0, 0, N * sizeof(double)));
     CK(dalloc(&P.bbox, (size_t)std::max(P.ntiles, 1) * 8));

@@ -547,8 +547,11 @@ __global__ void __launch_bounds__(128) near_list_kernel(const SgCloud* __restric
                                                         int n_leaves, int cap,
                                                         const float* __restrict__ bbox,
                                                         int* __restrict__ counts,
-                                                        unsigned short* __restrict__ lists) {
+                                                        unsigned short* __restrict__ lists,
+                                                        int* __restrict__ fix_list) {
     sg_griddep_wait();
+    // the fix-up lists of this call (a memset otherwise)
+    if (blockIdx.x == 0 && threadIdx.x < 2) fix_list[threadIdx.x] = 0;
     const int leaf = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (leaf >= n_leaves) return;
     const int c = leaf_cloud[leaf];
@@ -1387,11 +1390,11 @@ __global__ void __launch_bounds__(NT) coulomb_fp64_kernel(const double* __restri
 // kinds of fix-up of a flagged ion
 constexpr int kFixNear = 1, kFixFar = 2;
 
-// blocks of the fix-up kernel (each takes every kFixupBlocks-th work unit)
-constexpr int kFixupBlocks = 512;
-// work units of one listed ion in the fix-up kernel, and the listed ions that get them
-constexpr int kFarChunks = SG_FIX_UNITS;
-constexpr int kChunkedCap = SG_FIX_CHUNKED_CAP;
+// Blocks of the fix-up kernel, each with every grid-th work unit: three per SM are resident,
+// and the more there are the better the units even out (512 clouds of 500 to 1,000 ions, us
+// per attempt: 512 blocks 2,938, 2,048 2,768), but they all have to start (167 of <= 300: 335,
+// 339).
+inline int fixup_blocks(int n_total) { return std::min(2048, std::max(512, n_total / 128)); }
 // batches up to this many ions fix their flagged ions inside the reduction's blocks
 constexpr int kInBlockFixupMax = SG_FINISH_MAX_IONS;
 
@@ -1411,14 +1414,11 @@ struct Corr3 {
     double x, y, z;
 };
 
-// Block-wide sum of one value per thread and component; the result is thread 0's.
-template <int NTH>
-__device__ Corr3 block_sum3(double ax, double ay, double az, FixupShared<NTH>& sh) {
-    // An FP64 addition takes a warp 64 cycles whatever its lanes hold: 32 lanes x 3
-    // components in six (the upper half-warp takes y while the lower sums x, then every other
-    // 8 lanes z), the warps' parts in three.
-    static_assert(NTH == 256, "eight warps");
-    const int li = threadIdx.x, warp = li >> 5, lane = li & 31;
+// Sums of one value per lane and component: x in lane 0, y in lane 16, z in lane 8.  An FP64
+// addition takes a warp 64 cycles whatever its lanes hold: 32 lanes x 3 components in six
+// (the upper half-warp takes y while the lower sums x, then every other 8 lanes z).
+__device__ __forceinline__ double warp_sum3(double ax, double ay, double az) {
+    const int lane = threadIdx.x & 31;
     const bool up = lane & 16, odd = lane & 8;
     double a = up ? ay : ax;
     a += __shfl_xor_sync(0xffffffffu, up ? ax : ay, 16);
@@ -1426,6 +1426,15 @@ __device__ Corr3 block_sum3(double ax, double ay, double az, FixupShared<NTH>& s
     double v = odd ? az : a;
     v += __shfl_xor_sync(0xffffffffu, odd ? a : az, 8);
     for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Block-wide sum of one value per thread and component; the result is thread 0's.
+template <int NTH>
+__device__ Corr3 block_sum3(double ax, double ay, double az, FixupShared<NTH>& sh) {
+    static_assert(NTH == 256, "eight warps");
+    const int li = threadIdx.x, warp = li >> 5, lane = li & 31;
+    double v = warp_sum3(ax, ay, az);
     if (lane == 0) sh.wsum[warp][0] = v;
     if (lane == 16) sh.wsum[warp][1] = v;
     if (lane == 8) sh.wsum[warp][2] = v;
@@ -1657,8 +1666,13 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
     const double* __restrict__ c64, const float* __restrict__ bbox, float* __restrict__ risk,
     int* __restrict__ ran, const SgCheck* __restrict__ chk, int split, LeafSums leaf) {
     sg_griddep_wait();
-    // this block's share of its row block: cap / split rows
+    // this block's share of its row block: cap / split rows; leaf sums have no slots to
+    // share, so the first block of a leaf cloud's row block takes all of it, a thread per row
     SgRowBlock rb = rows[blockIdx.x / split];
+    if (F32 && !INBLOCK && clouds[rb.cloud].leafs) {
+        if (blockIdx.x % split) return;
+        split = 1;
+    }
     const int R = rb.cap / split, G = SG_ROWS / R;  // powers of two
     const int first = (int)(blockIdx.x % split) * R;
     rb.i0 += first;
@@ -1792,13 +1806,18 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
     if (!F32) return;
     if (!INBLOCK) {
         if (kind) {
-            // three lists: ions whose row is re-evaluated (kFixNear), the far-only ones, and
-            // the rows of small clouds
-            const int l = kind == kFixFar ? 1 : cl.npad <= SG_SMALL_ROW ? 2 : 0;
-            const int at = atomicAdd(fix_list + l, 1);
-            const size_t base = 4 + 2 * (size_t)n_total * l;
-            fix_list[base + 2 * at] = i;
-            fix_list[base + 2 * at + 1] = rb.cloud | (kind << 28);
+            // the ion's work units; past the list's end, the ion whole
+            const int U = sg_fix_units(cl.npad), at = atomicAdd(fix_list, U);
+            int4* units = reinterpret_cast<int4*>(fix_list + 4);
+            const int ck = rb.cloud | kind << 28;
+            const bool fits = at + U <= SG_FIX_CAP;
+            for (int c = 0; c < U && at + c < SG_FIX_CAP; c++)
+                units[at + c] = make_int4(fits ? i : -1, ck, c | U << 16, at);
+            if (!fits) {
+                int* whole = fix_list + 4 + 4 * SG_FIX_CAP + 2 * (size_t)atomicAdd(fix_list + 1, 1);
+                whole[0] = i;
+                whole[1] = ck;
+            }
             if (counters != nullptr) atomicAdd(counters, 1);
         }
         return;
@@ -1821,15 +1840,13 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
         fixup_ion(cl, flist[k], fkind[k], c32, c64, npad_total, out, n_total, bbox, sh);
 }
 
-// The flagged ions of a whole batch, in two lists: the ions whose row is re-evaluated in
-// FP64 (kFixNear) and the far-only ones (kFixFar).  Each of the first kChunkedCap ions of
-// a list is kFarChunks work units, so that the scan of a large cloud is spread over
-// blocks: each unit leaves its part in fix_part and the last unit of the ion (counted in
-// fix_done) combines them in unit order -- writing the row, or adding the far correction
-// -- so the result does not depend on the order the units ran in.  Units are numbered
-// so that every ion's first units come first.  Ions past the caps are one unit each.
-// Blocks of 256 threads, three per SM: the units of a 65,536-ion call run in one or two
-// waves.
+// The flagged ions of a whole batch: re-evaluated rows (kFixNear) and far corrections, in
+// units of ~1,024 j-ions (sg_fix_units).  Each unit of an ion leaves its part in fix_part and
+// the last of them (counted in fix_done) adds the parts in unit order -- writing the row,
+// or adding the far correction -- so the result does not depend on the order the units
+// ran in.  Ions that found the list full are one unit each.  FP64-bound: rows of up to
+// 4,096 ions as units of their own left the device waiting for the longest (128 clouds of
+// 64 to 8,192 ions, 596 rows a call: 84 us, 68 so).
 constexpr int kFixupThreads = 256;
 __global__ void __launch_bounds__(kFixupThreads, 3) coulomb_fixup_kernel(
     const SgCloud* __restrict__ clouds, const float* __restrict__ c32,
@@ -1839,69 +1856,60 @@ __global__ void __launch_bounds__(kFixupThreads, 3) coulomb_fixup_kernel(
     sg_griddep_wait();
     __shared__ FixupShared<kFixupThreads> sh;
     __shared__ int last;
-    constexpr int U = kFarChunks;
-    const int cn = fix_list[0], cf = fix_list[1], cs = fix_list[2];
-    const int* row_list = fix_list + 4;
-    const int* far_list = row_list + 2 * (size_t)n_total;
-    const int* small_list = far_list + 2 * (size_t)n_total;
-    const int cnc = min(cn, kChunkedCap), cfc = min(cf, kChunkedCap);
-    const int u_rows = cnc * U + (cn - cnc);
-    const int u_all = u_rows + cfc * U + (cf - cfc), units = u_all + cs;
-    for (int u = blockIdx.x; u < units; u += gridDim.x) {
-        if (u >= u_all) {  // a small cloud's row: one unit
-            const int i = small_list[2 * (u - u_all)], ck = small_list[2 * (u - u_all) + 1];
-            fixup_ion<kFixupThreads>(clouds[ck & 0x0FFFFFFF], i, kFixNear, c32, c64, npad_total,
-                                     out, n_total, bbox, sh);
-            continue;
-        }
-        const bool row = u < u_rows;
-        const int v = row ? u : u - u_rows;
-        const int nc = row ? cnc : cfc;
-        const int* list = row ? row_list : far_list;
-        if (v >= nc * U) {  // past the cap: the whole ion in this unit
-            const int k = nc + (v - nc * U);
-            const int ck = list[2 * k + 1];
-            fixup_ion<kFixupThreads>(clouds[ck & 0x0FFFFFFF], list[2 * k], ck >> 28, c32, c64,
+    const int units = min(fix_list[0], SG_FIX_CAP), whole = fix_list[1];
+    const int4* list = reinterpret_cast<const int4*>(fix_list + 4);
+    for (int u = blockIdx.x; u < units + whole; u += gridDim.x) {
+        if (u >= units) {
+            const int* w = fix_list + 4 + 4 * SG_FIX_CAP + 2 * (size_t)(u - units);
+            fixup_ion<kFixupThreads>(clouds[w[1] & 0x0FFFFFFF], w[0], w[1] >> 28, c32, c64,
                                      npad_total, out, n_total, bbox, sh);
             continue;
         }
-        const int k = v % nc, c = v / nc;
-        const int i = list[2 * k];
-        const SgCloud& cl = clouds[list[2 * k + 1] & 0x0FFFFFFF];
+        const int4 it = list[u];
+        const int i = it.x, c = it.z & 0xffff, U = it.z >> 16, base = it.w;
+        if (i < 0) continue;  // of an ion that did not fit
+        const SgCloud& cl = clouds[it.y & 0x0FFFFFFF];
+        const bool row = (it.y >> 28) & kFixNear;
         Corr3 r{0.0, 0.0, 0.0};
         if (row)
             r = fixup_row<kFixupThreads>(cl, i, c64, npad_total, c, U, sh);
         else if (bbox != nullptr)
             r = fixup_far<kFixupThreads>(cl, i, c32, npad_total, bbox, c, U, sh);
-        const size_t slot = (row ? 0 : (size_t)kChunkedCap) + (size_t)k;
         if (threadIdx.x == 0) {
-            double* fp = fix_part + (slot * U + c) * 3;
-            fp[0] = r.x;
-            fp[1] = r.y;
-            fp[2] = r.z;
-            __threadfence();
-            last = atomicAdd(&fix_done[slot], 1) == U - 1;
+            last = U == 1;
+            if (U > 1) {
+                double* fp = fix_part + 3 * (size_t)u;
+                fp[0] = r.x;
+                fp[1] = r.y;
+                fp[2] = r.z;
+                __threadfence();
+                last = atomicAdd(&fix_done[base], 1) == U - 1;
+            }
         }
         __syncthreads();
-        if (last && threadIdx.x == 0) {
-            __threadfence();
-            const volatile double* vp = fix_part + slot * U * 3;
-            double sx = 0.0, sy = 0.0, sz = 0.0;
-            for (int q = 0; q < U; q++) {
-                sx += vp[3 * q];
-                sy += vp[3 * q + 1];
-                sz += vp[3 * q + 2];
+        if (last && threadIdx.x < 32) {
+            if (U > 1) {
+                __threadfence();
+                const volatile double* vp = fix_part + 3 * (size_t)base;
+                r = {0.0, 0.0, 0.0};
+                for (int q = threadIdx.x; q < U; q += 32) {
+                    r.x += vp[3 * q];
+                    r.y += vp[3 * q + 1];
+                    r.z += vp[3 * q + 2];
+                }
+                const double v = warp_sum3(r.x, r.y, r.z);
+                r.x = v;
+                r.y = __shfl_sync(0xffffffffu, v, 16);
+                r.z = __shfl_sync(0xffffffffu, v, 8);
+                if (threadIdx.x == 0) fix_done[base] = 0;  // ready for the next call
             }
-            if (row) {
-                out[i] = sx;
-                out[(size_t)n_total + i] = sy;
-                out[2 * (size_t)n_total + i] = sz;
-            } else {
-                out[i] += sx;
-                out[(size_t)n_total + i] += sy;
-                out[2 * (size_t)n_total + i] += sz;
+            if (threadIdx.x == 0) {
+                double* o = out + i;
+                const size_t N = (size_t)n_total;
+                o[0] = row ? r.x : o[0] + r.x;
+                o[N] = row ? r.y : o[N] + r.y;
+                o[2 * N] = row ? r.z : o[2 * N] + r.z;
             }
-            fix_done[slot] = 0;  // ready for the next call
         }
         __syncthreads();
     }
@@ -2009,7 +2017,7 @@ cudaError_t sg_launch_coulomb_fp32c(const SgCoulombArgs& a, cudaStream_t s) {
                     a.c32, a.c64, a.items, a.clouds, a.ctrl, a.part, a.npad_total, a.errword);
             if (a.n_near <= 0) break;
             sg_launch(near_list_kernel, (a.n_leaves + 3) / 4, 128, 0, s, a.clouds, a.ctrl, a.leaf_cloud,
-                      a.n_leaves, a.near_cap, a.bbox, a.near_count, a.near_list);
+                      a.n_leaves, a.near_cap, a.bbox, a.near_count, a.near_list, a.fix_list);
             {
                 const LeafAcc acc{a.leaf_sum, a.leaf_fmx, a.leaf_n_close, a.leaf_close};
                 sg_launch(a.far_estimate ? coulomb_leaf_kernel<true> : coulomb_leaf_kernel<false>,
@@ -2049,9 +2057,8 @@ cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* r
                                      int row_cap, int fp32c, double* out, int n_total,
                                      int* counters, cudaStream_t s) {
     if (n_rows <= 0) return cudaSuccess;
-    // leaf sums have no slots to share: a thread per row
-    const bool whole = fp32c && a.variant == SG_C32_FAR_ONCE && a.n_items <= 0 && n_total > kInBlockFixupMax;
     const int take = n_total <= kInBlockFixupMax || a.max_slots > 24 ? 16 : 64;
+    const bool whole = fp32c && a.variant == SG_C32_FAR_ONCE && a.n_items <= 0 && n_total > kInBlockFixupMax;
     const int split = whole ? 1 : std::max(1, row_cap / take);
     if (fp32c) {
         const float* bbox = sg_variant_sorted(a.variant) ? a.bbox : nullptr;
@@ -2064,14 +2071,16 @@ cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* r
                 a.c32, a.c64, bbox, a.risk, a.ran, a.chk, split, leaf);
             return cudaGetLastError();
         }
-        cudaError_t e = cudaMemsetAsync(a.fix_list, 0, 3 * sizeof(int), s);
-        if (e != cudaSuccess) return e;
-        coulomb_reduce_kernel<true, false><<<n_rows * split, SG_ROWS, 0, s>>>(
+        if (a.n_near <= 0) {  // near_list_kernel has cleared it otherwise
+            cudaError_t e = cudaMemsetAsync(a.fix_list, 0, 2 * sizeof(int), s);
+            if (e != cudaSuccess) return e;
+        }
+        sg_launch(coulomb_reduce_kernel<true, false>, n_rows * split, SG_ROWS, 0, s, 
             rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, a.fix_list,
             a.c32, a.c64, nullptr, a.risk, a.ran, a.chk, split, leaf);
         // a fixed grid that strides over however many work units there are (a batch of
         // small clouds can flag a few percent of its ions; unused blocks exit at once)
-        const int grid = kFixupBlocks;
+        const int grid = fixup_blocks(n_total);
         sg_launch(coulomb_fixup_kernel, grid, kFixupThreads, 0, s, 
             a.clouds, a.c32, a.c64, a.npad_total, out, n_total, a.fix_list, bbox,
             a.fix_part, a.fix_done);

@@ -10,6 +10,32 @@ namespace {
 
 typedef SgDpArgs DpArgs;
 
+// u as float-float: h = u rounded to 24 bits (ties away from zero), l = the rest rounded.
+// By integers: a conversion between FP64 and FP32 takes a warp 64 cycles, like any FP64
+// instruction, and the three here with the difference were 4 of the ~30 a component of a
+// stage takes; the integer path is 10 instructions of 1 to 8 cycles.
+__device__ __forceinline__ void split_double(double u, float& h, float& l) {
+    const long long b = __double_as_longlong(u);
+    const int e = (int)((unsigned long long)b >> 52) & 0x7ff;
+    if (e >= 1023 - 70 && e <= 1023 + 100) {
+        // the fraction's low 29 bits, as a signed distance from the nearest multiple of 2^29
+        const long long r = b + 0x10000000ll;  // a carry into the exponent is the rounded value
+        const int d = (int)(b & 0x1fffffffll) - ((b & 0x10000000ll) ? 0x20000000 : 0);
+        const unsigned top = (unsigned)((unsigned long long)r >> 32);
+        // sign, exponent rebased by 1023 - 127, 23 fraction bits
+        const unsigned hb = (top & 0x80000000u) |
+                            ((((top & 0x7fffffffu) << 3) | (unsigned)((unsigned long long)r >> 29 & 7)) -
+                             ((1023u - 127u) << 23));
+        h = __uint_as_float(hb);
+        // d units of 2^(e - 1075), with u's sign
+        const float s = __uint_as_float((unsigned)(e - 1075 + 127) << 23 | (top & 0x80000000u));
+        l = __fmul_rn(__int2float_rn(d), s);
+    } else {  // zero, tiny, huge or not finite
+        h = __double2float_rn(u);
+        l = __double2float_rn(u - (double)h);
+    }
+}
+
 // Frame coordinate of one component: high part and remainder.
 __device__ __forceinline__ float write_coord(const DpArgs& a, const SgCloud& cl, int c, int ig,
                                              double x) {
@@ -17,9 +43,10 @@ __device__ __forceinline__ float write_coord(const DpArgs& a, const SgCloud& cl,
     a.c64[c * NP + ig] = x;
     if (!a.fp32c) return 0.f;
     const double u = (x - (c == 0 ? cl.cx : c == 1 ? cl.cy : cl.cz)) * cl.invL;
-    const float h = __double2float_rn(u);
+    float h, l;
+    split_double(u, h, l);
     a.c32[c * NP + ig] = h;
-    a.c32[(4 + c) * NP + ig] = __double2float_rn(u - (double)h);
+    a.c32[(4 + c) * NP + ig] = l;
     return h;
 }
 

@@ -204,7 +204,8 @@ __device__ __forceinline__ void store_state(const SgFusedArgs& f, const FusedArr
         if (c < 3) {
             const int li = lo + w.row[u];
             const double v = (w.st[u] - (c == 0 ? cl.cx : c == 1 ? cl.cy : cl.cz)) * cl.invL;
-            const float hi = __double2float_rn(v), low = __double2float_rn(v - (double)hi);
+            float hi, low;
+            split_double(v, hi, low);
             if (WIDE) {
                 float* C = f.c32 + set * 7 * NP + cl.poff + li;
                 C[c * NP] = hi;

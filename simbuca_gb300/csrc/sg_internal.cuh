@@ -74,9 +74,13 @@ inline cudaError_t sg_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 #define SG_SYM_IB 128
 #define SG_SYM_JT 32
 #define SG_SYM_MAX_IONS 131072
-// FP32c fix-up kernel: work units per listed ion, and the listed ions that get them
-#define SG_FIX_UNITS 16
-#define SG_FIX_CHUNKED_CAP 4096
+// FP32c fix-up: work units of a flagged ion of a cloud of npad ions (1,024 j-ions each, at
+// most 64 of them), and units the list of a call holds.
+#define SG_FIX_CAP 32768
+__host__ __device__ inline int sg_fix_units(int npad) {
+    const int u = (npad + 1023) / 1024;
+    return u < 64 ? u : 64;
+}
 
 // Bounded device waits: a wait gives up after this many nanoseconds of
 // %globaltimer and raises SG_TIMEOUT in the context's error word.

@@ -176,3 +176,27 @@ def test_flagged_ion_gets_its_exact_row(ctx, n, variant):
     print(n, variant, "planted ion", e0, "all ions", summary(e))
     assert e0 <= 1e-12
     assert e.max() <= BOUND
+
+
+@pytest.mark.parametrize("n", [9000, 70000])
+def test_more_flagged_ions_than_the_unit_list_holds(ctx, n):
+    """A lattice of alternating charges: the terms of an inner ion cancel, so that most ions
+    are flagged -- more work units than their list holds, the rest whole.  Every flagged
+    row is exact to FP64 rounding: n terms whose magnitudes add up to ~4 pi R in units of a
+    neighbour's field (R = 21, 41 spacings across): 1e-16 sqrt(n) 250 < 1e-11 of that field,
+    in either form's order of summation.  The others keep the FP32c bound (of fields of the
+    order of a neighbour's)."""
+    side = int(np.ceil(n ** (1 / 3)))
+    g = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    pos = 1e-5 * g.astype(np.float64)
+    q = np.where(g.sum(1) % 2 == 0, 1.0, -1.0)
+    kq = np.abs(kq_of(np.full(n, configs.M_CS), np.ones(n)))
+    ctx.fixup_count()
+    a32 = ctx.coulomb_accel(pos, q, kq, SG_PREC_FP32C)
+    flagged = ctx.fixup_count()
+    a64 = ctx.coulomb_accel(pos, q, kq, SG_PREC_FP64)
+    err = np.abs(a32 - a64).max(1) / (kq[0] / 1e-10)
+    print(n, "flagged", flagged, "largest", err.max())
+    assert flagged > 4000
+    assert err.max() <= BOUND
+    assert (err <= 1e-11).sum() >= flagged
