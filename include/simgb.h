@@ -261,8 +261,8 @@ int sg_batch_set_proposer(sg_ctx* ctx, const float* w, double safety);
  * clouds are small, in the plain ion order and without a recorder, operations,
  * dissociation, step log or proposer, run whole attempts in one launch, one thread-block
  * cluster of up to 16 CTAs per cloud.  sg_set_fused(ctx, mode): 1 (default) where it is
- * faster than the tiled kernels (one cloud of up to ~800 ions; several smaller ones while
- * their clusters fit on the device together); 2 for clouds of up to 2,048 ions; 0 never.
+ * faster than the tiled kernels (one cloud of up to ~4,000 ions; several smaller ones while
+ * their CTAs fit on the device together); 2 for clouds of up to 2,048 ions; 0 never.
  * sg_batch_fused gives the cluster size
  * the current batch runs with (0: the tiled kernels).  sg_fused_timing: CUDA-event time
  * of the fused launches while sg_set_kernel_timing is on. */

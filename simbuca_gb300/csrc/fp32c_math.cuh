@@ -94,6 +94,21 @@ __device__ __forceinline__ double inv_r3_fp64(double r2) {
     return fma(y3 * e, fma(e, 1.875, 1.5), y3);
 }
 
+// Sums of one value per lane and component: x in lane 0, y in lane 16, z in lane 8.  An FP64
+// addition takes a warp 64 cycles whatever its lanes hold: 32 lanes x 3 components in six
+// (the upper half-warp takes y while the lower sums x, then every other 8 lanes z).
+__device__ __forceinline__ double warp_sum3(double ax, double ay, double az) {
+    const int lane = threadIdx.x & 31;
+    const bool up = lane & 16, odd = lane & 8;
+    double a = up ? ay : ax;
+    a += __shfl_xor_sync(0xffffffffu, up ? ax : ay, 16);
+    az += __shfl_xor_sync(0xffffffffu, az, 16);
+    double v = odd ? az : a;
+    v += __shfl_xor_sync(0xffffffffu, odd ? a : az, 8);
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // ---- float-float (unevaluated sums hi + lo of two floats, ~48 bits) ------------------
 struct ff {
     float h, l;

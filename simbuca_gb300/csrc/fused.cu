@@ -17,7 +17,7 @@
 //     (float-float differences, SFU 1/r, 1/r^3 capped with float-float close pairs, partial
 //     sums folded into Kahan accumulators every 16 j-ions, the G parts added in
 //     float-float); an ion whose terms cancel strongly (sqrt(s2) > 1.5 |P|) gets its whole
-//     row in FP64 instead, spread over the CTA's warps;
+//     row in FP64 instead, spread over the CTA's warps or (larger wide clouds) all CTAs;
 //   * control: error partials go to every CTA, and every CTA decides alike
 //     (error_succes and step(), sg_error_succes; bin/ode.cpp:426-494), so the commit
 //     pos <- pos2, vel <- vel2 (bin/ode.cpp:488-489) needs no second barrier.
@@ -28,19 +28,18 @@
 // A cloud of many hundred ions has more pairs than 16 SMs take quickly: the wide form spreads
 // it over up to all SMs of the device (a cooperative launch).  There the coordinates go
 // through the batch's two global sets and the barrier is a counter in global memory, waited
-// for with a limit (SG_TIMEOUT); the rest is the same.  1,000 ions: 69 us per attempt, 124
-// in a cluster of 16, 121 in the tiled kernels.
+// for with a limit (SG_TIMEOUT); the rest is the same.  1,000 ions: 67 us per attempt, 124
+// in a cluster of 16, 121 in the tiled kernels; 4,096 ions 193, 223 in the tiled kernels.
 //
 // Measured, one cloud, us per attempt (state, coordinates and sums through global memory
 // with 15 barriers, close pairs found by a second scan, a flagged row per warp -> this
-// form): 64 ions 70 -> 34, 300 131 -> 60, 512 155 -> 72.  What is left is the
+// form): 64 ions 70 -> 34, 300 131 -> 56, 512 155 -> 67.  What is left is the
 // chain stage - barrier - pairs of dependent instructions.
 #include <cooperative_groups.h>
 #include <math.h>
 
 #include <algorithm>
-
-#include <algorithm>
+#include <type_traits>
 
 #include "dp_stage.cuh"
 #include "fp32c_math.cuh"
@@ -66,6 +65,7 @@ struct FusedShared {
     SgFieldCoef fk[SG_MAX_STAGES];
     FusedNote note[2];
     int expired;  // wide: a wait ran out
+    float part[kWarps][8];     // parts of the ions that several warps share
     double red[2][kWarps][3];  // parts of a flagged row; [0][w][0]: error partials
     double x0;
     int ew, hold, wtest;  // at the launch
@@ -226,45 +226,62 @@ __device__ __forceinline__ void store_state(const SgFusedArgs& f, const FusedArr
 __device__ __forceinline__ void load_coords(const SgFusedArgs& f, const FusedArrays& s,
                                             const SgCloud& cl, int set) {
     const size_t NP = (size_t)f.npad;
-    const int nv = s.npc / 4;
-#pragma unroll 4
-    for (int q = threadIdx.x; q < 6 * nv; q += kThreads) {
-        const int a = q / nv, v = q - a * nv;
-        const float4* src = reinterpret_cast<const float4*>(
-            f.c32 + (set * 7 + (a < 3 ? a : a + 1)) * NP + cl.poff);
-        reinterpret_cast<float4*>(s.C + a * s.npc)[v] = __ldcg(src + v);
+    const float4* src = reinterpret_cast<const float4*>(f.c32 + set * 7 * NP + cl.poff);
+    const size_t row = NP / 4;  // rows of whole 16-byte words
+#pragma unroll 2
+    for (int v = threadIdx.x; v < s.npc / 4; v += kThreads) {
+        float4 x[6];
+#pragma unroll
+        for (int a = 0; a < 6; a++) x[a] = __ldcg(src + (a < 3 ? a : a + 1) * row + v);
+#pragma unroll
+        for (int a = 0; a < 6; a++) reinterpret_cast<float4*>(s.C + a * s.npc)[v] = x[a];
     }
     __syncthreads();
 }
 
-// Wide: the barrier of a cloud's CTAs, a counter that each raises by one.  All of them are
+// Wide: a cloud's CTAs and their barrier, a counter that each raises by one.  All of them are
 // resident (cooperative launch); a wait gives up after SG_WAIT_NS.
-__device__ __forceinline__ void wide_arrive(int* count) {
-    __syncthreads();  // the CTA's stores come before its arrival
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(count, 1);
-    }
-}
-__device__ __forceinline__ bool wide_wait(const int* count, int target, FusedShared& sh,
-                                          unsigned long long limit_ns = SG_WAIT_NS) {
-    if (threadIdx.x == 0) {
-        int seen;
-        unsigned long long t0 = 0, t;
-        for (;;) {
-            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
-            if (seen >= target) break;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (t0 == 0) t0 = t;
-            if (t - t0 > limit_ns) {
-                sh.expired = 1;
-                break;
-            }
+struct WideGroup {
+    int* count;   // arrivals, departures
+    int R, r;     // CTAs of the cloud, this one's rank
+    int target;   // arrivals so far
+    int* flag_n;  // [2] flagged ions of the stage in either coordinate set ...
+    int* flags;   // [2][SG_WIDE_FLAGS] ... cloud indices
+
+    __device__ __forceinline__ void arrive() {
+        __syncthreads();  // the CTA's stores come before its arrival
+        target += R;
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(count, 1);
         }
     }
-    __syncthreads();
-    return sh.expired == 0;
-}
+    // past: arrivals beyond the last ones to wait for (the wait test)
+    __device__ __forceinline__ bool wait(FusedShared& sh, int past = 0,
+                                         unsigned long long limit_ns = SG_WAIT_NS) {
+        if (threadIdx.x == 0) {
+            int seen;
+            unsigned long long t0 = 0, t;
+            for (;;) {
+                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
+                if (seen >= target + past) break;
+                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+                if (t0 == 0) t0 = t;
+                if (t - t0 > limit_ns) {
+                    sh.expired = 1;
+                    break;
+                }
+            }
+        }
+        __syncthreads();
+        return sh.expired == 0;
+    }
+};
+// Wide clouds of more padded ions share a flagged ion's FP64 row between all their CTAs, two
+// more barriers a stage with a flagged ion and one without (~1.5 us each); a row in one CTA
+// takes 4 us per 1,000 ions, and the others wait for it (3,000 ions, us per attempt: 205
+// with rows in one CTA, 157 shared; 1,500 112 / 112).
+constexpr int kShareRows = 1536;
 
 // This CTA's rows [lo, lo + m) of set `set` into the other CTAs' shared memory, 16 bytes a
 // store: 6 m / 4 words of frame coordinates and 3 m / 2 of SI ones for each.
@@ -287,64 +304,55 @@ __device__ __forceinline__ void push_coords(cg::cluster_group& cluster, const Fu
     }
 }
 
-// Coulomb sums of the CTA's mo ions (cloud indices lo ...) at coordinate set `set` into
-// s.P, in the FP32-compensated form; risk: where the in-run check's inputs go (null: not
-// written).
-template <bool WIDE>
-__device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedArrays& s,
-                                              const SgCloud& cl, int lo, int mo, int set,
-                                              float* risk, FusedShared& sh) {
-    const int tid = threadIdx.x;
-    const int npc = s.npc;
-    const float* X = s.C + (WIDE ? 0 : set * 6 * npc);
+// The sums of one thread: every G-th packed j-pair (j = 2p, 2p + 1) from pair q on against ion
+// li, so that the G threads of an ion read consecutive 8-byte words of shared memory (no bank
+// conflicts; the ions of a warp read the same words).  Every 8 pairs (16 j-ions) the FP32
+// partial sums are folded into the Kahan accumulators.  GT: G where it is known.
+//
+// Bound by the issue and latency of a warp's instructions (18 packed FP32x2, 7 loads, ~6 ALU
+// per packed pair, four warps a sub-partition): close pairs are looked for once per four
+// packed pairs, and only the last ones of a cloud test for its end.  us per attempt, both
+// tests for each pair / so: 300 ions 60 / 56, 1,000 72 / 67, 4,096 206 / 193.  Two ions a
+// thread (half the loads per pair) spilled and gave 190 at 4,096, 65 at 300.
+struct IonSums {
+    ff x, y, z;
+    float s2;
+};
+template <int GT, class Load>
+__device__ __forceinline__ IonSums ion_pairs(const float* X, const float* Q, int npc, int q, int G0,
+                                             int li, float wc, const double* SX, const double* SQ,
+                                             size_t ND, double psc, const Load& ld) {
+    const int G = GT ? GT : G0;
+    const int npair = npc / 2;
     const float* Y = X + npc;
     const float* Z = X + 2 * npc;
     const float* XL = X + 3 * npc;
     const float* YL = X + 4 * npc;
     const float* ZL = X + 5 * npc;
-    const float* Q = s.Q;
-    const size_t ND = WIDE ? (size_t)f.npad : (size_t)npc;
-    const double* SX = WIDE ? f.c64 + set * 4 * ND + cl.poff : s.D + set * 3 * npc;
-    const double* SY = SX + ND;
-    const double* SZ = SX + 2 * ND;
-    // other CTAs write the global coordinates: through L2
-    auto ld = [](const double* p) { return WIDE ? __ldcg(p) : *p; };
-    const double* SQ = f.c64 + 3 * (size_t)f.npad + cl.poff;  // charges: never rewritten here
-    // G threads per ion.  Thread q of an ion takes the packed j-pairs q, q + G, q + 2G, ...
-    // (j = 2p, 2p + 1), so the G threads of an ion read consecutive 8-byte words of
-    // shared memory (no bank conflicts; the ions of a warp read the same words); every 8
-    // pairs (16 j-ions) its FP32 partial sums are folded into the Kahan accumulators.
-    int G = 1;
-    while (2 * G * mo <= kThreads && 2 * G <= 32) G *= 2;
-    const int il = tid / G, q = tid - il * G;
-    const int npair = npc / 2;
-    const float wc = cl.wc;
-    ff px{0.f, 0.f}, py{0.f, 0.f}, pz{0.f, 0.f};
-    float ps2 = 0.f;
-    const int li = lo + il;  // index in the cloud's coordinate arrays
-    if (il < mo) {
-        const float xih = X[li], yih = Y[li], zih = Z[li];
-        const float xil = XL[li], yil = YL[li], zil = ZL[li];
-        const f2 xh = pk(xih, xih), yh = pk(yih, yih), zh = pk(zih, zih);
-        const f2 xl = pk(xil, xil), yl = pk(yil, yil), zl = pk(zil, zil);
-        const f2 tiny2 = pk(kTiny, kTiny);
-        float ks[3] = {0.f, 0.f, 0.f}, kc[3] = {0.f, 0.f, 0.f}, s2 = 0.f, fmx = 0.f;
-        ff cx{0.f, 0.f}, cy{0.f, 0.f}, cz{0.f, 0.f};
-        for (int b0 = q; b0 < npair; b0 += 2 * kFold * G) {
-            // close pairs of these 32 j-ions, a bit each (the self pair, dx = 0, with them)
-            unsigned close = 0u;
+    const float xih = X[li], yih = Y[li], zih = Z[li];
+    const float xil = XL[li], yil = YL[li], zil = ZL[li];
+    const f2 xh = pk(xih, xih), yh = pk(yih, yih), zh = pk(zih, zih);
+    const f2 xl = pk(xil, xil), yl = pk(yil, yil), zl = pk(zil, zil);
+    const f2 tiny2 = pk(kTiny, kTiny);
+    float ks[3] = {0.f, 0.f, 0.f}, kc[3] = {0.f, 0.f, 0.f}, s2 = 0.f, fmx = 0.f;
+    ff cx{0.f, 0.f}, cy{0.f, 0.f}, cz{0.f, 0.f};
+    for (int b0 = q; b0 < npair; b0 += 2 * kFold * G) {
+        // close pairs of these 32 j-ions, a bit each (the self pair, dx = 0, with them)
+        unsigned close = 0u;
 #pragma unroll
-            for (int hb = 0; hb < 2; hb++) {
-                f2 ax = 0ull, ay = 0ull, az = 0ull;
+        for (int hb = 0; hb < 2; hb++) {
+            f2 ax = 0ull, ay = 0ull, az = 0ull;
 #pragma unroll
-                for (int u0 = 0; u0 < kFold; u0 += 4) {
-                    if (b0 + (hb * kFold + u0) * G >= npair) break;
+            for (int u0 = 0; u0 < kFold; u0 += 4) {
+                const int p0 = b0 + (hb * kFold + u0) * G;
+                if (p0 >= npair) break;
+                float y3[8], m4 = 0.f;
+                auto four = [&](auto tail) {
 #pragma unroll
-                    for (int u = u0; u < u0 + 4; u++) {
+                    for (int u = 0; u < 4; u++) {
                         // past the cloud's last pair: pair 0 again, with no weight
-                        const int p = b0 + (hb * kFold + u) * G;
-                        const bool ok = p < npair;
-                        const int jj = ok ? 2 * p : 0;
+                        const bool ok = !decltype(tail)::value || p0 + u * G < npair;
+                        const int jj = ok ? 2 * (p0 + u * G) : 0;
                         const f2 Xj = *reinterpret_cast<const f2*>(X + jj);
                         const f2 Yj = *reinterpret_cast<const f2*>(Y + jj);
                         const f2 Zj = *reinterpret_cast<const f2*>(Z + jj);
@@ -358,78 +366,128 @@ __device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedA
                         f2 r2 = fma2(dx, dx, tiny2);
                         r2 = fma2(dy, dy, r2);
                         r2 = fma2(dz, dz, r2);
-                        float ra, rb;
+                        float ra, rb, ua, ub;
                         upk(r2, ra, rb);
                         const f2 yv = pk(rsqrt_approx(ra), rsqrt_approx(rb));
-                        const f2 y3 = mul2(mul2(yv, yv), yv);
-                        float ua, ub;
-                        upk(y3, ua, ub);
-                        // the strongest term below the cap; a capped one counts below
-                        const bool ca = ua > wc, cb = ub > wc;
-                        fmx = fmaxf(fmx, ok ? fmaxf(ca ? 0.f : ua, cb ? 0.f : ub) : 0.f);
-                        if (ok && ca) close |= 1u << (2 * (hb * kFold + u));
-                        if (ok && cb) close |= 2u << (2 * (hb * kFold + u));
+                        upk(mul2(mul2(yv, yv), yv), ua, ub);
                         const f2 w = mul2(ok ? Qj : 0ull, pk(fminf(ua, wc), fminf(ub, wc)));
                         ax = fma2(w, dx, ax);
                         ay = fma2(w, dy, ay);
                         az = fma2(w, dz, az);
+                        y3[2 * u] = ok ? ua : 0.f;
+                        y3[2 * u + 1] = ok ? ub : 0.f;
+                        m4 = fmaxf(m4, fmaxf(y3[2 * u], y3[2 * u + 1]));
                     }
-                }
-                float a, b;
-                upk(ax, a, b);
-                const float tx = __fadd_rn(a, b);
-                upk(ay, a, b);
-                const float ty = __fadd_rn(a, b);
-                upk(az, a, b);
-                const float tz = __fadd_rn(a, b);
-                kahan_add(ks[0], kc[0], tx);
-                kahan_add(ks[1], kc[1], ty);
-                kahan_add(ks[2], kc[2], tz);
-                s2 = fmaf(tx, tx, fmaf(ty, ty, fmaf(tz, tz, s2)));
-            }
-            // close pairs: the exact term minus the capped FP32 one (close_term_ff; the
-            // closest in FP64 from the SI coordinates); a capped term is a candidate for
-            // the strongest
-            while (close) {
-                const int bit = __ffs(close) - 1;
-                close &= close - 1u;
-                const int jj = 2 * (b0 + (bit >> 1) * G) + (bit & 1);
-                if (jj == li || Q[jj] == 0.f) continue;
-                const PairF pr = pair_f32(X[jj], Y[jj], Z[jj], XL[jj], YL[jj], ZL[jj], xih, yih,
-                                          zih, xil, yil, zil);
-                fmx = fmaxf(fmx, capped_term_y3(pr.y3, wc));
-                const float wf = __fmul_rn(Q[jj], wc);
-                ff dx, dy, dz;
-                if (pr.y3 <= kVeryClose) {
-                    close_term_ff(ff_diff(X[jj], XL[jj], xih, xil), ff_diff(Y[jj], YL[jj], yih, yil),
-                                  ff_diff(Z[jj], ZL[jj], zih, zil), Q[jj], wf, pr, dx, dy, dz);
+                };
+                if (p0 + 3 * G < npair)
+                    four(std::false_type{});
+                else
+                    four(std::true_type{});
+                if (m4 > wc) {
+                    // which, and the strongest of the others (a capped one counts below)
+#pragma unroll
+                    for (int e = 0; e < 8; e++) {
+                        if (y3[e] > wc)
+                            close |= 1u << (2 * (hb * kFold + u0) + e);
+                        else
+                            fmx = fmaxf(fmx, y3[e]);
+                    }
                 } else {
-                    const double rx = ld(SX + li) - ld(SX + jj), ry = ld(SY + li) - ld(SY + jj),
-                                 rz = ld(SZ + li) - ld(SZ + jj);
-                    const double w = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz) / cl.psc;
-                    const double c0 = w * rx - (double)wf * (double)pr.dx,
-                                 c1 = w * ry - (double)wf * (double)pr.dy,
-                                 c2 = w * rz - (double)wf * (double)pr.dz;
-                    dx.h = (float)c0;
-                    dx.l = (float)(c0 - (double)dx.h);
-                    dy.h = (float)c1;
-                    dy.l = (float)(c1 - (double)dy.h);
-                    dz.h = (float)c2;
-                    dz.l = (float)(c2 - (double)dz.h);
+                    fmx = fmaxf(fmx, m4);
                 }
-                cx = ff_add(cx, dx);
-                cy = ff_add(cy, dy);
-                cz = ff_add(cz, dz);
             }
+            float a, b;
+            upk(ax, a, b);
+            const float tx = __fadd_rn(a, b);
+            upk(ay, a, b);
+            const float ty = __fadd_rn(a, b);
+            upk(az, a, b);
+            const float tz = __fadd_rn(a, b);
+            kahan_add(ks[0], kc[0], tx);
+            kahan_add(ks[1], kc[1], ty);
+            kahan_add(ks[2], kc[2], tz);
+            s2 = fmaf(tx, tx, fmaf(ty, ty, fmaf(tz, tz, s2)));
         }
-        px = ff_add({ks[0], -kc[0]}, cx);
-        py = ff_add({ks[1], -kc[1]}, cy);
-        pz = ff_add({ks[2], -kc[2]}, cz);
-        ps2 = conditioning_s2(s2, fmx);
+        // close pairs: the exact term minus the capped FP32 one (close_term_ff; the
+        // closest in FP64 from the SI coordinates); a capped term is a candidate for
+        // the strongest
+        while (close) {
+            const int bit = __ffs(close) - 1;
+            close &= close - 1u;
+            const int jj = 2 * (b0 + (bit >> 1) * G) + (bit & 1);
+            if (jj == li || Q[jj] == 0.f) continue;
+            const PairF pr = pair_f32(X[jj], Y[jj], Z[jj], XL[jj], YL[jj], ZL[jj], xih, yih, zih, xil,
+                                      yil, zil);
+            fmx = fmaxf(fmx, capped_term_y3(pr.y3, wc));
+            const float wf = __fmul_rn(Q[jj], wc);
+            ff dx, dy, dz;
+            if (pr.y3 <= kVeryClose) {
+                close_term_ff(ff_diff(X[jj], XL[jj], xih, xil), ff_diff(Y[jj], YL[jj], yih, yil),
+                              ff_diff(Z[jj], ZL[jj], zih, zil), Q[jj], wf, pr, dx, dy, dz);
+            } else {
+                const double rx = ld(SX + li) - ld(SX + jj),
+                             ry = ld(SX + ND + li) - ld(SX + ND + jj),
+                             rz = ld(SX + 2 * ND + li) - ld(SX + 2 * ND + jj);
+                const double w = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz) / psc;
+                const double c0 = w * rx - (double)wf * (double)pr.dx,
+                             c1 = w * ry - (double)wf * (double)pr.dy,
+                             c2 = w * rz - (double)wf * (double)pr.dz;
+                dx.h = (float)c0;
+                dx.l = (float)(c0 - (double)dx.h);
+                dy.h = (float)c1;
+                dy.l = (float)(c1 - (double)dy.h);
+                dz.h = (float)c2;
+                dz.l = (float)(c2 - (double)dz.h);
+            }
+            cx = ff_add(cx, dx);
+            cy = ff_add(cy, dy);
+            cz = ff_add(cz, dz);
+        }
     }
-    // the G parts of each ion (G consecutive lanes of one warp), in a fixed order, still in
-    // float-float; lane 0 of the G holds the ion
-    for (int o = G / 2; o > 0; o >>= 1) {
+    return IonSums{ff_add({ks[0], -kc[0]}, cx), ff_add({ks[1], -kc[1]}, cy),
+                   ff_add({ks[2], -kc[2]}, cz), conditioning_s2(s2, fmx)};
+}
+
+// Coulomb sums of the CTA's mo ions (cloud indices lo ...) at coordinate set `set` into
+// s.P, in the FP32-compensated form; risk: where the in-run check's inputs go (null: not
+// written).
+// One copy for the six stages of an attempt (inlined, they took minutes to compile).
+template <bool WIDE>
+__device__ __noinline__ bool coulomb_phase(const SgFusedArgs& f, const SgCloud& cl, int mc, int lo,
+                                           int mo, int set, float* risk, FusedShared& sh,
+                                           WideGroup& g) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    const FusedArrays s = carve<WIDE>(dyn, cl.npad, mc);
+    const int tid = threadIdx.x;
+    const int npc = s.npc;
+    const float* X = s.C + (WIDE ? 0 : set * 6 * npc);
+    const size_t ND = WIDE ? (size_t)f.npad : (size_t)npc;
+    const double* SX = WIDE ? f.c64 + set * 4 * ND + cl.poff : s.D + set * 3 * npc;
+    const double* SY = SX + ND;
+    const double* SZ = SX + 2 * ND;
+    // other CTAs write the global coordinates: through L2
+    auto ld = [](const double* p) { return WIDE ? __ldcg(p) : *p; };
+    const double* SQ = f.c64 + 3 * (size_t)f.npad + cl.poff;  // charges: never rewritten here
+    // G threads per ion: as many as the CTA has, up to four warps of them
+    int G = 1;
+    while (2 * G * mo <= kThreads && 2 * G <= 128 && 4 * G <= npc) G *= 2;
+    const int il = tid / G, q = tid - il * G;
+    const int li = lo + il;  // index in the cloud's coordinate arrays
+    IonSums p{{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, 0.f};
+    if (il < mo) {
+        switch (G) {
+            case 128: p = ion_pairs<128>(X, s.Q, npc, q, G, li, cl.wc, SX, SQ, ND, cl.psc, ld); break;
+            case 64: p = ion_pairs<64>(X, s.Q, npc, q, G, li, cl.wc, SX, SQ, ND, cl.psc, ld); break;
+            case 32: p = ion_pairs<32>(X, s.Q, npc, q, G, li, cl.wc, SX, SQ, ND, cl.psc, ld); break;
+            case 16: p = ion_pairs<16>(X, s.Q, npc, q, G, li, cl.wc, SX, SQ, ND, cl.psc, ld); break;
+            default: p = ion_pairs<0>(X, s.Q, npc, q, G, li, cl.wc, SX, SQ, ND, cl.psc, ld);
+        }
+    }
+    // the G parts of each ion, in a fixed order, still in float-float: first those of a warp
+    // (consecutive lanes), then the warps'; the first thread of the G holds the ion
+    ff px = p.x, py = p.y, pz = p.z;
+    float ps2 = p.s2;
+    for (int o = min(G, 32) / 2; o > 0; o >>= 1) {
         ff v;
         v.h = __shfl_down_sync(0xffffffffu, px.h, o);
         v.l = __shfl_down_sync(0xffffffffu, px.l, o);
@@ -442,6 +500,27 @@ __device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedA
         pz = ff_add(pz, v);
         ps2 += __shfl_down_sync(0xffffffffu, ps2, o);
     }
+    if (G > 32) {
+        float* v = sh.part[tid >> 5];
+        if ((tid & 31) == 0) {
+            v[0] = px.h;
+            v[1] = px.l;
+            v[2] = py.h;
+            v[3] = py.l;
+            v[4] = pz.h;
+            v[5] = pz.l;
+            v[6] = ps2;
+        }
+        __syncthreads();
+        if (q == 0)
+            for (int w = 1; w < G / 32; w++) {
+                v += 8;
+                px = ff_add(px, {v[0], v[1]});
+                py = ff_add(py, {v[2], v[3]});
+                pz = ff_add(pz, {v[4], v[5]});
+                ps2 += v[6];
+            }
+    }
     // the conditioning test (frame units for a unit charge)
     if (il < mo && q == 0) {
         const float pf2 = fmaf(px.h, px.h, fmaf(py.h, py.h, pz.h * pz.h));
@@ -449,6 +528,11 @@ __device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedA
         s.flag[il] = flagged;
         if (flagged) {
             s.list[atomicAdd(&sh.nflag, 1)] = il;
+            if (WIDE && npc > kShareRows) {
+                const int at = atomicAdd(g.flag_n + set, 1);
+                if (at < SG_WIDE_FLAGS) g.flags[set * SG_WIDE_FLAGS + at] = li;
+                s.flag[il] = at + 1;
+            }
         } else {
             s.P[il] = make_float2(px.h, px.l);
             s.P[s.mc + il] = make_float2(py.h, py.l);
@@ -461,6 +545,57 @@ __device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedA
         }
     }
     __syncthreads();
+    if (WIDE && npc > kShareRows) {
+        // shared rows: every CTA of the cloud takes its j-ions of each flagged ion, a warp an
+        // ion, and the owners add the parts in rank order
+        g.arrive();
+        if (!g.wait(sh)) return false;
+        const int all = __ldcg(g.flag_n + set);
+        if (all == 0) return true;
+        if (all <= SG_WIDE_FLAGS) {
+            const int warp = tid >> 5, lane = tid & 31;
+            const int len = (npc / 32 + g.R - 1) / g.R * 32;
+            const int j0 = g.r * len, j1 = min(npc, j0 + len);
+            double* parts = f.flag_part + (size_t)set * SG_WIDE_FLAGS * SG_FUSED_MAX_WIDE * 3;
+            for (int k = warp; k < all; k += kWarps) {
+                const int lf = __ldcg(g.flags + set * SG_WIDE_FLAGS + k);
+                const double xi = ld(SX + lf), yi = ld(SY + lf), zi = ld(SZ + lf);
+                double ax = 0.0, ay = 0.0, az = 0.0;
+                for (int jj = j0 + lane; jj < j1; jj += 32) {
+                    if (jj == lf) continue;
+                    const double rx = xi - ld(SX + jj), ry = yi - ld(SY + jj), rz = zi - ld(SZ + jj);
+                    const double wq = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz);
+                    ax = fma(wq, rx, ax);
+                    ay = fma(wq, ry, ay);
+                    az = fma(wq, rz, az);
+                }
+                __syncwarp();
+                const double v = j0 < j1 ? warp_sum3(ax, ay, az) : 0.0;
+                if (lane == 0 || lane == 8 || lane == 16)
+                    parts[((size_t)k * SG_FUSED_MAX_WIDE + blockIdx.x) * 3 +
+                          (lane == 0 ? 0 : lane == 16 ? 1 : 2)] = v;
+            }
+            g.arrive();
+            if (!g.wait(sh)) return false;
+            for (int k = warp; k < sh.nflag; k += kWarps) {
+                const int fi = s.list[k];
+                const double* p = parts + ((size_t)(s.flag[fi] - 1) * SG_FUSED_MAX_WIDE +
+                                           (blockIdx.x - g.r)) * 3;
+                double ax = 0.0, ay = 0.0, az = 0.0;
+                for (int q = lane; q < g.R; q += 32) {
+                    ax += __ldcg(p + 3 * q);
+                    ay += __ldcg(p + 3 * q + 1);
+                    az += __ldcg(p + 3 * q + 2);
+                }
+                __syncwarp();
+                const double v = warp_sum3(ax, ay, az);
+                if (lane == 0 || lane == 8 || lane == 16)
+                    *reinterpret_cast<double*>(s.P + (lane == 0 ? 0 : lane == 16 ? 1 : 2) * s.mc + fi) = v;
+            }
+            __syncthreads();
+            return true;
+        }
+    }
     // Flagged ions: the whole row in FP64 from the SI coordinates, which replaces the ion's
     // sum (re-evaluating only its dominant pairs would keep the rounding of the FP32
     // additions made while they were in a partial sum).  The CTA's warps share a row by 32
@@ -482,16 +617,7 @@ __device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedA
                 az = fma(wq, rz, az);
             }
             __syncwarp();
-            // 32 lanes x 3 components in six additions: the upper half-warp takes y while
-            // the lower sums x, then every other 8 lanes z
-            const bool up = lane & 16;
-            double a = up ? ay : ax;
-            a += __shfl_xor_sync(0xffffffffu, up ? ax : ay, 16);
-            az += __shfl_xor_sync(0xffffffffu, az, 16);
-            const bool odd = lane & 8;
-            double v = odd ? az : a;
-            v += __shfl_xor_sync(0xffffffffu, odd ? a : az, 8);
-            for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            const double v = warp_sum3(ax, ay, az);
             if (lane == 0) red[warp][0] = v;
             if (lane == 16) red[warp][1] = v;
             if (lane == 8) red[warp][2] = v;
@@ -505,6 +631,7 @@ __device__ __forceinline__ void coulomb_phase(const SgFusedArgs& f, const FusedA
         }
     }
     if (nf > 0) __syncthreads();
+    return true;
 }
 
 // Control of an attempt with error norm err (thread 0 of every CTA alike): error_succes,
@@ -538,7 +665,8 @@ __device__ __forceinline__ void control_phase(FusedShared& sh, const SgCloud& cl
 }
 
 template <int PASSES, bool WIDE>
-__global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs f, int mc) {
+__global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(const __grid_constant__ SgFusedArgs f,
+                                                                     int mc) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ FusedShared sh;
     cg::cluster_group cluster = cg::this_cluster();
@@ -591,16 +719,20 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
         }
     }
     // wide: the cloud's barrier counter and notes
-    int* count = WIDE ? f.barrier + 2 * c : nullptr;
+    WideGroup g{};
     double* notes = WIDE ? f.notes + (size_t)c * 2 * (SG_FUSED_MAX_WIDE + 1) : nullptr;
-    int arrived = 0;
     bool ok = true;
     if (WIDE) {
-        wide_arrive(count);
-        arrived += R;
-        ok = sh.wtest != 1 ? wide_wait(count, arrived, sh)
-                           : wide_wait(count, arrived + 1, sh,  // the wait test: never
-                                       1000ull * max(f.flags[SG_FLAG_WAIT_US], 1));
+        g.count = f.barrier + 2 * c;
+        g.R = R;
+        g.r = r;
+        g.flag_n = f.flag_n + 2 * c;
+        g.flags = f.flag_list + 2 * SG_WIDE_FLAGS * c;
+        if (r == 0 && tid == 0) g.flag_n[0] = g.flag_n[1] = 0;
+        g.arrive();
+        ok = sh.wtest != 1 ? g.wait(sh)
+                           : g.wait(sh, 1,  // the wait test: never
+                                    1000ull * max(f.flags[SG_FLAG_WAIT_US], 1));
     } else {
         cluster.sync();  // every CTA runs, and has read the control block
     }
@@ -632,19 +764,21 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
         stage_before<S>(s, cl, sh.fk[S], w);                                           \
         __syncthreads();                                                               \
     } else if (WIDE) {                                                                 \
-        wide_arrive(count);                                                            \
+        g.arrive();                                                                    \
         stage_before<S>(s, cl, sh.fk[S], w);                                           \
-        ok = wide_wait(count, (arrived += R), sh);                                     \
+        ok = g.wait(sh);                                                               \
         if (!ok) break;                                                                \
+        if (r == 0 && tid == 0) g.flag_n[((S) & 1) ^ 1] = 0;                           \
         load_coords(f, s, cl, (S) & 1);                                                \
-        coulomb_phase<WIDE>(f, s, cl, lo, mo, (S) & 1, (S) == 7 ? f.risk : nullptr, sh); \
+        ok = coulomb_phase<WIDE>(f, cl, mc, lo, mo, (S) & 1, (S) == 7 ? f.risk : nullptr, sh, g); \
+        if (!ok) break;                                                                \
     } else {                                                                           \
         __syncthreads();                                                               \
         if (mo > 0) push_coords(cluster, s, lo, m, (S) & 1, ctas, r);                  \
         auto token = cluster.barrier_arrive();                                         \
         stage_before<S>(s, cl, sh.fk[S], w);                                           \
         cluster.barrier_wait(std::move(token));                                        \
-        coulomb_phase<WIDE>(f, s, cl, lo, mo, (S) & 1, (S) == 7 ? f.risk : nullptr, sh); \
+        coulomb_phase<WIDE>(f, cl, mc, lo, mo, (S) & 1, (S) == 7 ? f.risk : nullptr, sh, g); \
     }
         SG_FUSED_STAGE(2)
         stage_after<2>(s, cl, h, atol, rtol, coul, w);
@@ -681,8 +815,8 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
                     if (own0) nt[SG_FUSED_MAX_WIDE] = sh.x0;
                 }
             }
-            wide_arrive(count);
-            ok = wide_wait(count, (arrived += R), sh);
+            g.arrive();
+            ok = g.wait(sh);
             if (!ok) break;
             if (tid < 32) {
                 double v = 0.0;
@@ -733,9 +867,9 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(SgFusedArgs
                     f.ctrl[c].done = 1;
                 }
             }
-            if (atomicAdd(count + 1, 1) == R - 1) {
-                count[0] = 0;
-                count[1] = 0;
+            if (atomicAdd(g.count + 1, 1) == R - 1) {
+                g.count[0] = 0;
+                g.count[1] = 0;
             }
         }
         if (!ok) return;

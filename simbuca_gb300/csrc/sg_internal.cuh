@@ -495,17 +495,19 @@ cudaError_t sg_dp_finish(const SgFinishArgs& f, int stage, int fp32c, cudaStream
 #define SG_FUSED_MAX_CTAS 16
 #define SG_FUSED_MAX_IONS 2048
 #define SG_FUSED_MAX_WIDE 160    // CTAs of a cloud in the wide form
-#define SG_FUSED_WIDE_IONS 4096  // ions of a cloud in the wide form
+#define SG_FUSED_WIDE_IONS 7168  // ions of a cloud in the wide form
+#define SG_WIDE_FLAGS 64         // shared flagged rows of a stage (more: each in its CTA)
 // Ordered pairs per CTA (its ions times the cloud's).  Up to SG_FUSED_CLUSTER_PAIRS a cluster
 // is faster than the wide form with more CTAs; the wide form is taken by default (sg_set_fused
 // mode 1) up to SG_FUSED_WIDE_PAIRS, clusters up to SG_FUSED_AUTO_PAIRS.  Measured on GB300, us
-// per attempt (pairs per CTA), cluster / wide / tiled kernels: one cloud of 300 ions 60 (6,000)
-// / 62 / 142, 512 71 (16,000) / 69 (2,000) / 131, 1,000 125 / 69 (8,000) / 121, 1,344 225 / 108
-// (16,000) / 156, 2,048 400 / 126 to 214 (33,000) / 150, 3,000 - / 205 (60,000) / 182; 8 of
-// 300 77 (12,000) / 60 (5,000) / 166, 16 of 300 101 (23,000) / 82 / 227, 4 of 1,000 139 / 108
-// (28,000) / 154; 70 of 100 on 2 CTAs each 67 (5,000) / 76 / 224.
+// per attempt (pairs per CTA), cluster / wide / tiled kernels: one cloud of 300 ions 56 (6,000)
+// / 62 / 142, 512 67 (16,000) / 66 (2,000) / 131, 1,000 120 / 67 (7,000) / 121, 2,048 400 / 98 to
+// 126 (29,000) / 150, 3,000 - / 155 to 171 (60,000) / 170 to 179, 4,096 - / 193 (111,000) / 223,
+// 5,000 - / 313 (165,000) / 239; 8 of 300 77 (12,000) / 60 (5,000) / 166, 16 of 300 101 (23,000)
+// / 82 / 227, 4 of 2,000 - / 192 (106,000) / 245, 2 of 4,000 - / 299 (212,000) / 309; 70 of 100 on
+// 2 CTAs each 66 (5,000) / 76 / 224.
 #define SG_FUSED_CLUSTER_PAIRS 8000
-#define SG_FUSED_WIDE_PAIRS 30000
+#define SG_FUSED_WIDE_PAIRS 120000
 #define SG_FUSED_AUTO_PAIRS 40000
 struct SgFusedArgs {
     const SgCloud* clouds;
@@ -523,6 +525,8 @@ struct SgFusedArgs {
     int ctas;
     int* barrier;   // [clouds][2] arrivals, departures; zero between launches
     double* notes;  // [clouds][2][SG_FUSED_MAX_WIDE + 1] error partials, x of the first ion
+    int *flag_n, *flag_list;  // [clouds][2], [clouds][2][SG_WIDE_FLAGS] flagged ions of a stage
+    double* flag_part;        // [2][SG_WIDE_FLAGS][SG_FUSED_MAX_WIDE][3] parts of their rows
 };
 // The cluster size (16, 8, 4 or 2) for n_clouds clouds of up to max_npad padded ions: the
 // largest with which all of them are on the device at once (clusters of 16 take the SMs of

@@ -72,7 +72,8 @@ def test_clusters_with_several_slots_per_thread(ctx):
         assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
 
 
-@pytest.mark.parametrize("counts", [[500], [1000], [1825], [1826], [300] * 8, [1000, 16, 999, 64]])
+@pytest.mark.parametrize("counts", [[500], [1000], [1536], [1537], [4096], [4500], [300] * 8,
+                                    [1000, 16, 999, 64], [2000, 40, 1900, 3]])
 def test_wide_form_against_fp64(ctx, counts):
     """The form that spreads a cloud over many CTAs: sizes of its automatic range and its
     edges, equal and uneven batches, with a close pair in every cloud; bounds as above."""
@@ -87,7 +88,7 @@ def test_wide_form_against_fp64(ctx, counts):
     out = []
     for prec in (SG_PREC_FP32C, SG_PREC_FP64):
         b = Batch(ctx, counts, [fp] * len(counts), [op] * len(counts), prec)
-        if prec == SG_PREC_FP32C and counts[0] <= 1824:
+        if prec == SG_PREC_FP32C and counts[0] <= 4096:
             assert b.fused() > 16
         b.upload(np.concatenate([c.pos for c in clouds]), np.concatenate([c.vel for c in clouds]),
                  np.concatenate([c.mass for c in clouds]),
