@@ -1225,7 +1225,7 @@ bool fused_eligible(sg_ctx* ctx, Problem& P) { return fused_form(ctx, P) != 0; }
 
 // n attempts of every active cloud at most (a cloud stops early once done or held);
 // `counted`: attempts counted towards the in-run check's interval.
-int run_fused(sg_ctx* ctx, Problem& P, int n, int counted) {
+int run_fused(sg_ctx* ctx, Problem& P, int n, int counted, int one_step = 0) {
     const bool wide = fused_form(ctx, P) == 2;
     SgFusedArgs f;
     f.clouds = P.dc;
@@ -1244,6 +1244,7 @@ int run_fused(sg_ctx* ctx, Problem& P, int n, int counted) {
     f.npad = P.npad;
     f.n_clouds = P.n_clouds;
     f.max_attempts = n;
+    f.one_step = one_step;
     f.ctas = wide ? P.fused_wide : 0;
     f.barrier = P.fused_barrier;
     f.notes = P.fused_notes;
@@ -1826,26 +1827,28 @@ int sg_dp45_step(sg_ctx* ctx, sg_step_info* info) {
     Problem& P = ctx->batch;
     if (!P.uploaded) return SG_NOT_READY;
     CK(cudaSetDevice(ctx->device));
-    // hold-on-accept on (any nonzero word) without a host-to-device copy
-    CK(cudaMemsetAsync(P.flags + 1, 1, sizeof(int), ctx->stream));
     int st = SG_OK;
-    // every cloud that is active now takes exactly one accepted step (or fails); the
-    // fused path loops over a cloud's attempts inside one launch until it holds
+    // every cloud that is active now takes exactly one accepted step (or fails).  The fused
+    // path loops over a cloud's attempts inside one launch until it has; the tiled one holds
+    // a cloud that accepts, the switch (any nonzero word) set without a host-to-device copy.
     const bool fused = fused_eligible(ctx, P);
+    if (!fused) CK(cudaMemsetAsync(P.flags + 1, 1, sizeof(int), ctx->stream));
     for (long long guard = 0; guard < (1ll << 40); guard++) {
-        st = fused ? run_fused(ctx, P, 64, 1) : run_attempts(ctx, P, 1);
+        st = fused ? run_fused(ctx, P, 64, 1, guard ? 2 : 1) : run_attempts(ctx, P, 1);
         if (st != SG_OK) break;
         st = sync_ctrl(ctx, P);
         if (st != SG_OK) break;
         bool all = true;
         for (int c = 0; c < P.n_clouds; c++) {
             const SgCtrl& s = P.hctrl[c];
-            if (!(s.done || s.hold || s.status != SG_OK)) all = false;
+            if (!(s.done || s.hold || s.status != SG_OK || (fused && s.stepped))) all = false;
         }
         if (all) break;
     }
-    CK(cudaMemsetAsync(P.flags + 1, 0, sizeof(int), ctx->stream));
-    CK(sg_clear_hold(P.dctrl, P.n_clouds, ctx->stream));
+    if (!fused) {
+        CK(cudaMemsetAsync(P.flags + 1, 0, sizeof(int), ctx->stream));
+        CK(sg_clear_hold(P.dctrl, P.n_clouds, ctx->stream));
+    }
     if (st == SG_OK) {
         // the host copy is current from the last sync: clear its hold bit the same way
         // instead of reading the control blocks back once more

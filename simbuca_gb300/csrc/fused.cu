@@ -68,7 +68,7 @@ struct FusedShared {
     float part[kWarps][8];     // parts of the ions that several warps share
     double red[2][kWarps][3];  // parts of a flagged row; [0][w][0]: error partials
     double x0;
-    int ew, hold, wtest;  // at the launch
+    int ew, wtest;  // at the launch
     int nflag;
 };
 
@@ -657,9 +657,9 @@ __device__ __forceinline__ void control_phase(FusedShared& sh, const SgCloud& cl
         cs.t = cs.t + cs.h;
         cs.h = cs.hnext;
         cs.steps++;
+        cs.stepped = 1;
         cs.rejects_here = 0;
         if (cs.t >= cs.t_end) cs.done = 1;
-        if (sh.hold) cs.hold |= 1;
     }
     cs.accepted = accepted;
 }
@@ -685,8 +685,8 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(const __gri
     const size_t N = (size_t)f.n, NP = (size_t)f.npad;
     if (tid == 0) {
         sh.cs = f.ctrl[c];
+        if (f.one_step == 1) sh.cs.stepped = 0;
         sh.ew = f.flags[SG_FLAG_ERR];
-        sh.hold = f.flags[SG_FLAG_HOLD];
         sh.wtest = f.flags[SG_FLAG_WAIT_TILE];
         sh.expired = 0;
     }
@@ -738,7 +738,9 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(const __gri
     }
     int att = 0;
     for (; ok && att < f.max_attempts; att++) {
-        if (sh.cs.done || sh.cs.hold || sh.cs.status != SG_OK || sh.ew != 0) break;
+        if (sh.cs.done || sh.cs.hold || sh.cs.status != SG_OK || sh.ew != 0 ||
+            (f.one_step && sh.cs.stepped))
+            break;
         const double t0 = sh.cs.t, h = sh.cs.h, atol = sh.cs.atol, rtol = sh.cs.rtol;
         // every stage's field coefficients, a lane each
         if (tid < MethodDP::stages) {

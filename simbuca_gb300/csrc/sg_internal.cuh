@@ -171,7 +171,8 @@ struct SgCtrl {
     // hold: bit 0 = one step per call taken, bit 1 = record ring full; either stops the
     // cloud's kernels until the host clears it
     int32_t reject, adaptive, max_rejects, status, done, accepted, rejects_here, hold;
-    int32_t method, pad2;  // 5 Dormand-Prince, 4 Cash-Karp, 1 Gear
+    int32_t method;   // 5 Dormand-Prince, 4 Cash-Karp, 1 Gear
+    int32_t stepped;  // fused path, one step per call: taken in this call
     double hf[4];          // Gear: h^2/2, h^3/6, h^4/24, h^5/120 of the initial step
     long long steps, rejects, force_evals, coulomb_evals;
     // recorder: the reference's print rule (bin/ion_fly.cpp:103-108), record due now
@@ -521,6 +522,7 @@ struct SgFusedArgs {
     int* ran;
     int n, npad, n_clouds;
     int max_attempts;  // attempts per launch at most
+    int one_step;      // 1: each cloud stops after an accepted attempt; 2: those that have not yet
     // wide form: CTAs per cloud (0: clusters), c64 and c32 hold two coordinate sets
     int ctas;
     int* barrier;   // [clouds][2] arrivals, departures; zero between launches
