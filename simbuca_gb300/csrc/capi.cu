@@ -1225,6 +1225,13 @@ bool fused_eligible(sg_ctx* ctx, Problem& P) { return fused_form(ctx, P) != 0; }
 
 // n attempts of every active cloud at most (a cloud stops early once done or held);
 // `counted`: attempts counted towards the in-run check's interval.
+// ions of the largest cloud
+int big_fused(const Problem& P) {
+    int big = 0;
+    for (const SgCloud& cl : P.hc) big = std::max(big, cl.n);
+    return big;
+}
+
 int run_fused(sg_ctx* ctx, Problem& P, int n, int counted, int one_step = 0) {
     const bool wide = fused_form(ctx, P) == 2;
     SgFusedArgs f;
@@ -1245,6 +1252,8 @@ int run_fused(sg_ctx* ctx, Problem& P, int n, int counted, int one_step = 0) {
     f.n_clouds = P.n_clouds;
     f.max_attempts = n;
     f.one_step = one_step;
+    f.kappa2 = big_fused(P) <= SG_FUSED_LOOSE_IONS && P.n_clouds * SG_FUSED_MAX_CTAS <= ctx->n_sm
+                   ? 2.25f : 1.21f;
     f.ctas = wide ? P.fused_wide : 0;
     f.barrier = P.fused_barrier;
     f.notes = P.fused_notes;

@@ -16,7 +16,7 @@
 //     interleaved G-ths of the cloud, in the FP32-compensated form of the tiled kernels
 //     (float-float differences, SFU 1/r, 1/r^3 capped with float-float close pairs, partial
 //     sums folded into Kahan accumulators every 16 j-ions, the G parts added in
-//     float-float); an ion whose terms cancel strongly (sqrt(s2) > 1.5 |P|) gets its whole
+//     float-float); an ion whose terms cancel strongly (s2 > kappa2 |P|^2) gets its whole
 //     row in FP64 instead, spread over the CTA's warps or (larger wide clouds) all CTAs;
 //   * control: error partials go to every CTA, and every CTA decides alike
 //     (error_succes and step(), sg_error_succes; bin/ode.cpp:426-494), so the commit
@@ -28,7 +28,7 @@
 // A cloud of many hundred ions has more pairs than 16 SMs take quickly: the wide form spreads
 // it over up to all SMs of the device (a cooperative launch).  There the coordinates go
 // through the batch's two global sets and the barrier is a counter in global memory, waited
-// for with a limit (SG_TIMEOUT); the rest is the same.  1,000 ions: 67 us per attempt, 124
+// for with a limit (SG_TIMEOUT); the rest is the same.  1,000 ions: 93 us per attempt, 124
 // in a cluster of 16, 121 in the tiled kernels; 4,096 ions 193, 223 in the tiled kernels.
 //
 // Measured, one cloud, us per attempt (state, coordinates and sums through global memory
@@ -51,7 +51,6 @@ namespace {
 constexpr int kThreads = SG_FUSED_THREADS;
 constexpr int kWarps = kThreads / 32;
 constexpr int kFold = 8;          // packed j-pairs per FP32 partial sum before the Kahan fold
-constexpr float kKappa2 = 2.25f;  // FP64 row when s2 > 2.25 |P|^2 (the tiled reduction's for large clouds)
 
 // What the CTAs of a cluster tell each other at the end of an attempt, two attempts in
 // turn: a CTA may be one barrier ahead of another's reads.
@@ -247,6 +246,7 @@ struct WideGroup {
     int target;   // arrivals so far
     int* flag_n;  // [2] flagged ions of the stage in either coordinate set ...
     int* flags;   // [2][SG_WIDE_FLAGS] ... cloud indices
+    bool share;   // flagged rows
 
     __device__ __forceinline__ void arrive() {
         __syncthreads();  // the CTA's stores come before its arrival
@@ -277,11 +277,13 @@ struct WideGroup {
         return sh.expired == 0;
     }
 };
-// Wide clouds of more padded ions share a flagged ion's FP64 row between all their CTAs, two
-// more barriers a stage with a flagged ion and one without (~1.5 us each); a row in one CTA
-// takes 4 us per 1,000 ions, and the others wait for it (3,000 ions, us per attempt: 205
-// with rows in one CTA, 157 shared; 1,500 112 / 112).
-constexpr int kShareRows = 1536;
+// Wide clouds of more padded ions, or of more ions a CTA, share a flagged ion's FP64 row
+// between all their CTAs: two more barriers a stage with a flagged ion and one without
+// (~1.5 us each), where a row in one CTA takes 4 us per 1,000 ions, two in the same CTA twice
+// that, and the others wait for it.  us per attempt, rows in one CTA / shared: 700 ions (5 a
+// CTA) 78 / 90, 850 83 / 90, 1,200 136 / 96, 3,000 205 / 157; 2 clouds of 700 (10 a CTA) 75 / 82,
+// 4 of 700 (19) 110 / 91, 8 of 600 (32) 113 / 90.
+constexpr int kShareIons = 896, kShareOwn = 12;
 
 // This CTA's rows [lo, lo + m) of set `set` into the other CTAs' shared memory, 16 bytes a
 // store: 6 m / 4 words of frame coordinates and 3 m / 2 of SI ones for each.
@@ -524,11 +526,11 @@ __device__ __noinline__ bool coulomb_phase(const SgFusedArgs& f, const SgCloud& 
     // the conditioning test (frame units for a unit charge)
     if (il < mo && q == 0) {
         const float pf2 = fmaf(px.h, px.h, fmaf(py.h, py.h, pz.h * pz.h));
-        const bool flagged = ps2 > kKappa2 * pf2;
+        const bool flagged = ps2 > f.kappa2 * pf2;
         s.flag[il] = flagged;
         if (flagged) {
             s.list[atomicAdd(&sh.nflag, 1)] = il;
-            if (WIDE && npc > kShareRows) {
+            if (WIDE && g.share) {
                 const int at = atomicAdd(g.flag_n + set, 1);
                 if (at < SG_WIDE_FLAGS) g.flags[set * SG_WIDE_FLAGS + at] = li;
                 s.flag[il] = at + 1;
@@ -545,7 +547,7 @@ __device__ __noinline__ bool coulomb_phase(const SgFusedArgs& f, const SgCloud& 
         }
     }
     __syncthreads();
-    if (WIDE && npc > kShareRows) {
+    if (WIDE && g.share) {
         // shared rows: every CTA of the cloud takes its j-ions of each flagged ion, a warp an
         // ion, and the owners add the parts in rank order
         g.arrive();
@@ -726,6 +728,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(const __gri
         g.count = f.barrier + 2 * c;
         g.R = R;
         g.r = r;
+        g.share = npc > kShareIons || m > kShareOwn;
         g.flag_n = f.flag_n + 2 * c;
         g.flags = f.flag_list + 2 * SG_WIDE_FLAGS * c;
         if (r == 0 && tid == 0) g.flag_n[0] = g.flag_n[1] = 0;

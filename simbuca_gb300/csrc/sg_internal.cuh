@@ -502,12 +502,18 @@ cudaError_t sg_dp_finish(const SgFinishArgs& f, int stage, int fp32c, cudaStream
 // is faster than the wide form with more CTAs; the wide form is taken by default (sg_set_fused
 // mode 1) up to SG_FUSED_WIDE_PAIRS, clusters up to SG_FUSED_AUTO_PAIRS.  Measured on GB300, us
 // per attempt (pairs per CTA), cluster / wide / tiled kernels: one cloud of 300 ions 56 (6,000)
-// / 62 / 142, 512 67 (16,000) / 66 (2,000) / 131, 1,000 120 / 67 (7,000) / 121, 2,048 400 / 98 to
-// 126 (29,000) / 150, 3,000 - / 155 to 171 (60,000) / 170 to 179, 4,096 - / 193 (111,000) / 223,
-// 5,000 - / 313 (165,000) / 239; 8 of 300 77 (12,000) / 60 (5,000) / 166, 16 of 300 101 (23,000)
-// / 82 / 227, 4 of 2,000 - / 192 (106,000) / 245, 2 of 4,000 - / 299 (212,000) / 309; 70 of 100 on
+// / 62 / 142, 512 67 (16,000) / 66 (2,000) / 131, 1,000 120 / 93 (7,000) / 121, 2,048 400 / 108
+// (29,000) / 150, 3,000 - / 151 to 166 (60,000) / 172 to 180, 4,096 - / 189 (111,000) / 223,
+// 5,000 - / 310 (165,000) / 239; 8 of 300 77 (12,000) / 60 (5,000) / 166, 16 of 300 101 (23,000)
+// / 82 / 227, 4 of 2,000 - / 195 (106,000) / 245, 2 of 4,000 - / 301 (212,000) / 309; 70 of 100 on
 // 2 CTAs each 66 (5,000) / 76 / 224.
 #define SG_FUSED_CLUSTER_PAIRS 8000
+// Conditioning threshold of the fused path: sqrt(s2) > 1.5 |P| for a few clouds of up to so
+// many ions, > 1.1 |P| for the others, whose largest errors are then the tiled kernels' at
+// their 1.0 (the fused partial sums interleave the cloud's ions): 1,000 ions 3.9e-7 (3.8e-7;
+// at 1.5 4.5e-7), 1,500 3.9e-7 (3.4e-7; 5.0e-7), 3,000 3.9e-7 (4.7e-7; 5.3e-7), 24 of 300
+// 4.6e-7 (4.1e-7; 5.4e-7), largest of 5,000 to 58,000 probes each.
+#define SG_FUSED_LOOSE_IONS 512
 #define SG_FUSED_WIDE_PAIRS 120000
 #define SG_FUSED_AUTO_PAIRS 40000
 struct SgFusedArgs {
@@ -522,6 +528,7 @@ struct SgFusedArgs {
     int* ran;
     int n, npad, n_clouds;
     int max_attempts;  // attempts per launch at most
+    float kappa2;      // conditioning threshold
     int one_step;      // 1: each cloud stops after an accepted attempt; 2: those that have not yet
     // wide form: CTAs per cloud (0: clusters), c64 and c32 hold two coordinate sets
     int ctas;

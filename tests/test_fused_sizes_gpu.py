@@ -72,7 +72,7 @@ def test_clusters_with_several_slots_per_thread(ctx):
         assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
 
 
-@pytest.mark.parametrize("counts", [[500], [1000], [1536], [1537], [4096], [4500], [300] * 8,
+@pytest.mark.parametrize("counts", [[500], [896], [897], [1000], [4096], [4500], [300] * 8, [500] * 7,
                                     [1000, 16, 999, 64], [2000, 40, 1900, 3]])
 def test_wide_form_against_fp64(ctx, counts):
     """The form that spreads a cloud over many CTAs: sizes of its automatic range and its
