@@ -66,7 +66,7 @@ def parse():
     ap.add_argument("--proposer-safety", type=float, default=None,
                     help="safety factor of the proposer (default: the trained one's)")
     ap.add_argument("--fused", default="auto", choices=["auto", "on", "off"],
-                    help="fused small-cloud path: automatic (clouds of up to 512 ions), on "
+                    help="fused small-cloud path: automatic (where it is faster), on "
                          "(up to 2,048: sg_set_fused 2) or off")
     ap.add_argument("--settle", type=int, default=60,
                     help="at most this many steps to let the step size settle before warm-up")

@@ -47,7 +47,8 @@ enum {
     SG_PREC_FP64 = 0,   /* plain form: every operation in FP64                          */
     SG_PREC_FP32C = 1   /* FP32 pair terms on cloud-centre-relative float-float
                            coordinates, Kahan-compensated per-ion accumulation across
-                           j-tiles, and FP64 evaluation of close pairs                  */
+                           j-tiles, float-float close pairs (the closest in FP64) and
+                           FP64 rows of ions whose terms cancel                         */
 };
 
 /* ---- field terms (bit flags of sg_field_params.flags) ---------------------- */

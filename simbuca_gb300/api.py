@@ -149,8 +149,8 @@ class Context:
         check(self._L.sg_set_use_graph(self._h, int(bool(on))), "sg_set_use_graph")
 
     def set_fused(self, mode):
-        """Whole attempts of small clouds in one cluster launch: 1 (default, True) for
-        clouds of up to 512 ions, 2 up to 2,048 ions, 0 (False) never."""
+        """Whole attempts of small clouds in one cluster launch: 1 (default, True)
+        where it is faster, 2 clouds of up to 2,048 ions, 0 (False) never."""
         check(self._L.sg_set_fused(self._h, int(mode)), "sg_set_fused")
 
     def fused_timing(self):

@@ -12,12 +12,13 @@
 // u_j - u_i = (hi_j - hi_i) + (lo_j - lo_i) keeps the pair distance accurate to an
 // FP32 rounding even for ions far from the frame centre.  1/r is the SFU
 // approximation (rsqrt.approx), 1/r^3 is capped at wc: the rare close pairs whose
-// 1/r^3 exceeds wc are re-evaluated in FP64 once the tile is done, and the capped
-// FP32 contribution is taken out again exactly.  Within a 128-ion j-tile the terms
+// 1/r^3 exceeds wc are re-evaluated in float-float (the very closest in FP64) once the
+// tile is done, and the capped FP32 contribution is taken out again exactly.  Within a 128-ion j-tile the terms
 // are summed in FP32; tile sums are added with Kahan compensation.  Arithmetic uses
 // the packed FP32x2 instructions of sm_100+ (add/mul/fma.rn.f32x2) on pairs of
 // consecutive j-ions.  j-tiles are fetched with TMA bulk copies (cp.async.bulk) into
-// a 4-stage shared-memory ring guarded by mbarriers.
+// a 4-stage shared-memory ring guarded by mbarriers.  Clouds in k-d order (shape 17) take
+// each unordered pair of 128-ion leaves once instead (coulomb_leaf_kernel).
 //
 // FP64 (coulomb_fp64_sym_kernel, fp64_pairs.cuh): the plain form, every operation in
 // FP64, each unordered pair evaluated once; 1/r^3 is the SFU's FP64 seed refined by one
