@@ -302,7 +302,7 @@ void plan_sym(Problem& P, int n_sm) {
         if (!(P.hc[c].fp.flags & SG_F_COULOMB)) continue;
         const int nj = P.hc[c].npad / SG_SYM_JT;
         for (int b = 0; b * TB < nj; b++) tiles += nj - b * TB;
-        tile_pairs += 0.5 * nj * (nj + 1.0);
+        tile_pairs += 0.5 * nj * nj;
     }
     const bool pairs = tiles < kSymTilePairs * n_sm;
     const int parts = pairs ? sym_parts(tile_pairs, n_sm) : 1;

@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "fp32c_math.cuh"
 #include "sg_internal.cuh"
@@ -196,16 +197,26 @@ __device__ __forceinline__ void fp64_sym_tile_block(const Load& ld, int n, int i
     }
 }
 
-// Sets with fewer 128 x 32 blocks than this per SM take tile pairs, and share each between
-// up to four blocks while those find an SM each.  A Dormand-Prince attempt, us, 128 x 32
-// items (in eighths where there are few) / tile pairs: 64 ions 78 / 65, 300 92 / 83, 1,000
-// 231 / 196, 1,500 323 / 320, 2,000 567 / 503, 3,000 1,036 / 1,015, 4,000 1,749 / 1,707, 5,003
-// 2,615 / 2,670.
+// Sets with fewer 128 x 32 blocks than this per SM take tile pairs.  A Dormand-Prince
+// attempt, us, 128 x 32 items (in eighths where there are few) / tile pairs: 64 ions 78 / 64,
+// 300 92 / 83, 1,000 231 / 187, 1,500 323 / 320, 2,000 567 / 503, 3,000 1,036 / 1,015, 4,000 1,749
+// / 1,707, 5,003 2,615 / 2,670.
 constexpr double kSymTilePairs = 16.0;
+// Blocks that share a tile pair: what makes the last round of blocks over the SMs shortest,
+// at 8 % a doubling for the slots it adds (a diagonal pair counts half).  us per attempt in one / two / four parts: 64 ions
+// 91 / 73 / 64, 400 99 / 95 / 91, 600 128 / 116 / 114, 700 128 / 134 / 134, 1,000 198 / 187 /
+// 204, 1,200 229 / 239 / 263, 32 clouds of 100 148 / 153 / 155.
 inline int sym_parts(double tile_pairs, int n_sm) {
-    int parts = 1;
-    while (parts < 4 && 2 * parts * tile_pairs <= n_sm) parts *= 2;
-    return parts;
+    int best = 1;
+    double least = 1e300;
+    for (int parts = 1; parts <= 4; parts *= 2) {
+        const double cost = std::ceil(parts * tile_pairs / n_sm) / parts * (parts == 1 ? 1.0 : parts == 2 ? 1.08 : 1.17);
+        if (cost < least) {
+            least = cost;
+            best = parts;
+        }
+    }
+    return best;
 }
 
 // ---- one set of ions on its own (allocation-free entry point, CUNBODY slot) -----------
@@ -225,7 +236,7 @@ inline SymPlan sym_plan(int npad, int n_sm, size_t cap) {
     const int nb = (npad + SG_SYM_IB - 1) / SG_SYM_IB, nt = npad / SG_SYM_JT;
     double tiles = 0.0;
     for (int b = 0; b < nb; b++) tiles += sym_chunks(npad, b, 1);
-    const int parts = sym_parts(0.5 * nt * (nt + 1), n_sm);
+    const int parts = sym_parts(0.5 * nt * nt, n_sm);
     if (tiles < kSymTilePairs * n_sm && (size_t)(nt + 1) * parts * 3 * npad <= cap)
         return SymPlan{0, parts, nt * (nt + 1) / 2 * parts, (nt + 1) * parts};
     SymPlan p{std::max(1, (int)(tiles / (16.0 * n_sm))), 1, 0, 0};

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("mixed", [False, True])
-@pytest.mark.parametrize("n", [2, 33, 64, 200, 257, 300, 417, 700, 4416, 4500])
+@pytest.mark.parametrize("n", [2, 33, 64, 200, 257, 300, 417, 600, 700, 1000, 4416, 4500])
 def test_sums_against_the_oracle(ctx, n, mixed):
     """1e-12 of the ion's sum, as for every size: FP64 terms to an ulp or so, sums of n terms
     whose rounding grows with sqrt(n) at most (sqrt(4,500) 1.1e-16 = 7e-15, times the
