@@ -188,17 +188,18 @@ def coulomb_kernel_name(prec, variant):
     return "coulomb_fp32c_sorted_kernel" if variant in sorted_shapes else "coulomb_fp32c_kernel"
 
 
-def launches_per_attempt(prec, n_total, variant):
+def launches_per_attempt(prec, n_total, variant, mixed=False):
     """Our kernel launches of one Dormand-Prince attempt: stage 1, then per Coulomb sum
     the pair kernel and, up to 8,192 ions in the plain order, the finish kernel (slot sums,
     flagged rows, stage), else the reduction, with FP32c the fix-up, and the stage; shape
-    17 lists its near leaves before each pair kernel.  Control and commit."""
+    17 lists its near leaves before each pair kernel, and takes the small clouds of a mixed
+    batch with one more.  Control and commit."""
     from simbuca_gb300 import abi
     fp32c = prec == abi.SG_PREC_FP32C
     plain = not fp32c or variant < 4 or variant in (5, 6, 10, 11)
     if n_total <= 8192 and plain:
         return 1 + 6 * 2 + 2
-    per_sum = 3 + (1 if fp32c and n_total > 8192 else 0) + (1 if fp32c and variant == 17 else 0)
+    per_sum = 3 + (1 if fp32c and n_total > 8192 else 0) + ((2 if mixed else 1) if fp32c and variant == 17 else 0)
     return 1 + 6 * per_sum + 2
 
 
@@ -556,6 +557,7 @@ def run_batched(args, dist: Dist):
     ctx.set_fused({"auto": 1, "on": 2, "off": 0}[args.fused])
     batch = Batch(ctx, w.counts, w.fields, w.odes, prec)
     batch.upload(allc.pos, allc.vel, allc.mass, allc.charge)
+    variant = batch.variant()  # before the one-cloud batches take the context
     step_control = apply_step_control(args, batch)
     per_step = 10  # attempts of every cloud per bench step (one graph replay each)
 
@@ -622,7 +624,7 @@ def run_batched(args, dist: Dist):
                    "step_control": step_control,
                    "parallelism": f"replicas x{dist.world}",
                    "l2": "flushed (256 MB write) between timed steps"},
-        "gpu_launches": int((launches_per_attempt(prec, w.n_total, batch.variant())
+        "gpu_launches": int((launches_per_attempt(prec, w.n_total, variant, min(w.counts) <= 2500)
                              + (2 if args.proposer == "on" else 0)) * per_step * args.steps
                             + (3 * (per_step * args.steps // CHECK_EVERY)
                                if args.precision == "fp32c" else 0)),
@@ -634,7 +636,7 @@ def run_batched(args, dist: Dist):
         "one_at_a_time": {"value": seq_value, "unit": "sim-us/wall-s",
                           "ms_total": seq_ms, "sim_us_total": seq_sim},
         "speedup_vs_one_at_a_time": value / seq_value if seq_value else None,
-        "coulomb_variant": batch.variant(),
+        "coulomb_variant": variant,
         "clocks": clk,
     }
     ctx.close()
