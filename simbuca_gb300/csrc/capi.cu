@@ -112,7 +112,7 @@ struct Problem {
     bool fused_known = false, fused_resident = false;
     int fused_wide = 0;       // CTAs per cloud of the wide form (0: not launchable)
     int* fused_barrier = nullptr;
-    double *fused_notes = nullptr, *fused_part = nullptr;
+    double *fused_notes = nullptr, *fused_part = nullptr, *fused_list = nullptr;
     int* fused_flags = nullptr;
     int fused_cluster = 0;    // cluster size for this batch (0: none can be launched)
     int max_npad = 0;         // largest padded cloud
@@ -221,6 +221,7 @@ void free_problem(Problem& P) {
     cudaFree(P.fused_notes);
     cudaFree(P.fused_flags);
     cudaFree(P.fused_part);
+    cudaFree(P.fused_list);
     cudaFree(P.leaf_sum);
     cudaFree(P.leaf_fmx);
     cudaFree(P.leaf_n_close);
@@ -708,7 +709,8 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
         CK(dalloc(&P.fused_barrier, 2 * (size_t)std::max(P.n_clouds, 1)));
         CK(cudaMemset(P.fused_barrier, 0, 2 * sizeof(int) * (size_t)std::max(P.n_clouds, 1)));
         CK(dalloc(&P.fused_notes, 2 * (SG_FUSED_MAX_WIDE + 1) * (size_t)std::max(P.n_clouds, 1)));
-        CK(dalloc(&P.fused_flags, 2 * (SG_WIDE_FLAGS + 1) * (size_t)std::max(P.n_clouds, 1)));
+        CK(dalloc(&P.fused_flags, 2 * (size_t)std::max(P.n_clouds, 1)));
+        CK(dalloc(&P.fused_list, 8 * SG_WIDE_FLAGS * (size_t)std::max(P.n_clouds, 1)));
         CK(dalloc(&P.fused_part, (size_t)2 * SG_WIDE_FLAGS * SG_FUSED_MAX_WIDE * 3));
     }
     CK(dalloc(&P.c32, (P.finish ? 14 : 7) * NP));
@@ -1258,7 +1260,7 @@ int run_fused(sg_ctx* ctx, Problem& P, int n, int counted, int one_step = 0) {
     f.barrier = P.fused_barrier;
     f.notes = P.fused_notes;
     f.flag_n = P.fused_flags;
-    f.flag_list = P.fused_flags + 2 * P.n_clouds;
+    f.flag_list = P.fused_list;
     f.flag_part = P.fused_part;
     TimedLaunch tl{nullptr, nullptr, 0.0, 1};
     if (ctx->timing) {

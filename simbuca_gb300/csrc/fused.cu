@@ -245,16 +245,14 @@ struct WideGroup {
     int R, r;     // CTAs of the cloud, this one's rank
     int target;   // arrivals so far
     int* flag_n;  // [2] flagged ions of the stage in either coordinate set ...
-    int* flags;   // [2][SG_WIDE_FLAGS] ... cloud indices
+    double* flags;  // [2][SG_WIDE_FLAGS][4] ... x, y, z, index in the cloud
     bool share;   // flagged rows
 
     __device__ __forceinline__ void arrive() {
         __syncthreads();  // the CTA's stores come before its arrival
         target += R;
-        if (threadIdx.x == 0) {
-            __threadfence();
-            atomicAdd(count, 1);
-        }
+        if (threadIdx.x == 0)
+            asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(count) : "memory");
     }
     // past: arrivals beyond the last ones to wait for (the wait test)
     __device__ __forceinline__ bool wait(FusedShared& sh, int past = 0,
@@ -532,7 +530,11 @@ __device__ __noinline__ bool coulomb_phase(const SgFusedArgs& f, const SgCloud& 
             s.list[atomicAdd(&sh.nflag, 1)] = il;
             if (WIDE && g.share) {
                 const int at = atomicAdd(g.flag_n + set, 1);
-                if (at < SG_WIDE_FLAGS) g.flags[set * SG_WIDE_FLAGS + at] = li;
+                if (at < SG_WIDE_FLAGS) {
+                    double* e = g.flags + 4 * (set * SG_WIDE_FLAGS + at);
+                    for (int c = 0; c < 3; c++) e[c] = s.ST[c * s.mc + il];
+                    e[3] = (double)li;
+                }
                 s.flag[il] = at + 1;
             }
         } else {
@@ -550,23 +552,40 @@ __device__ __noinline__ bool coulomb_phase(const SgFusedArgs& f, const SgCloud& 
     if (WIDE && g.share) {
         // shared rows: every CTA of the cloud takes its j-ions of each flagged ion, a warp an
         // ion, and the owners add the parts in rank order
+        const int warp = tid >> 5, lane = tid & 31;
+        const int len = (npc / 32 + g.R - 1) / g.R * 32;
+        const int j0 = g.r * len, j1 = min(npc, j0 + len);
         g.arrive();
+        // this lane's first j-ion arrives while the barrier completes, the warp's first
+        // flagged ion with their number
+        double jx = 0.0, jy = 0.0, jz = 0.0, jq = 0.0;
+        if (j0 < j1) {
+            jx = ld(SX + j0 + lane);
+            jy = ld(SY + j0 + lane);
+            jz = ld(SZ + j0 + lane);
+            jq = SQ[j0 + lane];
+        }
         if (!g.wait(sh)) return false;
+        const double2* flags = reinterpret_cast<const double2*>(g.flags + 4 * set * SG_WIDE_FLAGS);
+        double2 e0 = __ldcg(flags + 2 * warp), e1 = __ldcg(flags + 2 * warp + 1);
         const int all = __ldcg(g.flag_n + set);
         if (all == 0) return true;
         if (all <= SG_WIDE_FLAGS) {
-            const int warp = tid >> 5, lane = tid & 31;
-            const int len = (npc / 32 + g.R - 1) / g.R * 32;
-            const int j0 = g.r * len, j1 = min(npc, j0 + len);
             double* parts = f.flag_part + (size_t)set * SG_WIDE_FLAGS * SG_FUSED_MAX_WIDE * 3;
             for (int k = warp; k < all; k += kWarps) {
-                const int lf = __ldcg(g.flags + set * SG_WIDE_FLAGS + k);
-                const double xi = ld(SX + lf), yi = ld(SY + lf), zi = ld(SZ + lf);
+                if (k != warp) {
+                    e0 = __ldcg(flags + 2 * k);
+                    e1 = __ldcg(flags + 2 * k + 1);
+                }
+                const int lf = (int)e1.y;
                 double ax = 0.0, ay = 0.0, az = 0.0;
                 for (int jj = j0 + lane; jj < j1; jj += 32) {
+                    const bool first = jj == j0 + lane;
                     if (jj == lf) continue;
-                    const double rx = xi - ld(SX + jj), ry = yi - ld(SY + jj), rz = zi - ld(SZ + jj);
-                    const double wq = SQ[jj] * inv_r3_fp64(rx * rx + ry * ry + rz * rz);
+                    const double rx = e0.x - (first ? jx : ld(SX + jj)),
+                                 ry = e0.y - (first ? jy : ld(SY + jj)),
+                                 rz = e1.x - (first ? jz : ld(SZ + jj));
+                    const double wq = (first ? jq : SQ[jj]) * inv_r3_fp64(rx * rx + ry * ry + rz * rz);
                     ax = fma(wq, rx, ax);
                     ay = fma(wq, ry, ay);
                     az = fma(wq, rz, az);
@@ -730,7 +749,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_attempts_kernel(const __gri
         g.r = r;
         g.share = npc > kShareIons || m > kShareOwn;
         g.flag_n = f.flag_n + 2 * c;
-        g.flags = f.flag_list + 2 * SG_WIDE_FLAGS * c;
+        g.flags = f.flag_list + 8 * SG_WIDE_FLAGS * c;
         if (r == 0 && tid == 0) g.flag_n[0] = g.flag_n[1] = 0;
         g.arrive();
         ok = sh.wtest != 1 ? g.wait(sh)

@@ -534,7 +534,8 @@ struct SgFusedArgs {
     int ctas;
     int* barrier;   // [clouds][2] arrivals, departures; zero between launches
     double* notes;  // [clouds][2][SG_FUSED_MAX_WIDE + 1] error partials, x of the first ion
-    int *flag_n, *flag_list;  // [clouds][2], [clouds][2][SG_WIDE_FLAGS] flagged ions of a stage
+    int* flag_n;        // [clouds][2] flagged ions of a stage
+    double* flag_list;  // [clouds][2][SG_WIDE_FLAGS][4] their x, y, z and index in the cloud
     double* flag_part;        // [2][SG_WIDE_FLAGS][SG_FUSED_MAX_WIDE][3] parts of their rows
 };
 // The cluster size (16, 8, 4 or 2) for n_clouds clouds of up to max_npad padded ions: the
