@@ -2061,7 +2061,8 @@ cudaError_t sg_launch_coulomb_reduce(const SgCoulombArgs& a, const SgRowBlock* r
             cudaError_t e = cudaMemsetAsync(a.fix_list, 0, 2 * sizeof(int), s);
             if (e != cudaSuccess) return e;
         }
-        sg_launch(coulomb_reduce_kernel<true, false>, n_rows * split, SG_ROWS, 0, s, 
+        // a plain launch: nothing programmatic may follow the memset
+        coulomb_reduce_kernel<true, false><<<n_rows * split, SG_ROWS, 0, s>>>(
             rows, a.clouds, a.ctrl, a.part, a.npad_total, out, n_total, counters, a.fix_list,
             a.c32, a.c64, nullptr, a.risk, a.ran, a.chk, split, leaf);
         // a fixed grid that strides over however many work units there are (a batch of
