@@ -489,9 +489,9 @@ struct SgFinishArgs {
 cudaError_t sg_dp_finish(const SgFinishArgs& f, int stage, int fp32c, cudaStream_t st);
 
 // ---- fused small-cloud attempts (fused.cu) -----------------------------------------
-// One thread-block cluster per cloud runs whole Dormand-Prince attempts (FP32c, no
-// recorder, operations or proposer) for clouds of at most SG_FUSED_MAX_IONS ions, and
-// at most SG_FUSED_THREADS ions per CTA of the cluster.
+// A cloud's CTAs run whole Dormand-Prince attempts (FP32c, no recorder, operations or
+// proposer): a thread-block cluster per cloud of at most SG_FUSED_MAX_IONS ions, at most
+// SG_FUSED_THREADS of them per CTA, or the wide form on up to SG_FUSED_MAX_WIDE CTAs.
 #define SG_FUSED_THREADS 512
 #define SG_FUSED_MAX_CTAS 16
 #define SG_FUSED_MAX_IONS 2048
