@@ -38,7 +38,7 @@ def _stale(out: str, deps: list[str]) -> bool:
 
 def build(verbose: bool = False, force: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
-    headers = [os.path.join(CSRC, "sg_internal.cuh"), os.path.join(CSRC, "fp32c_math.cuh"),
+    headers = [os.path.join(CSRC, "sg_internal.cuh"), os.path.join(CSRC, "sg_rules.h"), os.path.join(CSRC, "fp32c_math.cuh"),
                os.path.join(CSRC, "dp_tableau.cuh"), os.path.join(CSRC, "fp64_pairs.cuh"), os.path.join(CSRC, "dp_stage.cuh"),
                os.path.join(os.path.dirname(PKG), "include", "simgb.h")]
     procs, objs = [], []

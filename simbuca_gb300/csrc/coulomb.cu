@@ -790,7 +790,7 @@ __device__ __forceinline__ void far_warp(const float* __restrict__ c32, const Sg
                 cp_async16(&t[a][4 * lane], c32 + a * NP + j0 + 4 * lane);
             else  // a cloud's last leaf: far away, no charge
 #pragma unroll
-                for (int q = 0; q < 4; q++) t[a][4 * lane + q] = a < 3 ? 2.0e4f : 0.f;
+                for (int q = 0; q < 4; q++) t[a][4 * lane + q] = a < 3 ? sg_leaf_fill(false) : 0.f;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -857,7 +857,7 @@ struct NearSide {
 
 template <bool NOQ, bool TWO>
 __device__ __forceinline__ void near_leaf(const float (*tj)[SG_TILE], NearWarpShared& sh,
-                                          NearSide& w, float wc, int i0, int j0,
+                                          NearSide& w, float wc, int i0, int j0, int end,
                                           const LeafAcc& acc) {
     const int lane = threadIdx.x & 31, next = (lane + 1) & 31;
     const f2 tiny2 = pk(kTiny, kTiny);
@@ -959,7 +959,7 @@ __device__ __forceinline__ void near_leaf(const float (*tj)[SG_TILE], NearWarpSh
             close &= close - 1u;
             const int i = i0 + 2 * lane + ((bit >> 1) & 1);
             const int j = j0 + 64 * sub + 2 * ((lane + s0 + (bit >> 2)) & 31) + (bit & 1);
-            if (i == j) continue;
+            if (!sg_lists_pair(i, j, end)) continue;
             int at = atomicAdd(acc.n_close + i, 1);
             if (at < kCloseCap) acc.close[(size_t)i * kCloseCap + at] = j;
             if (!TWO) continue;
@@ -991,7 +991,7 @@ __device__ __forceinline__ void near_warp(const float* __restrict__ c32, const S
         const bool in = i < pend;  // past a cloud's last leaf: far from everything, no charge
 #pragma unroll
         for (int c = 0; c < 6; c++) {
-            const float x = in ? c32[(c < 3 ? c : c + 1) * NP + i] : c < 3 ? 3.0e4f : 0.f;
+            const float x = in ? c32[(c < 3 ? c : c + 1) * NP + i] : c < 3 ? sg_leaf_fill(true) : 0.f;
             w.x[c][k] = pk(x, x);
         }
         const float q = in ? c32[3 * NP + i] : 0.f;
@@ -1009,7 +1009,7 @@ __device__ __forceinline__ void near_warp(const float* __restrict__ c32, const S
                 cp_async16(&t[a][4 * lane], c32 + a * NP + j0 + 4 * lane);
             else
 #pragma unroll
-                for (int q = 0; q < 4; q++) t[a][4 * lane + q] = a < 3 ? 2.0e4f : 0.f;
+                for (int q = 0; q < 4; q++) t[a][4 * lane + q] = a < 3 ? sg_leaf_fill(false) : 0.f;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -1028,14 +1028,14 @@ __device__ __forceinline__ void near_warp(const float* __restrict__ c32, const S
         const bool noq = cl.quniform && j0 + SG_TILE <= end;
         if (J == leaf) {  // every ordered pair of the half, one side
             if (noq)
-                near_leaf<true, false>(sh.j[slot], sh, w, cl.wc, i0, j0, acc);
+                near_leaf<true, false>(sh.j[slot], sh, w, cl.wc, i0, j0, end, acc);
             else
-                near_leaf<false, false>(sh.j[slot], sh, w, cl.wc, i0, j0, acc);
+                near_leaf<false, false>(sh.j[slot], sh, w, cl.wc, i0, j0, end, acc);
         } else {
             if (noq)
-                near_leaf<true, true>(sh.j[slot], sh, w, cl.wc, i0, j0, acc);
+                near_leaf<true, true>(sh.j[slot], sh, w, cl.wc, i0, j0, end, acc);
             else
-                near_leaf<false, true>(sh.j[slot], sh, w, cl.wc, i0, j0, acc);
+                near_leaf<false, true>(sh.j[slot], sh, w, cl.wc, i0, j0, end, acc);
 #pragma unroll 1
             for (int k = 0; k < 4; k++) {
                 const int p = lane + 32 * k, jg = j0 + p;

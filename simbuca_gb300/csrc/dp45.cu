@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(SG_ROWS) coords_from_state_kernel(DpArgs a,
             a.c64[2 * (size_t)a.npad + ig] = far;
             a.c64[3 * (size_t)a.npad + ig] = 0.0;
             if (a.fp32c) {
-                const float ff = 1.0e4f + (float)g;
+                const float ff = sg_pad_frame(g);
                 a.c32[ig] = ff;
                 a.c32[a.npad + ig] = ff;
                 a.c32[2 * (size_t)a.npad + ig] = ff;

@@ -7,6 +7,7 @@
 #include <utility>
 
 #include "../../include/simgb.h"
+#include "sg_rules.h"
 
 // ---- constants of the reference (bin/globals.h:4-16) -------------------------
 #define SG_PI 3.14159265358979323
