@@ -243,26 +243,26 @@ __device__ __forceinline__ void load_coords(const SgFusedArgs& f, const FusedArr
 struct WideGroup {
     int* count;   // arrivals, departures
     int R, r;     // CTAs of the cloud, this one's rank
-    int target;   // arrivals so far
+    unsigned target;  // arrivals so far (modulo 2^32)
     int* flag_n;  // [2] flagged ions of the stage in either coordinate set ...
     double* flags;  // [2][SG_WIDE_FLAGS][4] ... x, y, z, index in the cloud
     bool share;   // flagged rows
 
     __device__ __forceinline__ void arrive() {
         __syncthreads();  // the CTA's stores come before its arrival
-        target += R;
+        target += (unsigned)R;
         if (threadIdx.x == 0)
-            asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(count) : "memory");
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
     }
     // past: arrivals beyond the last ones to wait for (the wait test)
-    __device__ __forceinline__ bool wait(FusedShared& sh, int past = 0,
+    __device__ __forceinline__ bool wait(FusedShared& sh, unsigned past = 0,
                                          unsigned long long limit_ns = SG_WAIT_NS) {
         if (threadIdx.x == 0) {
-            int seen;
+            unsigned seen;
             unsigned long long t0 = 0, t;
             for (;;) {
-                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
-                if (seen >= target + past) break;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
+                if (sg_reached(seen, target + past)) break;
                 asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
                 if (t0 == 0) t0 = t;
                 if (t - t0 > limit_ns) {

@@ -18,3 +18,8 @@ SG_HD float sg_leaf_fill(bool i_side) { return i_side ? -3.0e4f : -2.0e4f; }
 // ions (of a cloud whose real ions end at `end`).  Only real ions' lists are emptied again,
 // and indices past the padded end are another cloud's or none.
 SG_HD bool sg_lists_pair(int i, int j, int end) { return i != j && i < end && j < end; }
+
+// Whether a counter that only rises by one has reached `target`, both modulo 2^32: the
+// difference of the two stays far below 2^31, the counts of a long launch do not (a barrier
+// of 152 blocks, up to 19 times an attempt, passes 2^31 after 0.74 million attempts).
+SG_HD bool sg_reached(unsigned seen, unsigned target) { return (int)(seen - target) >= 0; }

@@ -39,3 +39,20 @@ def test_only_real_ions_are_listed(tmp_path, n):
         for (int j = leaf0; j < leaf0 + 128; j++)
             if (sg_lists_pair(i, j, end) != (i != j && i < poff + n && j < poff + n)) printf("%d %d\\n", i, j);
     """) == ""
+
+
+@pytest.mark.parametrize("blocks,past", [(152, 0), (152, 1), (1, 0), (160, 0)])
+def test_a_barrier_count_may_wrap(tmp_path, blocks, past):
+    """A block waits for every arrival of its barrier, and no longer, wherever the count
+    stands: at the start, across 2^31 and across 2^32."""
+    assert run(tmp_path, f"""
+    const unsigned R = {blocks}, past = {past};
+    for (unsigned base : {{0u, 0x7fffffffu - R, 0x7fffffffu, 0x80000000u, 0xffffffffu - R, 0xffffffffu}}) {{
+        const unsigned target = base + R;
+        for (unsigned a = 0; a < R + past; a++)
+            if (sg_reached(base + a, target + past)) printf("early %u %u\\n", base, a);
+        // the others may be one barrier further on
+        for (unsigned a = R + past; a <= 2 * R; a++)
+            if (!sg_reached(base + a, target + past)) printf("late %u %u\\n", base, a);
+    }}
+    """) == ""
