@@ -290,13 +290,23 @@ int auto_variant(const std::vector<int>& counts, int requested, bool resident) {
     return big <= 6000 && total <= 32768 ? 11 : 5;
 }
 
+// Whether the partial sums of the unordered FP64 pairs may take so many bytes: 4 GiB, and of
+// a nearly full device half of what it has left.
+bool sym_fits(size_t bytes) {
+    if (bytes <= (size_t)1 << 28) return true;
+    size_t left = 0, total = 0;
+    return bytes <= (size_t)1 << 32 && cudaMemGetInfo(&left, &total) == cudaSuccess && bytes <= left / 2;
+}
+
 // FP64 items that take each unordered pair once: i-block b (128 ions) against the j-tiles
 // (32 ions) from its own diagonal up, K tiles per item, or pairs of 32-ion tiles when that
 // leaves the device short of items.  A block keeps all four FP64 pipes of an SM busy
 // whatever else it does, so the items only have to be small against one SM's share of
 // the work and large against the ~1 us it takes to start one (a 128 x 32 tile is 20 us of
-// FP64).
-void plan_sym(Problem& P, int n_sm) {
+// FP64).  An ion's slots grow with the i-blocks of the largest cloud (one of 131,072 ions:
+// 1,025 slots, 3.2 GB) and every ion of a batch has room for as many: false, and the
+// ordered pairs with their few slots, where that does not fit (sym_fits).
+bool plan_sym(Problem& P, int n_sm) {
     const int TB = SG_SYM_IB / SG_SYM_JT;
     double tiles = 0.0, tile_pairs = 0.0;
     for (int c = 0; c < P.n_clouds; c++) {
@@ -309,6 +319,17 @@ void plan_sym(Problem& P, int n_sm) {
     const int parts = pairs ? sym_parts(tile_pairs, n_sm) : 1;
     const int K = (int)std::min(64.0, std::max(1.0, std::floor(tiles / (16.0 * n_sm))));
     P.max_slots = 0;
+    for (int c = 0; c < P.n_clouds; c++) {
+        if (!(P.hc[c].fp.flags & SG_F_COULOMB)) continue;
+        const int nj = P.hc[c].npad / SG_SYM_JT;
+        if (pairs) P.max_slots = std::max(P.max_slots, (nj + 1) * parts);
+        for (int b = 0; !pairs && b * TB < nj; b++)
+            P.max_slots = std::max(P.max_slots, b + 1 + (nj - b * TB + K - 1) / K);
+    }
+    if (!sym_fits(3 * sizeof(double) * (size_t)P.max_slots * P.npad)) {
+        P.max_slots = 0;
+        return false;
+    }
     for (int c = 0; c < P.n_clouds; c++) {
         SgCloud& cl = P.hc[c];
         cl.nslots = 0;
@@ -335,7 +356,6 @@ void plan_sym(Problem& P, int n_sm) {
                     cl.nslots = std::max(cl.nslots, it.slot + 1);
                     P.hitems.push_back(it);
                 }
-        P.max_slots = std::max(P.max_slots, cl.nslots);
         P.cloud_inter[c] = (double)cl.n * (cl.n - 1);
     }
     // diagonal items (about half a tile's work each) last
@@ -343,6 +363,7 @@ void plan_sym(Problem& P, int n_sm) {
         return (a.j0 >= a.i0 + a.ni) > (b.j0 >= b.i0 + b.ni);
     });
     P.n_items = (int)P.hitems.size();
+    return true;
 }
 
 // Shape 17: near items (half a leaf, one in C of its near leaves) and far items (leaf
@@ -461,8 +482,8 @@ void plan(Problem& P, int n_sm) {
             if (P.hc[c].npad > SG_SYM_MAX_IONS) P.sym = false;
     }
     if (P.sym) {
-        plan_sym(P, n_sm);
-        return;
+        P.sym = plan_sym(P, n_sm);
+        if (P.sym) return;
     }
     if (f32 && P.variant == SG_C32_FAR_ONCE) {
         for (int c = 0; c < C; c++)
@@ -696,7 +717,8 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     CK(dalloc(&P.y, 6 * N));
     CK(dalloc(&P.ys, 6 * N));
     CK(dalloc(&P.k, 42 * N));
-    CK(dalloc(&P.part, (size_t)std::max(P.max_slots, 1) * SG_PART_DOUBLES * NP));
+    const size_t part = (size_t)std::max(P.max_slots, 1) * sg_part_doubles(P.precision == SG_PREC_FP32C) * NP;
+    CK(dalloc(&P.part, part));
     CK(dalloc(&P.coulS, 3 * N));
     CK(dalloc(&P.coul1, 3 * N));
     CK(dalloc(&P.coul7, 3 * N));
@@ -764,7 +786,7 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     for (int i = 0; i < P.n; i++) P.perm[i] = i;
     CK(cudaMemcpy(P.dperm, P.perm.data(), sizeof(int) * P.n, cudaMemcpyHostToDevice));
     CK(cudaMemset(P.coul1, 0, 3 * N * sizeof(double)));
-    CK(cudaMemset(P.part, 0, (size_t)std::max(P.max_slots, 1) * SG_PART_DOUBLES * NP * sizeof(double)));
+    CK(cudaMemset(P.part, 0, part * sizeof(double)));
     CK(cudaMemset(P.coulS, 0, 3 * N * sizeof(double)));
     CK(cudaMallocHost((void**)&P.hctrl, sizeof(SgCtrl) * (size_t)std::max(P.n_clouds, 1)));
     CK(cudaMemcpy(P.drows, P.hrows.data(), sizeof(SgRowBlock) * P.hrows.size(),

@@ -68,10 +68,10 @@ inline cudaError_t sg_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 // sums hi x, y, z, lo x, y, z in frame units, and the conditioning estimates of the near
 // tiles and of the far tiles (sums of squared partial sums).  FP64: three doubles (SI).
 #define SG_PART_F32 8
-#define SG_PART_DOUBLES 4  // allocated per ion and slot: the larger of the two
+__host__ __device__ inline int sg_part_doubles(bool fp32c) { return fp32c ? SG_PART_F32 / 2 : 3; }
 // FP64 Coulomb, each unordered pair once (fp64_pairs.cuh): ions per i-block, ions per
 // j-tile, and the largest cloud it takes (its j-side partial sums need a slot per i-block:
-// 3 GB there; larger clouds sum ordered pairs).
+// 3.2 GB there; larger clouds, and batches that need more than 4 GiB, sum ordered pairs).
 #define SG_SYM_IB 128
 #define SG_SYM_JT 32
 #define SG_SYM_MAX_IONS 131072
