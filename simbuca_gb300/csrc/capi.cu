@@ -2762,7 +2762,8 @@ int cb_begin(double xj[][3], double mj[], double xi[][3], double eps2, int ni, i
     // one set against itself, bit for bit, takes each unordered pair once; comparing the
     // arrays costs the host ~10 us per 10,000 ions, the pairs it saves milliseconds
     const int same = ni == nj && ni <= SG_SYM_MAX_IONS &&
-                     memcmp(xj, xi, 3 * sizeof(double) * (size_t)ni) == 0;
+                     memcmp(xj, xi, 3 * sizeof(double) * (size_t)ni) == 0 &&
+                     sym_fits(sizeof(double) * sg_cunbody_scratch(ni, nj, 1, ctx->n_sm));
     int uniform = same && mj[0] != 0.0 && std::isfinite(mj[0]);
     for (int j = 1; uniform && j < nj; j++) uniform = mj[j] == mj[0];
     const size_t need = sg_cunbody_scratch(ni, nj, same, ctx->n_sm);
@@ -2786,6 +2787,13 @@ int cb_end(double ai[][3], int ni) {
     if (!ctx) return SG_NOT_READY;
     CK(cudaStreamSynchronize(ctx->stream));
     memcpy(ai, ctx->cb_host, 3 * sizeof(double) * (size_t)ni);
+    // partial sums of large sets (3.2 GB at 131,072 ions, 0.3 s of work) are given back;
+    // up to 256 MB are kept for the next call
+    if (ctx->cb_part_cap > ((size_t)1 << 28) / sizeof(double)) {
+        cudaFree(ctx->cb_part);
+        ctx->cb_part = nullptr;
+        ctx->cb_part_cap = 0;
+    }
     return SG_OK;
 }
 }  // namespace

@@ -69,3 +69,23 @@ def test_set_sizes_and_coincident_pairs(ni, nj, eps2):
         ai = call("cunbody1_force", xj, mj, xi, eps2)
         ref = reference_sum(xj, mj, xi, eps2)
         np.testing.assert_allclose(ai, ref, rtol=1e-11, atol=1e-11 * np.abs(ref).max())
+
+
+def test_scratch_of_a_large_set_is_given_back():
+    """Partial sums of one set against itself: 0.8 GB at 65,536 ions while the call runs, at most
+    256 MB of them kept for the next one (with the buffers and the runtime's own granularity:
+    512 MB); sums checked on a few rows."""
+    torch = pytest.importorskip("torch")
+    n = 65536
+    rng = np.random.default_rng(n)
+    x = rng.normal(0, 1e-3, (n, 3))
+    mj = np.ones(n)
+    call("cunbody1_force", x[:256].copy(), mj[:256], x[:256].copy(), 0.0)  # the context exists
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    ai = call("cunbody1_force", x, mj, x.copy(), 0.0)
+    assert before - torch.cuda.mem_get_info()[0] <= 512 << 20
+    for i in (0, 127, 128, 40000, n - 1):
+        d = np.delete(x, i, axis=0) - x[i]
+        ref = (d / (d * d).sum(1)[:, None] ** 1.5).sum(0)
+        np.testing.assert_allclose(ai[i], ref, rtol=1e-11, atol=1e-11 * np.abs(ref).max())
