@@ -124,7 +124,7 @@ __device__ __forceinline__ float close_pairs_warp(const float (*tl)[TL], int jb,
             }
             if (close) {
                 const float wf = __fmul_rn(q, wc);
-                if (p.y3 <= kVeryClose) {
+                if (!very_close(p.y3, xih, yih, zih)) {
                     close_term_ff(ff_diff(xh, xl, xih, xil), ff_diff(yh, yl, yih, yil),
                                   ff_diff(zh, zl, zih, zil), q, wf, p, cx, cy, cz);
                 } else {
@@ -1595,7 +1595,7 @@ __device__ float close_list_terms(const SgCloud& cl, int ig, int m, const int* _
         fmx = fmaxf(fmx, capped_term_y3(pr.y3, cl.wc));
         const float wf = __fmul_rn(q, cl.wc);
         ff dx, dy, dz;
-        if (pr.y3 <= kVeryClose) {
+        if (!very_close(pr.y3, xih, yih, zih)) {
             close_term_ff(ff_diff(xjh, xjl, xih, xil), ff_diff(yjh, yjl, yih, yil),
                           ff_diff(zjh, zjl, zih, zil), q, wf, pr, dx, dy, dz);
         } else {

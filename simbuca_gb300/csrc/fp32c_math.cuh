@@ -145,9 +145,16 @@ __device__ __forceinline__ ff ff_mul(ff a, ff b) {
 }
 
 // Beyond this 1/r^3 (frame units: closer than 1e-5 of the cloud's spread) a close pair's
-// distance is taken from the SI coordinates in FP64; float-float frame coordinates
-// (absolute error ~1e-14) give the others to better than ~1e-9.
+// distance is taken from the SI coordinates in FP64.  Float-float frame coordinates have an
+// error of ~2^-49 |u|, so the distance grows with the ion's |u| where that is above 1 (the
+// frame stays where the cloud was uploaded, the cloud need not): a pair farther apart than
+// 1e-5 max(1, |u|) has its distance to ~4e-10 and its term to ~1e-9.  (Without the factor a
+// pair 1.2e-5 spreads apart, 10,000 spreads away from the frame: 6e-7; so: 1e-11.)
 constexpr float kVeryClose = 1e15f;
+__device__ __forceinline__ bool very_close(float y3, float x, float y, float z) {
+    const float m = fmaxf(fmaxf(1.0f, fabsf(x)), fmaxf(fabsf(y), fabsf(z)));
+    return y3 * m * m * m > kVeryClose;  // infinity: the FP64 form
+}
 
 // A close pair's exact term q u / |u|^3 (u = u_j - u_i in float-float; q the normalized
 // charge) minus the capped FP32 term wf d the main loop has summed, per component, in

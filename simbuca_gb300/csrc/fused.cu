@@ -421,7 +421,7 @@ __device__ __forceinline__ IonSums ion_pairs(const float* X, const float* Q, int
             fmx = fmaxf(fmx, capped_term_y3(pr.y3, wc));
             const float wf = __fmul_rn(Q[jj], wc);
             ff dx, dy, dz;
-            if (pr.y3 <= kVeryClose) {
+            if (!very_close(pr.y3, xih, yih, zih)) {
                 close_term_ff(ff_diff(X[jj], XL[jj], xih, xil), ff_diff(Y[jj], YL[jj], yih, yil),
                               ff_diff(Z[jj], ZL[jj], zih, zil), Q[jj], wf, pr, dx, dy, dz);
             } else {
