@@ -42,6 +42,7 @@ struct Problem {
     std::vector<SgWorkItem> hitems;
     std::vector<SgFarItem> hfar, hnear;   // shape 17
     int leaf_min = 0;              // ... its clouds of more ions; smaller ones are plain
+    bool leaf_strict = false;      // ... flag as the ordered-pair k-d shapes do (leaf_kappa)
     SgFarItem *dfar = nullptr, *dnear = nullptr;
     std::vector<int> hleaf;        // cloud of each leaf
     int near_cap = 0;              // leaves of the largest cloud
@@ -266,6 +267,29 @@ constexpr int kFarOnceMax = 1 << 21;
 // 1,101, 20 of 3,000 1,156 / 994, 10 of 4,096 1,009 / 812; below ~3,000 ions the leaves' errors
 // are 4 % larger (RMS), above smaller.
 constexpr int kLeafMin = 2500;
+// Clouds of this many ions, and batches of this many ordered pairs, take k-d ordered leaves
+// throughout and hold the errors of the ordered-pair shapes 9 and 14.
+constexpr int kLeafAlways = 24000;
+constexpr double kLeafAlwaysPairs = 2e9;
+
+// Conditioning threshold sqrt(s2) / |P| of a leaf sum.  Its partial sums have 16 terms and
+// are coherent, so the estimate differs from that of the other forms at the same error; the
+// thresholds are set by the tails.  Ions above 3e-7 per million, over 1.8 to 6.6 million ions
+// of a size (Gaussian / uniform / elongated clouds):
+//   strict, against shapes 9 and 14 (at 1.0 up to 4,096 ions, 1.5 above):
+//     2,600 ions 0.2 / 0.3 / 35, leaves at 1.0 0.0 / 0.6 / 29, at 2.0 60 / 187 / 615;
+//     4,096 0.3 / 1.1 / 21, at 1.0 0.3 / 1.5 / 20; 1,000 0.0 / 2.5 / 41, at 1.0 0.0 / 5.5 / 44;
+//     6,000 2.7 / 26 / 105, at 1.25 1.0 / 12 / 51; 8,192 2.3 / 16 / 79, at 1.25 0.4 / 8 / 41;
+//     30,000 1.7 / 21 / 39, at 1.15 1.7 / 6 / 24, at 1.5 7.8 / 36 / 52;
+//     65,536 2.4 / 32 / 30, at 1.15 1.0 / 21 / 16; 140,000 2.1 / 35 / 46, at 1.15 0.0 / 23 / 36.
+//   other automatic clouds, against the plain order they would have (1.0, 1.5 above 4,096):
+//     2,600 99 / 339 / 755, leaves at 1.5 8 / 41 / 219; 4,096 65 / 229 / 491, at 1.5 5.5 / 42 / 125;
+//     6,000 189 / 617 / 1,282, at 2.0 32 / 150 / 277; 20,001 83 / 326 / 523, at 2.0 21 / 120 / 142.
+float leaf_kappa(int npad, bool strict) {
+    if (npad <= SG_SMALL_ROW) return strict ? 1.0f : 1.5f;
+    if (npad <= kLeafAlways) return strict ? 1.25f : 2.0f;
+    return 1.15f;
+}
 
 // Measured on GB300 (us per Coulomb call, shapes 5 / 9 / 14 / 17): 8,000 ions 57 / 52 / 62 /
 // 53, 20,001 ions 250 / 195 / 203 / 151, 65,536 ions 2,483 / 1,755 / 1,756 / 1,245.  One
@@ -279,13 +303,16 @@ constexpr int kLeafMin = 2500;
 int auto_variant(const std::vector<int>& counts, int requested, bool resident) {
     int big = 0;
     long long total = 0;
+    double pairs = 0.0;
     for (int n : counts) {
         big = std::max(big, n);
         total += n;
+        pairs += (double)n * n;
     }
     if (requested >= 0) return requested == SG_C32_FAR_ONCE && big > kFarOnceMax ? 14 : requested;
     if (big > kFarOnceMax) return 14;
-    if (big > (resident ? SG_FINISH_MAX_IONS : 24000)) return SG_C32_FAR_ONCE;
+    if (big > (resident ? SG_FINISH_MAX_IONS : kLeafAlways)) return SG_C32_FAR_ONCE;
+    if (resident && pairs >= kLeafAlwaysPairs) return SG_C32_FAR_ONCE;
     if (resident && total > SG_FINISH_MAX_IONS && big > kLeafMin) return SG_C32_FAR_ONCE;
     return big <= 6000 && total <= 32768 ? 11 : 5;
 }
@@ -296,6 +323,18 @@ bool sym_fits(size_t bytes) {
     if (bytes <= (size_t)1 << 28) return true;
     size_t left = 0, total = 0;
     return bytes <= (size_t)1 << 32 && cudaMemGetInfo(&left, &total) == cudaSuccess && bytes <= left / 2;
+}
+
+// Which clouds of a shape-17 problem are leaves, and their thresholds.
+void set_leaf_rule(Problem& P, int requested) {
+    double pairs = 0.0;
+    bool big = false;
+    for (int n : P.counts) {
+        pairs += (double)n * n;
+        big = big || n >= kLeafAlways;
+    }
+    P.leaf_strict = requested == SG_C32_FAR_ONCE || big || pairs >= kLeafAlwaysPairs;
+    P.leaf_min = P.leaf_strict ? 0 : kLeafMin;
 }
 
 // FP64 items that take each unordered pair once: i-block b (128 ions) against the j-tiles
@@ -488,6 +527,10 @@ void plan(Problem& P, int n_sm) {
     if (f32 && P.variant == SG_C32_FAR_ONCE) {
         for (int c = 0; c < C; c++)
             P.hc[c].leafs = (P.hc[c].fp.flags & SG_F_COULOMB) && P.hc[c].n > P.leaf_min;
+        for (int c = 0; c < C; c++) {
+            const float k = leaf_kappa(P.hc[c].npad, P.leaf_strict);
+            P.hc[c].kleaf2 = k * k;
+        }
         plan_far_once(P, n_sm);
     }
     const int ib = f32 ? sg_coulomb_fp32c_ib(P.variant == SG_C32_FAR_ONCE ? SG_C32_PLAIN : P.variant)
@@ -1521,7 +1564,7 @@ int solo_prepare(sg_ctx* ctx, int n, int precision, const sg_field_params& fp) {
         P.counts.assign(1, n);
         P.precision = precision;
         P.variant = auto_variant(P.counts, ctx->c32_variant, false);
-        P.leaf_min = ctx->c32_variant == SG_C32_FAR_ONCE ? 0 : kLeafMin;
+        set_leaf_rule(P, ctx->c32_variant);
         P.hc.assign(1, SgCloud());
         P.hc[0].fp = fp;
         plan(P, ctx->n_sm);
@@ -1714,7 +1757,7 @@ int sg_batch_create(sg_ctx* ctx, int n_clouds, const int* counts, const sg_field
     P.counts.assign(counts, counts + n_clouds);
     P.precision = precision;
     P.variant = auto_variant(P.counts, ctx->c32_variant, true);
-    P.leaf_min = ctx->c32_variant == SG_C32_FAR_ONCE ? 0 : kLeafMin;
+    set_leaf_rule(P, ctx->c32_variant);
     P.method = op[0].method == 0 ? 5 : op[0].method;
     P.hc.assign(n_clouds, SgCloud());
     for (int c = 0; c < n_clouds; c++) P.hc[c].fp = fp[c];

@@ -1746,7 +1746,7 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
             const float pf2 = fmaf(px.h, px.h, fmaf(py.h, py.h, pz.h * pz.h));
             // the far threshold: the prior of the frame set-up, or the measured one
             const float kf2 = chk ? fminf(cl.kfar2, chk[rb.cloud].kfar2) : cl.kfar2;
-            const float kap2 = cl.leafs ? sg_kappa2_leaf(cl.npad) : sg_kappa2(cl.npad);
+            const float kap2 = cl.leafs ? cl.kleaf2 : sg_kappa2(cl.npad);
             kind = (many || s2 > kap2 * pf2 ? kFixNear : 0) | (s2f > kf2 * pf2 ? kFixFar : 0);
             if (risk != nullptr) {
                 const float pf = sqrtf(pf2);

@@ -154,7 +154,7 @@ struct SgCloud {
     float far_fs, far_fs2, near_fs2;
     int32_t leafs;  // shape 17: k-d ordered leaf pairs (else the plain kernel)
     int32_t sym_k;  // FP64 unordered items of K j-tiles (0: every ion has nslots slots)
-    int32_t pad4;
+    float kleaf2;   // shape 17: conditioning threshold of the leaf sums (leaf_kappa in capi.cu)
 };
 
 // Partial-sum slots of the FP64 symmetric form that hold a part of local padded ion p: one
@@ -459,17 +459,10 @@ struct SgDpArgs {
 // > |P| in clouds of up to SG_SMALL_ROW padded ions, whose FP64 row is cheap and whose
 // error per unit of sqrt(s2)/|P| ran up to ~9e-7 with their few terms per ion (an
 // unflagged ion at 1.37 measured 1.2e-6 in the 512-cloud scan's small clouds; 2.5e-7 at
-// most on the 65,536-ion cloud).  Their flagged rows are one work unit each.
+// most on the 65,536-ion cloud).  The leaf sums have thresholds of their own
+// (SgCloud::kleaf2), and so has the fused path (SG_FUSED_LOOSE_IONS).
 #define SG_SMALL_ROW 4096
 __device__ __forceinline__ float sg_kappa2(int npad) { return npad <= SG_SMALL_ROW ? 1.0f : 2.25f; }
-// k-d ordered leaves (shape 17): their partial sums are coherent, so sqrt(s2)/|P| is larger
-// for the same error.  Largest errors over 2 to 40 Gaussian and uniform clouds of a size,
-// plain order at its threshold / leaves at 1.5 / at 2: 1,000 ions 3.3e-7 / 3.6e-7 / 5.2e-7,
-// 2,000 4.0e-7 / 3.7e-7 / 3.7e-7, 4,000 4.8e-7 / 3.3e-7 / 4.0e-7, 8,000 7.1e-7 / 3.4e-7 /
-// 3.9e-7, 20,001 6.8e-7 / 3.2e-7 / 3.7e-7; the larger clouds had k-d order and 1.5 before.
-__device__ __forceinline__ float sg_kappa2_leaf(int npad) {
-    return npad <= 1024 ? 1.5625f : npad <= 24000 ? 4.0f : 2.25f;
-}
 // Close pairs listed per ion (shape 17); an ion with more gets its FP64 row.
 #define SG_CLOSE_CAP 8
 
