@@ -1319,8 +1319,7 @@ int run_fused(sg_ctx* ctx, Problem& P, int n, int counted, int one_step = 0) {
     f.n_clouds = P.n_clouds;
     f.max_attempts = n;
     f.one_step = one_step;
-    f.kappa2 = big_fused(P) <= SG_FUSED_LOOSE_IONS && P.n_clouds * SG_FUSED_MAX_CTAS <= ctx->n_sm
-                   ? 2.25f : 1.21f;
+    f.loose = big_fused(P) <= SG_FUSED_LOOSE_IONS && P.n_clouds * SG_FUSED_MAX_CTAS <= ctx->n_sm;
     f.ctas = wide ? P.fused_wide : 0;
     f.barrier = P.fused_barrier;
     f.notes = P.fused_notes;

@@ -16,7 +16,7 @@
 //     interleaved G-ths of the cloud, in the FP32-compensated form of the tiled kernels
 //     (float-float differences, SFU 1/r, 1/r^3 capped with float-float close pairs, partial
 //     sums folded into Kahan accumulators every 16 j-ions, the G parts added in
-//     float-float); an ion whose terms cancel strongly (s2 > kappa2 |P|^2) gets its whole
+//     float-float); an ion whose terms cancel strongly (s2 > kappa2 |P|^2, sg_kappa2_fused) gets its whole
 //     row in FP64 instead, spread over the CTA's warps or (larger wide clouds) all CTAs;
 //   * control: error partials go to every CTA, and every CTA decides alike
 //     (error_succes and step(), sg_error_succes; bin/ode.cpp:426-494), so the commit
@@ -524,7 +524,7 @@ __device__ __noinline__ bool coulomb_phase(const SgFusedArgs& f, const SgCloud& 
     // the conditioning test (frame units for a unit charge)
     if (il < mo && q == 0) {
         const float pf2 = fmaf(px.h, px.h, fmaf(py.h, py.h, pz.h * pz.h));
-        const bool flagged = ps2 > f.kappa2 * pf2;
+        const bool flagged = ps2 > sg_kappa2_fused(npc, f.loose) * pf2;
         s.flag[il] = flagged;
         if (flagged) {
             s.list[atomicAdd(&sh.nflag, 1)] = il;

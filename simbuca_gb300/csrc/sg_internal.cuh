@@ -502,12 +502,18 @@ cudaError_t sg_dp_finish(const SgFinishArgs& f, int stage, int fp32c, cudaStream
 // / 82 / 227, 4 of 2,000 - / 195 (106,000) / 245, 2 of 4,000 - / 301 (212,000) / 309; 70 of 100 on
 // 2 CTAs each 66 (5,000) / 76 / 224.
 #define SG_FUSED_CLUSTER_PAIRS 8000
-// Conditioning threshold of the fused path: sqrt(s2) > 1.5 |P| for a few clouds of up to so
-// many ions, > 1.1 |P| for the others, whose largest errors are then the tiled kernels' at
-// their 1.0 (the fused partial sums interleave the cloud's ions): 1,000 ions 3.9e-7 (3.8e-7;
-// at 1.5 4.5e-7), 1,500 3.9e-7 (3.4e-7; 5.0e-7), 3,000 3.9e-7 (4.7e-7; 5.3e-7), 24 of 300
-// 4.6e-7 (4.1e-7; 5.4e-7), largest of 5,000 to 58,000 probes each.
+// Conditioning threshold of the fused path (its partial sums interleave the cloud's ions):
+// sqrt(s2) > 1.5 |P| for a few clouds of up to SG_FUSED_LOOSE_IONS ions, which it always
+// took; for those it has from the tiled kernels their 1.0, or 1.1 above 2,048 padded ions,
+// where the tiled partial sums are 128 terms long and not 16.  Ions above 3e-7 per million,
+// tiled / fused at 1.0 / at 1.1, over 2 to 4 million ions each: 600 ions 23 / 10 / 23, uniform
+// density 89 / 39 / 83; 1,000 9 / 6.5 / 18, 66 / 43 / 90; 2,000 9 / 4.5 / 11, 38 / 32 / 65;
+// 24 of 300 31 / 33 / 64, 138 / 103 / 191; 8 of 700 16 / 13 / 32, 84 / 74 / 138; 3,000 90 / 8 / 16,
+// 303 / 29 / 57; 4,000 73 / 6 / 17, 269 / 25 / 48.
 #define SG_FUSED_LOOSE_IONS 512
+__device__ __forceinline__ float sg_kappa2_fused(int npad, bool loose) {
+    return loose ? 2.25f : npad <= 2048 ? 1.0f : 1.21f;
+}
 #define SG_FUSED_WIDE_PAIRS 120000
 #define SG_FUSED_AUTO_PAIRS 40000
 struct SgFusedArgs {
@@ -522,7 +528,7 @@ struct SgFusedArgs {
     int* ran;
     int n, npad, n_clouds;
     int max_attempts;  // attempts per launch at most
-    float kappa2;      // conditioning threshold
+    int loose;         // conditioning threshold: sg_kappa2_fused
     int one_step;      // 1: each cloud stops after an accepted attempt; 2: those that have not yet
     // wide form: CTAs per cloud (0: clusters), c64 and c32 hold two coordinate sets
     int ctas;
