@@ -408,7 +408,12 @@ bool plan_sym(Problem& P, int n_sm) {
 // Shape 17: near items (half a leaf, one in C of its near leaves) and far items (leaf
 // against up to 32 later leaves).  C so that a warp slot of the device (18 warps per SM)
 // gets at least ~8 near items, far runs so that it gets at least ~8 far ones, unless the
-// cloud is large enough for whole runs of 32.
+// cloud is large enough for whole runs of 32.  C up to 20: once the ions have mixed, every
+// leaf of a small cloud is near every other (set_state with the ions permuted), and a leaf's
+// list is as long as the cloud has later leaves; in eighths the first leaves' items held up
+// the rest.  us per attempt, mixed, plain order before the leaves / C <= 8 / <= 20: 9,000 ions
+// 615 / 762 / 540, 12,000 905 / 1,023 / 679, 20,001 1,793 / 2,009 / 1,568, 3 clouds of 8,000
+// 1,035 / 1,190 / 963; in order 478 / 491 / 488, 583 / 584, 1,101 / 1,114, 770 / 781.
 void plan_far_once(Problem& P, int n_sm) {
     double leaves = 0.0, pairs = 0.0;
     for (int c = 0; c < P.n_clouds; c++) {
@@ -419,7 +424,7 @@ void plan_far_once(Problem& P, int n_sm) {
     }
     if (leaves == 0.0) pairs = 1.0;
     const double slots = 18.0 * n_sm * 8.0;
-    const int C = (int)std::min(8.0, std::max(1.0, std::ceil(0.5 * slots / std::max(leaves, 1.0))));
+    const int C = (int)std::min(20.0, std::max(1.0, std::ceil(0.5 * slots / std::max(leaves, 1.0))));
     const int K = (int)std::min(32.0, std::max(1.0, std::floor(pairs / slots)));
     P.hfar.clear();
     P.hnear.clear();

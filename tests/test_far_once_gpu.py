@@ -196,3 +196,33 @@ def test_batches_of_two_billion_pairs_flag_as_shape_9(ctx):
     part = ctx.fixup_count() / len(pos)
     print(part)
     assert part >= 0.006
+
+
+@pytest.mark.parametrize("counts", [[9001], [20001], [40007], [8000, 100, 3001, 2600]])
+def test_set_state_on_a_mixed_order(ctx, counts):
+    """set_state keeps the ion order of the upload: with the ions permuted within each cloud
+    every leaf spans its cloud and all leaf pairs are near, the longest lists there are.  Each
+    ion then goes where it goes from an upload of that state (fixed steps, bounds as above), and
+    its sums do not depend on the run."""
+    rng = configs.rng_for(sum(counts) + 1)
+    clouds = [configs.gaussian_cloud(rng, n, 5e-4, 300.0, np.full(n, configs.M_CS)) for n in counts]
+    fp = configs.penning_field(quad=(0.5, configs.nu_c(configs.M_CS), 0.0, 0.0, 1.0), delta=1e3)
+    op = configs.ode(1e-9, 1e-15, 2e-9, 1.0, adaptive=False)
+    first = np.cumsum([0] + counts[:-1])
+    perm = np.concatenate([at + np.random.default_rng(1).permutation(n) for at, n in zip(first, counts)])
+    pos, vel = np.concatenate([c.pos for c in clouds]), np.concatenate([c.vel for c in clouds])
+    mass, q = np.concatenate([c.mass for c in clouds]), np.concatenate([c.charge for c in clouds]).astype(np.int32)
+    b = Batch(ctx, counts, [fp] * len(counts), [op] * len(counts), SG_PREC_FP32C)
+    assert b.variant() == 17
+    out = []
+    for _ in range(2):
+        b.upload(pos, vel, mass, q)
+        b.set_state(pos[perm], vel[perm])
+        b.attempts(3)
+        out.append(b.download())
+    assert all(np.array_equal(x, y) for x, y in zip(*out))
+    b.upload(pos[perm], vel[perm], mass, q)
+    b.attempts(3)
+    for got, ref in zip(out[0], b.download()):
+        for at, n in zip(first, counts):
+            assert np.abs(got[at:at + n] - ref[at:at + n]).max() <= 1e-9 * np.abs(ref[at:at + n]).max()
