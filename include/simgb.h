@@ -311,8 +311,10 @@ int sg_batch_set_far_threshold(sg_ctx* ctx, double kfar);
  * `tile` has arrived, also waits on a barrier that nothing arrives at until limit_us
  * microseconds (1 .. 1e6) have passed, and then takes its timeout path: it raises
  * SG_TIMEOUT, waits (bounded) for the copies it has issued, and returns without writing
- * sums.  (The small-cloud kernel that spreads a cloud over many CTAs does so at its first
- * barrier, for tile 0.)  The attempt is then neither accepted nor used for step control: every cloud
+ * sums.  (The leaf-pair kernel of shape 17 has no wait that could run out: its warps with
+ * more than `tile` leaf pairs wait for the limit before the first and add nothing.  The
+ * small-cloud kernel that spreads a cloud over many CTAs gives up at its first barrier,
+ * for tile 0; the cluster form has no bounded wait.)  The attempt is then neither accepted nor used for step control: every cloud
  * stops with status SG_TIMEOUT and the call returns it.  tile < 0 turns the test off;
  * sg_batch_upload clears the error word.  No copy is left in flight and no device
  * state is lost: the context stays usable. */

@@ -615,6 +615,19 @@ __device__ __forceinline__ void leaf_add(const LeafAcc& A, size_t NP, int c, int
     atomicAdd(A.sum + c * NP + ig, (unsigned long long)far_fixed(h, l, fs));
 }
 
+// The wait test (flags[SG_FLAG_WAIT_TILE] = t + 1) in a warp of the leaf kernel with more than
+// t leaf pairs to take: it waits until the test's limit has passed, raises SG_TIMEOUT and adds
+// nothing.  Its copies are cp.async groups, which have no wait that could run out.
+__device__ __forceinline__ bool leaf_wait_test(int* flags, int pairs) {
+    const int t = flags[SG_FLAG_WAIT_TILE];
+    if (t == 0 || t > pairs) return false;
+    const uint64_t limit = 1000ull * (uint64_t)max(flags[SG_FLAG_WAIT_US], 1), t0 = globaltimer();
+    while (globaltimer() - t0 <= limit) {
+    }
+    if ((threadIdx.x & 31) == 0) atomicExch(flags, SG_TIMEOUT);
+    return true;
+}
+
 // Far pairs of leaf I against up to 32 leaves J > I, by one warp, each unordered pair
 // once, from the high parts.  Bound by the FMA pipe: 8 packed FP32x2 operations shared by
 // the two ions and 3 for each, 7 lane operations per ordered pair where summing each
@@ -752,7 +765,8 @@ __device__ __forceinline__ void far_leaf(const float (*tj)[SG_TILE], FarWarpShar
 template <bool S2F>
 __device__ __forceinline__ void far_warp(const float* __restrict__ c32, const SgFarItem& it,
                                          const SgCloud& cl, const LeafAcc& acc, int npad_total,
-                                         const float* __restrict__ bbox, FarWarpShared<S2F>& sh) {
+                                         const float* __restrict__ bbox, int* flags,
+                                         FarWarpShared<S2F>& sh) {
     const int lane = threadIdx.x & 31;
     const size_t NP = (size_t)npad_total;
     // far leaves of the item: a lane each
@@ -764,7 +778,7 @@ __device__ __forceinline__ void far_warp(const float* __restrict__ c32, const Sg
         for (int q = 0; q < 6; q++) jb[q] = bbox[8 * (size_t)(cl.tile0 + J) + q];
         m = __ballot_sync(0xffffffffu, lane < it.n && box_dist2(ib, jb) > cl.dfar * cl.dfar);
     }
-    if (m == 0) return;
+    if (m == 0 || leaf_wait_test(flags, __popc(m))) return;
     // leaf I is whole: only the last leaf of a cloud may not be, and I < J
     const int i0 = cl.poff + it.leaf * SG_TILE;
     f2 xi[3][4];
@@ -976,13 +990,14 @@ __device__ __forceinline__ void near_warp(const float* __restrict__ c32, const S
                                           const SgCloud& cl, const LeafAcc& acc, int npad_total,
                                           const int* __restrict__ counts,
                                           const unsigned short* __restrict__ lists, int cap,
-                                          NearWarpShared& sh) {
+                                          int* flags, NearWarpShared& sh) {
     const int lane = threadIdx.x & 31;
     const size_t NP = (size_t)npad_total;
     const int leaf = it.leaf >> 1, i0 = cl.poff + leaf * SG_TILE + (it.leaf & 1) * (SG_TILE / 2);
     const int end = cl.poff + cl.n, pend = cl.poff + cl.npad;
     const int count = counts[cl.tile0 + leaf];
     if (i0 >= end || it.j0 >= count) return;
+    if (leaf_wait_test(flags, (count - it.j0 + it.n - 1) / it.n)) return;
     const unsigned short* L = lists + (size_t)(cl.tile0 + leaf) * cap;
     NearSide w;
 #pragma unroll
@@ -1070,7 +1085,7 @@ __global__ void __launch_bounds__(32, 19) coulomb_leaf_kernel(
     const float* __restrict__ c32, const SgFarItem* __restrict__ near_items, int n_near,
     const SgFarItem* __restrict__ far_items, int n_far, const SgCloud* __restrict__ clouds,
     const SgCtrl* __restrict__ ctrl, LeafAcc acc, int npad_total, const float* __restrict__ bbox,
-    const int* __restrict__ counts, const unsigned short* __restrict__ lists, int cap) {
+    const int* __restrict__ counts, const unsigned short* __restrict__ lists, int cap, int* flags) {
     sg_griddep_wait();
     typedef FarWarpShared<S2F> Far;
     constexpr size_t kWarp = sizeof(NearWarpShared) > sizeof(Far) ? sizeof(NearWarpShared) : sizeof(Far);
@@ -1081,10 +1096,10 @@ __global__ void __launch_bounds__(32, 19) coulomb_leaf_kernel(
         (ctrl[it.cloud].done || ctrl[it.cloud].hold || ctrl[it.cloud].status != SG_OK))
         return;
     if (near)
-        near_warp(c32, it, clouds[it.cloud], acc, npad_total, counts, lists, cap,
+        near_warp(c32, it, clouds[it.cloud], acc, npad_total, counts, lists, cap, flags,
                   *reinterpret_cast<NearWarpShared*>(raw));
     else
-        far_warp<S2F>(c32, it, clouds[it.cloud], acc, npad_total, bbox,
+        far_warp<S2F>(c32, it, clouds[it.cloud], acc, npad_total, bbox, flags,
                       *reinterpret_cast<Far*>(raw));
 }
 
@@ -2009,7 +2024,8 @@ cudaError_t sg_launch_coulomb_fp32c(const SgCoulombArgs& a, cudaStream_t s) {
                 sg_launch(a.far_estimate ? coulomb_leaf_kernel<true> : coulomb_leaf_kernel<false>,
                           a.n_near + a.n_far, 32, 0, s, a.c32, a.near_items, a.n_near, a.far_items,
                           a.n_far, a.clouds, a.ctrl, acc, a.npad_total, a.bbox,
-                          (const int*)a.near_count, (const unsigned short*)a.near_list, a.near_cap);
+                          (const int*)a.near_count, (const unsigned short*)a.near_list, a.near_cap,
+                          a.errword);
             }
             break;
         case 10:

@@ -52,3 +52,36 @@ def test_ring_wait_times_out_and_context_recovers(ctx, variant):
     finally:
         ctx.set_coulomb_variant(-1)
         ctx.set_fused(True)
+
+
+@pytest.mark.parametrize("counts,tile", [([9001], 0), ([30000], 0), ([30000], 1), ([7000, 100, 1500, 900], 0)])
+def test_leaf_pairs_time_out_and_context_recovers(ctx, counts, tile):
+    """The automatic form above 8,192 ions: leaf pairs, alone and beside plain clouds, at the
+    first and the second leaf of a warp.  The accumulators of the refused attempt must not
+    reach the next one: after the new upload the step is the first run's to the last bit."""
+    n = sum(counts)
+    c = configs.penning_1k(n=n, seed=6).clouds[0]
+    fp = configs.penning_field(quad=(0.5, configs.nu_c(132.905), 0.0, 0.0, 1.0), delta=1e3)
+    b = Batch(ctx, counts, [fp] * len(counts), [configs.ode(1e-9, 1e-15, 1e-9, 1e-6)] * len(counts),
+              SG_PREC_FP32C)
+    assert b.variant() == 17
+    try:
+        b.upload(c.pos, c.vel, c.mass, c.charge)
+        _, st = b.step()
+        assert st == abi.SG_OK
+        ref_p, ref_v = b.download()
+        b.upload(c.pos, c.vel, c.mass, c.charge)
+        ctx.set_wait_test(tile, 100)
+        info, st = b.step(raise_on_error=False)
+        assert st == abi.SG_TIMEOUT
+        assert all(i["status"] == abi.SG_TIMEOUT and i["steps"] == 0 and i["t"] == 0.0 for i in info)
+        p, v = b.download()
+        assert np.array_equal(p, c.pos) and np.array_equal(v, c.vel)
+        ctx.set_wait_test(-1)
+        b.upload(c.pos, c.vel, c.mass, c.charge)
+        info, st = b.step()
+        assert st == abi.SG_OK and all(i["steps"] == 1 for i in info)
+        p, v = b.download()
+        assert np.array_equal(p, ref_p) and np.array_equal(v, ref_v)
+    finally:
+        ctx.set_wait_test(-1)
