@@ -14,13 +14,15 @@ namespace {
 // Two different sets: ordered pairs, 128 i-rows a block against one of the j-chunks, which
 // go to a partial-sum slot each ([chunk][3][ni], sums of xi - xj).  FP64-bound (16
 // instructions a pair, 64 cycles each): the j-chunks give every SM several blocks, where a
-// block per 128 rows alone left half of them idle (10,007 x 10,007: 7,535 us).
+// block per 128 rows alone left half of them idle (10,007 x 10,007: 7,535 us).  A single
+// chunk's sums go straight to ai (null otherwise): one launch for up to 128 j-ions.
 constexpr int kCbThreads = 128;
 __global__ void __launch_bounds__(kCbThreads) cunbody_kernel(const double* __restrict__ xj,
                                                              const double* __restrict__ mj,
                                                              const double* __restrict__ xi,
                                                              double eps2, double* __restrict__ part,
-                                                             int ni, int nj, int jc) {
+                                                             int ni, int nj, int jc,
+                                                             double* __restrict__ ai) {
     sg_griddep_wait();
     __shared__ double t[4][kCbThreads];
     const int i = blockIdx.x * kCbThreads + threadIdx.x;
@@ -53,7 +55,11 @@ __global__ void __launch_bounds__(kCbThreads) cunbody_kernel(const double* __res
                 az = fma(w, dz, az);
             }
     }
-    if (act) {
+    if (act && ai != nullptr) {
+        ai[3 * (size_t)i] = -ax;
+        ai[3 * (size_t)i + 1] = -ay;
+        ai[3 * (size_t)i + 2] = -az;
+    } else if (act) {
         double* P = part + (size_t)blockIdx.y * 3 * ni;
         P[i] = ax;
         P[ni + i] = ay;
@@ -167,7 +173,8 @@ cudaError_t sg_cunbody_launch(const double* xj, const double* mj, const double* 
         int jc = 0;
         p = SymPlan{0, 1, 0, cb_chunks(ni, nj, n_sm, &jc)};
         sg_launch(cunbody_kernel, dim3((ni + kCbThreads - 1) / kCbThreads, p.slots), kCbThreads, 0,
-                  st, xj, mj, xi, eps2, part, ni, nj, jc);
+                  st, xj, mj, xi, eps2, part, ni, nj, jc, p.slots == 1 ? ai : nullptr);
+        if (p.slots == 1) return cudaGetLastError();
     }
     sg_launch(sym_sum_kernel<16>, (ni + 15) / 16, 256, 0, st, (const double*)part, ni, stride, p,
               (const double*)nullptr, -1.0, ai);

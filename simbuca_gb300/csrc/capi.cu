@@ -2807,8 +2807,9 @@ int cb_begin(double xj[][3], double mj[], double xi[][3], double eps2, int ni, i
     CK(cudaMemcpyAsync(ctx->cb_mj, mj, sizeof(double) * nj, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->cb_xi, xi, 3 * sizeof(double) * ni, cudaMemcpyHostToDevice, ctx->stream));
     // one set against itself, bit for bit, takes each unordered pair once; comparing the
-    // arrays costs the host ~10 us per 10,000 ions, the pairs it saves milliseconds
-    const int same = ni == nj && ni <= SG_SYM_MAX_IONS &&
+    // arrays costs the host ~10 us per 10,000 ions, the pairs it saves milliseconds.  Up to 32
+    // ions the one launch of the ordered form is the faster (1 ion: 26 us, 37 with two).
+    const int same = ni == nj && ni > 32 && ni <= SG_SYM_MAX_IONS &&
                      memcmp(xj, xi, 3 * sizeof(double) * (size_t)ni) == 0 &&
                      sym_fits(sizeof(double) * sg_cunbody_scratch(ni, nj, 1, ctx->n_sm));
     int uniform = same && mj[0] != 0.0 && std::isfinite(mj[0]);

@@ -89,3 +89,37 @@ def test_scratch_of_a_large_set_is_given_back():
         d = np.delete(x, i, axis=0) - x[i]
         ref = (d / (d * d).sum(1)[:, None] ** 1.5).sum(0)
         np.testing.assert_allclose(ai[i], ref, rtol=1e-11, atol=1e-11 * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("ni,nj", [(1, 1), (2, 2), (31, 31), (32, 32), (33, 33), (1, 128), (300, 128),
+                                   (300, 129), (7, 1), (1, 0), (64, 33)])
+def test_one_launch_and_two_launch_sizes(ni, nj):
+    """Up to 128 j-ions the sums go straight to ai, beyond through partial sums; one set against
+    itself takes unordered pairs above 32 ions.  Both sides of each line; no j-ions give 0."""
+    rng = np.random.default_rng(100 * ni + nj)
+    xj = rng.normal(0, 1e-3, (nj, 3))
+    xi = xj.copy() if ni == nj else rng.normal(0, 1e-3, (ni, 3))
+    mj = rng.uniform(0.5, 2.0, nj)
+    for _ in range(2):
+        ai = call("cunbody1_force", xj, mj, xi, 1e-14)
+        ref = reference_sum(xj, mj, xi, 1e-14)
+        np.testing.assert_allclose(ai, ref, rtol=1e-11, atol=1e-11 * np.abs(ref).max())
+
+
+def test_a_single_ion_takes_one_launch():
+    """The call time of one ion against itself, which two launches made 10 us longer, against
+    that of 33 ions, which take two: shorter by at least a launch's few microseconds."""
+    import time
+
+    def best(n):
+        x, m = np.random.default_rng(n).normal(0, 1e-3, (n, 3)), np.ones(n)
+        t = []
+        for _ in range(200):
+            t0 = time.perf_counter()
+            call("cunbody1_force", x, m, x, 1e-14)
+            t.append(time.perf_counter() - t0)
+        return min(t) * 1e6
+
+    one, two = best(1), best(33)
+    print(one, two)
+    assert one <= two - 2.0
