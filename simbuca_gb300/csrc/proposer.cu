@@ -65,13 +65,13 @@ __device__ float mlp_warp(const __nv_bfloat16* __restrict__ w, const float* x) {
     return o + __bfloat162float(w[SG_MLP_B3]);
 }
 
-// Per-cloud features from the row-block moment partials of moments_kernel.
+// Per-cloud features from the moment partials of moments_kernel.
 __device__ void cloud_features(const SgCloud& cl, const SgCtrl& cs, const double* mom,
                                const SgProposerState& ps, float* f) {
     double s[11];
     for (int q = 0; q < 11; q++) s[q] = 0.0;
-    for (int b = 0; b < cl.nrb; b++)
-        for (int q = 0; q < 11; q++) s[q] += mom[(size_t)(cl.rb0 + b) * 11 + q];
+    for (int b = 0; b < cl.nmb; b++)
+        for (int q = 0; q < 11; q++) s[q] += mom[(size_t)(cl.mb0 + b) * 11 + q];
     const double n = cl.n;
     const double L = cl.L, v0 = cl.vref > 0.0 ? cl.vref : 1.0;
     for (int c = 0; c < 3; c++) {

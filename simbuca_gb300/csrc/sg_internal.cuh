@@ -131,6 +131,7 @@ struct SgCloud {
     int32_t npad;    // padded ions (multiple of SG_PAD)
     int32_t nslots;  // Coulomb partial-sum slots (j-chunks) of this cloud
     int32_t rb0, nrb;  // row blocks [rb0, rb0+nrb)
+    int32_t mb0, nmb;  // blocks of the moment sums, SG_ROWS ions each
     int32_t ion0;      // device index of the caller's first ion of the cloud (k-d order
                        // moves it; the step-size underflow test reads its x)
     double cx, cy, cz;   // centre of the FP32 frame (m)
@@ -597,6 +598,7 @@ cudaError_t sg_aos_to_soa(const double* pos, const double* vel, const int* perm,
 cudaError_t sg_soa_to_aos(const double* y, const int* perm, double* pos, double* vel, int n,
                           cudaStream_t st);
 cudaError_t sg_gather(const double* src, const int* perm, double* dst, int n, cudaStream_t st);
+// a.rows: the moment blocks
 cudaError_t sg_moments(const SgDpArgs& a, const double* mass, double* out, int n_rows,
                        cudaStream_t st);
 // same: xi is the set xj itself (ni = nj); uniform: every mass is m0; part: at least

@@ -200,3 +200,46 @@ def test_ragged_edges(ctx, prec):
         ep, ev = replay_error(c, fields[k], ts[k], hs[k], p[off:off + n], v[off:off + n])
         assert ep <= tol and ev <= tol, (k, ep, ev)
         off += n
+
+
+@pytest.mark.parametrize("counts", [[1], [255, 256, 257], [8192], [8193], [16, 300, 5000, 31]])
+def test_moments_at_block_edges(ctx, counts):
+    """Moments of clouds of any size against numpy, whatever rows the other kernels' blocks hold
+    (16 ions up to 8,192 in all): sums of n terms in FP64."""
+    rng = np.random.default_rng(sum(counts))
+    n = sum(counts)
+    pos, vel = rng.normal(1e-4, 5e-4, (n, 3)), rng.normal(0, 100.0, (n, 3))
+    mass = rng.uniform(100, 140, n) * 1.6605402e-27
+    b = Batch(ctx, counts, [configs.penning_field()] * len(counts),
+              [configs.ode(1e-9, 1e-15, 1e-9, 1e-6)] * len(counts), SG_PREC_FP64)
+    b.upload(pos, vel, mass, np.ones(n, np.int32))
+    at = 0
+    for c, m in zip(counts, b.moments()):
+        p, v = pos[at:at + c], vel[at:at + c]
+        np.testing.assert_allclose(m[:3], p.mean(0), rtol=1e-11, atol=1e-18)
+        np.testing.assert_allclose(m[3:6], np.sqrt(np.maximum((p * p).mean(0) - p.mean(0) ** 2, 0)),
+                                   rtol=1e-9, atol=1e-11)
+        np.testing.assert_allclose(m[6:9], (v * v).mean(0), rtol=1e-11)
+        assert m[11] == c
+        at += c
+
+
+def test_moments_of_a_small_batch_add_few_partials(ctx):
+    """8,000 ions in 32 partial sums, not 500: the call takes a few microseconds more than for
+    64 ions (15 more with a partial per 16 ions)."""
+    import time
+
+    def best(n):
+        rng = np.random.default_rng(n)
+        b = Batch(ctx, [n], [configs.penning_field()], [configs.ode(1e-9, 1e-15, 1e-9, 1e-6)], SG_PREC_FP64)
+        b.upload(rng.normal(0, 5e-4, (n, 3)), np.zeros((n, 3)), np.full(n, 2e-25), np.ones(n, np.int32))
+        t = []
+        for _ in range(200):
+            t0 = time.perf_counter()
+            b.moments()
+            t.append(time.perf_counter() - t0)
+        return min(t) * 1e6
+
+    small, large = best(64), best(8000)
+    print(small, large)
+    assert large <= small + 8.0
