@@ -23,6 +23,7 @@
 
 #include <algorithm>
 
+#include "fp32c_math.cuh"
 #include "sg_internal.cuh"
 
 namespace {
@@ -300,20 +301,26 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_grad_kernel(
     }
 }
 
+// Sum of the nb block partials p[b * stride], in order and compensated: 64 to 128 plain FP32
+// additions added more rounding than the pass before them (relative l2 error of a gradient over
+// 256 / 2,000 samples 1.4e-7 / 1.7e-7, so 0.7e-7 / 0.4e-7; 0.8 us of an iteration's 30).
+__device__ __forceinline__ float block_partials(const float* __restrict__ p, int stride, int nb) {
+    float s = 0.f, c = 0.f;
+#pragma unroll 16
+    for (int b = 0; b < nb; b++) kahan_add(s, c, p[(size_t)b * stride]);
+    return s;
+}
+
 // grad[k] = sum_b gpart[b][k] (fixed order); loss = sum_b lpart[b] / B.
 __global__ void mlp_reduce_kernel(const float* __restrict__ gpart, const float* __restrict__ lpart,
                                   int nb, int B, float* __restrict__ grad, float* __restrict__ loss) {
     sg_griddep_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < SG_MLP_NP) {
-        float s = 0.f;
-        for (int b = 0; b < nb; b++) s += gpart[(size_t)b * SG_MLP_NP + k];
-        grad[k] = s;
+        grad[k] = block_partials(gpart + k, SG_MLP_NP, nb);
     }
     if (k == 0) {
-        float s = 0.f;
-        for (int b = 0; b < nb; b++) s += lpart[b];
-        *loss = s / (float)B;
+        *loss = block_partials(lpart, 1, nb) / (float)B;
     }
 }
 
@@ -329,9 +336,7 @@ __global__ void mlp_adam_kernel(float* __restrict__ wm, __nv_bfloat16* __restric
     sg_griddep_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < SG_MLP_NP) {
-        float g = 0.f;
-#pragma unroll 16
-        for (int b = 0; b < nb; b++) g += gpart[(size_t)b * SG_MLP_NP + k];
+        const float g = block_partials(gpart + k, SG_MLP_NP, nb);
         const float a = b1 * m1[k] + (1.f - b1) * g;
         const float v = b2 * m2[k] + (1.f - b2) * g * g;
         m1[k] = a;
@@ -342,9 +347,7 @@ __global__ void mlp_adam_kernel(float* __restrict__ wm, __nv_bfloat16* __restric
         wm[k] = nw;
         wb[k] = __float2bfloat16_rn(nw);
     } else if (k == SG_MLP_NP) {  // a thread of its own
-        float s = 0.f;
-        for (int b = 0; b < nb; b++) s += lpart[b];
-        *loss = s / (float)B;
+        *loss = block_partials(lpart, 1, nb) / (float)B;
     }
 }
 
