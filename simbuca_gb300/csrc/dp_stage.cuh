@@ -87,12 +87,13 @@ struct MethodCK {
 // 1/x from the SFU's FP64 reciprocal (rcp.approx.ftz.f64, ~2^-20) and the geometric series
 // 1/(x y0) = 1 + e + e^2 + ..., e = 1 - x y0: 3 FP64 instructions where the IEEE division's
 // sequence takes ~14, 64 cycles each, for every component of every ion.  |e|^3 < 2^-57: the
-// result is within an ulp or so, far inside the error norm's own conditioning (~1e-8).
+// result is within an ulp or so, far inside the error norm's own conditioning (~1e-8).  An
+// infinite x (a tolerance that accepts everything) has the reciprocal 0, not the series' NaN.
 __device__ __forceinline__ double stage_rcp(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
+    return __double2hiint(y) == 0 ? y : fma(y, fma(e, e, e), y);
 }
 
 // Component c of ion i at stage S: finishes its force (P: the Coulomb sum along the axis

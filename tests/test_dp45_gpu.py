@@ -471,3 +471,16 @@ def test_integrators_in_kd_order(ctx, variant, method):
         ep = np.abs(p - pr).max() / np.abs(pr).max()
         ev = np.abs(v - vr).max() / np.abs(vr).max()
         assert ep <= 1e-7 and ev <= 1e-7, (ep, ev)
+
+
+@pytest.mark.parametrize("n,prec", [(5, SG_PREC_FP64), (5, SG_PREC_FP32C), (300, SG_PREC_FP32C), (1000, SG_PREC_FP32C),
+                                    (1000, SG_PREC_FP64), (9001, SG_PREC_FP32C)])
+def test_a_tolerance_that_accepts_everything(ctx, n, prec):
+    """An infinite absolute tolerance makes every scaled error 0: the step is accepted with error
+    norm 0 and the next step is the largest allowed, ten times as long (bin/ode.cpp:439-443)."""
+    c = configs.gaussian_cloud(configs.rng_for(n), n, 0.5e-3, 300.0, np.full(n, configs.M_CS))
+    b = Batch(ctx, [n], [configs.penning_field()], [configs.ode(1e-9, float("inf"), 1e-10, 1e-6)], prec)
+    b.upload(c.pos, c.vel, c.mass, c.charge)
+    info, _ = b.step()
+    assert info[0]["steps"] == 1 and info[0]["rejects"] == 0 and info[0]["err"] == 0.0
+    assert info[0]["h"] == pytest.approx(1e-9, rel=1e-15)
