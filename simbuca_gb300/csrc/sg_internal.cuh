@@ -189,17 +189,21 @@ struct SgCtrl {
     double beta;  // PI term of error_succes (0: the reference's I-controller)
 };
 
-// x^(-1/5) for a positive finite x: an FP32 estimate and two Newton steps
-// y <- y + y (1 - x y^5) / 5, each squaring the relative error (times 3): below the
+// pow(x, -0.2) for a positive finite x: an FP32 estimate and two Newton steps for the fifth
+// root, y <- y + y (1 - x y^5) / 5, each squaring the relative error (times 3): below the
 // rounding of the last one.  ~15 FP64 operations where pow takes ~100, 64 cycles each, on
-// the one lane that every block of the next attempt waits for.
+// the one lane that every block of the next attempt waits for.  The double 0.2 is 1/5 +
+// 1.11e-17: x^-0.2 = x^(-1/5) (1 - 1.11e-17 ln x), 7e-16 at the ends of the range.
 __device__ inline double sg_inv_fifth_root(double x) {
     if (!(x > 1e-30 && x < 1e30)) return pow(x, -0.2);
-    double y = (double)exp2f(-0.2f * log2f((float)x));
+    const float l2 = log2f((float)x);
+    double y = (double)exp2f(-0.2f * l2);
+    const double less = 5.0 * 1.1102230246251565e-17 * 0.6931471805599453 * (double)l2;
 #pragma unroll
     for (int k = 0; k < 2; k++) {
         const double y2 = y * y;
-        y = fma(y * 0.2, fma(-x * y, y2 * y2, 1.0), y);
+        const double r = fma(-x * y, y2 * y2, 1.0);
+        y = fma(y * 0.2, k ? r - less : r, y);
     }
     return y;
 }
