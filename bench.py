@@ -67,7 +67,7 @@ def parse():
                     help="safety factor of the proposer (default: the trained one's)")
     ap.add_argument("--fused", default="auto", choices=["auto", "on", "off"],
                     help="fused small-cloud path: automatic (where it is faster), on "
-                         "(up to 2,048: sg_set_fused 2) or off")
+                         "(wherever it can run: sg_set_fused 2) or off")
     ap.add_argument("--settle", type=int, default=60,
                     help="at most this many steps to let the step size settle before warm-up")
     return ap.parse_args()
@@ -201,6 +201,12 @@ def launches_per_attempt(prec, n_total, variant, mixed=False):
         return 1 + 6 * 2 + 2
     per_sum = 3 + (1 if fp32c and n_total > 8192 else 0) + ((2 if mixed else 1) if fp32c and variant == 17 else 0)
     return 1 + 6 * per_sum + 2
+
+
+def mixed_leaves(counts):
+    """Whether a batch of shape 17 has clouds in the plain kernel too: those of up to 2,500
+    ions, unless a cloud of 24,000 ions or 2e9 pairs make all of them leaves."""
+    return min(counts) <= 2500 and max(counts) < 24000 and sum(n * n for n in counts) < 2e9
 
 
 # Algorithmic HBM traffic of one Dormand-Prince attempt per ion in the O(N) kernels:
@@ -451,12 +457,12 @@ def run_ours(args, dist: Dist):
                 "mean_h": sum(a["t"] - b["t"] for a, b in zip(e_after, e_before)) /
                 max(1, sum(a["steps"] - b["steps"] for a, b in zip(e_after, e_before)))},
         "mean_h": sim_us * 1e-6 / max(1, sum(a["steps"] - b["steps"] for a, b in zip(s_after, s_before))),
-        # per step one hold reset (+2 per attempt with the proposer: cloud moments and the
+        # tiled kernels: per step one hold reset (+2 per attempt with the proposer: cloud moments and the
         # MLP); fused small-cloud path: one launch per step (its attempts inside it)
         "gpu_launches": int((args.steps if fused_cluster else
                              attempts * (launches_per_attempt(prec, w.n_total, batch.variant())
                                          + (2 if args.proposer == "on" else 0)))
-                            + args.steps
+                            + (0 if fused_cluster else args.steps)
                             + (3 * (attempts // CHECK_EVERY) if prec == abi.SG_PREC_FP32C else 0)),
         "fixup_ions_per_coulomb_call": fixups / max(1, 6 * attempts),
         "force_check": checks,
@@ -624,7 +630,7 @@ def run_batched(args, dist: Dist):
                    "step_control": step_control,
                    "parallelism": f"replicas x{dist.world}",
                    "l2": "flushed (256 MB write) between timed steps"},
-        "gpu_launches": int((launches_per_attempt(prec, w.n_total, variant, min(w.counts) <= 2500)
+        "gpu_launches": int((launches_per_attempt(prec, w.n_total, variant, mixed_leaves(w.counts))
                              + (2 if args.proposer == "on" else 0)) * per_step * args.steps
                             + (3 * (per_step * args.steps // CHECK_EVERY)
                                if args.precision == "fp32c" else 0)),
