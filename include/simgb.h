@@ -260,12 +260,14 @@ int sg_mlp_train(sg_ctx* ctx, int n, const float* X, const float* Y, int iters, 
 int sg_batch_set_proposer(sg_ctx* ctx, const float* w, double safety);
 /* Small clouds (no counterpart in the reference): FP32c Dormand-Prince batches whose
  * clouds are small, in the plain ion order and without a recorder, operations,
- * dissociation, step log or proposer, run whole attempts in one launch, one thread-block
- * cluster of up to 16 CTAs per cloud.  sg_set_fused(ctx, mode): 1 (default) where it is
- * faster than the tiled kernels (one cloud of up to ~4,000 ions; several smaller ones while
- * their CTAs fit on the device together); 2 for clouds of up to 2,048 ions; 0 never.
- * sg_batch_fused gives the cluster size
- * the current batch runs with (0: the tiled kernels).  sg_fused_timing: CUDA-event time
+ * dissociation, step log or proposer, run whole attempts in one launch: a thread-block
+ * cluster of up to 16 CTAs per cloud (clouds of up to 2,048 ions), or the wide form, which
+ * spreads each cloud over up to 160 CTAs (batches of up to 8,192 ions, clouds of up to
+ * 7,168, while all their CTAs fit on the device).  sg_set_fused(ctx, mode): 1 (default) where
+ * it is faster than the tiled kernels (one cloud of up to ~4,000 ions; several smaller ones
+ * while their CTAs fit on the device together); 2 wherever one of the two can run; 0 never.
+ * sg_batch_fused gives the CTAs per cloud that the current batch runs with (0: the tiled
+ * kernels; above 16: the wide form).  sg_fused_timing: CUDA-event time
  * of the fused launches while sg_set_kernel_timing is on. */
 int sg_set_fused(sg_ctx* ctx, int on);
 int sg_batch_fused(sg_ctx* ctx, int* cluster);

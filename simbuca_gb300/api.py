@@ -149,8 +149,9 @@ class Context:
         check(self._L.sg_set_use_graph(self._h, int(bool(on))), "sg_set_use_graph")
 
     def set_fused(self, mode):
-        """Whole attempts of small clouds in one cluster launch: 1 (default, True)
-        where it is faster, 2 clouds of up to 2,048 ions, 0 (False) never."""
+        """Whole attempts of small clouds in one launch: 1 (default, True) where it is faster,
+        2 wherever it can run (clouds of up to 2,048 ions; batches of up to 8,192 ions whatever
+        their clouds, up to 7,168 ions each), 0 (False) never."""
         check(self._L.sg_set_fused(self._h, int(mode)), "sg_set_fused")
 
     def fused_timing(self):
@@ -221,7 +222,8 @@ class Batch:
         check(self._L.sg_batch_attempts(self.ctx.handle, int(n)), "sg_batch_attempts")
 
     def fused(self) -> int:
-        """Cluster size of the fused small-cloud path this batch runs with (0: tiled)."""
+        """CTAs per cloud of the fused small-cloud path this batch runs with: up to 16 a
+        thread-block cluster, more (or one) the wide form; 0 the tiled kernels."""
         self._live()
         v = ctypes.c_int()
         check(self._L.sg_batch_fused(self.ctx.handle, ctypes.byref(v)), "sg_batch_fused")

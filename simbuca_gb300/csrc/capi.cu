@@ -312,7 +312,7 @@ int auto_variant(const std::vector<int>& counts, int requested, bool resident) {
     }
     if (requested >= 0) return requested == SG_C32_FAR_ONCE && big > kFarOnceMax ? 14 : requested;
     if (big > kFarOnceMax) return 14;
-    if (big > (resident ? SG_FINISH_MAX_IONS : kLeafAlways)) return SG_C32_FAR_ONCE;
+    if (resident ? big > SG_FINISH_MAX_IONS : big >= kLeafAlways) return SG_C32_FAR_ONCE;
     if (resident && pairs >= kLeafAlwaysPairs) return SG_C32_FAR_ONCE;
     if (resident && total > SG_FINISH_MAX_IONS && big > kLeafMin) return SG_C32_FAR_ONCE;
     return big <= 6000 && total <= 32768 ? 11 : 5;
@@ -829,7 +829,7 @@ int alloc_problem(sg_ctx* ctx, Problem& P) {
     CK(cudaMemset(P.spec, 0, N * sizeof(int)));
     CK(dalloc(&P.pmass, N));
     CK(dalloc(&P.pmass0, N));
-    // two lists (near-only ions; ions with a far fix-up): counts, then N pairs each
+    // counts, work units (int4), then the ions that found the unit list full (pairs)
     CK(dalloc(&P.fix_list, 4 + 4 * SG_FIX_CAP + 2 * N));
     CK(cudaMemset(P.fix_list, 0, 4 * sizeof(int)));
     CK(dalloc(&P.fix_part, (size_t)3 * SG_FIX_CAP));
@@ -1314,8 +1314,6 @@ int fused_form(sg_ctx* ctx, Problem& P) {
 }
 bool fused_eligible(sg_ctx* ctx, Problem& P) { return fused_form(ctx, P) != 0; }
 
-// n attempts of every active cloud at most (a cloud stops early once done or held);
-// `counted`: attempts counted towards the in-run check's interval.
 // ions of the largest cloud
 int big_fused(const Problem& P) {
     int big = 0;
@@ -1323,6 +1321,8 @@ int big_fused(const Problem& P) {
     return big;
 }
 
+// n attempts of every active cloud at most (a cloud stops early once done or held);
+// `counted`: attempts counted towards the in-run check's interval.
 int run_fused(sg_ctx* ctx, Problem& P, int n, int counted, int one_step = 0) {
     const bool wide = fused_form(ctx, P) == 2;
     SgFusedArgs f;
@@ -2578,7 +2578,7 @@ int sg_mlp_train(sg_ctx* ctx, int n, const float* X, const float* Y, int iters, 
     CK(cudaMemcpyAsync(ctx->mlp_X, X, sizeof(float) * n * SG_MLP_IN, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->mlp_Y, Y, sizeof(float) * n, cudaMemcpyHostToDevice, ctx->stream));
     // minibatches: a seeded permutation per epoch (splitmix64), drawn and uploaded for
-    // kMlpRun iterations at a time, so that the host waits once per run of iterations
+    // `run` iterations at a time, so that the host waits once per run of iterations
     std::vector<int> perm(n);
     for (int i = 0; i < n; i++) perm[i] = i;
     uint64_t s = seed;

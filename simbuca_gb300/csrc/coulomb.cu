@@ -1298,7 +1298,7 @@ __global__ void __launch_bounds__(NT, MINB) coulomb_fp32c_sorted_kernel(const fl
 // ---------------------------------------------------------------------------
 
 // Every unordered pair once (fp64_pairs.cuh): a work item is one 128-ion i-block against
-// nj j-ions, rotation steps [s0, s1) of each 32-ion j-tile.
+// nj j-ions, or a part of a pair of 32-ion tiles (tile_pair).
 __global__ void __launch_bounds__(SG_SYM_IB) coulomb_fp64_sym_kernel(
     const double* __restrict__ c64, const SgWorkItem* __restrict__ items,
     const SgCloud* __restrict__ clouds, const SgCtrl* __restrict__ ctrl,
@@ -1648,11 +1648,12 @@ struct SlotShared64 {
 //
 // FP32c: the slots hold float-float sums in frame units (store_partial); they are added
 // in float-float and converted once.  An ion whose near terms cancel strongly
-// (sqrt(s2) > 1.5 |P|, > |P| in clouds of up to SG_SMALL_ROW ions) or whose far terms are
+// (sqrt(s2) > 1.5 |P|, > |P| in clouds of up to SG_SMALL_ROW ions, leaf sums: leaf_kappa in
+// capi.cu) or whose far terms are
 // large next to |P| (s2f > SgCloud::kfar2 |P|^2) is fixed up (fixup_ion): INBLOCK, by this
 // block right away (small batches, where a second launch costs more than the work);
-// otherwise it is put on a work list of coulomb_fixup_kernel (ion index; cloud | kind <<
-// 28): the ions whose row is re-evaluated in one list, the far-only ones in the other.
+// otherwise its work units are put on the list of coulomb_fixup_kernel (ion index; cloud |
+// kind << 28; unit and their count; first unit), or the ion whole once that is full.
 //
 // Latency-bound for small clouds: an FP64 addition takes a warp 64 cycles, so one thread
 // per row over 32 slots of five FP64 values spent ~5 us on additions alone.  Batches of

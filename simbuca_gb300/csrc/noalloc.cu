@@ -42,8 +42,8 @@ constexpr int kNaMaxIons = 8192;
 constexpr int kNaMaxContexts = 64;
 constexpr int kNaSms = 152;  // GB300
 
-// the partial-sum slots: 66 at the largest size (64 i-blocks, 128 ions each, on the j
-// side of the last one), more for smaller sets
+// the partial-sum slots: room for 66 at the largest size, which takes 65 (64 i-blocks, 128
+// ions each, on the j side of the last one); smaller sets use more of them
 constexpr size_t kNaSlotDoubles = (size_t)66 * 3 * kNaMaxIons;
 constexpr size_t kScratchBytes = kNaSlotDoubles * sizeof(double);
 

@@ -159,8 +159,8 @@ struct SgCloud {
 };
 
 // Partial-sum slots of the FP64 symmetric form that hold a part of local padded ion p: one
-// per i-block up to its own (j-side) and band, one per j-chunk of its own i-block (i-side)
-// and band.
+// per i-block up to its own (j-side), one per j-chunk of its own i-block (i-side).  (Tile
+// pairs, sym_k = 0: all slots of the cloud.)
 __host__ __device__ inline int sg_sym_slots(const SgCloud& cl, int p) {
     const int b = p / SG_SYM_IB;
     const int tiles = cl.npad / SG_SYM_JT - b * (SG_SYM_IB / SG_SYM_JT);

@@ -157,3 +157,37 @@ def test_tail_of_the_wide_forms_errors(ctx, n, kind, most):
         above += int((rel_err_per_ion(a, ctx.coulomb_accel(p, q, kq, SG_PREC_FP64)) > 3e-7).sum())
     print(n, kind, above)
     assert above <= most
+
+
+@pytest.mark.parametrize("counts", [[900], [2000], [4000], [1000, 60], [300] * 8])
+def test_more_flagged_ions_than_the_shared_list_holds(ctx, counts):
+    """A lattice of alternating charges: every ion's terms cancel, so that hundreds are flagged in
+    a stage, more than the 64 rows the wide form's CTAs share; each CTA then takes its own.
+    From rest, two tiny steps: the velocity of the second one is the step times the force
+    (bound as for such lattices in the tiled kernels: n terms that add up to ~250 of a
+    neighbour's field, 1e-16 sqrt(n) 250 < 1e-11 of it)."""
+    d, h = 1e-5, 1e-16
+    pos, q = [], []
+    for n in counts:
+        side = int(np.ceil(n ** (1 / 3)))
+        g = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+        pos.append(d * g.astype(np.float64))
+        q.append(np.where(g.sum(1) % 2 == 0, 1, -1))
+    pos, q = np.concatenate(pos), np.concatenate(q).astype(np.int32)
+    fp = abi.FieldParams()
+    fp.flags, fp.coulomb_scale = abi.SG_F_COULOMB, 1.0
+    op = configs.ode(1e-9, 1e-15, h, 1.0, adaptive=False)
+    mass = np.full(len(q), 132.905 * oracle.AMU)
+    out = []
+    for prec in (SG_PREC_FP32C, SG_PREC_FP64):
+        b = Batch(ctx, counts, [fp] * len(counts), [op] * len(counts), prec)
+        assert (b.fused() > 16) == (prec == SG_PREC_FP32C)
+        b.upload(pos, np.zeros_like(pos), mass, q)
+        b.attempts(1)
+        v1 = b.download()[1]
+        b.attempts(1)
+        out.append((b.download()[1] - v1) / h)
+    field = kq_of(mass, np.ones(len(q)))[0] / d ** 2
+    err = np.abs(out[0] - out[1]).max() / field
+    print(counts, err)
+    assert err <= 1e-11
