@@ -303,12 +303,16 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_grad_kernel(
 
 // Sum of the nb block partials p[b * stride], in order and compensated: 64 to 128 plain FP32
 // additions added more rounding than the pass before them (relative l2 error of a gradient over
-// 256 / 2,000 samples 1.4e-7 / 1.7e-7, so 0.7e-7 / 0.4e-7; 0.8 us of an iteration's 30).
+// 256 / 2,000 samples 1.4e-7 / 1.7e-7, so 0.7e-7 / 0.4e-7; 0.4 us of an iteration's 30).
 __device__ __forceinline__ float block_partials(const float* __restrict__ p, int stride, int nb) {
-    float s = 0.f, c = 0.f;
+    float s = 0.f, c = 0.f;  // the roundings of s in c, off its chain of additions
 #pragma unroll 16
-    for (int b = 0; b < nb; b++) kahan_add(s, c, p[(size_t)b * stride]);
-    return s;
+    for (int b = 0; b < nb; b++) {
+        const ff t = ff_two_sum(s, p[(size_t)b * stride]);
+        s = t.h;
+        c += t.l;
+    }
+    return s + c;
 }
 
 // grad[k] = sum_b gpart[b][k] (fixed order); loss = sum_b lpart[b] / B.
