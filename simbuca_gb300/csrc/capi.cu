@@ -8,9 +8,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <ctime>
+#include <exception>
 #include <mutex>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -698,7 +698,9 @@ int kd_split(KdIon* p, int n) {
     return m;
 }
 
-// Segments to split, shared by the threads of one call.
+// Segments to split, shared by the threads of one call.  Nothing in work() allocates (`open` is
+// reserved for the disjoint segments of more than kAlone ions that it can hold), so no thread
+// can end in an exception.
 struct KdQueue {
     static constexpr int kAlone = 2048;  // ions a thread splits on its own
     std::mutex mu;
@@ -715,20 +717,21 @@ struct KdQueue {
             open.pop_back();
             busy++;
             lk.unlock();
-            std::vector<KdSegment> own(1, s);
-            while (!own.empty()) {
-                s = own.back();
-                own.pop_back();
+            KdSegment own[64];  // two per level of halving at most
+            int m_own = 0;
+            own[m_own++] = s;
+            while (m_own > 0) {
+                s = own[--m_own];
                 if (s.n <= 128) continue;
                 const int m = kd_split(s.p, s.n);
                 const KdSegment low{s.p, m}, high{s.p + m, s.n - m};
-                own.push_back(low);
+                own[m_own++] = low;
                 if (high.n > kAlone) {
                     std::lock_guard<std::mutex> g(mu);
                     open.push_back(high);
                     cv.notify_one();
                 } else {
-                    own.push_back(high);
+                    own[m_own++] = high;
                 }
             }
             lk.lock();
@@ -744,6 +747,7 @@ void kd_order(const double* pos, const std::vector<std::pair<int, int>>& clouds,
     for (const auto& c : clouds) total += c.second;
     std::vector<KdIon> ions(total);
     KdQueue queue;
+    queue.open.reserve(clouds.size() + total / KdQueue::kAlone + 1);
     KdIon* p = ions.data();
     for (const auto& c : clouds) {
         for (int i = 0; i < c.second; i++) {
@@ -757,8 +761,9 @@ void kd_order(const double* pos, const std::vector<std::pair<int, int>>& clouds,
     const int extra = std::min(most, (int)(total / 4096)) - 1;
     std::vector<std::thread> threads;
     try {
+        threads.reserve(std::max(extra, 0));
         for (int t = 0; t < extra; t++) threads.emplace_back([&queue] { queue.work(); });
-    } catch (const std::system_error&) {
+    } catch (const std::exception&) {
         // fewer threads than asked for
     }
     queue.work();

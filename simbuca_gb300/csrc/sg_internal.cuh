@@ -505,7 +505,8 @@ cudaError_t sg_dp_finish(const SgFinishArgs& f, int stage, int fp32c, cudaStream
 // (29,000) / 150, 3,000 - / 151 to 166 (60,000) / 172 to 180, 4,096 - / 189 (111,000) / 223,
 // 5,000 - / 310 (165,000) / 239; 8 of 300 77 (12,000) / 60 (5,000) / 166, 16 of 300 101 (23,000)
 // / 82 / 227, 4 of 2,000 - / 195 (106,000) / 245, 2 of 4,000 - / 301 (212,000) / 309; 70 of 100 on
-// 2 CTAs each 66 (5,000) / 76 / 224.
+// 2 CTAs each 66 (5,000) / 76 / 224.  (At a conditioning threshold of 1.1 |P|; at the 1.0 of
+// sg_kappa2_fused 8 of 300 take 74 in the wide form, 135 tiled, 32 of 300 128 in clusters, 256.)
 #define SG_FUSED_CLUSTER_PAIRS 8000
 // Conditioning threshold of the fused path (its partial sums interleave the cloud's ions):
 // sqrt(s2) > 1.5 |P| for a few clouds of up to SG_FUSED_LOOSE_IONS ions, which it always
