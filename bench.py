@@ -205,8 +205,9 @@ def launches_per_attempt(prec, n_total, variant, mixed=False):
 
 def mixed_leaves(counts):
     """Whether a batch of shape 17 has clouds in the plain kernel too: those of up to 2,500
-    ions, unless a cloud of 24,000 ions or 2e9 pairs make all of them leaves."""
-    return min(counts) <= 2500 and max(counts) < 24000 and sum(n * n for n in counts) < 2e9
+    ions, or 2,048 with a cloud of 24,000 ions or 2e9 pairs in the batch."""
+    strict = max(counts) >= 24000 or sum(n * n for n in counts) >= 2e9
+    return min(counts) <= (2048 if strict else 2500)
 
 
 # Algorithmic HBM traffic of one Dormand-Prince attempt per ion in the O(N) kernels:

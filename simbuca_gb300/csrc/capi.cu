@@ -43,7 +43,7 @@ struct Problem {
     std::vector<SgWorkItem> hitems;
     std::vector<SgFarItem> hfar, hnear;   // shape 17
     int leaf_min = 0;              // ... its clouds of more ions; smaller ones are plain
-    bool leaf_strict = false;      // ... flag as the ordered-pair k-d shapes do (leaf_kappa)
+    bool leaf_strict = false;      // ... flag as the ordered-pair k-d shapes do (sum_kappa)
     SgFarItem *dfar = nullptr, *dnear = nullptr;
     std::vector<int> hleaf;        // cloud of each leaf
     int near_cap = 0;              // leaves of the largest cloud
@@ -268,25 +268,33 @@ constexpr int kFarOnceMax = 1 << 21;
 // 1,101, 20 of 3,000 1,156 / 994, 10 of 4,096 1,009 / 812; below ~3,000 ions the leaves' errors
 // are 4 % larger (RMS), above smaller.
 constexpr int kLeafMin = 2500;
-// Clouds of this many ions, and batches of this many ordered pairs, take k-d ordered leaves
-// throughout and hold the errors of the ordered-pair shapes 9 and 14.
+// Batches with a cloud of this many ions, or of this many ordered pairs, hold the errors of the
+// ordered-pair k-d shapes 9 and 14: leaves above 2,048 ions (the plain partial sums of larger
+// clouds are 128 terms long, not 16) and stricter thresholds.
 constexpr int kLeafAlways = 24000;
 constexpr double kLeafAlwaysPairs = 2e9;
+constexpr int kLeafMinStrict = 2048;
 
-// Conditioning threshold sqrt(s2) / |P| of a leaf sum.  Its partial sums have 16 terms and
-// are coherent, so the estimate differs from that of the other forms at the same error; the
+// Conditioning threshold sqrt(s2) / |P|.  A leaf's partial sums have 16 terms and are
+// coherent, so the estimate differs from that of the other forms at the same error; the
 // thresholds are set by the tails.  Ions above 3e-7 per million, over 1.8 to 6.6 million ions
 // of a size (Gaussian / uniform / elongated clouds):
 //   strict, against shapes 9 and 14 (at 1.0 up to 4,096 ions, 1.5 above):
-//     2,600 ions 0.2 / 0.3 / 35, leaves at 1.0 0.0 / 0.6 / 29, at 2.0 60 / 187 / 615;
-//     4,096 0.3 / 1.1 / 21, at 1.0 0.3 / 1.5 / 20; 1,000 0.0 / 2.5 / 41, at 1.0 0.0 / 5.5 / 44;
+//     300 ions 5.6 / 24 / 233, plain order at 0.65 1.1 / 1.1 / 3, at 0.75 4.5 / 7 / 18;
+//     1,000 0.0 / 2.5 / 41, at 0.65 0.0 / 0.5 / 1.5, at 0.75 0.5 / 4.5 / 6.5 (at 1.0 10 / 56 / 80);
+//     2,040 0.4 / 1.1 / 29, at 0.65 0.0 / 0.4 / 0.0, at 0.75 0.0 / 3.0 / 5.3;
+//     2,600 0.2 / 0.3 / 35, leaves at 1.0 0.0 / 0.6 / 29, at 2.0 60 / 187 / 615;
+//     4,096 0.3 / 1.1 / 21, at 1.0 0.3 / 1.5 / 20;
 //     6,000 2.7 / 26 / 105, at 1.25 1.0 / 12 / 51; 8,192 2.3 / 16 / 79, at 1.25 0.4 / 8 / 41;
 //     30,000 1.7 / 21 / 39, at 1.15 1.7 / 6 / 24, at 1.5 7.8 / 36 / 52;
 //     65,536 2.4 / 32 / 30, at 1.15 1.0 / 21 / 16; 140,000 2.1 / 35 / 46, at 1.15 0.0 / 23 / 36.
 //   other automatic clouds, against the plain order they would have (1.0, 1.5 above 4,096):
 //     2,600 99 / 339 / 755, leaves at 1.5 8 / 41 / 219; 4,096 65 / 229 / 491, at 1.5 5.5 / 42 / 125;
 //     6,000 189 / 617 / 1,282, at 2.0 32 / 150 / 277; 20,001 83 / 326 / 523, at 2.0 21 / 120 / 142.
-float leaf_kappa(int npad, bool strict) {
+// (3,000 clouds of 850 ions: 23.6 ms per attempt with the plain order at 0.75, 27.3 at 0.65, 29.3
+// with leaves at 1.0, 40.5 with shape 9.)
+float sum_kappa(int npad, bool leafs, bool strict) {
+    if (!leafs) return strict ? 0.7f : std::sqrt(sg_kappa2(npad));
     if (npad <= SG_SMALL_ROW) return strict ? 1.0f : 1.5f;
     if (npad <= kLeafAlways) return strict ? 1.25f : 2.0f;
     return 1.15f;
@@ -335,7 +343,7 @@ void set_leaf_rule(Problem& P, int requested) {
         big = big || n >= kLeafAlways;
     }
     P.leaf_strict = requested == SG_C32_FAR_ONCE || big || pairs >= kLeafAlwaysPairs;
-    P.leaf_min = P.leaf_strict ? 0 : kLeafMin;
+    P.leaf_min = requested == SG_C32_FAR_ONCE ? 0 : P.leaf_strict ? kLeafMinStrict : kLeafMin;
 }
 
 // FP64 items that take each unordered pair once: i-block b (128 ions) against the j-tiles
@@ -546,11 +554,11 @@ void plan(Problem& P, int n_sm) {
     if (f32 && P.variant == SG_C32_FAR_ONCE) {
         for (int c = 0; c < C; c++)
             P.hc[c].leafs = (P.hc[c].fp.flags & SG_F_COULOMB) && P.hc[c].n > P.leaf_min;
-        for (int c = 0; c < C; c++) {
-            const float k = leaf_kappa(P.hc[c].npad, P.leaf_strict);
-            P.hc[c].kleaf2 = k * k;
-        }
         plan_far_once(P, n_sm);
+    }
+    for (int c = 0; f32 && c < C; c++) {
+        const float k = sum_kappa(P.hc[c].npad, P.hc[c].leafs, P.variant == SG_C32_FAR_ONCE && P.leaf_strict);
+        P.hc[c].kappa2 = k * k;
     }
     const int ib = f32 ? sg_coulomb_fp32c_ib(P.variant == SG_C32_FAR_ONCE ? SG_C32_PLAIN : P.variant)
                        : SG_C64_IB;

@@ -1648,8 +1648,8 @@ struct SlotShared64 {
 //
 // FP32c: the slots hold float-float sums in frame units (store_partial); they are added
 // in float-float and converted once.  An ion whose near terms cancel strongly
-// (sqrt(s2) > 1.5 |P|, > |P| in clouds of up to SG_SMALL_ROW ions, leaf sums: leaf_kappa in
-// capi.cu) or whose far terms are
+// (sqrt(s2) > 1.5 |P|, > |P| in clouds of up to SG_SMALL_ROW ions, batches of shape 17:
+// sum_kappa in capi.cu) or whose far terms are
 // large next to |P| (s2f > SgCloud::kfar2 |P|^2) is fixed up (fixup_ion): INBLOCK, by this
 // block right away (small batches, where a second launch costs more than the work);
 // otherwise its work units are put on the list of coulomb_fixup_kernel (ion index; cloud |
@@ -1762,7 +1762,7 @@ __global__ void __launch_bounds__(SG_ROWS) coulomb_reduce_kernel(
             const float pf2 = fmaf(px.h, px.h, fmaf(py.h, py.h, pz.h * pz.h));
             // the far threshold: the prior of the frame set-up, or the measured one
             const float kf2 = chk ? fminf(cl.kfar2, chk[rb.cloud].kfar2) : cl.kfar2;
-            const float kap2 = cl.leafs ? cl.kleaf2 : sg_kappa2(cl.npad);
+            const float kap2 = cl.kappa2;
             kind = (many || s2 > kap2 * pf2 ? kFixNear : 0) | (s2f > kf2 * pf2 ? kFixFar : 0);
             if (risk != nullptr) {
                 const float pf = sqrtf(pf2);

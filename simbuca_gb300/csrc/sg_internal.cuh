@@ -155,7 +155,7 @@ struct SgCloud {
     float far_fs, far_fs2, near_fs2;
     int32_t leafs;  // shape 17: k-d ordered leaf pairs (else the plain kernel)
     int32_t sym_k;  // FP64 unordered items of K j-tiles (0: every ion has nslots slots)
-    float kleaf2;   // shape 17: conditioning threshold of the leaf sums (leaf_kappa in capi.cu)
+    float kappa2;   // conditioning threshold of the sums above 8,192 ions (sum_kappa in capi.cu)
 };
 
 // Partial-sum slots of the FP64 symmetric form that hold a part of local padded ion p: one
@@ -464,10 +464,10 @@ struct SgDpArgs {
 // > |P| in clouds of up to SG_SMALL_ROW padded ions, whose FP64 row is cheap and whose
 // error per unit of sqrt(s2)/|P| ran up to ~9e-7 with their few terms per ion (an
 // unflagged ion at 1.37 measured 1.2e-6 in the 512-cloud scan's small clouds; 2.5e-7 at
-// most on the 65,536-ion cloud).  The leaf sums have thresholds of their own
-// (SgCloud::kleaf2), and so has the fused path (SG_FUSED_LOOSE_IONS).
+// most on the 65,536-ion cloud).  Leaf sums and the batches that have them use
+// SgCloud::kappa2, and the fused path sg_kappa2_fused.
 #define SG_SMALL_ROW 4096
-__device__ __forceinline__ float sg_kappa2(int npad) { return npad <= SG_SMALL_ROW ? 1.0f : 2.25f; }
+__host__ __device__ __forceinline__ float sg_kappa2(int npad) { return npad <= SG_SMALL_ROW ? 1.0f : 2.25f; }
 // Close pairs listed per ion (shape 17); an ion with more gets its FP64 row.
 #define SG_CLOSE_CAP 8
 
